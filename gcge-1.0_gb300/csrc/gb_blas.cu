@@ -942,10 +942,12 @@ extern "C" int gb_residual_norms(gcge_gpu_ctx *ctx, int n, int k, const double *
 // 32-row slabs of V and W staged in shared memory.
 __global__ void __launch_bounds__(256)
 k_gram_partial(int n, int k1, int k2, const double *__restrict__ V, long ldv, const double *__restrict__ W,
-               long ldw, double *__restrict__ part, long rows_per_split, int sym)
+               long ldw, double *__restrict__ part, long rows_per_split, int sym,
+               const int *__restrict__ run = nullptr)
 {
     const int ti = blockIdx.x, tj = blockIdx.y, split = blockIdx.z;
     if (sym && ti > tj) return;
+    if (run && !*run) return;                              // the tensor-core form has the product
     const int i0 = ti * 32, j0 = tj * 32;
     const long rb = (long)split * rows_per_split;
     const long re = min((long)n, rb + rows_per_split);
@@ -981,13 +983,15 @@ k_gram_partial(int n, int k1, int k2, const double *__restrict__ V, long ldv, co
 }
 
 __global__ void k_gram_reduce(int k1, int k2, int nsplit, const double *__restrict__ part, double *a, int lda,
-                              int sym)
+                              int sym, const int *__restrict__ run = nullptr)
 {
+    if (run && !*run) return;
     const long total = (long)k1 * k2;
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
         const int i = (int)(t % k1), j = (int)(t / k1);
         if (sym && i > j) continue;
         double s = 0;
+#pragma unroll 8
         for (int q = 0; q < nsplit; ++q) s += part[(long)q * total + t];
         a[i + (long)j * lda] = s;
         if (sym && i != j) a[j + (long)i * lda] = s;
@@ -999,7 +1003,7 @@ extern "C" int gb_gram(gcge_gpu_ctx *ctx, int n, int k1, int k2, const double *V
 {
     if (k1 <= 0 || k2 <= 0) return GCGE_GPU_OK;
     if (ctx->tc) {
-        int st = gb_iscratch(ctx, (size_t)k1 + k2);
+        int st = gb_iscratch(ctx, gb_gram_tc_ints(k1, k2));
         if (st) return st;
         return gb_gram_tc(ctx, n, k1, k2, V, ldv, W, ldw, a_dev, lda, sym, ctx->iscratch);
     }
@@ -1144,35 +1148,54 @@ extern "C" int gb_scale_cols(gcge_gpu_ctx *ctx, int n, int k, const double *X, l
     return GCGE_GPU_OK;
 }
 
-// Gram V^T W with caller-provided partial-sum storage and stream (no context,
-// no allocation): the launcher behind the allocation-free entry point. part
-// must hold part_cap doubles; returns GCGE_GPU_ERR_ARG when k1*k2 does not fit
-// at least one row split.
-extern "C" int gb_gram_fixed_scratch(cudaStream_t stream, int num_sms, int n, int k1, int k2, const double *V,
-                                     long ldv, const double *W, long ldw, double *a_dev, int lda, int sym,
-                                     double *part, size_t part_cap)
+// Row splits of an FP64-pipe Gram that fit part_cap doubles of partials: the
+// splits and the rows of each; 0 when not even one fits. A block takes 8.2 us for a
+// slab of 32 rows (its SM's FP64 pipe), so few rows go out as one slab a block:
+// 1,000 x (64, 64) took 79 us in splits of 256 rows, 21 us in these.
+extern "C" long gb_gram_fixed_splits(int num_sms, int n, int k1, int k2, int sym, size_t part_cap, long *rps_out)
 {
     const int ti = (k1 + 31) / 32, tj = (k2 + 31) / 32;
     int tiles = sym ? ti * (ti + 1) / 2 : ti * tj;
     if (tiles < 1) tiles = 1;
     long nsplit = ((long)num_sms * 4) / tiles;
-    const long max_split = (n + 255) / 256;
+    const long max_split = ((long)n + 31) / 32;
     if (nsplit > max_split) nsplit = max_split;
     const long fit = (long)(part_cap / ((size_t)k1 * k2));
     if (nsplit > fit) nsplit = fit;
-    if (nsplit < 1) return GCGE_GPU_ERR_ARG;
+    if (nsplit < 1) return 0;
     long rps = ((n + nsplit - 1) / nsplit + 31) / 32 * 32;
     if (rps < 32) rps = 32;
+    *rps_out = rps;
     nsplit = (n + rps - 1) / rps;
-    if (nsplit < 1) nsplit = 1;
-    dim3 grid(ti, tj, (unsigned)nsplit);
-    k_gram_partial<<<grid, 256, 0, stream>>>(n, k1, k2, V, ldv, W, ldw, part, rps, sym);
-    if (cudaGetLastError() != cudaSuccess) return GCGE_GPU_ERR_CUDA;
+    return nsplit < 1 ? 1 : nsplit;
+}
+
+// Partials of the FP64-pipe Gram V^T W with caller-provided storage and stream (no
+// context, no allocation): the launcher behind the allocation-free entry point.
+// run (device, optional): the kernel does nothing where *run is zero. Returns the
+// number of row splits in part, or 0 (GCGE_GPU_ERR_ARG or GCGE_GPU_ERR_CUDA in *st).
+extern "C" int gb_gram_fixed_partials(cudaStream_t stream, int num_sms, int n, int k1, int k2, const double *V,
+                                      long ldv, const double *W, long ldw, int sym, double *part, size_t part_cap,
+                                      const int *run, int *st)
+{
+    long rps = 0;
+    const long nsplit = gb_gram_fixed_splits(num_sms, n, k1, k2, sym, part_cap, &rps);
+    *st = nsplit ? GCGE_GPU_OK : GCGE_GPU_ERR_ARG;
+    if (!nsplit) return 0;
+    dim3 grid((k1 + 31) / 32, (k2 + 31) / 32, (unsigned)nsplit);
+    k_gram_partial<<<grid, 256, 0, stream>>>(n, k1, k2, V, ldv, W, ldw, part, rps, sym, run);
+    if (cudaGetLastError() != cudaSuccess) *st = GCGE_GPU_ERR_CUDA;
+    return *st ? 0 : (int)nsplit;
+}
+
+// the partials' sum over the splits (run as above)
+extern "C" int gb_gram_fixed_reduce(cudaStream_t stream, int num_sms, int k1, int k2, int nsplit, const double *part,
+                                    double *a_dev, int lda, int sym, const int *run)
+{
     long g = ((long)k1 * k2 + 255) / 256;
     if (g > (long)num_sms * 16) g = (long)num_sms * 16;
-    k_gram_reduce<<<(int)(g > 0 ? g : 1), 256, 0, stream>>>(k1, k2, (int)nsplit, part, a_dev, lda, sym);
-    if (cudaGetLastError() != cudaSuccess) return GCGE_GPU_ERR_CUDA;
-    return GCGE_GPU_OK;
+    k_gram_reduce<<<(int)(g > 0 ? g : 1), 256, 0, stream>>>(k1, k2, nsplit, part, a_dev, lda, sym, run);
+    return cudaGetLastError() != cudaSuccess ? GCGE_GPU_ERR_CUDA : GCGE_GPU_OK;
 }
 
 // second stage of a Gram product whose per-split partials are already in part

@@ -120,9 +120,17 @@ int gb_pinned(gcge_gpu_ctx *ctx, size_t n);
 int gb_iscratch(gcge_gpu_ctx *ctx, size_t n);
 int gb_ozbuf(gcge_gpu_ctx *ctx, size_t bytes);
 int gb_check_device_error(gcge_gpu_ctx *ctx);
-/* FP64-accurate Gram on the tensor cores (gb_ozaki.cu); exps: int[k1 + k2] */
+/* FP64-accurate Gram on the tensor cores (gb_ozaki.cu); exps: int[gb_gram_tc_ints(k1, k2)] */
+size_t gb_gram_tc_ints(int k1, int k2);
 int gb_gram_tc(gcge_gpu_ctx *ctx, int n, int k1, int k2, const double *V, long ldv, const double *W, long ldw,
                double *a_dev, int lda, int sym, int *exps);
+/* the Gram on caller storage: part_cap doubles of partials, a control block of
+ * gb_gram_fixed_ctl_bytes() <= GB_GRAM_FIXED_CTL bytes, no context, no allocation */
+#define GB_GRAM_FIXED_COLS 2600
+#define GB_GRAM_FIXED_CTL 65536
+size_t gb_gram_fixed_ctl_bytes(void);
+int gb_gram_fixed(cudaStream_t stream, int num_sms, int n, int k1, int k2, const double *V, long ldv, const double *W,
+                  long ldw, double *a_dev, int lda, int sym, double *part, size_t part_cap, void *ctl_dev);
 /* FP64-accurate Y = alpha X C + beta Y on the tensor cores (gb_ozaki.cu), for k1 where
  * gb_lincomb_tc_ok(k1) holds */
 int gb_lincomb_tc_ok(int k1);

@@ -36,8 +36,9 @@
 //   per-row scales (of X equilibrated by the row scales of C), C split once per
 //   call by k_lc_coef_split;
 // k_gram_tc: V^T W, M = 128 columns of V, N = 64 columns of W, K = rows of a
-//   row split, per-column scales from a pre-pass (k_col_exponent); partial
-//   Grams of the splits are summed in a fixed order by k_gram_reduce.
+//   row split, per-column scales from a pre-pass (k_col_exponent); the splits'
+//   exact integer sums meet in atomics (any order, the same value) and the split
+//   that comes last rounds them to FP64.
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -244,11 +245,18 @@ __device__ __forceinline__ void tc_release(tc_hdr *h, uint32_t tmem, int mma_war
 // loads per row in flight) over 256-column chunks, so each row's bytes stream
 // once per chunk; each block reduces its warps and issues one atomic per column.
 #define CE_COLS 256
+// grid (blocks, 2): blockIdx.y = 0 the columns of V (exps[0:k1]), 1 those of W
+// (exps[k1:]) -- one launch, so that the two short passes share the chip.
 __global__ void __launch_bounds__(256)
-k_col_exponent(int n, int k, const double *__restrict__ X, long ldx, int *__restrict__ exps)
+k_col_exponent(int n, int k1, const double *__restrict__ V, long ldv, int k2, const double *__restrict__ W, long ldw,
+               int *__restrict__ exps)
 {
     __shared__ int se[8][CE_COLS];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int k = blockIdx.y ? k2 : k1;
+    const double *X = blockIdx.y ? W : V;
+    const long ldx = blockIdx.y ? ldw : ldv;
+    if (blockIdx.y) exps += k1;
     const long warp = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long nw = ((long)gridDim.x * blockDim.x) >> 5;
     for (int c0 = 0; c0 < k; c0 += CE_COLS) {
@@ -276,10 +284,14 @@ k_col_exponent(int n, int k, const double *__restrict__ X, long ldx, int *__rest
     }
 }
 
-__global__ void k_fill_int(int *p, int count, int v)
+// start of a Gram: column exponents unset, tickets and integer sums zero
+__global__ void k_gram_init(int *__restrict__ exps, int cols, unsigned *__restrict__ ticket, int tiles,
+                            ulonglong2 *__restrict__ sums, long total)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < count) p[i] = v;
+    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < cols) exps[i] = OZ_NO_EXP;
+    if (i < tiles) ticket[i] = 0;
+    for (long t = i; t < total; t += (long)gridDim.x * blockDim.x) sums[t] = make_ulonglong2(0, 0);
 }
 
 // ---------------------------------------------------------------- Gram V^T W (tcgen05)
@@ -294,14 +306,21 @@ __global__ void k_fill_int(int *p, int count, int v)
 #define GR_LEVELS 8
 #define GR_SMEM (2 * TC_STAGE + TC_HDR)
 
-// grid (ceil(k1 / 128), ceil(k2 / 64), splits); part[split][i + j k1] = the
-// split's exact integer sum of the digit products of sum_r V[r, i] W[r, j] as
-// (hi, lo), value (hi 2^40 + lo) 2^(e_i + f_j - 66) (sym: tiles wholly below
-// the diagonal are skipped).
+// grid (ceil(k1 / 128), ceil(k2 / 64), splits). A split's exact integer sum of the
+// digit products of sum_r V[r, i] W[r, j] is (hi, lo), value
+// (hi 2^40 + lo) 2^(e_i + f_j - 66). The splits add theirs to sums[i + j k1] by
+// atomics -- integers, so the order does not show: |hi| < 2^28.2 a row, below 2^60
+// over any n, and lo < 2^40 a split -- and the split that finishes last on a tile
+// rounds the tile to FP64 once, a[i + j lda]: the correctly rounded value of the
+// exact sum of the kept digit products, whatever the row split. (Partials per split
+// summed by a second kernel took 16 to 32 us at 76 splits of 178 x 64, and their
+// storage capped the splits of the allocation-free form at 46.)
+// sym: tiles wholly below the diagonal are skipped, entries above it mirrored.
 __global__ void __launch_bounds__(TC_THREADS, 1)
 k_gram_tc(int n, int k1, int k2, const double *__restrict__ V, long ldv, const double *__restrict__ W, long ldw,
-          const int *__restrict__ ev, const int *__restrict__ ew, long long *__restrict__ part, long rows_per_split,
-          int sym, int *__restrict__ err, int stall)
+          const int *__restrict__ ev, const int *__restrict__ ew, unsigned long long *__restrict__ sums,
+          unsigned *__restrict__ ticket, double *__restrict__ a, int lda, long rows_per_split, int sym,
+          int *__restrict__ err, int stall)
 {
     extern __shared__ __align__(1024) uint8_t tc_smem[];
     uint8_t *sm = tc_smem;
@@ -413,18 +432,55 @@ k_gram_tc(int n, int k1, int k2, const double *__restrict__ V, long ldv, const d
         if (*(volatile int *)&h->flag) break;
     }
 
+    __syncthreads();                                     // every wait of this CTA has ended: the flag is final
     if (!*(volatile int *)&h->flag) {
-        // the split's exact integer sums (level 0-2 part, level 3-7 part < 2^40),
-        // summed exactly over the splits and rounded once by k_gram_reduce_oz
         const int i = i0 + quarter * 32 + lane;
-        long long *P = part + 2 * (long)blockIdx.z * k1 * k2;
-        if (i < k1) {
+        bool last = gridDim.z == 1;
+        if (!last) {
 #pragma unroll
             for (int q = 0; q < TC_COLS_PER_WARP; ++q) {
                 const int j = j0 + col0 + q;
-                if (j < k2) {
-                    P[2 * (i + (long)j * k1)] = hi[q];
-                    P[2 * (i + (long)j * k1) + 1] = lo[q];
+                if (i < k1 && j < k2) {
+                    unsigned long long *P = sums + 2 * (i + (long)j * k1);
+                    atomicAdd(P, (unsigned long long)hi[q]);
+                    atomicAdd(P + 1, (unsigned long long)lo[q]);
+                }
+            }
+            __threadfence();
+            __syncthreads();
+            int *is_last = (int *)(sm + 2 * TC_STAGE + 64);
+            if (tid == 0) *is_last = atomicAdd(ticket + blockIdx.y * gridDim.x + blockIdx.x, 1u) == gridDim.z - 1;
+            __syncthreads();
+            last = *is_last != 0;
+            if (last) {
+                __threadfence();
+#pragma unroll
+                for (int q = 0; q < TC_COLS_PER_WARP; ++q) {
+                    const int j = j0 + col0 + q;
+                    if (i < k1 && j < k2) {
+                        const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2 *>(sums) + i + (long)j * k1);
+                        hi[q] = (long long)v.x;
+                        lo[q] = (long long)v.y;
+                    }
+                }
+            }
+        }
+        if (last) {
+#pragma unroll 1
+            for (int q = 0; q < TC_COLS_PER_WARP; ++q) {
+                const int j = j0 + col0 + q;
+                long long hq = 0, lq = 0;
+#pragma unroll
+                for (int u = 0; u < TC_COLS_PER_WARP; ++u)
+                    if (u == q) {
+                        hq = hi[u];
+                        lq = lo[u];
+                    }
+                if (i < k1 && j < k2 && !(sym && i > j)) {
+                    const __int128 z = (__int128)hq * ((__int128)1 << 40) + lq;
+                    const double s = z == 0 ? 0.0 : oz_i128_to_double(z, ev[i] + ew[j] - OZ_SCALE_OFFSET - 56);
+                    a[i + (long)j * lda] = s;
+                    if (sym && i != j) a[j + (long)i * lda] = s;
                 }
             }
         }
@@ -432,33 +488,36 @@ k_gram_tc(int n, int k1, int k2, const double *__restrict__ V, long ldv, const d
     tc_release(h, tmem, mma_warp, commits, nullptr);
 }
 
-// a[i + j lda] = the exact sum over the splits of their (hi 2^40 + lo) integer
-// sums, rounded once to FP64: every Gram entry is the correctly rounded value of
-// the exact sum of the split operands' kept digit products, whatever the row
-// split (sym: upper triangle computed, mirrored)
-__global__ void k_gram_reduce_oz(int k1, int k2, int nsplit, const long long *__restrict__ part,
-                                 const int *__restrict__ ev, const int *__restrict__ ew, double *__restrict__ a,
-                                 int lda, int sym)
+// Row splits of the tensor-core Gram and the rows of each: about one CTA per SM. int64 headroom: a row adds < 2^28.2 to the level 0-2 sum (units
+// of 2^-16), so a split holds at most GR_MAX_ROWS rows (the level 3-7 sum is
+// carried into it after every chunk).
+#define GR_MAX_ROWS (1L << 20)
+static long gram_tc_splits(int num_sms, int n, int k1, int k2, int sym, long *rps_out)
 {
-    const long total = (long)k1 * k2;
-    for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
-        const int i = (int)(t % k1), j = (int)(t / k1);
-        if (sym && i > j) continue;
-        __int128 hs = 0;
-        long long ls = 0;                                // nsplit < 2^23 terms below 2^40 each
-        for (int q = 0; q < nsplit; ++q) {
-            hs += part[2 * ((long)q * total + t)];
-            ls += part[2 * ((long)q * total + t) + 1];
-        }
-        const __int128 z = hs * ((__int128)1 << 40) + ls;
-        const double s = z == 0 ? 0.0 : oz_i128_to_double(z, ev[i] + ew[j] - OZ_SCALE_OFFSET - 56);
-        a[i + (long)j * lda] = s;
-        if (sym && i != j) a[j + (long)i * lda] = s;
-    }
+    const int ti = (k1 + TC_M - 1) / TC_M, tj = (k2 + TC_N - 1) / TC_N;
+    int tiles = 0;
+    for (int a = 0; a < ti; ++a)
+        for (int b = 0; b < tj; ++b)
+            if (!sym || a * TC_M <= b * TC_N + TC_N - 1) ++tiles;
+    if (tiles < 1) tiles = 1;
+    long nsplit = ((long)num_sms + tiles - 1) / tiles;
+    const long max_split = (n + 4 * TC_KS - 1) / (4 * TC_KS);
+    if (nsplit > max_split) nsplit = max_split;
+    const long min_split = (n + GR_MAX_ROWS - 1) / GR_MAX_ROWS;
+    if (nsplit < min_split) nsplit = min_split;
+    if (nsplit < 1) nsplit = 1;
+    const long rps = ((n + nsplit - 1) / nsplit + TC_KS - 1) / TC_KS * TC_KS;
+    *rps_out = rps;
+    nsplit = (n + rps - 1) / rps;
+    return nsplit < 1 ? 1 : nsplit;
 }
 
 // a[i + j*lda] = sum_r V[r,i] W[r,j] to FP64 accuracy on the tensor cores.
-// exps: device int[k1 + k2] scratch for the column scales.
+// exps: device scratch of gb_gram_tc_ints(k1, k2) ints (column scales, tickets).
+extern "C" size_t gb_gram_tc_ints(int k1, int k2)
+{
+    return (size_t)k1 + k2 + (size_t)((k1 + TC_M - 1) / TC_M) * ((k2 + TC_N - 1) / TC_N);
+}
 extern "C" int gb_gram_tc(gcge_gpu_ctx *ctx, int n, int k1, int k2, const double *V, long ldv, const double *W,
                           long ldw, double *a_dev, int lda, int sym, int *exps)
 {
@@ -471,40 +530,192 @@ extern "C" int gb_gram_tc(gcge_gpu_ctx *ctx, int n, int k1, int k2, const double
         attr = true;
     }
     const int ti = (k1 + TC_M - 1) / TC_M, tj = (k2 + TC_N - 1) / TC_N;
-    int tiles = 0;
-    for (int a = 0; a < ti; ++a)
-        for (int b = 0; b < tj; ++b)
-            if (!sym || a * TC_M <= b * TC_N + TC_N - 1) ++tiles;
-    if (tiles < 1) tiles = 1;
-    // about one CTA per SM; int64 headroom: a row adds < 2^28.2 to the level 0-2
-    // sum (units of 2^-16), so a split holds at most 2^20 rows (the level 3-7 sum
-    // is carried into it after every chunk)
-    long nsplit = ((long)ctx->num_sms + tiles - 1) / tiles;
-    const long max_split = (n + 4 * TC_KS - 1) / (4 * TC_KS);
-    if (nsplit > max_split) nsplit = max_split;
-    const long min_split = (n + (1L << 20) - 1) >> 20;
-    if (nsplit < min_split) nsplit = min_split;
-    if (nsplit < 1) nsplit = 1;
-    long rps = ((n + nsplit - 1) / nsplit + TC_KS - 1) / TC_KS * TC_KS;
-    nsplit = (n + rps - 1) / rps;
-    if (nsplit < 1) nsplit = 1;
-    int st = gb_scratch(ctx, (size_t)2 * nsplit * k1 * k2);
+    long rps = 0;
+    const long nsplit = gram_tc_splits(ctx->num_sms, n, k1, k2, sym, &rps);
+    const long total = (long)k1 * k2;
+    int st = gb_scratch(ctx, (size_t)2 * total);
     if (st) return st;
-    GB_LAUNCH(ctx, k_fill_int, (k1 + k2 + 127) / 128, 128, 0, exps, k1 + k2, OZ_NO_EXP);
-    const int eg = ctx->num_sms * 4;
-    GB_LAUNCH(ctx, k_col_exponent, eg, 256, 0, n, k1, V, ldv, exps);
-    GB_LAUNCH(ctx, k_col_exponent, eg, 256, 0, n, k2, W, ldw, exps + k1);
+    unsigned *ticket = (unsigned *)(exps + k1 + k2);
+    const long cols = k1 + k2, most = total > cols ? total : cols;
+    GB_LAUNCH(ctx, k_gram_init, (int)((most < 65536 ? most : 65536) + 255) / 256, 256, 0, exps, (int)cols, ticket,
+              ti * tj, (ulonglong2 *)ctx->scratch, nsplit > 1 ? total : 0);
+    GB_LAUNCH(ctx, k_col_exponent, dim3(ctx->num_sms * 4, 2), 256, 0, n, k1, V, ldv, k2, W, ldw, exps);
     dim3 grid(ti, tj, (unsigned)nsplit);
     GB_PROF(ctx, GB_K_GRAM, 8.0 * n * (k1 + k2), sym ? 1.0 * n * k1 * (k1 + 1) : 2.0 * n * k1 * k2);
     const int stall = ctx->tc_stall;
     ctx->tc_stall = 0;
-    long long *part = reinterpret_cast<long long *>(ctx->scratch);
-    GB_LAUNCH(ctx, k_gram_tc, grid, TC_THREADS, GR_SMEM, n, k1, k2, V, ldv, W, ldw, exps, exps + k1, part, rps, sym,
-              ctx->dev_err, stall);
-    long rg = ((long)k1 * k2 + 255) / 256;
-    if (rg > (long)ctx->num_sms * 16) rg = (long)ctx->num_sms * 16;
-    GB_LAUNCH(ctx, k_gram_reduce_oz, (int)rg, 256, 0, k1, k2, (int)nsplit, part, exps, exps + k1, a_dev, lda, sym);
+    GB_LAUNCH(ctx, k_gram_tc, grid, TC_THREADS, GR_SMEM, n, k1, k2, V, ldv, W, ldw, exps, exps + k1,
+              (unsigned long long *)ctx->scratch, ticket, a_dev, lda, rps, sym, ctx->dev_err, stall);
     return GCGE_GPU_OK;
+}
+
+// ---------------------------------------------------------------- Gram on fixed storage
+// The allocation-free Gram on the tensor cores. What the FP64-pipe form took at
+// 262,144 x (178, 64) was the FP64 pipe itself: 5.44 ms at 1.1 of 1.2 TFLOP/s.
+//
+// Column scales serve every row of a column, so an entry far below its column's
+// largest keeps fewer bits than FP64 would. k_col_stats therefore forms, beside the
+// scale e (max |x| < 2^e), the mean exponent of the nonzero entries, and the block
+// that finishes last sets ctl->skip when a column's mean lies more than
+// GN_SPREAD below its e, or an entry is not finite or subnormal: the FP64-pipe kernel that
+// follows then does the work, and nothing otherwise. With GN_SPREAD = 5 the digits
+// of a typical entry end 2^-49 below it and their roundings are independent, so
+// their sum over n rows stays under the FP64 form's own summation error (normal
+// and smooth columns, n from 1,000 to 600,000: 0.4 to 0.02 of it). A bounded wait
+// that runs out sets skip as well.
+#define GN_SPREAD 5
+struct gn_ctl {
+    int skip;
+    unsigned done;
+    unsigned ticket[GB_GRAM_FIXED_COLS];                 // tiles <= k1 + k2
+    int e[GB_GRAM_FIXED_COLS], cnt[GB_GRAM_FIXED_COLS];
+    long long sum[GB_GRAM_FIXED_COLS];
+};
+extern "C" size_t gb_gram_fixed_ctl_bytes(void) { return sizeof(gn_ctl); }
+
+__global__ void k_gn_init(gn_ctl *ctl, int cols, ulonglong2 *__restrict__ sums, long total)
+{
+    const long c = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (c == 0) {
+        ctl->skip = 0;
+        ctl->done = 0;
+    }
+    if (c < cols) {
+        ctl->ticket[c] = 0;
+        ctl->e[c] = OZ_NO_EXP;
+        ctl->cnt[c] = 0;
+        ctl->sum[c] = 0;
+    }
+    for (long t = c; t < total; t += (long)gridDim.x * blockDim.x) sums[t] = make_ulonglong2(0, 0);
+}
+
+// grid (blocks, 2): blockIdx.y = 0 the columns of V, 1 those of W. A warp reads
+// whole rows, eight independent loads per lane in flight, as k_col_exponent.
+__global__ void __launch_bounds__(256)
+k_col_stats(int n, int k1, const double *__restrict__ V, long ldv, int k2, const double *__restrict__ W, long ldw,
+            gn_ctl *ctl)
+{
+    __shared__ int se[8][CE_COLS], sc[8][CE_COLS], ss[8][CE_COLS];
+    __shared__ int done, wide;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int k = blockIdx.y ? k2 : k1, off = blockIdx.y ? k1 : 0;
+    const double *X = blockIdx.y ? W : V;
+    const long ldx = blockIdx.y ? ldw : ldv;
+    const long warp = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long nw = ((long)gridDim.x * blockDim.x) >> 5;
+    for (int c0 = 0; c0 < k; c0 += CE_COLS) {
+        int e[CE_COLS / 32], cnt[CE_COLS / 32], sum[CE_COLS / 32];   // a warp's rows: below 2^20
+#pragma unroll
+        for (int j = 0; j < CE_COLS / 32; ++j) {
+            e[j] = OZ_NO_EXP;
+            cnt[j] = 0;
+            sum[j] = 0;
+        }
+        for (long r = warp; r < n; r += nw) {
+            const double *xr = X + r * ldx + c0 + lane;
+            double v[CE_COLS / 32];
+#pragma unroll
+            for (int j = 0; j < CE_COLS / 32; ++j) v[j] = c0 + lane + 32 * j < k ? __ldg(xr + 32 * j) : 0.0;
+#pragma unroll
+            for (int j = 0; j < CE_COLS / 32; ++j) {
+                // a subnormal entry has no digits: counted as not finite
+                int x = oz_exponent(v[j]);
+                if (x == OZ_NO_EXP && (__double_as_longlong(v[j]) << 1)) x = 1025;
+                if (x != OZ_NO_EXP) {
+                    e[j] = max(e[j], x);
+                    ++cnt[j];
+                    sum[j] += x;
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < CE_COLS / 32; ++j) {
+            se[w][lane + 32 * j] = e[j];
+            sc[w][lane + 32 * j] = cnt[j];
+            ss[w][lane + 32 * j] = sum[j];
+        }
+        __syncthreads();
+        for (int c = threadIdx.x; c < CE_COLS; c += blockDim.x) {
+            int m = OZ_NO_EXP, q = 0;
+            long long t = 0;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                m = max(m, se[u][c]);
+                q += sc[u][c];
+                t += ss[u][c];
+            }
+            if (c0 + c < k && m > OZ_NO_EXP) {
+                atomicMax(&ctl->e[off + c0 + c], m);
+                atomicAdd(&ctl->cnt[off + c0 + c], q);
+                atomicAdd((unsigned long long *)&ctl->sum[off + c0 + c], (unsigned long long)t);
+            }
+        }
+        __syncthreads();
+    }
+    __threadfence();
+    if (threadIdx.x == 0) {
+        done = atomicAdd(&ctl->done, 1u) == gridDim.x * 2 - 1;
+        wide = 0;
+    }
+    __syncthreads();
+    if (!done) return;
+    __threadfence();
+    for (int c = threadIdx.x; c < k1 + k2; c += blockDim.x) {
+        const long long q = __ldcg(&ctl->cnt[c]), t = __ldcg(&ctl->sum[c]);
+        const int m = __ldcg(&ctl->e[c]);
+        if (m > 1024 || (long long)m * q - t > GN_SPREAD * q) wide = 1;   // e = 1025: not finite, or subnormal
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && wide) ctl->skip = 1;
+}
+
+extern "C" int gb_gram_fixed_partials(cudaStream_t stream, int num_sms, int n, int k1, int k2, const double *V,
+                                      long ldv, const double *W, long ldw, int sym, double *part, size_t part_cap,
+                                      const int *run, int *st);
+extern "C" int gb_gram_fixed_reduce(cudaStream_t stream, int num_sms, int k1, int k2, int nsplit, const double *part,
+                                    double *a_dev, int lda, int sym, const int *run);
+
+// Gram V^T W with caller-provided partials (part_cap doubles), control block and
+// stream: no context, no allocation; part_cap >= 2 k1 k2. The tensor-core form where
+// its estimate is the shorter one. Measured on the GB300: a CTA takes a stage of 32
+// rows in 2.6 us for a few columns and 4.6 us for a full tile, and the form has 40 us
+// of launches, scales and drain beside it; the FP64 pipe takes 8.2 us for 32 rows of
+// a 32 x 32 tile on each SM, and 12 us.
+extern "C" long gb_gram_fixed_splits(int num_sms, int n, int k1, int k2, int sym, size_t part_cap, long *rps_out);
+extern "C" int gb_gram_fixed(cudaStream_t stream, int num_sms, int n, int k1, int k2, const double *V, long ldv,
+                             const double *W, long ldw, double *a_dev, int lda, int sym, double *part,
+                             size_t part_cap, void *ctl_dev)
+{
+    gn_ctl *ctl = (gn_ctl *)ctl_dev;
+    int st = GCGE_GPU_OK;
+    const int *run = nullptr;
+    if (k1 + k2 <= GB_GRAM_FIXED_COLS) {
+        const int ti = (k1 + TC_M - 1) / TC_M, tj = (k2 + TC_N - 1) / TC_N;
+        long rps = 0;
+        const long nsplit = gram_tc_splits(num_sms, n, k1, k2, sym, &rps), total = (long)k1 * k2;
+        const double waves = (double)(((long)ti * tj * nsplit + num_sms - 1) / num_sms);
+        const double fill = (double)((k1 < TC_M ? k1 : TC_M) + (k2 < TC_N ? k2 : TC_N)) / (TC_M + TC_N);
+        const double t_tc = 40.0 + waves * (double)(rps / TC_KS) * (2.6 + 2.0 * fill);
+        long rps64 = 0;
+        const long n64 = gb_gram_fixed_splits(num_sms, n, k1, k2, sym, part_cap, &rps64);
+        const long b64 = n64 * ((k1 + 31) / 32) * ((k2 + 31) / 32);
+        const double t_64 = 12.0 + 8.2 * (double)(rps64 / 32) * (double)((b64 + num_sms - 1) / num_sms);
+        if (t_tc < t_64) {
+            if (cudaFuncSetAttribute(k_gram_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, GR_SMEM) != cudaSuccess)
+                return GCGE_GPU_ERR_CUDA;
+            const long most = total > k1 + k2 ? total : k1 + k2;
+            k_gn_init<<<(int)((most < 65536 ? most : 65536) + 255) / 256, 256, 0, stream>>>(
+                ctl, k1 + k2, (ulonglong2 *)part, nsplit > 1 ? total : 0);
+            k_col_stats<<<dim3(num_sms * 4, 2), 256, 0, stream>>>(n, k1, V, ldv, k2, W, ldw, ctl);
+            k_gram_tc<<<dim3(ti, tj, (unsigned)nsplit), TC_THREADS, GR_SMEM, stream>>>(
+                n, k1, k2, V, ldv, W, ldw, ctl->e, ctl->e + k1, (unsigned long long *)part, ctl->ticket, a_dev, lda,
+                rps, sym, &ctl->skip, 0);
+            if (cudaGetLastError() != cudaSuccess) return GCGE_GPU_ERR_CUDA;
+            run = &ctl->skip;
+        }
+    }
+    const int n64 = gb_gram_fixed_partials(stream, num_sms, n, k1, k2, V, ldv, W, ldw, sym, part, part_cap, run, &st);
+    return st ? st : gb_gram_fixed_reduce(stream, num_sms, k1, k2, n64, part, a_dev, lda, sym, run);
 }
 
 // ---------------------------------------------------------------- linear combination (tcgen05)

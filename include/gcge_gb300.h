@@ -316,8 +316,9 @@ int  GCGE_GPU_EigvecAdjoint(const gcge_gpu_mat *A, const gcge_gpu_mat *B, const 
  *          (the multivector layout of this library), n rows, k1 / k2 columns;
  *   a      device pointer, column major with leading dimension lda >= k1;
  *   stream a cudaStream_t (NULL: the default stream); the call is asynchronous.
- * Partial sums go to a fixed 8 MiB device array inside the library (held by
- * every GPU that loads it, until exit), so k1*k2 may be at most 262,144.
+ * Partial sums go to a fixed 8 MiB device array inside the library, with 64 KiB of
+ * column scales beside it (held by every GPU that loads it, until exit), so k1*k2
+ * may be at most 262,144.
  * Larger sizes are rejected with GCGE_GPU_ERR_ARG. The first call on a device
  * looks up the array's device address with that device current; make that
  * first call before any stream capture. All calls share the array and it keeps

@@ -221,3 +221,64 @@ def test_tensor_gram_at_full_size_against_exact(ctx, pattern):
             worst = max(worst, err / float(abs(ex)))
     # far inside the FP64 summation error of the same Gram (same sign: ~n eps / nsplit relative)
     assert worst < (1e-15 if pattern == "same_sign" else 1e-10), worst
+
+
+# ---- the allocation-free Gram: tensor cores or the FP64 pipe, chosen on the device
+def _no_alloc(torch, V, W, k1, k2, sym=0):
+    lib = G.load()
+    lda = k1 + 1
+    a = torch.full((k2, lda), float("nan"), dtype=torch.float64, device="cuda")
+    st = lib.GCGE_GPU_InnerProdNoAlloc(V.shape[0], k1, k2, V.data_ptr(), V.stride(0), W.data_ptr(), W.stride(0),
+                                       a.data_ptr(), lda, sym, torch.cuda.current_stream().cuda_stream)
+    assert st == 0
+    return a[:, :k1].T.cpu().numpy()
+
+
+@pytest.mark.parametrize("n,k1,k2", [(60001, 128, 64), (60017, 129, 65), (250007, 16, 8), (90000, 300, 40),
+                                     (33, 4, 3), (1 << 20, 17, 16), ((1 << 20) + 5, 16, 17)])
+def test_no_alloc_gram_sides_of_the_tiles(n, k1, k2):
+    """Widths at and past a tile's edge, rows with a remainder, both forms: every entry
+    within the summation bound n 2^-53 sum |v w| of the product in long double, taken
+    in runs (n 2^-64 of it more)."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(n + k1)
+    V = torch.from_numpy(rng.standard_normal((n, k1 + 2))).cuda()
+    W = torch.from_numpy(rng.uniform(-1, 1, (n, k2 + 1))).cuda()
+    got = _no_alloc(torch, V, W, k1, k2)
+    v, w = V.cpu().numpy(), W.cpu().numpy()
+    for i, j in [(0, 0), (k1 - 1, k2 - 1), (k1 // 2, k2 // 2), (min(127, k1 - 1), min(63, k2 - 1))]:
+        t = v[:, i].astype(np.longdouble) * w[:, j]
+        assert abs(got[i, j] - t.sum()) <= n * 2.0 ** -53 * float(np.abs(t).sum())
+    assert np.all(np.isfinite(got))
+
+
+@pytest.mark.parametrize("what", ["spike", "range", "nan", "inf", "subnormal", "zero"])
+def test_no_alloc_gram_columns_that_a_scale_does_not_serve(what):
+    """Columns whose entries lie far below the largest, and entries without digits, get
+    what plain FP64 sums give: exact integers, or NaN and infinities where FP64 has them."""
+    torch = pytest.importorskip("torch")
+    n, k1, k2 = 70000, 130, 66
+    rng = np.random.default_rng(3)
+    v, w = rng.integers(-3, 4, (n, k1)).astype(float), rng.integers(-3, 4, (n, k2)).astype(float)
+    if what == "spike":
+        v[5, 7], w[5] = 2.0 ** 80, 0.0
+    elif what == "range":
+        w[:, 3] *= 2.0 ** rng.integers(-40, 40, n)
+        v[:] = 0.0
+        v[11, 2] = 1.0
+    elif what == "nan":
+        v[9, 1] = np.nan
+    elif what == "inf":
+        w[69999, 65], v[69999] = np.inf, 1.0
+    elif what == "subnormal":
+        v[:, 4] = 2.0 ** -1070
+        w[:, 2] = 2.0 ** 1000
+    else:
+        v[:, 5] = w[:, 6] = 0.0
+    got = _no_alloc(torch, torch.from_numpy(v).cuda(), torch.from_numpy(w).cuda(), k1, k2)
+    with np.errstate(invalid="ignore"):
+        ref = v.T @ w
+    if what == "subnormal":
+        np.testing.assert_allclose(got, ref, rtol=n * 2.0 ** -53)
+    else:
+        np.testing.assert_array_equal(got, ref)
