@@ -153,6 +153,8 @@ extern "C" int GCGE_GPU_Init(int device, gcge_gpu_ctx **out)
     if (!st) st = gb_ozbuf(c, 1 << 20);
     if (!st && (cudaMalloc(&c->dev_err, sizeof(int)) != cudaSuccess ||
                 cudaMemsetAsync(c->dev_err, 0, sizeof(int), c->stream) != cudaSuccess ||
+                cudaMalloc(&c->dev_bar, 4 * sizeof(unsigned)) != cudaSuccess ||
+                cudaMemsetAsync(c->dev_bar, 0, 4 * sizeof(unsigned), c->stream) != cudaSuccess ||
                 cudaMalloc(&c->dev_pairflag, sizeof(int)) != cudaSuccess ||
                 cudaMemsetAsync(c->dev_pairflag, 0, sizeof(int), c->stream) != cudaSuccess))
         st = GCGE_GPU_ERR_NOMEM;
@@ -246,6 +248,7 @@ extern "C" int GCGE_GPU_Finalize(gcge_gpu_ctx *ctx)
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
     if (ctx->ozbuf) cudaFree(ctx->ozbuf);
     if (ctx->dev_err) cudaFree(ctx->dev_err);
+    if (ctx->dev_bar) cudaFree(ctx->dev_bar);
     if (ctx->dev_pairflag) cudaFree(ctx->dev_pairflag);
     if (ctx->pairbuf) cudaFree(ctx->pairbuf);
     cudaStreamDestroy(ctx->stream);
@@ -784,7 +787,7 @@ extern "C" int GCGE_GPU_BCG(const gcge_gpu_mat *A, gcge_gpu_mv *RHS, int r_start
     if (k <= 0) return GCGE_GPU_OK;
     size_t bytes = gb_bcg_work_bytes(A->n, k, precision);
     void *work = nullptr;
-    CUDA_TRY(ctx, cudaMalloc(&work, bytes));
+    if (gb_dev_alloc(ctx, &work, bytes)) return gb_fail(ctx, GCGE_GPU_ERR_CUDA);
     gb_bcg_args args;
     memset(&args, 0, sizeof(args));
     args.n = A->n;
@@ -794,7 +797,7 @@ extern "C" int GCGE_GPU_BCG(const gcge_gpu_mat *A, gcge_gpu_mv *RHS, int r_start
     args.rate = cg_rate;
     int st = gb_bcg(ctx, A, RHS->d + r_start, RHS->ld, W->d + w_start, W->ld, &args, work, bytes);
     cudaStreamSynchronize(ctx->stream);
-    cudaFree(work);
+    gb_dev_free(ctx, work);
     return st;
 }
 

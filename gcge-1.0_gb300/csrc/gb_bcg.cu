@@ -12,13 +12,14 @@
 // (src/gcge_cg.c:286-294 writes unlock[idx] = idx at position idx, and the
 // update loops walk unlock[0 .. num_unlock)).
 //
-// precision 0: FP64 vectors and values. precision 1: the residual of the initial
+// precision 0: FP64 vectors and values, all rounds in one launch (gb_bcg_persist.cu). precision 1: the residual of the initial
 // guess is formed in FP64, then CG runs on the correction with FP32 vectors and
 // the FP32 copy of the matrix values; products are formed in FP32 and summed in
 // FP32 over runs of 8 rows, then accumulated in FP64 (FP64-reduced dot products);
 // the correction is added to the FP64 solution at the end.
 #include <cuda_runtime.h>
 
+#include "gb_bcg.h"
 #include "gb_internal.h"
 
 #define RED_ROWS 128
@@ -38,11 +39,6 @@ static inline int cdiv(long a, long b) { return (int)((a + b - 1) / b); }
         int _st = gb_check_launch(ctx);                                                \
         if (_st) return _st;                                                           \
     } while (0)
-
-struct bcg_state {
-    double *rho1, *rho2, *err, *ptw, *part, *alpha, *beta, *sums;
-    int *nact;
-};
 
 // warp-per-row loop over an n x k block: lanes walk the columns of one row
 #define ROWS_BY_WARP(n, r)                                                             \
@@ -221,12 +217,20 @@ static int row_grid(gcge_gpu_ctx *ctx, long rows)
 // cdiv(n, RED_ROWS) rows of the other kernels)
 #define LONG_PART_ROWS 2048
 
+// the FP64 rounds may form p where it is gathered (a second buffer of p) up to this
+// many entries of a block; which calls do is decided at the launch, by their work
+#define FUSE_MAX 400000L
+static bool fuse_direction(int n, int k) { return (long)n * ((k + 3) & ~3) <= FUSE_MAX; }
+
 extern "C" size_t gb_bcg_work_bytes(int n, int k, int precision)
 {
     long ldk = (k + 3) & ~3;   // 16-byte rows for the vectorised SpMM
     size_t vec = precision ? sizeof(float) : sizeof(double);
     size_t nblk = (size_t)cdiv(n > 0 ? n : 1, RED_ROWS) + (precision ? LONG_PART_ROWS : 0);
-    size_t blocks = 4 * (size_t)n * ldk * vec;  // R, X, P, W
+    // FP32: R, X, P, W; FP64: P, W and, where it is used, P2 -- never less for more
+    // columns, as the solver sizes the workspace for its widest block
+    size_t blocks = (precision ? 4 : 2) * (size_t)n * ldk * vec;
+    if (!precision && blocks < 3 * vec * FUSE_MAX) blocks = 3 * vec * (fuse_direction(n, k) ? (size_t)n * ldk : FUSE_MAX);
     size_t state = (7 * (size_t)k + nblk * (size_t)k + 8) * sizeof(double) + 64;
     return blocks + state + 16 * 256;   // every sub-buffer is aligned to 256 bytes (10 of them)
 }
@@ -676,29 +680,23 @@ static int bcg_rounds32(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, float *R, floa
     return GCGE_GPU_OK;
 }
 
-template <typename T>
-static int bcg_rounds(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, T *R, T *X, T *P, T *W, long ld,
-                      const gb_bcg_args *a, bcg_state *s)
+// FP32 rounds of blocks wider than the fused kernels take (256 columns)
+static int bcg_rounds32_wide(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, float *R, float *X, float *P, float *W, long ld,
+                             const gb_bcg_args *a, bcg_state *s)
 {
     const int n = a->n, k = a->k, nblk = cdiv(n > 0 ? n : 1, RED_ROWS);
     dim3 rgrid(nblk, (k + 31) / 32);
-    const double es = sizeof(T);
-    const T *dv = sizeof(T) == sizeof(double) ? (const T *)(const void *)a->dinv : (const T *)(const void *)a->dinv32;
     for (int it = 1; it < a->max_it; ++it) {
-        GB_PROF(ctx, GB_K_BCGVEC, 3.0 * es * n * k, 2.0 * n * k);
-        GB_LAUNCH(ctx, k_pupdate<T>, row_grid(ctx, n), 256, 0, n, k, R, P, ld, s->beta, s->nact, it == 1, dv);
-        int st;
-        if (sizeof(T) == sizeof(double))
-            st = gb_spmm(ctx, A, (const double *)P, ld, (double *)W, ld, k, 1.0, nullptr, 0.0, s->nact);
-        else
-            st = gb_spmm32(ctx, A, (const float *)P, ld, (float *)W, ld, k, s->nact);
+        GB_PROF(ctx, GB_K_BCGVEC, 12.0 * n * k, 2.0 * n * k);
+        GB_LAUNCH(ctx, k_pupdate<float>, row_grid(ctx, n), 256, 0, n, k, R, P, ld, s->beta, s->nact, it == 1, a->dinv32);
+        int st = gb_spmm32(ctx, A, P, ld, W, ld, k, s->nact);
         if (st) return st;
-        GB_PROF(ctx, GB_K_BCGVEC, 2.0 * es * n * k, 2.0 * n * k);
-        GB_LAUNCH(ctx, k_dot_partial<T>, rgrid, 256, 0, n, k, P, W, ld, s->nact, s->part);
+        GB_PROF(ctx, GB_K_BCGVEC, 8.0 * n * k, 2.0 * n * k);
+        GB_LAUNCH(ctx, k_dot_partial<float>, rgrid, 256, 0, n, k, P, W, ld, s->nact, s->part);
         GB_LAUNCH(ctx, k_colsum, k, 256, 0, nblk, k, s->part, s->nact, s->ptw);
         GB_LAUNCH(ctx, k_sum_active, (k + 127) / 128, 128, 0, k, s->nact, s->ptw, s->rho2, s->alpha);
-        GB_PROF(ctx, GB_K_BCGVEC, 6.0 * es * n * k, 6.0 * n * k);
-        GB_LAUNCH(ctx, k_xr_update<T>, rgrid, 256, 0, n, k, X, R, P, W, ld, s->alpha, s->nact, s->part, dv);
+        GB_PROF(ctx, GB_K_BCGVEC, 24.0 * n * k, 6.0 * n * k);
+        GB_LAUNCH(ctx, k_xr_update<float>, rgrid, 256, 0, n, k, X, R, P, W, ld, s->alpha, s->nact, s->part, a->dinv32);
         GB_LAUNCH(ctx, k_colsum, k, 256, 0, nblk, k, s->part, s->nact, s->sums);
         GB_LAUNCH(ctx, k_finalize, 1, 256, 0, k, s->sums, s->rho1, s->rho2, s->err, s->nact, a->rate, s->beta);
     }
@@ -727,34 +725,14 @@ extern "C" int gb_bcg(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, double *RHS, lon
     s.sums = (double *)take(sizeof(double) * k);
     s.part = (double *)take(sizeof(double) * (size_t)(nblk + (a->precision ? LONG_PART_ROWS : 0)) * k);
     s.nact = (int *)take(64);
-    dim3 rgrid(nblk, (k + 31) / 32);
     if (a->precision == 0) {
         double *P = (double *)take((size_t)n * ld * vec);
         double *W = (double *)take((size_t)n * ld * vec);
-        (void)W;
+        double *P2 = fuse_direction(n, k) ? (double *)take((size_t)n * ld * vec) : nullptr;
+        if ((size_t)(w - (char *)work) > work_bytes) return gb_fail(ctx, GCGE_GPU_ERR_ARG);
         // R = RHS - A X, in place in RHS (the reference overwrites RHS with the residual)
         int st = a->rhs_is_residual ? 0 : gb_spmm(ctx, A, X, ldx, RHS, ldr, k, -1.0, nullptr, 1.0, nullptr);
-        if (st) return st;
-        // P and W use the compact ld; R and X keep their own ld through the copies below
-        if (ldr == ld && ldx == ld) {
-            GB_LAUNCH(ctx, k_dot_partial<double>, rgrid, 256, 0, n, k, RHS, RHS, ld, (const int *)nullptr, s.part,
-                      a->dinv);
-            GB_LAUNCH(ctx, k_colsum, k, 256, 0, nblk, k, s.part, (const int *)nullptr, s.sums);
-            GB_LAUNCH(ctx, k_init_state, 1, 256, 0, k, s.sums, s.rho2, s.err, s.nact);
-            return bcg_rounds<double>(ctx, A, RHS, X, P, W, ld, a, &s);
-        }
-        // general leading dimensions: stage R and X in compact blocks
-        double *R = (double *)take((size_t)n * ld * vec);
-        double *Xc = (double *)take((size_t)n * ld * vec);
-        if ((size_t)(w - (char *)work) > work_bytes) return gb_fail(ctx, GCGE_GPU_ERR_ARG);
-        if ((st = gb_axpby(ctx, n, k, 1.0, RHS, ldr, 0.0, R, ld))) return st;
-        if ((st = gb_axpby(ctx, n, k, 1.0, X, ldx, 0.0, Xc, ld))) return st;
-        GB_LAUNCH(ctx, k_dot_partial<double>, rgrid, 256, 0, n, k, R, R, ld, (const int *)nullptr, s.part, a->dinv);
-        GB_LAUNCH(ctx, k_colsum, k, 256, 0, nblk, k, s.part, (const int *)nullptr, s.sums);
-            GB_LAUNCH(ctx, k_init_state, 1, 256, 0, k, s.sums, s.rho2, s.err, s.nact);
-        if ((st = bcg_rounds<double>(ctx, A, R, Xc, P, W, ld, a, &s))) return st;
-        if ((st = gb_axpby(ctx, n, k, 1.0, Xc, ld, 0.0, X, ldx))) return st;
-        return gb_axpby(ctx, n, k, 1.0, R, ld, 0.0, RHS, ldr);
+        return st ? st : gb_bcg_persist64(ctx, A, a, &s, RHS, ldr, X, ldx, P, P2, W, ld);
     }
     // Mixed precision as defect correction: the residual r0 = RHS - A X is formed in
     // FP64, block CG runs in FP32 on A D = r0 from D = 0, and X += D in FP64. The
@@ -770,10 +748,11 @@ extern "C" int gb_bcg(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, double *RHS, lon
     if ((st = gb_convert_d2f(ctx, n, k, RHS, ldr, R, ld))) return st;
     if (cudaMemsetAsync(D, 0, (size_t)n * ld * sizeof(float), ctx->stream) != cudaSuccess)
         return gb_fail(ctx, GCGE_GPU_ERR_CUDA);
-    GB_LAUNCH(ctx, k_dot_partial<float>, rgrid, 256, 0, n, k, R, R, ld, (const int *)nullptr, s.part, a->dinv32);
+    GB_LAUNCH(ctx, k_dot_partial<float>, dim3(nblk, (k + 31) / 32), 256, 0, n, k, R, R, ld, (const int *)nullptr, s.part,
+              a->dinv32);
     GB_LAUNCH(ctx, k_colsum, k, 256, 0, nblk, k, s.part, (const int *)nullptr, s.sums);
     GB_LAUNCH(ctx, k_init_state, 1, 256, 0, k, s.sums, s.rho2, s.err, s.nact);
-    if ((st = k <= 256 ? bcg_rounds32(ctx, A, R, D, P, W, ld, a, &s) : bcg_rounds<float>(ctx, A, R, D, P, W, ld, a, &s)))
+    if ((st = k <= 256 ? bcg_rounds32(ctx, A, R, D, P, W, ld, a, &s) : bcg_rounds32_wide(ctx, A, R, D, P, W, ld, a, &s)))
         return st;
     GB_LAUNCH(ctx, k_add_f2d, row_grid(ctx, n), 256, 0, n, k, D, ld, X, ldx);
     return a->residual_unused ? GCGE_GPU_OK : gb_convert_f2d(ctx, n, k, R, ld, RHS, ldr);

@@ -291,3 +291,59 @@ def test_range_checks(ctx):
     x, y = ctx.multivec(100, 4), ctx.multivec(100, 4)
     with pytest.raises(G.GcgeGpuError):
         G.multivec_axpby(1.0, x, 0.0, y, (0, 2), (3, 5))
+
+
+def _block_cg(A, R0, W0, rounds, rate):
+    """GCGE_BCG's iteration in numpy: the first `count` columns are iterated, count taken
+    over all columns after each round."""
+    x, r = W0.copy(), R0 - A @ W0
+    rho = np.sum(r * r, axis=0)
+    err, p, act = np.sqrt(rho), np.zeros_like(r), r.shape[1]
+    beta = np.zeros(r.shape[1])
+    for _ in range(rounds):
+        if act == 0:
+            break
+        a = slice(0, act)
+        p[:, a] = r[:, a] + beta[a] * p[:, a]
+        w = A @ p[:, a]
+        alpha = rho[a] / np.sum(p[:, a] * w, axis=0)
+        x[:, a] += alpha * p[:, a]
+        r[:, a] -= alpha * w
+        new = np.sum(r[:, a] ** 2, axis=0)
+        beta[a], rho[a] = new / rho[a], new
+        act = int(np.sum(np.sqrt(rho) / err >= rate))
+    return x, r
+
+
+@pytest.mark.parametrize("shape,k,rounds,rate", [
+    ((1, 1), 1, 2, 1e-3), ((16, 8), 3, 6, 1e-2), ((43, 3), 17, 6, 1e-2), ((30, 30), 150, 5, 1e-2),
+    ((100, 100), 10, 8, 1e-3), ((200, 200), 5, 8, 1e-2), ((120, 90), 131, 4, 1e-30), ((300, 280), 33, 5, 1e-30),
+    ("graph", 6, 8, 1e-2), ("graph", 40, 4, 1e-30)])
+def test_bcg_fp64_on_the_sides_of_its_forms(ctx, shape, k, rounds, rate):
+    """One launch for all rounds: fewer rows than a slab, a slab and a row, more columns than
+    a chunk, sums by one block and by a block per column, p formed where it is gathered or
+    in a pass, rows past the long-row length, columns that leave the active range. The
+    matrices have condition numbers of at most 25, so rounding grows by little over
+    a few rounds: 1e-11 is four orders above it and far below any wrong term."""
+    if shape == "graph":
+        A, _ = P.powerlaw_graph(n=9000, seed=12, shift=100.0)
+        assert int(np.sum(np.diff(A.rowptr) > 64)) > 20
+    else:
+        A, _ = P.laplace2d(*shape)
+        A = P.CSR.from_scipy(A.to_scipy() + 4.0 * __import__("scipy.sparse").sparse.identity(A.n))
+    rng = np.random.default_rng(k)
+    R0 = rng.standard_normal((A.n, k)) * np.logspace(0, -3, k)
+    R0[:, ::3] = A.to_scipy() @ rng.standard_normal((A.n, (k + 2) // 3))
+    W0 = 0.1 * rng.standard_normal((A.n, k))
+    dA = ctx.matrix(A)
+    out = []
+    for _ in range(2):
+        r, w = ctx.multivec(A.n, k + 1), ctx.multivec(A.n, k + 3)
+        r.upload(R0, 1)
+        w.upload(W0, 3)
+        G.bcg(dA, r, 1, w, 3, k, cg_max_it=rounds + 1, cg_rate=rate, precision=0)
+        out.append((w.download(3, k), r.download(1, k)))
+    x, res = _block_cg(A.to_scipy(), R0, W0, rounds, rate)
+    assert rel(out[0][0], x) < 1e-11
+    assert np.linalg.norm(out[0][1] - res) < 1e-11 * np.linalg.norm(R0)
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
