@@ -12,6 +12,7 @@
 //   dL / d A_ij = -mu_i x_j,   dL / d B_ij = lambda mu_i x_j - (g^T x / 2) x_i x_j.
 // Both are sums of products U[i, t] V[j, t] over the sparsity pattern (an SDDMM),
 // which GCGE_GPU_PatternGrad evaluates; GCGE_GPU_EigvecAdjoint computes mu.
+#include "gb_coop.h"
 #include "gb_internal.h"
 
 #include <cuda_runtime.h>
@@ -248,7 +249,7 @@ struct ad_work {
     double *BX;        // B X (n x m, ld m) or NULL when B = I
     double *y, *r, *p, *q, *t, *u, *w;
     double *c;         // m coefficients
-    double *dot;       // one scalar
+    double *dot;       // one scalar, or the iteration's state
     double *part;      // block partials (grid x max(m, 1))
     double *h_c;       // host copy of m coefficients
 };
@@ -329,6 +330,344 @@ static int ad_apply(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, const gcge_gpu_mat
     return ad_project(ctx, n, m, X, ldx, BX, ldbx, W->u, W->u, q, W);
 }
 
+// ---------------------------------------------------------------- the CG iteration in one launch
+// An iteration is a projection (X^T p, p - X c), a product, a second projection, a dot
+// product, the updates and another dot. As launches that was fifteen kernels and two
+// host synchronisations, 167 us on 16,384 unknowns with ten vectors, of which the
+// arithmetic needs five. Here the phases are those of one cooperative grid and the
+// sums are formed in its barriers (five an iteration, six with B): 28 us. A block owns
+// tiles of 128 rows, a thread a row; for X^T v the lanes of a warp take columns
+// instead (32 / lanes-for-m rows at once), as one FP64 instruction costs a warp the
+// same 16 clocks for one lane as for 32.
+#define AC_ROWS 128
+#define AC_WARPS (AC_ROWS / 32)
+
+// scalars of the iteration, written by the block that ends a barrier
+struct ac_state {
+    double rr, alpha, beta, bnorm;
+    int it, status;
+};
+struct ac_args {
+    int n, m, max_it, warp_rows;             // warp_rows: products by a warp per row (long rows)
+    double lambda, tol;
+    const int *arp, *aci, *brp, *bci;
+    const double *av, *bv;                   // bv: NULL when B = I
+    const double *X, *BX;
+    long ldx, ldbx;
+    double *y, *r, *p, *q, *t, *u;
+    double *c, *part;                        // m sums; [m][grid] partials
+    ac_state *s;
+    unsigned *bar;
+    int *dev_err;
+};
+enum { AC_PLAIN, AC_COEF, AC_PQ, AC_RR };
+
+// grid barrier with ns column sums (fixed order) and what the op derives from them;
+// the message is 1 to go on, 0 to stop; -1: a wait ran out
+__device__ int ac_barrier(const ac_args &a, int op, int ns, unsigned &gen)
+{
+    __shared__ int last, res;
+    __shared__ double sum0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, G = gridDim.x;
+    __syncthreads();
+    if (threadIdx.x == 0) last = coop_arrive(a.bar) == (unsigned)G - 1;
+    __syncthreads();
+    if (last) {
+        for (int j = warp; j < ns; j += AC_WARPS) {
+            double s = 0;
+            for (int b = lane; b < G; b += 32) s += __ldcg(a.part + (size_t)j * G + b);
+#pragma unroll
+            for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane == 0) {
+                if (op == AC_COEF) a.c[j] = s;
+                else sum0 = s;
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            ac_state *s = a.s;
+            int go = 1;
+            if (op == AC_PQ || op == AC_RR) {
+                const double v = sum0, rr = __ldcg(&s->rr);
+                if (!isfinite(v)) {
+                    s->status = GCGE_GPU_ERR_NONFINITE;
+                    go = 0;
+                } else if (op == AC_PQ) {
+                    if (v > 0) s->alpha = rr / v;
+                    else go = 0;                         // left the SPD complement: stop
+                } else {
+                    const int it = __ldcg(&s->it) + 1;
+                    s->beta = v / rr;
+                    s->rr = v;
+                    s->it = it;
+                    go = sqrt(v) > a.tol * __ldcg(&s->bnorm) && it < a.max_it;
+                }
+            }
+            *(volatile unsigned *)a.bar = 0;
+            ++gen;
+            res = go;
+            coop_release(a.bar + 2, gen, (unsigned)go);
+        }
+    } else if (threadIdx.x == 0) {
+        const unsigned long long t0 = coop_now();
+        int spin = 0;
+        unsigned long long v;
+        while ((unsigned)((v = coop_ld64(a.bar + 2)) >> 32) == gen)
+            if ((++spin & 1023) == 0 && coop_now() - t0 > COOP_WAIT_NS) {
+                atomicExch(a.dev_err, 1);
+                v = 0xffffffffull;
+                break;
+            }
+        ++gen;
+        res = (int)(unsigned)v;
+    }
+    __syncthreads();
+    return res;
+}
+
+// row r of M v (one thread)
+__device__ __forceinline__ double ac_row(const int *rp, const int *ci, const double *val, const double *v, long r)
+{
+    double s = 0;
+    const int end = __ldg(rp + r + 1);
+#pragma unroll 4
+    for (int e = __ldg(rp + r); e < end; ++e) s = fma(__ldg(val + e), v[__ldg(ci + e)], s);
+    return s;
+}
+// row r of M v by a warp
+__device__ __forceinline__ double ac_row_warp(const int *rp, const int *ci, const double *val, const double *v, long r)
+{
+    double s = 0;
+    const int end = __ldg(rp + r + 1);
+    for (int e = __ldg(rp + r) + (threadIdx.x & 31); e < end; e += 32) s = fma(__ldg(val + e), v[__ldg(ci + e)], s);
+#pragma unroll
+    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+// M v for the tile's rows: this thread's row r0 + threadIdx.x (tile: scratch)
+__device__ __forceinline__ double ac_product(const ac_args &a, const int *rp, const int *ci, const double *val,
+                                             const double *v, long r0, double *tile)
+{
+    const long r = r0 + threadIdx.x;
+    if (!a.warp_rows) return r < a.n ? ac_row(rp, ci, val, v, r) : 0.0;
+    __syncthreads();
+    for (int i = threadIdx.x >> 5; i < AC_ROWS; i += AC_WARPS) {
+        const double s = r0 + i < a.n ? ac_row_warp(rp, ci, val, v, r0 + i) : 0.0;
+        if ((threadIdx.x & 31) == 0) tile[i] = s;
+    }
+    __syncthreads();
+    return tile[threadIdx.x];
+}
+
+// the tile's part of X^T v, v = this thread's value of row r0 + threadIdx.x: lane
+// (sub, c) adds rows sub, sub + 32 / W, ... of the warp's 32 for columns c and c + 32
+__device__ __forceinline__ void ac_xtv(const ac_args &a, double v, long r0, double *tile, int W, double acc[2])
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = lane & (W - 1), sub = lane / W;
+    __syncwarp();
+    tile[threadIdx.x] = v;
+    __syncwarp();
+    const long rw = r0 + warp * 32;
+    const double *vt = tile + warp * 32;
+    const int step = 32 / W;
+#pragma unroll 4
+    for (int i = sub; i < 32; i += step) {
+        const bool in = rw + i < a.n;
+        const double *xr = a.X + (rw + i) * a.ldx;
+        const double x0 = in && c < a.m ? xr[c] : 0.0;
+        acc[0] = fma(x0, vt[i], acc[0]);
+        if (a.m > 32) {
+            const double x1 = in && c + 32 < a.m ? xr[c + 32] : 0.0;
+            acc[1] = fma(x1, vt[i], acc[1]);
+        }
+    }
+}
+
+// the block's partials of X^T v from the lanes' sums
+__device__ __forceinline__ void ac_xtv_part(const ac_args &a, double acc[2], int W, double (*red)[64])
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+        for (int o = W; o < 32; o <<= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+    red[warp][lane] = acc[0];
+    red[warp][lane + 32] = acc[1];
+    __syncthreads();
+    for (int j = threadIdx.x; j < a.m; j += AC_ROWS) {
+        double t = 0;
+#pragma unroll
+        for (int w = 0; w < AC_WARPS; ++w) t += red[w][j];
+        a.part[(size_t)j * gridDim.x + blockIdx.x] = t;
+    }
+    __syncthreads();
+}
+
+__device__ __forceinline__ void ac_dot_part(const ac_args &a, double s, double (*red)[64])
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) red[warp][0] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0;
+        for (int w = 0; w < AC_WARPS; ++w) t += red[w][0];
+        a.part[blockIdx.x] = t;
+    }
+    __syncthreads();
+}
+
+// v - sum_j M[r, j] c_j
+__device__ __forceinline__ double ac_minus(const ac_args &a, const double *M, long ldm, long r, double v, const double *cs)
+{
+    const double *mr = M + r * ldm;
+    double s = 0;
+#pragma unroll 4
+    for (int j = 0; j < a.m; ++j) s = fma(mr[j], cs[j], s);
+    return v - s;
+}
+
+// CG on P^T (A - lambda B) P y = b, P = I - X X^T B, from y = 0 with r = p = b
+__global__ void __launch_bounds__(AC_ROWS, 4)
+k_adjoint_cg(const ac_args a)
+{
+    __shared__ double red[AC_WARPS][64], tile[AC_ROWS], cs[64];
+    const int n = a.n, m = a.m;
+    const long stride = (long)gridDim.x * AC_ROWS, first = (long)blockIdx.x * AC_ROWS;
+    if (*(volatile int *)a.dev_err) return;              // an earlier wait ran out: do nothing
+    unsigned gen = threadIdx.x == 0 ? (unsigned)(coop_ld64(a.bar + 2) >> 32) : 0;
+    int W = 1;
+    while (W < m && W < 32) W <<= 1;
+    double beta = 0;
+    for (bool start = true;; start = false) {
+        // p = r + beta p; c = X^T B p
+        double acc[2] = {0, 0};
+        for (long r0 = first; r0 < n; r0 += stride) {
+            const long r = r0 + threadIdx.x;
+            double p = 0;
+            if (r < n) {
+                p = a.p[r];
+                if (!start) a.p[r] = p = fma(beta, p, a.r[r]);
+            }
+            if (!a.bv) ac_xtv(a, p, r0, tile, W, acc);
+        }
+        if (a.bv) {
+            if (ac_barrier(a, AC_PLAIN, 0, gen) < 0) return;
+            for (long r0 = first; r0 < n; r0 += stride)
+                ac_xtv(a, ac_product(a, a.brp, a.bci, a.bv, a.p, r0, tile), r0, tile, W, acc);
+        }
+        ac_xtv_part(a, acc, W, red);
+        if (ac_barrier(a, AC_COEF, m, gen) < 0) return;
+        // t = P p
+        for (int j = threadIdx.x; j < m; j += AC_ROWS) cs[j] = __ldcg(a.c + j);
+        __syncthreads();
+        for (long r0 = first; r0 < n; r0 += stride) {
+            const long r = r0 + threadIdx.x;
+            if (r < n) a.t[r] = ac_minus(a, a.X, a.ldx, r, a.p[r], cs);
+        }
+        if (ac_barrier(a, AC_PLAIN, 0, gen) < 0) return;
+        // u = (A - lambda B) t; c = X^T u
+        acc[0] = acc[1] = 0;
+        for (long r0 = first; r0 < n; r0 += stride) {
+            const long r = r0 + threadIdx.x;
+            double u = ac_product(a, a.arp, a.aci, a.av, a.t, r0, tile);
+            const double bt = a.bv ? ac_product(a, a.brp, a.bci, a.bv, a.t, r0, tile) : r < n ? a.t[r] : 0.0;
+            u = fma(-a.lambda, bt, u);
+            if (r < n) a.u[r] = u;
+            else u = 0;
+            ac_xtv(a, u, r0, tile, W, acc);
+        }
+        ac_xtv_part(a, acc, W, red);
+        if (ac_barrier(a, AC_COEF, m, gen) < 0) return;
+        // q = P^T u; p.q
+        for (int j = threadIdx.x; j < m; j += AC_ROWS) cs[j] = __ldcg(a.c + j);
+        __syncthreads();
+        double s = 0;
+        for (long r0 = first; r0 < n; r0 += stride) {
+            const long r = r0 + threadIdx.x;
+            if (r < n) {
+                const double q = ac_minus(a, a.BX, a.ldbx, r, a.u[r], cs);
+                a.q[r] = q;
+                s = fma(a.p[r], q, s);
+            }
+        }
+        ac_dot_part(a, s, red);
+        if (ac_barrier(a, AC_PQ, 1, gen) <= 0) return;
+        // y += alpha p, r -= alpha q; r.r
+        const double alpha = __ldcg(&a.s->alpha);
+        s = 0;
+        for (long r0 = first; r0 < n; r0 += stride) {
+            const long r = r0 + threadIdx.x;
+            if (r < n) {
+                a.y[r] = fma(alpha, a.p[r], a.y[r]);
+                const double rn = fma(-alpha, a.q[r], a.r[r]);
+                a.r[r] = rn;
+                s = fma(rn, rn, s);
+            }
+        }
+        ac_dot_part(a, s, red);
+        if (ac_barrier(a, AC_RR, 1, gen) <= 0) return;
+        beta = __ldcg(&a.s->beta);
+    }
+}
+
+// the iteration from the right-hand side in W->r and W->p, y = 0, r.r = rr
+static int ad_iterate(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, const gcge_gpu_mat *B, int n, int m, const double *X,
+                      long ldx, const double *BX, long ldbx, double lambda, double rr, double tol, int max_it,
+                      int *iters, ad_work *W)
+{
+    ac_state s = {rr, 0.0, 0.0, sqrt(rr), 0, GCGE_GPU_OK};
+    AD_CUDA(ctx, cudaMemcpyAsync(W->dot, &s, sizeof(s), cudaMemcpyHostToDevice, ctx->stream));
+    ac_args a = {};
+    a.n = n;
+    a.m = m;
+    a.max_it = max_it;
+    // a thread per row leaves a warp waiting for its longest one
+    a.warp_rows = A->max_row_nnz > 64.0 || (B && B->max_row_nnz > 64.0);
+    a.lambda = lambda;
+    a.tol = tol;
+    a.arp = A->rp;
+    a.aci = A->ci;
+    a.av = A->v;
+    if (B) {
+        a.brp = B->rp;
+        a.bci = B->ci;
+        a.bv = B->v;
+    }
+    a.X = X;
+    a.ldx = ldx;
+    a.BX = BX;
+    a.ldbx = ldbx;
+    a.y = W->y;
+    a.r = W->r;
+    a.p = W->p;
+    a.q = W->q;
+    a.t = W->t;
+    a.u = W->u;
+    a.c = W->c;
+    a.part = W->part;
+    a.s = (ac_state *)W->dot;
+    a.bar = ctx->dev_bar;
+    a.dev_err = ctx->dev_err;
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_adjoint_cg, AC_ROWS, 0) != cudaSuccess || per_sm < 1)
+        return gb_fail(ctx, GCGE_GPU_ERR_CUDA);
+    if (per_sm > AV_BLOCKS_PER_SM) per_sm = AV_BLOCKS_PER_SM;   // the partials' room
+    long G = (long)ctx->num_sms * per_sm, tiles = ((long)n + AC_ROWS - 1) / AC_ROWS;
+    if (G > tiles) G = tiles;
+    void *args[] = {&a};
+    if (cudaLaunchCooperativeKernel(k_adjoint_cg, dim3((unsigned)G), dim3(AC_ROWS), args, 0, ctx->stream) != cudaSuccess) {
+        cudaGetLastError();
+        return gb_fail(ctx, GCGE_GPU_ERR_CUDA);
+    }
+    ctx->launches++;
+    AD_CUDA(ctx, cudaMemcpyAsync(&s, W->dot, sizeof(s), cudaMemcpyDeviceToHost, ctx->stream));
+    AD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    *iters = s.it;
+    if (s.status) return gb_fail(ctx, s.status);
+    return gb_check_device_error(ctx);
+}
+
 static int ad_solve(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, const gcge_gpu_mat *B, int n, int m, const double *X,
                     long ldx, const double *eval, int k, const double *g, long ldg, double *mu, long ldmu,
                     double cluster_tol, double tol, int max_it, int *iters, ad_work *W)
@@ -363,7 +702,10 @@ static int ad_solve(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, const gcge_gpu_mat
     if (!st) st = ad_axpby(ctx, n, 1.0, W->r, 0.0, W->p);
     if (!st) st = ad_dot(ctx, n, W->r, W->r, W, &rr);
     bnorm = sqrt(rr);
-    while (!st && bnorm > 0 && sqrt(rr) > tol * bnorm && it < max_it) {
+    if (!st && m <= AD_SKINNY_M && bnorm > 0 && bnorm > tol * bnorm && max_it > 0)
+        st = ad_iterate(ctx, A, B, n, m, X, ldx, BX, ldbx, lambda, rr, tol, max_it, &it, W);
+    // more vectors than the single launch takes
+    while (!st && m > AD_SKINNY_M && bnorm > 0 && sqrt(rr) > tol * bnorm && it < max_it) {
         double pq;
         if ((st = ad_apply(ctx, A, B, n, m, X, ldx, lambda, W->p, W->q, W))) break;
         if ((st = ad_dot(ctx, n, W->p, W->q, W, &pq))) break;
@@ -418,7 +760,7 @@ extern "C" int GCGE_GPU_EigvecAdjoint(const gcge_gpu_mat *A, const gcge_gpu_mat 
     const size_t vn = ((size_t)n + 31) & ~(size_t)31, vm = ((size_t)m + 31) & ~(size_t)31;
     const size_t np = (((size_t)ctx->num_sms * AV_BLOCKS_PER_SM * (size_t)(m > 1 ? m : 1)) + 31) & ~(size_t)31;
     const size_t nv = 7 * vn + vm + 32 + np + (B ? (((size_t)n * m + 31) & ~(size_t)31) : 0);
-    if (cudaMalloc(&base, sizeof(double) * nv) != cudaSuccess) return gb_fail(ctx, GCGE_GPU_ERR_NOMEM);
+    if (gb_dev_alloc(ctx, (void **)&base, sizeof(double) * nv)) return gb_fail(ctx, GCGE_GPU_ERR_NOMEM);
     W.y = base;
     W.r = W.y + vn;
     W.p = W.r + vn;
@@ -432,7 +774,7 @@ extern "C" int GCGE_GPU_EigvecAdjoint(const gcge_gpu_mat *A, const gcge_gpu_mat 
     W.BX = B ? W.part + np : nullptr;
     W.h_c = (double *)malloc(sizeof(double) * m);
     if (!W.h_c) {
-        cudaFree(base);
+        gb_dev_free(ctx, base);
         return gb_fail(ctx, GCGE_GPU_ERR_NOMEM);
     }
     // the projections are n x m by one column: FP64-pipe Gram and combination
@@ -443,7 +785,7 @@ extern "C" int GCGE_GPU_EigvecAdjoint(const gcge_gpu_mat *A, const gcge_gpu_mat 
                   tol, max_it, iters, &W);
     ctx->tc = tc;
     cudaStreamSynchronize(ctx->stream);
-    cudaFree(base);
+    gb_dev_free(ctx, base);
     free(W.h_c);
     return st;
 }

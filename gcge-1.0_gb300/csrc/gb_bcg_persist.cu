@@ -22,19 +22,19 @@
 // chunk), the shape with the fewest idle slots: the FP64 pipe issues for idle lanes
 // too. Only p crosses a barrier; x and r of an entry belong to one thread.
 //
-// Every wait is bounded (PB_WAIT_NS); a block whose wait runs out sets the
+// Every wait is bounded (COOP_WAIT_NS); a block whose wait runs out sets the
 // context's device error word and leaves, and so do the others in turn.
 #include <cstdint>
 #include <cuda_runtime.h>
 
-#include "gb_internal.h"
 #include "gb_bcg.h"
+#include "gb_coop.h"
+#include "gb_internal.h"
 
 #define PB_THREADS 256
 #define PB_WARPS (PB_THREADS / 32)
 #define PB_SLAB 128
 #define PB_FUSED_K 1024                                   // widest block of the fused form
-#define PB_WAIT_NS 20000000000ull
 // partials (slabs x columns) up to which the block that arrives last sums them all;
 // beyond, one block per column does (a trip more, but side by side)
 #define PB_ONE_BLOCK_SUMS 1024
@@ -59,13 +59,6 @@ struct pb_args {
     unsigned *bar;             // [0] arrivals, [1] columns' owners done, [2..3] generation and active columns
     int *dev_err;
 };
-
-__device__ __forceinline__ unsigned long long pb_now()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    return t;
-}
 
 // sqrt(|s|) / err >= rate (src/gcge_cg.c:286-294); far from the line, where rounding
 // cannot matter, without the square root and the division (0.7 us of the barrier)
@@ -135,25 +128,6 @@ __device__ __forceinline__ void pb_column(const pb_args &a, int op, int c, doubl
     }
 }
 
-__device__ __forceinline__ unsigned pb_arrive(unsigned *w)
-{
-    unsigned t;
-    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(t) : "l"(w) : "memory");
-    return t;
-}
-__device__ __forceinline__ unsigned long long pb_ld64(const unsigned *w)
-{
-    unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(w) : "memory");
-    return v;
-}
-__device__ __forceinline__ unsigned pb_ld32(const unsigned *w)
-{
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(w) : "memory");
-    return v;
-}
-
 // Grid barrier that forms the column sums of `ka` columns and what follows from them.
 // gen: the generation so far, in thread 0. Returns the active columns, -1 when a wait
 // ran out. The generation and the count travel in one 64-bit word, so that nobody
@@ -166,7 +140,7 @@ __device__ int pb_barrier(const pb_args &a, int op, int ka, double *sh, unsigned
     const unsigned owners = min((unsigned)ka, G);
     __syncthreads();
     if (threadIdx.x == 0) {
-        last = pb_arrive(a.bar) == G - 1;
+        last = coop_arrive(a.bar) == G - 1;
         res = 0;
     }
     __syncthreads();
@@ -190,10 +164,10 @@ __device__ int pb_barrier(const pb_args &a, int op, int ka, double *sh, unsigned
         }
     } else if (!one && blockIdx.x < owners) {
         if (threadIdx.x == 0) {
-            const unsigned long long t0 = pb_now();
+            const unsigned long long t0 = coop_now();
             int spin = 0;
-            while (pb_ld32(a.bar) != G)
-                if ((++spin & 1023) == 0 && pb_now() - t0 > PB_WAIT_NS) {
+            while (coop_ld32(a.bar) != G)
+                if ((++spin & 1023) == 0 && coop_now() - t0 > COOP_WAIT_NS) {
                     atomicExch(a.dev_err, 1);
                     res = -1;
                     break;
@@ -207,7 +181,7 @@ __device__ int pb_barrier(const pb_args &a, int op, int ka, double *sh, unsigned
             if (threadIdx.x == 0) pb_column(a, op, c, s, r1);
         }
         __syncthreads();
-        if (threadIdx.x == 0) last = pb_arrive(a.bar + 1) == owners - 1;
+        if (threadIdx.x == 0) last = coop_arrive(a.bar + 1) == owners - 1;
         __syncthreads();
         release = last;
         if (release && op == PB_BETA)
@@ -222,16 +196,14 @@ __device__ int pb_barrier(const pb_args &a, int op, int ka, double *sh, unsigned
             *(volatile unsigned *)(a.bar + 1) = 0;
             ++gen;
             res = cnt;
-            asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(a.bar + 2),
-                         "l"((unsigned long long)gen << 32 | (unsigned)cnt)
-                         : "memory");
+            coop_release(a.bar + 2, gen, (unsigned)cnt);
         }
     } else if (threadIdx.x == 0) {
-        const unsigned long long t0 = pb_now();
+        const unsigned long long t0 = coop_now();
         int spin = 0;
         unsigned long long v;
-        while ((unsigned)((v = pb_ld64(a.bar + 2)) >> 32) == gen)
-            if ((++spin & 1023) == 0 && pb_now() - t0 > PB_WAIT_NS) {
+        while ((unsigned)((v = coop_ld64(a.bar + 2)) >> 32) == gen)
+            if ((++spin & 1023) == 0 && coop_now() - t0 > COOP_WAIT_NS) {
                 atomicExch(a.dev_err, 1);
                 v = 0xffffffffull;
                 break;
@@ -331,7 +303,7 @@ k_bcg_persist(const pb_args a)
     const unsigned gmask = (L == 32) ? 0xffffffffu : (((1u << L) - 1u) << ((lane / L) * L));
     const int n = a.n, k = a.k;
     if (*(volatile int *)a.dev_err) return;              // an earlier wait ran out: do nothing
-    unsigned gen = threadIdx.x == 0 ? (unsigned)(pb_ld64(a.bar + 2) >> 32) : 0;
+    unsigned gen = threadIdx.x == 0 ? (unsigned)(coop_ld64(a.bar + 2) >> 32) : 0;
 
     // norms of the initial residual
     {

@@ -42,6 +42,32 @@ def test_pattern_grad_matches_numpy(ctx, r):
     assert rel(g2, ref + 1.0) < 1e-14
 
 
+@pytest.mark.parametrize("m,what", [(1, "grid"), (17, "grid"), (33, "B"), (64, "grid"), (65, "B"), (12, "graph")])
+def test_eigvec_adjoint_forms(ctx, m, what):
+    """Widths at the lanes' and the launch's limits, with and without B, and rows that take
+    a warp each: mu satisfies its equation and its constraint to the solve's tolerance."""
+    if what == "graph":
+        A, _ = P.powerlaw_graph(700, seed=9, dmax=300)
+        assert np.max(np.diff(A.rowptr)) > 64
+        B = None
+    else:
+        A, _ = P.varcoef2d(nc=15, seed=5, sigma=0.5)
+        B = AD.diag_csr(np.random.default_rng(6).uniform(1.0, 2.0, A.n)) if what == "B" else None
+    w, X = AD.eig_dense(A, B)
+    g = np.random.default_rng(m).standard_normal(A.n)
+    dA, dB = ctx.matrix(A), (ctx.matrix(B) if B is not None else None)
+    Gd, MU = ctx.multivec(A.n, 1, g), ctx.multivec(A.n, 1)
+    it = G.eigvec_adjoint(dA, dB, ctx.multivec(A.n, m, X[:, :m]), m, w[:m], 0, Gd, 0, MU, 0, tol=1e-12)
+    assert it > 0
+    mu = MU.download()[:, 0]
+    Bs = B.to_scipy() if B is not None else None
+    b = lambda v: v if Bs is None else Bs @ v  # noqa: E731
+    x = X[:, 0]
+    res = A.to_scipy() @ mu - w[0] * b(mu) - (g - b(x) * (x @ g))
+    assert np.linalg.norm(res) <= 1e-9 * np.linalg.norm(g)
+    assert abs(x @ b(mu)) <= 1e-10 * np.linalg.norm(mu)
+
+
 @pytest.mark.parametrize("generalized,k", [(False, 0), (True, 0), (True, 3)])
 def test_eigvec_adjoint_matches_dense(ctx, generalized, k):
     """mu of the GPU solve (explicit components along the m computed eigenvectors,
