@@ -35,70 +35,79 @@
     } while (0)
 
 #define PG_THREADS 256
-#define PG_LANE_MAX_R 8                 // r up to this: one lane per stored entry
+#define PG_ROWS 64                      // most rows of a block
+#define PG_CHUNK 2048                   // entries whose rows are listed at a time
+#define PG_SMEM (44 * 1024)             // scaled U rows of a block (48 KB with the lists)
+#define PG_MAX_R 768
 
 // grad[e] = (acc ? grad[e] : 0) + sum_t s[t] U[i, t] V[j, t], e = (i, j) stored.
-// One warp per row. Lane per stored entry (r <= PG_LANE_MAX_R): the row's scaled
-// U values sit in registers and each lane gathers its V row. Otherwise the warp
-// walks the row's entries and splits t over the lanes (scaled U row in shared
-// memory), reducing with a fixed shuffle tree: the result does not depend on
-// scheduling.
-template <bool LANE_PER_ENTRY>
+// A block owns a run of rows: their scaled U values in shared memory, and the row of
+// every entry of the run beside them, so that the entries -- not the rows -- are dealt
+// to the lanes, LPE consecutive lanes each, and every lane works whatever the
+// row lengths (an FP64 instruction costs a warp 16 clocks for one lane as for 32: a warp
+// per row with lanes over t and a shuffle tree per entry spent five adds of all lanes
+// on each, 502 us for the 5-point 512^2 pattern with r = 20; here 71 us). LPE: two
+// lanes read 16 consecutive bytes of a V row, four (r >= 32) a whole sector.
+// Sums in a fixed order: the result does not depend on scheduling.
+template <int LPE>
 __global__ void __launch_bounds__(PG_THREADS)
 k_pattern_grad(int n, const int *__restrict__ rp, const int *__restrict__ ci, const double *__restrict__ U,
                long ldu, const double *__restrict__ V, long ldv, int r, const double *__restrict__ s, int acc,
-               double *__restrict__ grad)
+               double *__restrict__ grad, int rows)
 {
-    extern __shared__ double us_all[];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const long nw = ((long)gridDim.x * PG_THREADS) >> 5;
-    for (long i = ((long)blockIdx.x * PG_THREADS + threadIdx.x) >> 5; i < n; i += nw) {
-        const int beg = rp[i], end = rp[i + 1];
-        if (LANE_PER_ENTRY) {
-            double us[PG_LANE_MAX_R];
+    extern __shared__ double us[];      // [rows][r | 1]
+    __shared__ unsigned char row_of[PG_CHUNK];
+    __shared__ int first[PG_ROWS + 1];
+    const int ldus = r | 1;             // odd: the lanes' rows fall in different banks
+    const long i0 = (long)blockIdx.x * rows;
+    const int nr = (int)min((long)rows, n - i0);
+    for (int t = threadIdx.x; t < nr * r; t += PG_THREADS) {
+        const int i = t / r, q = t - i * r;
+        us[i * ldus + q] = s[q] * U[(i0 + i) * ldu + q];
+    }
+    for (int i = threadIdx.x; i <= nr; i += PG_THREADS) first[i] = rp[i0 + i];
+    __syncthreads();
+    const int e0 = first[0], e1 = first[nr], sub = threadIdx.x % LPE;
+    for (int base = e0; base < e1; base += PG_CHUNK) {
+        const int cnt = min(PG_CHUNK, e1 - base);
+        // four threads list a row's entries
+        for (int i = threadIdx.x >> 2; i < nr; i += PG_THREADS / 4)
+            for (int e = max(first[i], base) + (threadIdx.x & 3); e < min(first[i + 1], base + cnt); e += 4)
+                row_of[e - base] = (unsigned char)i;
+        __syncthreads();
+        for (int k = threadIdx.x / LPE; k < cnt; k += PG_THREADS / LPE) {
+            const double *vr = V + (long)__ldg(ci + base + k) * ldv;
+            const double *ur = us + row_of[k] * ldus;
+            double sum = 0.0;
+#pragma unroll 4
+            for (int t = sub; t < r; t += LPE) sum = fma(ur[t], __ldg(vr + t), sum);
 #pragma unroll
-            for (int t = 0; t < PG_LANE_MAX_R; ++t) us[t] = t < r ? s[t] * U[i * ldu + t] : 0.0;
-            for (int e = beg + lane; e < end; e += 32) {
-                const double *vr = V + (long)ci[e] * ldv;
-                double sum = 0.0;
-#pragma unroll
-                for (int t = 0; t < PG_LANE_MAX_R; ++t)
-                    if (t < r) sum = fma(us[t], vr[t], sum);
-                grad[e] = acc ? grad[e] + sum : sum;
-            }
-        } else {
-            double *us = us_all + (size_t)w * r;
-            for (int t = lane; t < r; t += 32) us[t] = s[t] * U[i * ldu + t];
-            __syncwarp();
-            for (int e = beg; e < end; ++e) {
-                const double *vr = V + (long)ci[e] * ldv;
-                double sum = 0.0;
-                for (int t = lane; t < r; t += 32) sum = fma(us[t], vr[t], sum);
-#pragma unroll
-                for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-                if (lane == 0) grad[e] = acc ? grad[e] + sum : sum;
-            }
-            __syncwarp();
+            for (int o = 1; o < LPE; o <<= 1) sum += __shfl_xor_sync(__activemask(), sum, o, LPE);
+            if (sub == 0) grad[base + k] = acc ? grad[base + k] + sum : sum;
         }
+        __syncthreads();
     }
 }
 
 static int pg_launch(gcge_gpu_ctx *ctx, const gcge_gpu_mat *M, const double *U, long ldu, const double *V, long ldv,
                      int r, const double *s_dev, int acc, double *grad_dev)
 {
-    long blocks = ((long)M->n * 32 + PG_THREADS - 1) / PG_THREADS;
-    const long cap = (long)ctx->num_sms * 8;
-    if (blocks > cap) blocks = cap;
-    if (blocks < 1) blocks = 1;
-    if (r <= PG_LANE_MAX_R) {
-        GB_LAUNCH(ctx, k_pattern_grad<true>, (int)blocks, PG_THREADS, 0, M->n, M->rp, M->ci, U, ldu, V, ldv, r,
-                  s_dev, acc, grad_dev);
-    } else {
-        const size_t smem = sizeof(double) * (size_t)(PG_THREADS / 32) * r;
-        if (smem > 48 * 1024) return gb_fail(ctx, GCGE_GPU_ERR_ARG);
-        GB_LAUNCH(ctx, k_pattern_grad<false>, (int)blocks, PG_THREADS, smem, M->n, M->rp, M->ci, U, ldu, V, ldv, r,
-                  s_dev, acc, grad_dev);
-    }
+    int rows = PG_SMEM / 8 / (r | 1);
+    if (rows > PG_ROWS) rows = PG_ROWS;
+    // few rows: a block for every SM
+    if ((long)rows * ctx->num_sms > M->n) rows = (M->n + ctx->num_sms - 1) / ctx->num_sms;
+    if (rows < 1) return gb_fail(ctx, GCGE_GPU_ERR_ARG);
+    const int blocks = (int)(((long)M->n + rows - 1) / rows);
+    const size_t smem = sizeof(double) * (size_t)rows * (r | 1);
+    if (r < 4)
+        GB_LAUNCH(ctx, k_pattern_grad<1>, blocks, PG_THREADS, smem, M->n, M->rp, M->ci, U, ldu, V, ldv, r, s_dev, acc,
+                  grad_dev, rows);
+    else if (r < 32)
+        GB_LAUNCH(ctx, k_pattern_grad<2>, blocks, PG_THREADS, smem, M->n, M->rp, M->ci, U, ldu, V, ldv, r, s_dev, acc,
+                  grad_dev, rows);
+    else
+        GB_LAUNCH(ctx, k_pattern_grad<4>, blocks, PG_THREADS, smem, M->n, M->rp, M->ci, U, ldu, V, ldv, r, s_dev, acc,
+                  grad_dev, rows);
     return GCGE_GPU_OK;
 }
 
@@ -113,13 +122,13 @@ extern "C" int GCGE_GPU_PatternGrad(const gcge_gpu_mat *M, const gcge_gpu_mv *U,
     if (!M || !U || !V || !scale || !grad) return GCGE_GPU_ERR_ARG;
     gcge_gpu_ctx *ctx = M->ctx;
     if (r < 1 || !mv_cols_ok(U, u0, r) || !mv_cols_ok(V, v0, r) || U->n != M->n || V->n != M->n ||
-        (size_t)(PG_THREADS / 32) * r * sizeof(double) > 48 * 1024)
+        r > PG_MAX_R)
         return gb_fail(ctx, GCGE_GPU_ERR_ARG);
     if (M->nnz == 0) return GCGE_GPU_OK;
     double *g_dev = nullptr, *s_dev = nullptr;
     int st = GCGE_GPU_OK;
-    if (cudaMalloc(&g_dev, sizeof(double) * (size_t)M->nnz) != cudaSuccess ||
-        cudaMalloc(&s_dev, sizeof(double) * (size_t)r) != cudaSuccess) {
+    if (gb_dev_alloc(ctx, (void **)&g_dev, sizeof(double) * (size_t)M->nnz) ||
+        gb_dev_alloc(ctx, (void **)&s_dev, sizeof(double) * (size_t)r)) {
         st = gb_fail(ctx, GCGE_GPU_ERR_NOMEM);
         goto done;
     }
@@ -137,8 +146,8 @@ extern "C" int GCGE_GPU_PatternGrad(const gcge_gpu_mat *M, const gcge_gpu_mv *U,
         st = gb_fail(ctx, GCGE_GPU_ERR_CUDA);
 done:
     cudaStreamSynchronize(ctx->stream);
-    cudaFree(g_dev);
-    cudaFree(s_dev);
+    gb_dev_free(ctx, g_dev);
+    gb_dev_free(ctx, s_dev);
     return st;
 }
 

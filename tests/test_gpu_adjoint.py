@@ -42,6 +42,30 @@ def test_pattern_grad_matches_numpy(ctx, r):
     assert rel(g2, ref + 1.0) < 1e-14
 
 
+@pytest.mark.parametrize("r", [3, 4, 31, 32, 768])
+def test_pattern_grad_row_runs(ctx, r):
+    """Rows of no entries, of one and of more than a block lists at a time, and widths at the
+    changes of lanes per entry: within r 2^-53 of the sum of the products' magnitudes
+    (their scale's rounding among them: 2 r + 2 roundings at most)."""
+    import scipy.sparse as sp
+    n = 2611
+    rng = np.random.default_rng(r)
+    M = sp.random(n, n, density=8e-4, random_state=1, format="lil")
+    M[7, :] = rng.uniform(0.5, 1.0, n)
+    M[100:180, :] = 0
+    M = sp.csr_matrix(M)
+    M.eliminate_zeros()
+    A = P.CSR.from_scipy(M)
+    assert A.rowptr[8] - A.rowptr[7] > 2048 and A.rowptr[180] == A.rowptr[100]
+    U, V = rng.standard_normal((n, r)), rng.standard_normal((n, r))
+    s = rng.standard_normal(r)
+    g = G.pattern_grad(ctx.matrix(A), ctx.multivec(n, r, U), 0, ctx.multivec(n, r, V), 0, r, s, A.nnz)
+    rows, cols = AD.pattern(A)
+    for b in range(0, A.nnz, 2000):
+        t = (U[rows[b:b + 2000]].astype(np.longdouble) * V[cols[b:b + 2000]]) * s
+        assert np.all(np.abs(g[b:b + 2000] - t.sum(1)) <= (r + 2) * 2.0 ** -52 * np.abs(t).sum(1))
+
+
 @pytest.mark.parametrize("m,what", [(1, "grid"), (17, "grid"), (33, "B"), (64, "grid"), (65, "B"), (12, "graph")])
 def test_eigvec_adjoint_forms(ctx, m, what):
     """Widths at the lanes' and the launch's limits, with and without B, and rows that take
