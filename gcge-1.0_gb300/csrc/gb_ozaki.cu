@@ -23,15 +23,17 @@
 //    planes in shared memory (two stages of K = 32, no-swizzle K-major core
 //    matrices), lane 0 of warp 15 issues the digit-pair MMAs of a stage
 //    (M = 128, N = 64, K = 16, accumulators: 8 levels x 64 TMEM columns), and
-//    all 16 warps drain TMEM (warp w: lanes 32 (w % 4) .. +31, 16 columns from
-//    16 (w / 4));
+//    all 16 warps drain TMEM (warp w: lanes 32 (w % 4) .. +31, columns 4 (w / 4)
+//    .. +3 of every 16, so that a narrow output is shared by all of them);
 //  * hand-offs through mbarriers: full[b] (stage b written, 480 arrivals),
 //    empty[b] (MMAs of stage b done, tcgen05.commit), drained (TMEM read out,
 //    512 arrivals), copied[b] (bulk copy of the pre-split planes of stage b);
 //    every wait is bounded and reports a timeout through the context's device
 //    error word;
-//  * the split warps load the next stage's FP64 values while the MMAs of the
-//    current one run.
+//  * the next stage's FP64 values are on their way while the MMAs of the current one
+//    run: registers in k_lincomb_tc; in k_gram_tc, whose sums fill the registers, a
+//    lane's own slot of shared memory (cp.async, one group per core matrix, refilled as
+//    soon as it has been read).
 // k_lincomb_tc: Y = alpha X C + beta Y, M = 128 rows of X, K = columns of X,
 //   per-row scales (of X equilibrated by the row scales of C), C split once per
 //   call by k_lc_coef_split;
@@ -88,11 +90,11 @@ extern "C" int gb_gram_reduce_launch(gcge_gpu_ctx *ctx, int k1, int k2, int nspl
 
 // shared header of both kernels
 struct tc_hdr {
-    uint64_t bar[7];             // full[2], empty[2], drained, copied[2] (bulk copies of a stage)
+    uint64_t bar[8];             // full[2], empty[2], drained, copied[2] (bulk copies of a stage), scales
     uint32_t tmem;
     int flag;                    // a bounded wait ran out in this CTA
 };
-static_assert(sizeof(tc_hdr) <= 64, "header overlaps the scale arrays");
+static_assert(sizeof(tc_hdr) <= 80, "header overlaps the scale arrays");
 
 __device__ __forceinline__ void tc_fail(tc_hdr *h, int *err)
 {
@@ -113,6 +115,7 @@ __device__ __forceinline__ void tc_setup(tc_hdr *h)
         tc_mbar_init(b + 32, TC_THREADS);
         tc_mbar_init(b + 40, 1);
         tc_mbar_init(b + 48, 1);
+        tc_mbar_init(b + 56, TC_SPLIT_THREADS);
         h->flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -295,7 +298,11 @@ __global__ void k_gram_init(int *__restrict__ exps, int cols, unsigned *__restri
 }
 
 // ---------------------------------------------------------------- Gram V^T W (tcgen05)
-#define GR_CORES_PER_WARP ((TC_ACORES + TC_BCORES + TC_SPLIT_WARPS - 1) / TC_SPLIT_WARPS)
+// core matrices a warp splits per stage: of V, and of W (dealt from the last warp down, so
+// that no warp has the odd one of both)
+#define GR_A ((TC_ACORES + TC_SPLIT_WARPS - 1) / TC_SPLIT_WARPS)
+#define GR_B ((TC_BCORES + TC_SPLIT_WARPS - 1) / TC_SPLIT_WARPS)
+#define GR_CORES_PER_WARP (GR_A + GR_B)
 // Levels 0-7 (34 digit pairs, 8 x 64 TMEM columns), as the linear combination:
 // the dropped pairs (level >= 8) add at most 2^-57.4 of the column-scale product
 // 2^(e+f) per row, so over n rows the error stays below 2^-57.4 n 2^(e+f) even
@@ -304,9 +311,11 @@ __global__ void k_gram_init(int *__restrict__ exps, int cols, unsigned *__restri
 // (2^-56) and carried into the level 0-2 sum (units 2^-16) after every chunk, so
 // neither int64 sum can overflow for the 2^20 rows a split may hold.
 #define GR_LEVELS 8
-#define GR_SMEM (2 * TC_STAGE + TC_HDR)
+#define GR_SMEM (2 * TC_STAGE + TC_HDR + 512 * (TC_ACORES + TC_BCORES))   // and a slot of 16 bytes a lane and core
 
-// grid (ceil(k1 / 128), ceil(k2 / 64), splits). A split's exact integer sum of the
+// grid (tiles of mt <= 128 columns of V, ceil(k2 / 64), splits): V's columns are dealt
+// evenly to the tiles, as the widest one sets the time (178 as 96 + 82: 0.83 of 128 +
+// 50). A split's exact integer sum of the
 // digit products of sum_r V[r, i] W[r, j] is (hi, lo), value
 // (hi 2^40 + lo) 2^(e_i + f_j - 66). The splits add theirs to sums[i + j k1] by
 // atomics -- integers, so the order does not show: |hi| < 2^28.2 a row, below 2^60
@@ -319,12 +328,12 @@ __global__ void k_gram_init(int *__restrict__ exps, int cols, unsigned *__restri
 __global__ void __launch_bounds__(TC_THREADS, 1)
 k_gram_tc(int n, int k1, int k2, const double *__restrict__ V, long ldv, const double *__restrict__ W, long ldw,
           const int *__restrict__ ev, const int *__restrict__ ew, unsigned long long *__restrict__ sums,
-          unsigned *__restrict__ ticket, double *__restrict__ a, int lda, long rows_per_split, int sym,
+          unsigned *__restrict__ ticket, double *__restrict__ a, int lda, long rows_per_split, int mt, int sym,
           int *__restrict__ err, int stall)
 {
     extern __shared__ __align__(1024) uint8_t tc_smem[];
     uint8_t *sm = tc_smem;
-    const int i0 = blockIdx.x * TC_M, j0 = blockIdx.y * TC_N;
+    const int i0 = blockIdx.x * mt, j0 = blockIdx.y * TC_N, iend = min(k1, i0 + mt);
     if (sym && i0 > j0 + TC_N - 1) return;
     if (*(volatile int *)err) return;                    // an earlier launch timed out: do nothing
     tc_hdr *h = (tc_hdr *)(sm + 2 * TC_STAGE);
@@ -334,6 +343,11 @@ k_gram_tc(int n, int k1, int k2, const double *__restrict__ V, long ldv, const d
     const int nst = (int)((re - rb + TC_KS - 1) / TC_KS);
     const int N = min(TC_N, (k2 - j0 + 15) & ~15);
     tc_setup(h);
+    int *sbs = (int *)(sm + 2 * TC_STAGE + 128);         // shift bases of the tile's columns of V, then of W
+    for (int c = tid; c < TC_M + TC_N; c += TC_THREADS) {
+        const int col = c < TC_M ? i0 + c : j0 + c - TC_M;
+        sbs[c] = col < (c < TC_M ? iend : k2) ? (c < TC_M ? ev : ew)[col] + OZ_SHIFT0 : OZ_SHIFT_NONE;
+    }
     // digit planes of both buffers start at zero: core matrices wholly outside the
     // columns of V or W (the padding of a short tile) are never split and keep
     // zero digits; the split threads' first proxy fence covers these writes
@@ -345,35 +359,51 @@ k_gram_tc(int n, int k1, int k2, const double *__restrict__ V, long ldv, const d
     tc_fence_after_sync();
     const uint32_t tmem = h->tmem, sbase = tc_smem_addr(sm);
     const bool mma_warp = warp == TC_SPLIT_WARPS;
-    const int quarter = warp & 3, col0 = (warp >> 2) * TC_COLS_PER_WARP;
+    const int quarter = warp & 3, col0 = (warp >> 2) * 4;    // drained: columns col0 .. +3 of every 16
     const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16) + col0;
     int commits[3] = {0, 0, 0};                          // empty[0], empty[1], drained chunks
     long long hi[TC_COLS_PER_WARP], lo[TC_COLS_PER_WARP];
 #pragma unroll
     for (int q = 0; q < TC_COLS_PER_WARP; ++q) hi[q] = lo[q] = 0;
 
-    // split-warp geometry: core q = warp + 15 cc; A cores (V) first, then B cores (W);
-    // lane (i8, rp): column 8g + i8, rows 8c + 2 rp and 8c + 2 rp + 1
-    const int i8 = lane & 7, rp = lane >> 3;
-    double xv[GR_CORES_PER_WARP][2];
-    auto load_stage = [&](int s) {
-        const long r = rb + (long)s * TC_KS + 2 * rp;
+    // split-warp geometry: A cores (V) warp + 15 cc, B cores (W) 14 - warp + 15 cc, those that
+    // hold columns; lane (i8, rp): column 8g + i8, rows 8c + 2 rp and 8c + 2 rp + 1.
+    // Lanes past the last column read it again; their shift base leaves them no digits.
+    const int i8 = lane & 7, rp = lane >> 3, rwarp = TC_SPLIT_WARPS - 1 - warp;
+    const int cmaxV = iend - 1 - i0, cmaxW = min(TC_N, k2 - j0) - 1;
+    const int ncA = 4 * (cmaxV / 8 + 1), ncB = 4 * (cmaxW / 8 + 1);
+    // a core's copy of stage s: cc < GR_A of V, the others of W
+    int off[GR_CORES_PER_WARP];                          // of the lane's entry from the stage's first row
 #pragma unroll
-        for (int cc = 0; cc < GR_CORES_PER_WARP; ++cc) {
-            const int q = warp + TC_SPLIT_WARPS * cc;
-            const bool isA = q < TC_ACORES;
-            const int qq = isA ? q : q - TC_ACORES;
-            const int col = (isA ? i0 : j0) + 8 * (qq >> 2) + i8;
-            const long rr = r + 8 * (qq & 3);
-            const double *src = isA ? V : W;
-            const long ld = isA ? ldv : ldw;
-            const bool in = q < TC_ACORES + TC_BCORES && col < (isA ? k1 : k2);
-            xv[cc][0] = (in && rr < re) ? src[rr * ld + col] : 0.0;
-            xv[cc][1] = (in && rr + 1 < re) ? src[(rr + 1) * ld + col] : 0.0;
+    for (int cc = 0; cc < GR_CORES_PER_WARP; ++cc) {
+        const bool isA = cc < GR_A;
+        const int q = isA ? warp + TC_SPLIT_WARPS * cc : rwarp + TC_SPLIT_WARPS * (cc - GR_A);
+        off[cc] = (8 * (q & 3) + 2 * rp) * (int)(isA ? ldv : ldw) + min(8 * (q >> 2) + i8, isA ? cmaxV : cmaxW);
+    }
+    auto copy_core = [&](int s, int cc) {
+        const bool isA = cc < GR_A;
+        const int q = isA ? warp + TC_SPLIT_WARPS * cc : rwarp + TC_SPLIT_WARPS * (cc - GR_A);
+        const long r = rb + (long)s * TC_KS, ld = isA ? ldv : ldw;
+        if (s < nst && q < (isA ? ncA : ncB)) {
+            const double *src = (isA ? V + i0 : W + j0) + r * ld + off[cc];
+            const uint32_t dst = sbase + 2 * TC_STAGE + TC_HDR + 512 * ((isA ? 0 : TC_ACORES) + q) + 16 * lane;
+            if (r + TC_KS <= re) {
+                tc_cp8(dst, src, 8);
+                tc_cp8(dst + 8, src + ld, 8);
+            } else {
+                const long left = re - r - (8 * (q & 3) + 2 * rp);   // rows of this lane before the split's end
+                tc_cp8(dst, left > 0 ? src : V, left > 0 ? 8 : 0);
+                tc_cp8(dst + 8, left > 1 ? src + ld : V, left > 1 ? 8 : 0);
+            }
         }
+        tc_cp_commit();
     };
-    if (!mma_warp) load_stage(0);
+    if (!mma_warp) {
+#pragma unroll
+        for (int cc = 0; cc < GR_CORES_PER_WARP; ++cc) copy_core(0, cc);
+    }
 
+    const uint8_t *raw = sm + 2 * TC_STAGE + TC_HDR + 16 * lane;
     for (int s = 0; s < nst; ++s) {
         const int buf = s & 1, cs = s % TC_CHUNK_STAGES;
         const bool chunk_end = cs == TC_CHUNK_STAGES - 1 || s == nst - 1;
@@ -387,37 +417,38 @@ k_gram_tc(int n, int k1, int k2, const double *__restrict__ V, long ldv, const d
             uint8_t *B = A + OZ_DIGITS * TC_APLANE;
 #pragma unroll
             for (int cc = 0; cc < GR_CORES_PER_WARP; ++cc) {
-                const int q = warp + TC_SPLIT_WARPS * cc;
-                const bool isA = q < TC_ACORES;
-                const int qq = isA ? q : q - TC_ACORES;
-                if (q < TC_ACORES + TC_BCORES && (isA ? i0 : j0) + 8 * (qq >> 2) < (isA ? k1 : k2)) {
-                    const int col = (isA ? i0 : j0) + 8 * (qq >> 2) + i8;
-                    const int e = col < (isA ? k1 : k2) ? (isA ? ev : ew)[col] : OZ_NO_EXP;
-                    const unsigned long long u0 = oz_bias(xv[cc][0], e), u1 = oz_bias(xv[cc][1], e);
-                    uint32_t *dst = (uint32_t *)((isA ? A : B) + qq * 128 + i8 * 16 + rp * 4);
-                    const int pl = (isA ? TC_APLANE : TC_BPLANE) / 4;
+                const bool isA = cc < GR_A;
+                const int q = isA ? warp + TC_SPLIT_WARPS * cc : rwarp + TC_SPLIT_WARPS * (cc - GR_A);
+                tc_cp_wait<GR_CORES_PER_WARP - 1>();     // this core's copy, the oldest in flight
+                if (q < (isA ? ncA : ncB)) {
+                    const int sb = sbs[(isA ? 0 : TC_M) + 8 * (q >> 2) + i8];
+                    const double2 xv = *reinterpret_cast<const double2 *>(raw + 512 * ((isA ? 0 : TC_ACORES) + q));
+                    uint32_t d[OZ_DIGITS];
+                    oz_pack(oz_bias(xv.x, sb), oz_bias(xv.y, sb), d);
+                    uint32_t *dst = (uint32_t *)((isA ? A : B) + q * 128 + i8 * 16 + rp * 4);
+                    constexpr int pl[2] = {TC_BPLANE / 4, TC_APLANE / 4};
 #pragma unroll
-                    for (int p = 0; p < OZ_DIGITS; ++p) dst[p * pl] = oz_pack(u0, u1, p);
+                    for (int p = 0; p < OZ_DIGITS; ++p) dst[p * pl[isA]] = d[p];
                 }
+                copy_core(s + 1, cc);
             }
             tc_fence_async_smem();
             tc_mbar_arrive(tc_smem_addr(h->bar) + 8 * buf);
-            if (s + 1 < nst) load_stage(s + 1);          // in flight while the MMAs run
         }
         if (chunk_end) {
             if (!tc_wait_chunk(h, s, err)) break;
 #pragma unroll
             for (int g4 = 0; g4 < TC_COLS_PER_WARP / 4; ++g4) {
-                if (col0 + g4 * 4 < N) {
+                if (col0 + g4 * 16 < N) {
                     uint32_t v[GR_LEVELS][4];
-                    tc_load_levels4<GR_LEVELS>(trow + g4 * 4, v);
+                    tc_load_levels4<GR_LEVELS>(trow + g4 * 16, v);
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         float lev[GR_LEVELS];
 #pragma unroll
                         for (int L = 0; L < GR_LEVELS; ++L) lev[L] = __uint_as_float(v[L][q]);
                         long long a, b;
-                        oz_levels_to_int<GR_LEVELS>(lev, a, b);
+                        oz_levels_to_int(lev, a, b);
                         // lo < 2^40 before the chunk and a chunk's level 3-7 sum is < 2^56.1
                         const long long l = lo[g4 * 4 + q] + b;
                         hi[g4 * 4 + q] += a + (l >> 40);
@@ -432,6 +463,7 @@ k_gram_tc(int n, int k1, int k2, const double *__restrict__ V, long ldv, const d
         if (*(volatile int *)&h->flag) break;
     }
 
+    tc_cp_wait<0>();
     __syncthreads();                                     // every wait of this CTA has ended: the flag is final
     if (!*(volatile int *)&h->flag) {
         const int i = i0 + quarter * 32 + lane;
@@ -439,8 +471,8 @@ k_gram_tc(int n, int k1, int k2, const double *__restrict__ V, long ldv, const d
         if (!last) {
 #pragma unroll
             for (int q = 0; q < TC_COLS_PER_WARP; ++q) {
-                const int j = j0 + col0 + q;
-                if (i < k1 && j < k2) {
+                const int j = j0 + col0 + (q >> 2) * 16 + (q & 3);
+                if (i < iend && j < k2) {
                     unsigned long long *P = sums + 2 * (i + (long)j * k1);
                     atomicAdd(P, (unsigned long long)hi[q]);
                     atomicAdd(P + 1, (unsigned long long)lo[q]);
@@ -448,7 +480,7 @@ k_gram_tc(int n, int k1, int k2, const double *__restrict__ V, long ldv, const d
             }
             __threadfence();
             __syncthreads();
-            int *is_last = (int *)(sm + 2 * TC_STAGE + 64);
+            int *is_last = (int *)(sm + 2 * TC_STAGE + 80);
             if (tid == 0) *is_last = atomicAdd(ticket + blockIdx.y * gridDim.x + blockIdx.x, 1u) == gridDim.z - 1;
             __syncthreads();
             last = *is_last != 0;
@@ -456,8 +488,8 @@ k_gram_tc(int n, int k1, int k2, const double *__restrict__ V, long ldv, const d
                 __threadfence();
 #pragma unroll
                 for (int q = 0; q < TC_COLS_PER_WARP; ++q) {
-                    const int j = j0 + col0 + q;
-                    if (i < k1 && j < k2) {
+                    const int j = j0 + col0 + (q >> 2) * 16 + (q & 3);
+                    if (i < iend && j < k2) {
                         const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2 *>(sums) + i + (long)j * k1);
                         hi[q] = (long long)v.x;
                         lo[q] = (long long)v.y;
@@ -468,7 +500,7 @@ k_gram_tc(int n, int k1, int k2, const double *__restrict__ V, long ldv, const d
         if (last) {
 #pragma unroll 1
             for (int q = 0; q < TC_COLS_PER_WARP; ++q) {
-                const int j = j0 + col0 + q;
+                const int j = j0 + col0 + (q >> 2) * 16 + (q & 3);
                 long long hq = 0, lq = 0;
 #pragma unroll
                 for (int u = 0; u < TC_COLS_PER_WARP; ++u)
@@ -476,7 +508,7 @@ k_gram_tc(int n, int k1, int k2, const double *__restrict__ V, long ldv, const d
                         hq = hi[u];
                         lq = lo[u];
                     }
-                if (i < k1 && j < k2 && !(sym && i > j)) {
+                if (i < iend && j < k2 && !(sym && i > j)) {
                     const __int128 z = (__int128)hq * ((__int128)1 << 40) + lq;
                     const double s = z == 0 ? 0.0 : oz_i128_to_double(z, ev[i] + ew[j] - OZ_SCALE_OFFSET - 56);
                     a[i + (long)j * lda] = s;
@@ -492,13 +524,18 @@ k_gram_tc(int n, int k1, int k2, const double *__restrict__ V, long ldv, const d
 // of 2^-16), so a split holds at most GR_MAX_ROWS rows (the level 3-7 sum is
 // carried into it after every chunk).
 #define GR_MAX_ROWS (1L << 20)
+static int gram_tc_mt(int k1)
+{
+    const int ti = (k1 + TC_M - 1) / TC_M;
+    return ((k1 + ti - 1) / ti + 7) / 8 * 8;
+}
 static long gram_tc_splits(int num_sms, int n, int k1, int k2, int sym, long *rps_out)
 {
     const int ti = (k1 + TC_M - 1) / TC_M, tj = (k2 + TC_N - 1) / TC_N;
     int tiles = 0;
     for (int a = 0; a < ti; ++a)
         for (int b = 0; b < tj; ++b)
-            if (!sym || a * TC_M <= b * TC_N + TC_N - 1) ++tiles;
+            if (!sym || a * gram_tc_mt(k1) <= b * TC_N + TC_N - 1) ++tiles;
     if (tiles < 1) tiles = 1;
     long nsplit = ((long)num_sms + tiles - 1) / tiles;
     const long max_split = (n + 4 * TC_KS - 1) / (4 * TC_KS);
@@ -545,7 +582,8 @@ extern "C" int gb_gram_tc(gcge_gpu_ctx *ctx, int n, int k1, int k2, const double
     const int stall = ctx->tc_stall;
     ctx->tc_stall = 0;
     GB_LAUNCH(ctx, k_gram_tc, grid, TC_THREADS, GR_SMEM, n, k1, k2, V, ldv, W, ldw, exps, exps + k1,
-              (unsigned long long *)ctx->scratch, ticket, a_dev, lda, rps, sym, ctx->dev_err, stall);
+              (unsigned long long *)ctx->scratch, ticket, a_dev, lda, rps, gram_tc_mt(k1), sym, ctx->dev_err,
+              stall);
     return GCGE_GPU_OK;
 }
 
@@ -709,7 +747,7 @@ extern "C" int gb_gram_fixed(cudaStream_t stream, int num_sms, int n, int k1, in
             k_col_stats<<<dim3(num_sms * 4, 2), 256, 0, stream>>>(n, k1, V, ldv, k2, W, ldw, ctl);
             k_gram_tc<<<dim3(ti, tj, (unsigned)nsplit), TC_THREADS, GR_SMEM, stream>>>(
                 n, k1, k2, V, ldv, W, ldw, ctl->e, ctl->e + k1, (unsigned long long *)part, ctl->ticket, a_dev, lda,
-                rps, sym, &ctl->skip, 0);
+                rps, gram_tc_mt(k1), sym, &ctl->skip, 0);
             if (cudaGetLastError() != cudaSuccess) return GCGE_GPU_ERR_CUDA;
             run = &ctl->skip;
         }
@@ -720,7 +758,8 @@ extern "C" int gb_gram_fixed(cudaStream_t stream, int num_sms, int n, int k1, in
 
 // ---------------------------------------------------------------- linear combination (tcgen05)
 #define LC_MAX_K 4096                                // inner dimension handled by the tensor-core path
-#define LC_HDR 2048                                  // tc_hdr, er, er_next, ecs
+#define LC_ER 8                                      // tiles whose row scales are kept
+#define LC_HDR (80 + 4 * (LC_ER * TC_M + TC_N) + 48) // tc_hdr, er, ecs
 #define LC_SMEM (2 * TC_STAGE + LC_HDR + 4 * LC_MAX_K)
 #define LC_OUT_LD (TC_N + 1)                         // doubles per staged output row
 #define LC_CORES_PER_WARP ((TC_ACORES + TC_SPLIT_WARPS - 1) / TC_SPLIT_WARPS)
@@ -782,14 +821,16 @@ k_lc_coef_split(int k1, int k2, const double *__restrict__ C, int ldc, int upper
     for (int cc = 0; cc < 4; ++cc) {
         const int core = warp * 4 + cc, g = core >> 2, c = core & 3;
         const int jj = g * 8 + n8, j = j0 + jj, i = s * TC_KS + c * 8 + 2 * kp;
-        unsigned long long u0 = OZ_BIAS, u1 = OZ_BIAS;
+        unsigned long long u0 = OZ_ZERO, u1 = OZ_ZERO;
         if (j < k2) {
-            if (i < k1 && (!upper || i <= j)) u0 = oz_bias(C[i + (long)j * ldc], fs[jj] + gs[i]);
-            if (i + 1 < k1 && (!upper || i + 1 <= j)) u1 = oz_bias(C[i + 1 + (long)j * ldc], fs[jj] + gs[i + 1]);
+            if (i < k1 && (!upper || i <= j)) u0 = oz_bias(C[i + (long)j * ldc], fs[jj] + gs[i] + OZ_SHIFT0);
+            if (i + 1 < k1 && (!upper || i + 1 <= j)) u1 = oz_bias(C[i + 1 + (long)j * ldc], fs[jj] + gs[i + 1] + OZ_SHIFT0);
         }
         const int w = (core * 128 + n8 * 16 + kp * 4) / 4;
+        uint32_t d[OZ_DIGITS];
+        oz_pack(u0, u1, d);
 #pragma unroll
-        for (int q = 0; q < OZ_DIGITS; ++q) out[q * (TC_BPLANE / 4) + w] = oz_pack(u0, u1, q);
+        for (int q = 0; q < OZ_DIGITS; ++q) out[q * (TC_BPLANE / 4) + w] = d[q];
     }
 }
 
@@ -815,9 +856,8 @@ k_lincomb_tc(int n, int k1, int k2, const double *__restrict__ X, long ldx, cons
     uint8_t *sm = tc_smem;
     if (*(volatile int *)err) return;                    // an earlier launch timed out: do nothing
     tc_hdr *h = (tc_hdr *)(sm + 2 * TC_STAGE);
-    int *er = (int *)(sm + 2 * TC_STAGE + 64);           // [TC_M] row scales of X 2^g, this tile
-    int *er_next = er + TC_M;                            // [TC_M] the same for the next tile
-    int *ecs = er_next + TC_M;                           // [TC_N] column scales of 2^-g C
+    int *er = (int *)(sm + 2 * TC_STAGE + 80);           // [LC_ER][TC_M] row scales of X 2^g, tile by tile
+    int *ecs = er + LC_ER * TC_M;                            // [TC_N] column scales of 2^-g C
     int *gs = (int *)(sm + 2 * TC_STAGE + LC_HDR);       // [k1] inner-dimension scales g
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int jt = blockIdx.y, j0 = jt * TC_N;
@@ -827,9 +867,13 @@ k_lincomb_tc(int n, int k1, int k2, const double *__restrict__ X, long ldx, cons
     const int chunk_stages = k1 <= OZ_EXACT_TERMS ? nst : TC_CHUNK_STAGES;
 
     tc_setup(h);
-    for (int i = tid; i < k1; i += TC_THREADS) gs[i] = g_in[i];
+    // a zero row of C contributes nothing, nor do the entries past k1: no digits
+    for (int i = tid; i < nst * TC_KS; i += TC_THREADS) {
+        const int g = i < k1 ? g_in[i] : OZ_NO_EXP;
+        gs[i] = g != OZ_NO_EXP ? g : -OZ_SHIFT_NONE;
+    }
     if (tid < TC_N) ecs[tid] = j0 + tid < k2 ? ec[j0 + tid] : OZ_NO_EXP;
-    if (tid < TC_M) er_next[tid] = OZ_NO_EXP;
+    for (int i = tid; i < (LC_ER - 1) * TC_M; i += TC_THREADS) er[TC_M + i] = OZ_NO_EXP;
     __syncthreads();
     // row scales of the first tile: 4 threads per row, up to LC_SCALE_LOADS
     // independent loads of the high words (sign, exponent) in flight per thread
@@ -850,8 +894,7 @@ k_lincomb_tc(int n, int k1, int k2, const double *__restrict__ X, long ldx, cons
             for (int j = 0; j < LC_SCALE_LOADS; ++j) {
                 const int i = i0 + 4 * j;
                 const int ex = (int)((w[j] >> 20) & 0x7ff);
-                const int gi = i < k1 ? gs[i] : OZ_NO_EXP;
-                if (ex && gi != OZ_NO_EXP) e = max(e, ex - 1022 + gi);
+                if (ex && i < k1) e = max(e, ex - 1022 + gs[i]);
             }
         }
         e = max(e, __shfl_xor_sync(0xffffffffu, e, 1));
@@ -863,12 +906,13 @@ k_lincomb_tc(int n, int k1, int k2, const double *__restrict__ X, long ldx, cons
     tc_fence_after_sync();
     const uint32_t tmem = h->tmem, sbase = tc_smem_addr(sm);
     const bool mma_warp = warp == TC_SPLIT_WARPS;
-    const int quarter = warp & 3, col0 = (warp >> 2) * TC_COLS_PER_WARP;
+    const int quarter = warp & 3, col0 = (warp >> 2) * 4;    // drained: columns col0 .. +3 of every 16
     const int my_row = quarter * 32 + lane;
     const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16) + col0;
     // alpha = +-1, beta = 0: the output is the drained value with its sign bit
     // flipped or not, an integer operation (the FP64 pipe runs at 1/64 rate)
     const bool plain = beta == 0.0 && (alpha == 1.0 || alpha == -1.0);
+    const bool unit = beta == 1.0 && (alpha == 1.0 || alpha == -1.0);   // one FP64 addition: fma(1, y, +-v)
     const unsigned long long sflip = alpha == -1.0 ? 0x8000000000000000ull : 0ull;
     int commits[3] = {0, 0, 0};
     int copies[2] = {0, 0};                              // bulk copies per buffer (thread 0)
@@ -877,174 +921,172 @@ k_lincomb_tc(int n, int k1, int k2, const double *__restrict__ X, long ldx, cons
     // row 8g + r8, entries 8c + 2 kp and 8c + 2 kp + 1
     const int r8 = lane >> 2, kp = lane & 3;
     double xv[LC_CORES_PER_WARP][2];
-    auto load_stage = [&](long row0, int s) {
-        const int ib = s * TC_KS + 2 * kp;
+    unsigned pw[LC_CORES_PER_WARP][2];                   // high words of the next tile's entries, in flight
+    int off[LC_CORES_PER_WARP];                          // of the lane's entries from the stage's first one
 #pragma unroll
-        for (int cc = 0; cc < LC_CORES_PER_WARP; ++cc) {
-            const int q = warp + TC_SPLIT_WARPS * cc;
-            const long r = row0 + 8 * (q >> 2) + r8;
-            const int i = ib + 8 * (q & 3);
-            const bool in = q < TC_ACORES && r < n;
-            xv[cc][0] = (in && i < k1) ? X[r * ldx + i] : 0.0;
-            xv[cc][1] = (in && i + 1 < k1) ? X[r * ldx + i + 1] : 0.0;
+    for (int cc = 0; cc < LC_CORES_PER_WARP; ++cc) {
+        const int q = warp + TC_SPLIT_WARPS * cc;
+        off[cc] = (8 * (q >> 2) + r8) * (int)ldx + 8 * (q & 3) + 2 * kp;
+    }
+    auto load_stage = [&](long row0, int s) {
+        const double *Xs = X + row0 * ldx + s * TC_KS;
+        if (row0 + TC_M <= n && (s + 1) * TC_KS <= k1) {
+#pragma unroll
+            for (int cc = 0; cc < LC_CORES_PER_WARP; ++cc)
+                if (warp + TC_SPLIT_WARPS * cc < TC_ACORES) {
+                    xv[cc][0] = Xs[off[cc]];
+                    xv[cc][1] = Xs[off[cc] + 1];
+                }
+        } else {
+#pragma unroll
+            for (int cc = 0; cc < LC_CORES_PER_WARP; ++cc) {
+                const int q = warp + TC_SPLIT_WARPS * cc, left = k1 - s * TC_KS - (8 * (q & 3) + 2 * kp);
+                const bool in = q < TC_ACORES && row0 + 8 * (q >> 2) + r8 < n;
+                xv[cc][0] = in && left > 0 ? Xs[off[cc]] : 0.0;
+                xv[cc][1] = in && left > 1 ? Xs[off[cc] + 1] : 0.0;
+            }
         }
     };
-    if (!mma_warp) load_stage((long)blockIdx.x * TC_M, 0);
-    // high words (sign, exponent) of the next tile's entries of one stage, in flight
-    unsigned pw[LC_CORES_PER_WARP][2];
-    int pw_stage = -1;
-    auto fold_scales = [&](int ps) {
-        const int ib = ps * TC_KS + 2 * kp;
+    auto load_words = [&](long row0, int s) {
+        const unsigned *Xs = reinterpret_cast<const unsigned *>(X + row0 * ldx + s * TC_KS) + 1;
+        const bool full = row0 + TC_M <= n && (s + 1) * TC_KS <= k1;
+#pragma unroll
+        for (int cc = 0; cc < LC_CORES_PER_WARP; ++cc) {
+            const int q = warp + TC_SPLIT_WARPS * cc, left = k1 - s * TC_KS - (8 * (q & 3) + 2 * kp);
+            const bool in = q < TC_ACORES && (full || row0 + 8 * (q >> 2) + r8 < n);
+            pw[cc][0] = in && (full || left > 0) ? __ldg(Xs + 2 * off[cc]) : 0u;
+            pw[cc][1] = in && (full || left > 1) ? __ldg(Xs + 2 * off[cc] + 2) : 0u;
+        }
+    };
+    auto fold_words = [&](int *scales, int s) {          // into the scales of the words' tile
 #pragma unroll
         for (int cc = 0; cc < LC_CORES_PER_WARP; ++cc) {
             const int q = warp + TC_SPLIT_WARPS * cc;
             if (q < TC_ACORES) {
-                const int i = ib + 8 * (q & 3);
-                int e = OZ_NO_EXP;
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const int ex = (int)((pw[cc][u] >> 20) & 0x7ff);
-                    const int gi = i + u < k1 ? gs[i + u] : OZ_NO_EXP;
-                    if (ex && gi != OZ_NO_EXP) e = max(e, ex - 1022 + gi);
-                }
+                const int2 g = *reinterpret_cast<const int2 *>(gs + s * TC_KS + 8 * (q & 3) + 2 * kp);
+                const int x0 = (int)((pw[cc][0] >> 20) & 0x7ff), x1 = (int)((pw[cc][1] >> 20) & 0x7ff);
+                int e = max(x0 ? x0 + g.x : OZ_NO_EXP, x1 ? x1 + g.y : OZ_NO_EXP);
                 e = max(e, __shfl_xor_sync(0xffffffffu, e, 1));
                 e = max(e, __shfl_xor_sync(0xffffffffu, e, 2));
-                if (kp == 0 && e > OZ_NO_EXP) atomicMax(er_next + 8 * (q >> 2) + r8, e);
+                if (kp == 0 && e > OZ_NO_EXP + 1022) atomicMax(scales + 8 * (q >> 2) + r8, e - 1022);
             }
         }
     };
+    if (!mma_warp) load_stage((long)blockIdx.x * TC_M, 0);
 
-    int gsc = 0;                                         // stages issued by this CTA, over all tiles
-    bool stop = false;
-    for (long t = blockIdx.x; t < ntiles && !stop; t += gridDim.x) {
-        const long row0 = t * TC_M, nrow0 = row0 + (long)gridDim.x * TC_M;
-        const bool has_next = t + gridDim.x < ntiles;
-        const int my_e = er[my_row];
-        double acc[MULTI ? TC_COLS_PER_WARP : 1];
+    // Stages g of this CTA over all its tiles (lt: its tile, s: the stage in it). A chunk
+    // is drained after the next stage has been split: the split of that one -- the next
+    // tile's first, mostly -- runs while the chunk's last MMAs do, and the next MMAs are
+    // ready to go when the drain ends.
+    const int mytiles = (int)((ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x), total = mytiles * nst;
+    const uint32_t scales_bar = tc_smem_addr(h->bar) + 56;
+    double acc[MULTI ? TC_COLS_PER_WARP : 1];
+    int s = 0, lt = 0, ps = 0, plt = 0;                  // this stage, the one before
+    for (int g = 0; g <= total; ++g) {
+        const int buf = g & 1;
+        const long row0 = ((long)blockIdx.x + (long)lt * gridDim.x) * TC_M, nrow0 = row0 + (long)gridDim.x * TC_M;
+        if (g < total && !mma_warp) {
+            const bool has_next = lt + 1 < mytiles;
+            if (g >= 2 && !tc_mbar_wait(tc_smem_addr(h->bar) + 16 + 8 * buf, ((g >> 1) - 1) & 1, TC_WAIT_NS))
+                tc_fail(h, err);
+            if (s == 0 && lt > 0) {
+                // the tile's scales: the last words loaded for it, then every split lane's are in.
+                // The slot cleared for the tile after the next held those of six tiles back: the
+                // MMAs just waited for, of tile lt - 2 at the earliest, were issued after every
+                // thread's drain of the tile before theirs.
+                fold_words(er + lt % LC_ER * TC_M, nst - 1);
+                if (tid < TC_M) er[(lt + 2) % LC_ER * TC_M + tid] = OZ_NO_EXP;
+                tc_mbar_arrive(scales_bar);
+                if (!tc_mbar_wait(scales_bar, (lt - 1) & 1, TC_WAIT_NS)) tc_fail(h, err);
+            }
+            const int *ert = er + lt % LC_ER * TC_M;
+            uint8_t *A = sm + buf * TC_STAGE;
+            uint8_t *B = A + OZ_DIGITS * TC_APLANE;
+            // the pre-split C planes of this stage: one bulk copy, completing on copied[buf]
+            if (tid == 0) {
+                const uint32_t copied = tc_smem_addr(h->bar) + 40 + 8 * buf;
+                tc_mbar_arrive_expect_tx(copied, OZ_DIGITS * TC_BPLANE);
+                tc_bulk_g2s(tc_smem_addr(B), Bd + (size_t)(jt * nst + s) * (OZ_DIGITS * TC_BPLANE / 16),
+                            OZ_DIGITS * TC_BPLANE, copied);
+                ++copies[buf];
+            }
 #pragma unroll
-        for (int q = 0; q < (MULTI ? TC_COLS_PER_WARP : 1); ++q) acc[q] = 0.0;
-        for (int s = 0; s < nst; ++s, ++gsc) {
-            const int buf = gsc & 1, cs = s % chunk_stages;
-            const bool chunk_end = cs == chunk_stages - 1 || s == nst - 1;
-            if (mma_warp) {
-                if (lane == 0) tc_issue_stage<LC_LEVELS, true>(h, sbase, tmem, N, gsc, cs, commits, err, stall);
-                __syncwarp();
-            } else {
-                if (gsc >= 2 && !tc_mbar_wait(tc_smem_addr(h->bar) + 16 + 8 * buf, ((gsc >> 1) - 1) & 1,
-                                              TC_WAIT_NS))
-                    tc_fail(h, err);
-                uint8_t *A = sm + buf * TC_STAGE;
-                uint8_t *B = A + OZ_DIGITS * TC_APLANE;
-                const uint32_t full = tc_smem_addr(h->bar) + 8 * buf;
-                // the pre-split C planes of this stage: one bulk copy, completing on copied[buf]
-                if (tid == 0) {
-                    const uint32_t copied = tc_smem_addr(h->bar) + 40 + 8 * buf;
-                    tc_mbar_arrive_expect_tx(copied, OZ_DIGITS * TC_BPLANE);
-                    tc_bulk_g2s(tc_smem_addr(B), Bd + (size_t)(jt * nst + s) * (OZ_DIGITS * TC_BPLANE / 16),
-                                OZ_DIGITS * TC_BPLANE, copied);
-                    ++copies[buf];
-                }
-                const int ib = s * TC_KS + 2 * kp;
+            for (int cc = 0; cc < LC_CORES_PER_WARP; ++cc) {
+                const int q = warp + TC_SPLIT_WARPS * cc;
+                if (q < TC_ACORES) {
+                    const int sb = ert[8 * (q >> 2) + r8] + OZ_SHIFT0;
+                    const int2 gg = *reinterpret_cast<const int2 *>(gs + s * TC_KS + 8 * (q & 3) + 2 * kp);
+                    uint32_t d[OZ_DIGITS];
+                    oz_pack(oz_bias(xv[cc][0], sb - gg.x), oz_bias(xv[cc][1], sb - gg.y), d);
+                    uint32_t *dst = (uint32_t *)(A + q * 128 + r8 * 16 + kp * 4);
 #pragma unroll
-                for (int cc = 0; cc < LC_CORES_PER_WARP; ++cc) {
-                    const int q = warp + TC_SPLIT_WARPS * cc;
-                    if (q < TC_ACORES) {
-                        const int i = ib + 8 * (q & 3);
-                        const int e = er[8 * (q >> 2) + r8];
-                        // a zero row of C (g = OZ_NO_EXP) contributes nothing: its digits stay zero
-                        const int g0 = i < k1 ? gs[i] : OZ_NO_EXP, g1 = i + 1 < k1 ? gs[i + 1] : OZ_NO_EXP;
-                        const unsigned long long u0 = g0 != OZ_NO_EXP ? oz_bias(xv[cc][0], e - g0) : OZ_BIAS;
-                        const unsigned long long u1 = g1 != OZ_NO_EXP ? oz_bias(xv[cc][1], e - g1) : OZ_BIAS;
-                        uint32_t *dst = (uint32_t *)(A + q * 128 + r8 * 16 + kp * 4);
-#pragma unroll
-                        for (int p = 0; p < OZ_DIGITS; ++p) dst[p * (TC_APLANE / 4)] = oz_pack(u0, u1, p);
-                    }
-                }
-                tc_fence_async_smem();
-                tc_mbar_arrive(full);
-                // in flight while the MMAs run: the next stage's values (or the next
-                // tile's first stage), and the next tile's entries of this stage for its scales
-                if (s + 1 < nst) load_stage(row0, s + 1);
-                else if (has_next) load_stage(nrow0, 0);
-                // the next tile's high words of the previous stage arrived while this
-                // stage was split: fold them into its row scales now, then issue this
-                // stage's (consumed one stage later, so no load latency is waited on)
-                if (pw_stage >= 0) fold_scales(pw_stage);
-                pw_stage = -1;
-                if (has_next) {
-#pragma unroll
-                    for (int cc = 0; cc < LC_CORES_PER_WARP; ++cc) {
-                        const int q = warp + TC_SPLIT_WARPS * cc;
-                        const long r = nrow0 + 8 * (q >> 2) + r8;
-                        const int i = ib + 8 * (q & 3);
-                        const bool in = q < TC_ACORES && r < n;
-                        const unsigned *xh = reinterpret_cast<const unsigned *>(X + (in ? r : 0) * ldx + i) + 1;
-                        pw[cc][0] = (in && i < k1) ? __ldg(xh) : 0u;
-                        pw[cc][1] = (in && i + 1 < k1) ? __ldg(xh + 2) : 0u;
-                    }
-                    pw_stage = s;
+                    for (int p = 0; p < OZ_DIGITS; ++p) dst[p * (TC_APLANE / 4)] = d[p];
                 }
             }
-            if (chunk_end) {
-                if (!tc_wait_chunk(h, gsc, err)) {
-                    stop = true;
-                    break;
+            tc_fence_async_smem();
+            tc_mbar_arrive(tc_smem_addr(h->bar) + 8 * buf);
+            // in flight while the MMAs run: the next stage's values (or the next tile's first
+            // ones), and the next tile's words of this stage; those of the stage before
+            // have arrived and are folded first
+            if (has_next && s > 0) fold_words(er + (lt + 1) % LC_ER * TC_M, s - 1);
+            if (s + 1 < nst) load_stage(row0, s + 1);
+            else if (has_next) load_stage(nrow0, 0);
+            if (has_next) load_words(nrow0, s);
+        }
+        // ---- drain of the chunk that ended with the stage before
+        if (g > 0 && (ps == nst - 1 || ps % chunk_stages == chunk_stages - 1)) {
+            const bool first = ps < chunk_stages, last = ps == nst - 1;
+            const long r = ((long)blockIdx.x + (long)plt * gridDim.x) * TC_M + my_row;
+            double *y = Y + r * ldy + j0 + col0;
+            const bool rin = r < n;
+            double yv[TC_COLS_PER_WARP];                 // the old values, on their way while the MMAs end
+            if (last && !plain) {
+#pragma unroll
+                for (int c = 0; c < TC_COLS_PER_WARP; ++c) {
+                    const int j = 16 * (c >> 2) + (c & 3);
+                    yv[c] = rin && j0 + col0 + j < k2 ? y[j] : 0.0;
                 }
-                const bool first = s < chunk_stages, last = s == nst - 1;
-                const long r = row0 + my_row;
+            }
+            if (!tc_wait_chunk(h, g - 1, err)) break;
+            const int my_e = er[plt % LC_ER * TC_M + my_row] - OZ_SCALE_OFFSET;
 #pragma unroll
-                for (int g4 = 0; g4 < TC_COLS_PER_WARP / 4; ++g4) {
-                    if (col0 + g4 * 4 < N) {
-                        uint32_t v[LC_LEVELS][4];
-                        tc_load_levels4<LC_LEVELS>(trow + g4 * 4, v);
+            for (int g4 = 0; g4 < TC_COLS_PER_WARP / 4; ++g4) {
+                if (col0 + g4 * 16 < N) {
+                    uint32_t v[LC_LEVELS][4];
+                    tc_load_levels4<LC_LEVELS>(trow + g4 * 16, v);
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            float lev[LC_LEVELS];
+                    for (int q = 0; q < 4; ++q) {
+                        int lev[LC_LEVELS];
 #pragma unroll
-                            for (int L = 0; L < LC_LEVELS; ++L) lev[L] = __uint_as_float(v[L][q]);
-                            long long a, b;
-                            oz_levels_to_int<LC_LEVELS>(lev, a, b);
-                            const double d =
-                                oz_to_double40(a, b, my_e + ecs[col0 + g4 * 4 + q] - OZ_SCALE_OFFSET);
-                            double v2 = d;
-                            if (MULTI) {
-                                acc[g4 * 4 + q] = first ? d : acc[g4 * 4 + q] + d;
-                                v2 = acc[g4 * 4 + q];
-                            }
-                            const int j = j0 + col0 + g4 * 4 + q;
-                            if (last && r < n && j < k2) {
-                                double *y = Y + r * ldy + j;
-                                if (plain)
-                                    *y = __longlong_as_double(__double_as_longlong(v2) ^ (long long)sflip);
-                                else
-                                    *y = fma(beta, *y, alpha * v2);
-                            }
+                        for (int L = 0; L < LC_LEVELS; ++L) lev[L] = __float2int_rn(__uint_as_float(v[L][q]));
+                        double v2 = oz_levels_to_double(lev, my_e + ecs[col0 + g4 * 16 + q]);
+                        if (MULTI) {
+                            acc[g4 * 4 + q] = first ? v2 : acc[g4 * 4 + q] + v2;
+                            v2 = acc[g4 * 4 + q];
+                        }
+                        if (last && rin && j0 + col0 + g4 * 16 + q < k2) {
+                            const double sv = __longlong_as_double(__double_as_longlong(v2) ^ (long long)sflip);
+                            const double yo = yv[g4 * 4 + q];
+                            y[16 * g4 + q] = plain ? sv : unit ? yo + sv : fma(beta, yo, alpha * v2);
                         }
                     }
                 }
-                tc_fence_before_sync();
-                tc_mbar_arrive(tc_smem_addr(h->bar) + 32);
-                ++commits[2];
             }
-            if (*(volatile int *)&h->flag) {
-                stop = true;
-                break;
-            }
+            tc_fence_before_sync();
+            tc_mbar_arrive(tc_smem_addr(h->bar) + 32);
+            ++commits[2];
         }
-        // tile end: fold the last stage's words (they arrived during the drain); then
-        // every scale atomic of the next tile is done; er <- er_next
-        if (!mma_warp && pw_stage >= 0) {
+        if (g < total && mma_warp) {
+            if (lane == 0) tc_issue_stage<LC_LEVELS, true>(h, sbase, tmem, N, g, s % chunk_stages, commits, err, stall);
             __syncwarp();
-            fold_scales(pw_stage);
-            pw_stage = -1;
         }
-        __syncthreads();
-        if (tid < TC_M) {
-            er[tid] = er_next[tid];
-            er_next[tid] = OZ_NO_EXP;
+        if (*(volatile int *)&h->flag) break;
+        ps = s;
+        plt = lt;
+        if (++s == nst) {
+            s = 0;
+            ++lt;
         }
-        __syncthreads();
-        if (*(volatile int *)&h->flag) stop = true;
     }
     tc_release(h, tmem, mma_warp, commits, copies);
 }

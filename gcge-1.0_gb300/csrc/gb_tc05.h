@@ -79,6 +79,22 @@ __device__ __forceinline__ void tc_bulk_g2s(uint32_t dst_smem, const void *src, 
                  "l"(src), "r"(bytes), "r"(bar)
                  : "memory");
 }
+// asynchronous copies of the issuing thread: global -> shared, zero filled past src_bytes
+__device__ __forceinline__ void tc_cp8(uint32_t dst_smem, const void *src, uint32_t src_bytes)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst_smem), "l"(src), "r"(src_bytes) : "memory");
+}
+__device__ __forceinline__ void tc_cp16(uint32_t dst_smem, const void *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
+}
+__device__ __forceinline__ void tc_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// until at most PENDING of this thread's groups are in flight
+template <int PENDING>
+__device__ __forceinline__ void tc_cp_wait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
+}
 // barrier over the first `count` threads of the CTA (named barrier `id`, 1..15)
 __device__ __forceinline__ void tc_bar_sync(int id, int count)
 {
@@ -146,53 +162,47 @@ __device__ __forceinline__ void tc_mma_commit(uint32_t bar)
 // -- an exact FP32 integer -- for up to OZ_EXACT_TERMS terms.
 #define OZ_DIGITS 7
 #define OZ_NO_EXP (-2000)          // scale of an all-zero row or column
-#define OZ_BIAS 0x80808080808080ULL
 #define OZ_EXACT_TERMS 186
 #define OZ_SCALE_OFFSET 10         // a digit product of level 0 carries 2^(e + f - 10)
 
-__device__ __forceinline__ unsigned long long oz_bias(double x, int e)
-{
-    const long long b = __double_as_longlong(x);
-    const int ex = (int)((b >> 52) & 0x7ff);
-    long long T = 0;
-    const int r = e + 1022 - ex;                          // T = mant 2^-r, r >= 0
-    if (ex && r < 60) {
-        const long long mant = (b & 0xFFFFFFFFFFFFFLL) | (1LL << 52);
-        T = (mant + ((1LL << r) >> 1)) >> r;
-        if (b < 0) T = -T;
-    }
-    return (unsigned long long)T + OZ_BIAS;
-}
 // exponent contribution of one entry: |x| < 2^(ex - 1022); OZ_NO_EXP for 0 and subnormals
 __device__ __forceinline__ int oz_exponent(double x)
 {
     const int ex = (int)((__double_as_longlong(x) >> 52) & 0x7ff);
     return ex ? ex - 1022 : OZ_NO_EXP;
 }
-// digit p of two biased values as one f16x2 word (u0 in the low half): the
-// bytes b are placed as 0x64bb = 1024 + b and 1152 is subtracted, both exact
-__device__ __forceinline__ uint32_t oz_pack(unsigned long long u0, unsigned long long u1, int p)
+#include "gb_ozconv.h"
+// U 2^8 of one entry, sb = its scale + OZ_SHIFT0 (OZ_SHIFT_NONE: no digits)
+__device__ __forceinline__ unsigned long long oz_bias(double x, int sb)
 {
-    const int byte = 6 - p, b = byte & 3;
-    const uint32_t w0 = byte < 4 ? (uint32_t)u0 : (uint32_t)(u0 >> 32);
-    const uint32_t w1 = byte < 4 ? (uint32_t)u1 : (uint32_t)(u1 >> 32);
-    const uint32_t t = __byte_perm(w0, w1, (uint32_t)(b | (b << 4) | ((b + 4) << 8) | ((b + 4) << 12)));
-    const uint32_t h = (t & 0x00FF00FFu) | 0x64006400u;
-    uint32_t r;
-    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(h), "r"(0x64806480u));
-    return r;
+    return oz_digits((uint32_t)__double2hiint(x), (uint32_t)__double2loint(x), sb);
+}
+// the seven digits of two entries (oz_digits) as f16x2 words, u0's in the low half, most
+// significant first: byte b goes under 0x64 as 0x64bb = 1024 + b, from which 1152 is
+// subtracted, both exact. A byte permute pairs two bytes of both entries, a second one
+// spreads each pair over the constant: 11 for seven digits.
+#define OZ_ZERO 0x8080808080808080ULL                // oz_digits of nothing
+__device__ __forceinline__ void oz_pack(unsigned long long u0, unsigned long long u1, uint32_t d[OZ_DIGITS])
+{
+    const uint32_t l0 = (uint32_t)u0, h0 = (uint32_t)(u0 >> 32), l1 = (uint32_t)u1, h1 = (uint32_t)(u1 >> 32);
+    const uint32_t ha = __byte_perm(h0, h1, 0x7362), hb = __byte_perm(h0, h1, 0x5140);
+    const uint32_t la = __byte_perm(l0, l1, 0x7373), lb = __byte_perm(l0, l1, 0x6251);
+    d[0] = __byte_perm(ha, 0x64646464u, 0x4342);
+    d[1] = __byte_perm(ha, 0x64646464u, 0x4140);
+    d[2] = __byte_perm(hb, 0x64646464u, 0x4342);
+    d[3] = __byte_perm(hb, 0x64646464u, 0x4140);
+    d[4] = __byte_perm(la, 0x64646464u, 0x4140);
+    d[5] = __byte_perm(lb, 0x64646464u, 0x4342);
+    d[6] = __byte_perm(lb, 0x64646464u, 0x4140);
+#pragma unroll
+    for (int p = 0; p < OZ_DIGITS; ++p) asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d[p]) : "r"(d[p]), "r"(0x64806480u));
 }
 
-#include "gb_ozconv.h"
-
-// levels (exact FP32 integers) -> hi (levels 0-2, units 2^-16) and lo (levels
-// 3 .. LEVELS-1 in units of the lowest level) of one output
-template <int LEVELS>
+// levels (exact FP32 integers) -> hi (levels 0-2, units 2^-16) and lo (levels 3-7,
+// units 2^-56) of one output
 __device__ __forceinline__ void oz_levels_to_int(const float *v, long long &hi, long long &lo)
 {
-    hi = ((long long)__float2int_rn(v[0]) << 16) + ((long long)__float2int_rn(v[1]) << 8) +
-         (long long)__float2int_rn(v[2]);
-    lo = 0;
-#pragma unroll
-    for (int L = 3; L < LEVELS; ++L) lo += (long long)__float2int_rn(v[L]) << (8 * (LEVELS - 1 - L));
+    hi = ((long long)__float2int_rn(v[1]) * 256 + __float2int_rn(v[2])) + (long long)__float2int_rn(v[0]) * 65536;
+    lo = (((long long)__float2int_rn(v[6]) * 256 + __float2int_rn(v[7])) + (long long)__float2int_rn(v[5]) * 65536) +
+         (long long)__float2int_rn(v[4]) * 16777216 + ((long long)__float2int_rn(v[3]) << 32);
 }
