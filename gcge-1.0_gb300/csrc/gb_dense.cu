@@ -221,84 +221,158 @@ extern "C" int gb_p_coef_assemble(gcge_gpu_ctx *ctx, double *coef, int ldc, int 
 // dropped when d <= rel_tol * G[j,j] or sqrt(d) <= zero_tol (or not finite).
 // Kept: R[j, j:] = S[j, j:] / sqrt(d), trailing update. Then U = R restricted to
 // the kept rows/columns is inverted; T[K_q, p] = inv(U)[q, p] (zeros elsewhere).
-__global__ void __launch_bounds__(512)
-k_chol_deflate(int k, const double *__restrict__ G, int ldg, double *__restrict__ T, int *kept_out,
-               double zero_tol, double rel_tol, double *__restrict__ S, double *__restrict__ R,
-               double *__restrict__ min_ratio)
+//
+// A step's pivot is a chain of a square root and a reciprocal (0.7 us of the FP64
+// pipe's latency), so warp 0 updates the next row first and forms the next pivot while
+// the other warps update the rest: one barrier a step. S and R share one array
+// (a row is scaled in place), and T's columns go into the triangle below it, all in
+// shared memory up to CD_SMEM_K columns (odd leading dimension: rows and columns
+// free of bank conflicts); wider blocks use the caller's work array. (One thread's
+// pivot, a reciprocal in all 512 threads, integer divisions for the indices and
+// global arrays took 474 us on average of 64 and 114 columns; this form 170 and 437, 259 on that average.)
+#define CD_THREADS 256
+#define CD_SMEM_K 160
+
+// n / b rounded as IEEE division, y = 1 / b correctly rounded: two corrections of n y by
+// the exact remainder (Markstein, IBM J. Res. Dev. 34, 1990; with a quotient within
+// one ulp and a correctly rounded reciprocal the second is exact), a chain of five
+// operations. Outside the middle of the exponent range the division itself.
+__device__ __forceinline__ double div_by(double n, double b, double y)
 {
-    extern __shared__ int shm[];
-    int *keep = shm;            // k
-    int *pos = shm + k;         // k: packed index of kept column
-    __shared__ int s_drop;
-    __shared__ double s_r;
-    const int tid = threadIdx.x, nt = blockDim.x;
-    for (long t = tid; t < (long)k * k; t += nt) {
-        const int i = (int)(t % k), j = (int)(t / k);
-        S[t] = G[i + (long)j * ldg];
-        R[t] = 0.0;
-    }
+    const int en = __double2hiint(n) & 0x7ff00000, eb = __double2hiint(b) & 0x7ff00000;
+    if (en < (123 << 20) || en > (1923 << 20) || eb < (723 << 20) || eb > (1323 << 20)) return n / b;
+    double q = __dmul_rn(n, y);
+    q = fma(fma(-b, q, n), y, q);
+    return fma(fma(-b, q, n), y, q);
+}
+
+__global__ void __launch_bounds__(CD_THREADS)
+k_chol_deflate(int k, const double *__restrict__ G, int ldg, double *__restrict__ T, int *kept_out,
+               double zero_tol, double rel_tol, double *work, double *__restrict__ min_ratio)
+{
+    extern __shared__ double cd_sm[];
+    const int ld = k | 1;
+    double *piv = cd_sm, *diag = piv + k, *rinv = diag + k;      // pivots d, G's diagonal, 1 / R[j, j]
+    int *keep = (int *)(rinv + k), *pos = keep + k;
+    double *A = work ? work : rinv + 2 * k;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = CD_THREADS / 32;
+    for (int j = warp; j < k; j += nw)
+        for (int i = lane; i <= j; i += 32) A[i + (long)j * ld] = G[i + (long)j * ldg];
+    for (int j = tid; j < k; j += CD_THREADS) diag[j] = G[j + (long)j * ldg];
     __syncthreads();
-    double mr = 1.0;                                     // thread 0: smallest pivot / diagonal
-    for (int j = 0; j < k; ++j) {
-        if (tid == 0) {
-            const double d = S[j + (long)j * k];
-            const double g = G[j + (long)j * ldg];
-            const bool ok = isfinite(d) && isfinite(g) && g > 0.0 && d > rel_tol * g && sqrt(d) > zero_tol;
-            if (g > 0.0) mr = fmin(mr, d / g);
-            s_drop = ok ? 0 : 1;
-            s_r = ok ? sqrt(d) : 0.0;
+    // pivot of row j (all lanes of a warp) and the row scaled into R
+    auto pivot = [&](int j) {
+        const double d = A[j + (long)j * ld], g = diag[j], r = sqrt(d);
+        const bool ok = isfinite(d) && isfinite(g) && g > 0.0 && d > rel_tol * g && r > zero_tol;
+        const double ri = 1.0 / r;
+        __syncwarp();
+        if (ok) {
+            for (int m = j + 1 + lane; m < k; m += 32) A[j + (long)m * ld] *= ri;
+            if (lane == 0) A[j + (long)j * ld] = r;
+        }
+        if (lane == 0) {
+            piv[j] = d;
+            rinv[j] = ri;
             keep[j] = ok;
         }
+    };
+    if (warp == 0) pivot(0);
+    for (int j = 0; j + 1 < k; ++j) {
         __syncthreads();
-        if (!s_drop) {
-            const double r = s_r, ri = 1.0 / r;
-            for (int m = j + tid; m < k; m += nt) R[j + (long)m * k] = (m == j) ? r : S[j + (long)m * k] * ri;
-            __syncthreads();
-            const int len = k - j - 1;
-            for (long t = tid; t < (long)len * len; t += nt) {
-                const int a = j + 1 + (int)(t % len), b = j + 1 + (int)(t / len);
-                if (a <= b) S[a + (long)b * k] -= R[j + (long)a * k] * R[j + (long)b * k];
+        const bool kj = keep[j];
+        if (warp == 0) {
+            if (kj) {
+                const double f = A[j + (long)(j + 1) * ld];
+                for (int m = j + 1 + lane; m < k; m += 32) {
+                    double *a = A + j + 1 + (long)m * ld;
+                    *a = fma(-f, A[j + (long)m * ld], *a);
+                }
+                __syncwarp();
+            }
+            pivot(j + 1);
+        } else if (kj) {
+            for (int b = j + 1 + warp; b < k; b += nw - 1) {
+                const double rb = A[j + (long)b * ld];
+                for (int a = j + 2 + lane; a <= b; a += 32) {
+                    double *t = A + a + (long)b * ld;
+                    *t = fma(-A[j + (long)a * ld], rb, *t);
+                }
             }
         }
-        __syncthreads();
     }
+    __syncthreads();
     if (tid == 0) {
         int c = 0;
         for (int j = 0; j < k; ++j) { pos[j] = keep[j] ? c : -1; c += keep[j]; }
         *kept_out = c;
-        if (min_ratio) *min_ratio = mr;
     }
-    __syncthreads();
-    // T = 0, then column p of inv(U) for each kept column j (p = pos[j]):
-    // x[p] = 1/U[p,p]; x[q] = -(sum_{l=q+1..p} U[q,l] x[l]) / U[q,q], walking kept rows.
-    for (long t = tid; t < (long)k * k; t += nt) T[t] = 0.0;
-    __syncthreads();
-    for (int jc = tid; jc < k; jc += nt) {
-        if (!keep[jc]) continue;
-        const int p = pos[jc];
-        T[jc + (long)p * k] = 1.0 / R[jc + (long)jc * k];
+    if (min_ratio && tid == 32) {
+        double mr = 1.0;
+        for (int j = 0; j < k; ++j)
+            if (diag[j] > 0.0) mr = fmin(mr, piv[j] / diag[j]);
+        *min_ratio = mr;
+    }
+    // column p of inv(U) for each kept column j (p = pos[j]):
+    // x[p] = 1/U[p,p]; x[q] = -(sum_{l=q+1..p} U[q,l] x[l]) / U[q,q], walking kept
+    // rows. x[l] of column jc is A[jc, l], zero for a dropped l. The sum is two chains (odd
+    // and even l - q), one in each of two lanes, as the pipe takes as long for one
+    // chain's instruction as for both; 16 columns a warp, a long and a short run of them
+    // on every quarter of the SM.
+    const int h = lane & 1, run = warp < 4 ? 7 - warp : warp - 4;
+    const unsigned pair = 3u << (lane & 30);
+    for (int j0 = (k - 1) / (16 * nw) * (16 * nw); j0 >= 0; j0 -= 16 * nw) {
+        const int jc = j0 + 16 * run + (lane >> 1);
+        if (jc >= k || !keep[jc]) continue;
+        double *x = A + jc;
         for (int q = jc - 1; q >= 0; --q) {
-            if (!keep[q]) continue;
-            double s0 = 0, s1 = 0;
-            int l = q + 1;
-            for (; l + 1 <= jc; l += 2) {
-                s0 = fma(R[q + (long)l * k], T[l + (long)p * k], s0);
-                s1 = fma(R[q + (long)(l + 1) * k], T[l + 1 + (long)p * k], s1);
+            double s = 0, z = 0.0;
+            if (keep[q]) {
+                const double *u = A + q;
+                int l = q + 1 + h;
+                for (; l < jc; l += 2) s = fma(u[(long)l * ld], x[(long)l * ld], s);
+                if (l == jc) s = fma(u[(long)jc * ld], rinv[jc], s);
+                s += __shfl_xor_sync(pair, s, 1);
+                z = div_by(-s, A[q + (long)q * ld], rinv[q]);
             }
-            if (l <= jc) s0 = fma(R[q + (long)l * k], T[l + (long)p * k], s0);
-            T[q + (long)p * k] = -(s0 + s1) / R[q + (long)q * k];
+            if (h == 0) x[(long)q * ld] = z;
+            __syncwarp(pair);
         }
     }
+    __syncthreads();
+    const int kept = *(volatile int *)kept_out;
+    for (int c = kept + warp; c < k; c += nw)                // columns past the kept ones
+        for (int i = lane; i < k; i += 32) T[i + (long)c * k] = 0.0;
+    for (int j = warp; j < k; j += nw) {
+        if (!keep[j]) continue;
+        double *t = T + (long)pos[j] * k;
+        for (int i = lane; i < k; i += 32) t[i] = i < j ? A[j + (long)i * ld] : i == j ? rinv[j] : 0.0;
+    }
+}
+
+static size_t cd_smem(int k, bool array)
+{
+    return sizeof(double) * (3 * (size_t)k + (array ? (size_t)k + (size_t)k * (k | 1) : 0)) + 2 * sizeof(int) * (size_t)k;
+}
+
+// work: at least k (k + 1) doubles
+static int cd_launch(gcge_gpu_ctx *ctx, int k, const double *G, int ldg, double *T, int *kept_dev, double zero_tol,
+                     double rel_tol, double *work, double *ratio_dev)
+{
+    if (k <= CD_SMEM_K) {
+        if (cudaFuncSetAttribute(k_chol_deflate, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)cd_smem(CD_SMEM_K, true)) != cudaSuccess)
+            return gb_fail(ctx, GCGE_GPU_ERR_CUDA);
+        work = nullptr;
+    }
+    GB_LAUNCH(ctx, k_chol_deflate, 1, CD_THREADS, cd_smem(k, !work), k, G, ldg, T, kept_dev, zero_tol, rel_tol, work,
+              ratio_dev);
+    return GCGE_GPU_OK;
 }
 
 extern "C" int gb_chol_deflate(gcge_gpu_ctx *ctx, int k, const double *G, int ldg, double *T, int *kept_dev,
                                double zero_tol, double rel_tol, double *work)
 {
-    if (k <= 0) return GCGE_GPU_OK;
-    double *S = work, *R = work + (size_t)k * k;
-    GB_LAUNCH(ctx, k_chol_deflate, 1, 512, 2 * k * sizeof(int), k, G, ldg, T, kept_dev, zero_tol, rel_tol, S, R,
-              (double *)nullptr);
-    return GCGE_GPU_OK;
+    return k <= 0 ? GCGE_GPU_OK : cd_launch(ctx, k, G, ldg, T, kept_dev, zero_tol, rel_tol, work, nullptr);
 }
 
 // ---------------------------------------------------------------- eigensolver
@@ -520,6 +594,174 @@ k_tridiag_smem(int m, const double *__restrict__ H, int ldh, double *__restrict_
     // reflectors (and the rest of the lower triangle) back to Aw for the back-transformation
     for (int c = wid; c < m; c += nw)
         for (int r = c + lane; r < m; r += 32) Aw[r + (long)c * m] = L[off(c) + (r - c)];
+}
+
+// The same reduction for m <= TS_MAX_M, with the matrix in full in shared memory and FP64
+// instructions counted: one keeps its quarter of the SM busy for 64 clocks whatever the
+// lanes that take part, so few of them, and on all four quarters. (A warp per row of
+// p = A22 v -- an FMA per 32 columns, then the five additions of a shuffle tree -- and a
+// warp per column of the update, lanes below the diagonal idle, spend most of
+// theirs on idle lanes.)
+//  * p = A22 v: a lane per row; of the 32 partial sums that are the lanes of that tree
+//    a warp takes the eight of one residue mod 4 and the tree's first three levels,
+//    and the row's thread the last two: 15 instructions a warp per 32 rows and columns.
+//  * The update walks the lower triangle folded into a rectangle, and mirrors it.
+//  * Warp 0 updates the next pivot column first and forms its reflector (a square root,
+//    and both quotients as two lanes of one division) while the others update the rest.
+// The same operations in the same order as k_tridiag with 256 threads. m = 33:
+// 134 -> 94 us.
+#define TS_MAX_M 127
+#define TS_THREADS 512
+static size_t ts_smem_bytes(int m) { return sizeof(double) * ((size_t)m * (m | 1) + 7 * (size_t)m); }
+
+__global__ void __launch_bounds__(TS_THREADS)
+k_tridiag_small(int m, const double *__restrict__ H, int ldh, double *__restrict__ Aw, double *__restrict__ d,
+                double *__restrict__ e, double *__restrict__ tau)
+{
+    extern __shared__ double sm[];
+    const int ld = m | 1;
+    double *A = sm, *vb = sm + (size_t)m * ld, *w = vb + 2 * m, *part = w + m;   // v of both parities, w, partials [4][m]
+    __shared__ double s_tau[2], red[4];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = TS_THREADS >> 5;
+    for (int c = wid; c < m; c += nw)
+        for (int r = c + lane; r < m; r += 32) {
+            const double h = H[r + (long)c * ldh];
+            A[r + c * ld] = h;
+            A[c + r * ld] = h;
+        }
+    __syncthreads();
+    auto tree = [&](double s) {
+#pragma unroll
+        for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
+        return s;
+    };
+    // reflector of column i (warp 0): v, tau, d, e
+    auto reflector = [&](int i) {
+        const int len = m - i - 1;
+        double *col = A + i * ld + i + 1, *v = vb + (i & 1) * m;  // x = A[i+1:m, i]
+        double t = 0;
+        for (int r0 = 1; r0 < len; r0 += 32) {
+            const double x = r0 + lane < len ? col[r0 + lane] : 0.0;
+            t += tree(x * x);
+        }
+        const double alpha = col[0];
+        double tv = 0.0, beta = alpha, sc = 0.0;
+        if (t != 0.0) {
+            beta = -copysign(sqrt(alpha * alpha + t), alpha);
+            const double q = (lane ? 1.0 : beta - alpha) / (lane ? alpha - beta : beta);
+            tv = __shfl_sync(FULL, q, 0);
+            sc = __shfl_sync(FULL, q, 1);
+        }
+        if (lane == 0) {
+            d[i] = A[i * ld + i];
+            e[i] = beta;
+            tau[i] = tv;
+            s_tau[i & 1] = tv;
+        }
+        __syncwarp();
+        for (int r = lane; r < len; r += 32) {
+            const double vr = tv == 0.0 ? 0.0 : col[r] * sc;   // a zero reflector is stored as zeros
+            if (r > 0) col[r] = vr;
+            v[r] = r == 0 ? 1.0 : vr;
+        }
+    };
+    if (wid == 0 && m > 2) reflector(0);
+    for (int i = 0; i + 2 < m; ++i) {
+        const int len = m - i - 1, b = i + 1;
+        const double *v = vb + (i & 1) * m;
+        double *A22 = A + b * ld + b;
+        __syncthreads();
+        const double tv = s_tau[i & 1];
+        if (tv == 0.0) {                                   // uniform: nothing to apply
+            if (wid == 0 && i + 3 < m) reflector(i + 1);
+            continue;
+        }
+        // the partial sums of p = A22 v: (32 rows, residue) per warp
+        for (int k = wid; k < 4 * ((len + 31) / 32); k += nw) {
+            const int q = k & 3, r = 32 * (k >> 2) + lane;
+            double P[8];
+#pragma unroll
+            for (int l = 0; l < 8; ++l) P[l] = 0;
+            const double *a = A22 + min(r, len - 1);
+            for (int c0 = q; c0 < len; c0 += 32) {
+#pragma unroll
+                for (int l = 0; l < 8; ++l)
+                    if (c0 + 4 * l < len) P[l] = fma(a[(c0 + 4 * l) * ld], v[c0 + 4 * l], P[l]);
+            }
+#pragma unroll
+            for (int o = 4; o; o >>= 1)
+#pragma unroll
+                for (int l = 0; l < o; ++l)
+                    if (q + 4 * (l + o) < len) P[l] += P[l + o];
+            if (r < len) part[q * m + r] = P[0];
+        }
+        __syncthreads();
+        // p = tau times the rows' sums, K = tau / 2 p.v, w = p - K v: 32 rows a warp
+        if (wid < 4) {
+            const int r = 32 * wid + lane, n4 = min(4, (len + 31) / 32);
+            double p = 0, x = 0;
+            if (r < len) {
+                p = tv * ((part[r] + part[2 * m + r]) + (part[m + r] + part[3 * m + r]));
+                x = p * v[r];
+            }
+            if (32 * wid < len) {
+                x = tree(x);
+                if (lane == 0) red[wid] = x;
+            }
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+            double t = 0;
+            for (int q = 0; q < n4; ++q) t += red[q];
+            const double K = 0.5 * tv * t;
+            if (r < len) w[r] = p - K * v[r];
+        }
+        __syncthreads();
+        // A22 -= v w^T + w v^T
+        auto update = [&](int r, int c) {
+            const double vc = v[c], wc = w[c];
+            double t = A22[r + c * ld];
+            t -= v[r] * wc + w[r] * vc;
+            A22[r + c * ld] = t;
+            A22[c + r * ld] = t;
+        };
+        if (wid == 0) {
+            for (int r = lane; r < len; r += 32) update(r, 0);
+            __syncwarp();
+            if (i + 3 < m) reflector(i + 1);
+        } else {
+            // columns 1 .. len - 1 (len - c entries each) as rows of width len: column 1 + y
+            // and column len - 1 - y share one
+            const int n1 = len - 1, rows = (n1 + 1) / 2, width = n1 + 1;
+            int y = 0, xx = tid - 32;
+            while (xx >= width) {
+                xx -= width;
+                ++y;
+            }
+            while (y < rows) {
+                const int lc = n1 - y;                     // entries of column 1 + y
+                if (xx < lc) update(1 + y + xx, 1 + y);
+                else if (n1 - 1 - y != y) update(n1 - y + xx - lc, n1 - y);
+                xx += TS_THREADS - 32;
+                while (xx >= width) {
+                    xx -= width;
+                    ++y;
+                }
+            }
+        }
+    }
+    __syncthreads();
+    if (tid == 0) {
+        if (m >= 2) {
+            d[m - 2] = A[(m - 2) * ld + m - 2];
+            e[m - 2] = A[(m - 2) * ld + m - 1];
+            tau[m - 2] = 0.0;
+        }
+        d[m - 1] = A[(m - 1) * ld + m - 1];
+        e[m - 1] = 0.0;
+        tau[m - 1] = 0.0;
+    }
+    // reflectors (and the rest of the lower triangle) back to Aw for the back-transformation
+    for (int c = wid; c < m; c += nw)
+        for (int r = c + lane; r < m; r += 32) Aw[r + (long)c * m] = A[r + c * ld];
 }
 
 // 1/x by Newton-Raphson refinement of the hardware reciprocal approximation
@@ -822,23 +1064,53 @@ static int td_cluster_launch(gcge_gpu_ctx *ctx, int tc, int m, const double *H, 
     return gb_check_launch(ctx);
 }
 
+// n / b on the path of the Sturm counts: the hardware reciprocal refined once (Newton-
+// Raphson, about 2^-40), then the quotient corrected by its exact remainder, which
+// leaves an error of 2^-80 before the one rounding -- the IEEE quotient but for values
+// that close to the middle of two doubles. Five FP64 instructions; a quotient is most
+// of a Sturm step, and each instruction takes a quarter of the SM for 64 clocks.
+// Outside the middle of the exponent range the division itself.
+__device__ __forceinline__ double sturm_div(double n, double b)
+{
+    const int en = __double2hiint(n) & 0x7ff00000, eb = __double2hiint(b) & 0x7ff00000;
+    if (en < (323 << 20) || en > (1723 << 20) || eb < (323 << 20) || eb > (1723 << 20)) return n / b;
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
+    r = fma(fma(-b, r, 1.0), r, r);
+    const double q = __dmul_rn(n, r);
+    return fma(fma(-b, q, n), r, q);
+}
+
+// x = m 2^e with |m| in [1, 2) (x normal): m, and e added to ex
+__device__ __forceinline__ double take_exponent(double x, int &ex)
+{
+    const int hi = __double2hiint(x);
+    ex += ((hi >> 20) & 0x7ff) - 1023;
+    return __hiloint2double((hi & 0x800fffff) | 0x3ff00000, __double2loint(x));
+}
+
 // number of eigenvalues of the tridiagonal (d, e2 = e^2) smaller than x (the
 // ratio form of the Sturm sequence with the pivmin guard; its count is monotone
-// in x under IEEE arithmetic, which the bisection relies on inside clusters)
-__device__ __forceinline__ int sturm_count(int m, const double *d, const double *e2, double x, double pivmin)
+// in x under IEEE arithmetic, which the bisection relies on inside clusters);
+// det 2^ex: det(T - x I), the product of the ratios (off the chain of them)
+__device__ __forceinline__ int sturm_count(int m, const double *d, const double *e2, double x, double pivmin,
+                                           double &det, int &ex)
 {
     double q = d[0] - x;
     if (fabs(q) < pivmin) q = -pivmin;
     int cnt = q < 0.0;
+    ex = 0;
+    det = take_exponent(q, ex);
     for (int i = 1; i < m; ++i) {
-        q = (d[i] - x) - e2[i - 1] / q;
+        q = (d[i] - x) - sturm_div(e2[i - 1], q);
         if (fabs(q) < pivmin) q = -pivmin;
         cnt += q < 0.0;
+        det = take_exponent(__dmul_rn(det, take_exponent(q, ex)), ex);
     }
     return cnt;
 }
 
-// one warp per wanted eigenvalue index j (il-1+warp), 32-point multisection.
+// one block per wanted eigenvalue index j (il-1+block), 32-point multisection.
 // guess (may be NULL): an estimate of each wanted eigenvalue (the previous
 // Rayleigh-Ritz step's). Its first round counts at g -/+ |g| 2^-(3l+1), l = 0..15
 // (lanes 0-15 below, 16-31 above); the closest points whose counts still bracket
@@ -846,46 +1118,55 @@ __device__ __forceinline__ int sturm_count(int m, const double *d, const double 
 // guess within relative d of the eigenvalue leaves a bracket of relative width
 // ~16 d instead of the Gershgorin interval. The counts are monotone in x, so a
 // wrong guess only loses that round.
-__global__ void __launch_bounds__(256)
+//
+// A warp's 32 counts keep its quarter of the SM's FP64 pipe busy, so a pass of four
+// warps takes as long as one: warp L counts at the points of the L-th round from
+// here, along the path that an estimate of the eigenvalue predicts (at first the guess,
+// then the zero of det(T - x I) by inverse interpolation through the four points
+// around its sign change; the last ratio alone says nothing where T all but splits). Rounds whose predicted interval turns out to be the actual one are
+// done; the first always is. m = 33: 149 us (one round a pass, IEEE divisions) -> 92.
+#define BI_WARPS 4
+__global__ void __launch_bounds__(32 * BI_WARPS)
 k_bisect(int m, const double *__restrict__ dg, const double *__restrict__ eg, int il, int iu,
          double *__restrict__ eval, int *info, const double *__restrict__ guess)
 {
     extern __shared__ double sm[];
     double *d = sm, *e2 = sm + m;
-    __shared__ double s_gl, s_gu, s_piv;
-    const int tid = threadIdx.x, lane = tid & 31;
+    __shared__ double px[BI_WARPS][32], pq[BI_WARPS][32], plo[BI_WARPS], phi[BI_WARPS];
+    __shared__ unsigned pge[BI_WARPS];
+    __shared__ int pe[BI_WARPS][32];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     for (int i = tid; i < m; i += blockDim.x) {
         d[i] = dg[i];
         e2[i] = (i < m - 1) ? eg[i] * eg[i] : 0.0;
     }
     __syncthreads();
-    if (tid == 0) {
-        double gl = DBL_MAX, gu = -DBL_MAX, emax = 0;
-        for (int i = 0; i < m; ++i) {
-            const double r = (i > 0 ? fabs(eg[i - 1]) : 0.0) + (i < m - 1 ? fabs(eg[i]) : 0.0);
-            gl = fmin(gl, d[i] - r);
-            gu = fmax(gu, d[i] + r);
-            if (i < m - 1) emax = fmax(emax, e2[i]);
-        }
-        const double bn = fmax(fabs(gl), fabs(gu));
-        const double piv = DBL_MIN * fmax(1.0, emax);
-        const double fudge = 2.0 * DBL_EPSILON * bn * m + 2.0 * piv;
-        s_gl = gl - fudge;
-        s_gu = gu + fudge;
-        s_piv = piv;
+    // Gershgorin interval and pivot floor, every warp for itself
+    double gl = DBL_MAX, gu = -DBL_MAX, emax = 0;
+    for (int i = lane; i < m; i += 32) {
+        const double r = (i > 0 ? fabs(eg[i - 1]) : 0.0) + (i < m - 1 ? fabs(eg[i]) : 0.0);
+        gl = fmin(gl, d[i] - r);
+        gu = fmax(gu, d[i] + r);
+        if (i < m - 1) emax = fmax(emax, e2[i]);
     }
-    __syncthreads();
-    const int j = il + (int)((blockIdx.x * blockDim.x + tid) >> 5);   // 1-based wanted index
-    if (j > iu) return;                                                // warp-uniform
-    double lo = s_gl, hi = s_gu;
-    const double piv = s_piv;
+    for (int o = 16; o; o >>= 1) {
+        gl = fmin(gl, __shfl_xor_sync(FULL, gl, o));
+        gu = fmax(gu, __shfl_xor_sync(FULL, gu, o));
+        emax = fmax(emax, __shfl_xor_sync(FULL, emax, o));
+    }
+    const double bn = fmax(fabs(gl), fabs(gu));
+    const double piv = DBL_MIN * fmax(1.0, emax);
+    const double fudge = 2.0 * DBL_EPSILON * bn * m + 2.0 * piv;
+    const int j = il + (int)blockIdx.x;                               // 1-based wanted index
+    double lo = gl - fudge, hi = gu + fudge, est = 0.5 * (lo + hi), q;
+    int ex;
     if (guess) {
         const double g = guess[j - il];
-        if (isfinite(g) && g != 0.0) {
+        if (isfinite(g) && g != 0.0) {                                // every warp the same counts
             const int l = lane & 15;
             const double del = ldexp(fabs(g), -(3 * l + 1));
             const double x = lane < 16 ? g - del : g + del;
-            const int c = sturm_count(m, d, e2, x, piv);
+            const int c = sturm_count(m, d, e2, x, piv, q, ex);
             const unsigned below = __ballot_sync(FULL, lane < 16 && c < j) & 0xffffu;
             const unsigned above = __ballot_sync(FULL, lane >= 16 && c >= j) >> 16;
             if (below) {
@@ -896,38 +1177,91 @@ k_bisect(int m, const double *__restrict__ dg, const double *__restrict__ eg, in
                 const double xh = __shfl_sync(FULL, x, 16 + (31 - __clz(above)));
                 if (xh < hi) hi = xh;
             }
+            est = g;
         }
     }
-    for (int it = 0; it < 80; ++it) {
-        const double width = hi - lo;
-        const double tolv = 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + piv;
-        if (width <= tolv) break;
-        const double x = lo + width * (double)(lane + 1) / 33.0;
-        const int c = sturm_count(m, d, e2, x, piv);
-        const unsigned ge = __ballot_sync(FULL, c >= j);
-        double nlo, nhi;
+    // the round's next interval, given which of its points the eigenvalue lies below
+    auto next = [&](unsigned ge, double x, double &a, double &b) {
         if (ge == 0u) {
-            nlo = __shfl_sync(FULL, x, 31);
-            nhi = hi;
+            a = __shfl_sync(FULL, x, 31);
         } else {
             const int f = __ffs(ge) - 1;
-            nhi = __shfl_sync(FULL, x, f);
+            b = __shfl_sync(FULL, x, f);
             const double xm = __shfl_sync(FULL, x, f > 0 ? f - 1 : 0);
-            nlo = f > 0 ? xm : lo;
+            if (f > 0) a = xm;
         }
-        if (nlo == lo && nhi == hi) break;   // no representable progress
-        lo = nlo;
-        hi = nhi;
+    };
+    auto narrow = [&](double a, double b) { return b - a <= 2.0 * DBL_EPSILON * fmax(fabs(a), fabs(b)) + piv; };
+    bool more = true;
+    for (int it = 0; it < 80 && more && !narrow(lo, hi);) {
+        // this warp's round on the predicted path
+        double a = lo, b = hi, x = 0;
+        for (int L = 0;; ++L) {
+            x = a + (b - a) * (double)(lane + 1) / 33.0;
+            if (L == wid) break;
+            next(__ballot_sync(FULL, x >= est), x, a, b);
+        }
+        const int c = sturm_count(m, d, e2, x, piv, q, ex);
+        const unsigned ge = __ballot_sync(FULL, c >= j);
+        px[wid][lane] = x;
+        pq[wid][lane] = q;
+        pe[wid][lane] = ex;
+        if (lane == 0) {
+            pge[wid] = ge;
+            plo[wid] = a;
+            phi[wid] = b;
+        }
+        __syncthreads();
+        // the rounds that hold, in every warp
+        int deep = 0;
+        for (int L = 0; L < BI_WARPS && it < 80; ++L, ++it) {
+            if (narrow(lo, hi)) {
+                more = false;
+                break;
+            }
+            if (plo[L] != lo || phi[L] != hi) break;                  // not this way: L >= 1
+            double nlo = lo, nhi = hi;
+            next(pge[L], px[L][lane], nlo, nhi);
+            deep = L;
+            if (nlo == lo && nhi == hi) {                             // no representable progress
+                more = false;
+                break;
+            }
+            lo = nlo;
+            hi = nhi;
+        }
+        // the next estimate: inverse interpolation of the determinant around its sign change
+        if (more) {
+            const unsigned g = pge[deep];
+            const int f = g ? __ffs(g) - 1 : 32, f0 = min(max(f - 2, 0), 28);
+            double X[4], Q[4];
+            const int e0 = max(pe[deep][f0], pe[deep][f0 + 3]);       // a common scale, near enough
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                X[t] = px[deep][f0 + t];
+                Q[t] = ldexp(pq[deep][f0 + t], max(-1000, min(1000, pe[deep][f0 + t] - e0)));
+            }
+            est = 0.5 * (lo + hi);
+            const bool down = Q[0] > Q[1] && Q[1] > Q[2] && Q[2] > Q[3] && Q[0] > 0.0 && Q[3] < 0.0;
+            const bool up = Q[0] < Q[1] && Q[1] < Q[2] && Q[2] < Q[3] && Q[0] < 0.0 && Q[3] > 0.0;
+            if (down || up) {
+#pragma unroll
+                for (int s = 1; s < 4; ++s)
+#pragma unroll
+                    for (int t = 0; t + s < 4; ++t) X[t] = X[t] + (X[t + 1] - X[t]) * (Q[t] / (Q[t] - Q[t + s]));
+                if (X[0] > lo && X[0] < hi) est = X[0];
+            }
+        }
+        __syncthreads();                                              // before the points are overwritten
     }
-    if (lane == 0) {
+    if (tid == 0) {
         const double ev = 0.5 * (lo + hi);
         eval[j - il] = ev;
         if (!isfinite(ev)) atomicExch(info, 1);
     }
 }
 
-// inverse iteration: one thread per wanted eigenvalue; LU of T - lambda I with
-// partial pivoting (dgttrf layout) and three solves from a hashed start vector.
+// start vectors of inverse iteration, hashed
 __device__ __forceinline__ double start_value(int j, int i)
 {
     unsigned long long z = (unsigned long long)(j + 1) * 0x9E3779B97F4A7C15ULL ^ (unsigned long long)(i + 7) * 0xD1B54A32D192ED03ULL;
@@ -964,26 +1298,25 @@ extern "C" int gb_recip_check(int n, const double *x_host, double *r_host)
     return st;
 }
 
-// inverse iteration: one thread per wanted eigenvalue, IV per block (one warp);
-// LU of T - lambda I with partial pivoting (dgttrf layout) and three solves from
-// a hashed start vector. The working arrays of the block's eigenvalues sit in
-// shared memory, element i of lane l at [i * IV + l] (consecutive lanes,
-// consecutive words: no bank conflicts).
+// inverse iteration: a block of one warp per wanted eigenvalue, so that the chains
+// spread over the SMs (the FP64 pipe of an SM is narrow); LU of T - lambda I with
+// partial pivoting (dgttrf layout) and three solves from a hashed start vector, the
+// working arrays in shared memory. Lane 0 walks the recurrences, with the next
+// elements in registers; what has no recurrence (set-up, pivots' reciprocals, start
+// vector, maxima, scalings) is done by all lanes. (All by one lane: 71 us for 13
+// vectors of 30, here 34.)
 __global__ void __launch_bounds__(32)
 k_invit(int m, const double *__restrict__ d, const double *__restrict__ e, int nev,
-        const double *__restrict__ eval, double *__restrict__ Zt, int ldz, int IV)
+        const double *__restrict__ eval, double *__restrict__ Zt, int ldz)
 {
     extern __shared__ double ism[];
-    const int lane = threadIdx.x;
-    const int j = blockIdx.x * IV + lane;
-    if (lane >= IV || j >= nev) return;
-    double *dl = ism, *dd = dl + (size_t)m * IV, *du = dd + (size_t)m * IV, *du2 = du + (size_t)m * IV;
-    double *inv = du2 + (size_t)m * IV, *z = inv + (size_t)m * IV;
-    int *ip = (int *)(z + (size_t)m * IV);
-#define IX(i) ((size_t)(i) * IV + lane)
+    const int lane = threadIdx.x, j = blockIdx.x;
+    double *dl = ism, *dd = dl + m, *du = dd + m, *du2 = du + m, *inv = du2 + m, *z = inv + m;
+    int *ip = (int *)(z + m);
     double tnorm = 0;
-    for (int i = 0; i < m; ++i)
+    for (int i = lane; i < m; i += 32)
         tnorm = fmax(tnorm, fabs(d[i]) + (i > 0 ? fabs(e[i - 1]) : 0.0) + (i < m - 1 ? fabs(e[i]) : 0.0));
+    for (int o = 16; o; o >>= 1) tnorm = fmax(tnorm, __shfl_xor_sync(FULL, tnorm, o));
     // perturb a shift that repeats the previous one (dstein: separate close shifts)
     double lam = eval[j];
     const double pert = 10.0 * DBL_EPSILON * fmax(fabs(lam), tnorm * 1e-3);
@@ -992,77 +1325,104 @@ k_invit(int m, const double *__restrict__ d, const double *__restrict__ e, int n
         while (k > 0 && eval[k] - eval[k - 1] < pert) --k;
         lam = eval[k] + (double)(j - k) * pert;
     }
-    for (int i = 0; i < m; ++i) {
-        dd[IX(i)] = d[i] - lam;
-        dl[IX(i)] = (i < m - 1) ? e[i] : 0.0;
-        du[IX(i)] = (i < m - 1) ? e[i] : 0.0;
-        du2[IX(i)] = 0.0;
-        ip[IX(i)] = i;
+    for (int i = lane; i < m; i += 32) {
+        dd[i] = d[i] - lam;
+        const double ei = i < m - 1 ? e[i] : 0.0;
+        dl[i] = ei;
+        du[i] = ei;
+        du2[i] = 0.0;
+        ip[i] = i;
+        z[i] = start_value(j, i);
     }
-    for (int i = 0; i + 1 < m; ++i) {
-        const double di = dd[IX(i)], li = dl[IX(i)];
-        if (fabs(di) >= fabs(li)) {
-            if (di != 0.0) {
-                const double f = li * nr_recip(di);
-                dl[IX(i)] = f;
-                dd[IX(i + 1)] -= f * du[IX(i)];
+    __syncwarp();
+    if (lane == 0) {
+        double di = dd[0], ui = du[0];                   // row i of the partly reduced matrix
+        for (int i = 0; i + 1 < m; ++i) {
+            const double li = dl[i], dn = dd[i + 1], un = du[i + 1];
+            if (fabs(di) >= fabs(li)) {
+                dd[i] = di;
+                du[i] = ui;
+                double f = 0.0, t = dn;
+                if (di != 0.0) {
+                    f = li * nr_recip(di);
+                    t -= f * ui;
+                }
+                dl[i] = f;
+                di = t;
+                ui = un;
             } else {
-                dl[IX(i)] = 0.0;
+                const double f = di * nr_recip(li);
+                dd[i] = li;
+                dl[i] = f;
+                du[i] = dn;
+                di = ui - f * dn;
+                ui = un;
+                if (i + 2 < m) {
+                    du2[i] = un;
+                    ui = -f * un;
+                }
+                ip[i] = i + 1;
             }
-        } else {
-            const double f = di * nr_recip(li);
-            dd[IX(i)] = li;
-            dl[IX(i)] = f;
-            const double t = du[IX(i)];
-            const double dn = dd[IX(i + 1)];
-            du[IX(i)] = dn;
-            dd[IX(i + 1)] = t - f * dn;
-            if (i + 2 < m) {
-                du2[IX(i)] = du[IX(i + 1)];
-                du[IX(i + 1)] = -f * du[IX(i + 1)];
-            }
-            ip[IX(i)] = i + 1;
         }
+        dd[m - 1] = di;
     }
+    __syncwarp();
     const double tiny = DBL_EPSILON * fmax(tnorm, DBL_MIN);
-    for (int i = 0; i < m; ++i) {
-        double di = dd[IX(i)];
+    for (int i = lane; i < m; i += 32) {
+        double di = dd[i];
         if (fabs(di) < tiny) di = copysign(tiny, di == 0.0 ? 1.0 : di);
-        dd[IX(i)] = di;
-        inv[IX(i)] = nr_recip(di);
+        inv[i] = nr_recip(di);
     }
-    for (int i = 0; i < m; ++i) z[IX(i)] = start_value(j, i);
+    __syncwarp();
     for (int iter = 0; iter < 3; ++iter) {
         // solve L U x = z (dgttrs, no transpose)
-        for (int i = 0; i + 1 < m; ++i) {
-            if (ip[IX(i)] == i) {
-                z[IX(i + 1)] -= dl[IX(i)] * z[IX(i)];
-            } else {
-                const double t = z[IX(i)];
-                z[IX(i)] = z[IX(i + 1)];
-                z[IX(i + 1)] = t - dl[IX(i)] * z[IX(i)];
+        if (lane == 0) {
+            double zi = z[0];
+            for (int i = 0; i + 1 < m; ++i) {
+                const double f = dl[i], zn = z[i + 1];
+                if (ip[i] == i) {
+                    z[i] = zi;
+                    zi = zn - f * zi;
+                } else {
+                    z[i] = zn;
+                    zi = zi - f * zn;
+                }
+            }
+            double z1 = zi * inv[m - 1], z2 = 0.0;       // z[i + 1], z[i + 2]
+            z[m - 1] = z1;
+            if (m >= 2) {
+                z2 = z1;
+                z1 = (z[m - 2] - du[m - 2] * z2) * inv[m - 2];
+                z[m - 2] = z1;
+            }
+            for (int i = m - 3; i >= 0; --i) {
+                const double t = (z[i] - du[i] * z1 - du2[i] * z2) * inv[i];
+                z[i] = t;
+                z2 = z1;
+                z1 = t;
             }
         }
-        z[IX(m - 1)] *= inv[IX(m - 1)];
-        if (m >= 2) z[IX(m - 2)] = (z[IX(m - 2)] - du[IX(m - 2)] * z[IX(m - 1)]) * inv[IX(m - 2)];
-        for (int i = m - 3; i >= 0; --i)
-            z[IX(i)] = (z[IX(i)] - du[IX(i)] * z[IX(i + 1)] - du2[IX(i)] * z[IX(i + 2)]) * inv[IX(i)];
+        __syncwarp();
         double mx = 0;
-        for (int i = 0; i < m; ++i) mx = fmax(mx, fabs(z[IX(i)]));
+        for (int i = lane; i < m; i += 32) mx = fmax(mx, fabs(z[i]));
+        for (int o = 16; o; o >>= 1) mx = fmax(mx, __shfl_xor_sync(FULL, mx, o));
         const double sc = mx > 0 ? 1.0 / mx : 1.0;
-        for (int i = 0; i < m; ++i) z[IX(i)] *= sc;
+        for (int i = lane; i < m; i += 32) z[i] *= sc;
+        __syncwarp();
     }
-    double nn = 0;
-    for (int i = 0; i < m; ++i) nn = fma(z[IX(i)], z[IX(i)], nn);
+    double nn = 0;                                       // every lane the same chain
+    for (int i = 0; i < m; ++i) nn = fma(z[i], z[i], nn);
     const double sc = 1.0 / sqrt(nn);
     double *zo = Zt + (size_t)j * ldz;
-    for (int i = 0; i < m; ++i) zo[i] = z[IX(i)] * sc;
-#undef IX
+    for (int i = lane; i < m; i += 32) zo[i] = z[i] * sc;
 }
 
 // reorthogonalise inside clusters (gap <= 1e-3 ||T||_1, as dstein) by two
-// classical Gram-Schmidt passes, then normalise. One block, vectors in order;
-// with SMEM the nev vectors are worked on in shared memory (m * nev doubles).
+// classical Gram-Schmidt passes, then normalise; a block per cluster (the b-th run of
+// close eigenvalues to block b), vectors in order; with SMEM the cluster's vectors are
+// worked on in shared memory. m <= 1024: a thread per row. (All vectors in one block of
+// 1,024 threads spent 2.3 us on each, mostly barriers and a serial sum of 32 warps, although
+// most of them belong to no cluster: 73 us for 13 vectors of 30, here 12.)
 template <bool SMEM>
 __global__ void __launch_bounds__(1024)
 k_cluster_orth(int m, const double *__restrict__ d, const double *__restrict__ e, int nev,
@@ -1070,33 +1430,59 @@ k_cluster_orth(int m, const double *__restrict__ d, const double *__restrict__ e
 {
     extern __shared__ double zsm[];
     __shared__ double coef[1024];
-    __shared__ double s_tn;
     __shared__ double red[32];
+    __shared__ unsigned starts[32];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
-    double *Zt = Zg;
+    // ||T||: the largest row sum
+    double tn = 0;
+    for (int i = tid; i < m; i += blockDim.x)
+        tn = fmax(tn, fabs(d[i]) + (i > 0 ? fabs(e[i - 1]) : 0.0) + (i < m - 1 ? fabs(e[i]) : 0.0));
+    for (int o = 16; o; o >>= 1) tn = fmax(tn, __shfl_xor_sync(FULL, tn, o));
+    if (lane == 0) red[wid] = tn;
+    __syncthreads();
+    for (int q = 0; q < nw; ++q) tn = fmax(tn, red[q]);
+    const double ortol = 1e-3 * tn;
+    // the b-th run of eigenvalues: [first, end)
+    int first = -1, end = nev, seen = 0;
+    for (int j0 = 0; j0 < nev && first < 0; j0 += 1024) {
+        __syncthreads();
+        for (int w = wid; w < 32; w += nw) {
+            const int j = j0 + 32 * w + lane;
+            const unsigned b = __ballot_sync(FULL, j < nev && (j == 0 || eval[j] - eval[j - 1] > ortol));
+            if (lane == 0) starts[w] = b;
+        }
+        __syncthreads();
+        for (int w = 0; w < 32 && first < 0; ++w) {
+            unsigned b = starts[w];
+            const int c = __popc(b);
+            if (seen + c > (int)blockIdx.x) {
+                for (int q = blockIdx.x - seen; q > 0; --q) b &= b - 1;
+                first = j0 + 32 * w + __ffs(b) - 1;
+            }
+            seen += c;
+        }
+    }
+    if (first < 0) return;                               // fewer runs than blocks
+    for (int j = first + 1; j < nev; ++j)
+        if (eval[j] - eval[j - 1] > ortol) {
+            end = j;
+            break;
+        }
+    double *Zt = Zg + (size_t)first * ldz;
     long ld = ldz;
     if (SMEM) {
-        for (long t = tid; t < (long)m * nev; t += blockDim.x) zsm[t] = Zg[(t / m) * ldz + t % m];
+        for (int c = wid; c < end - first; c += nw)
+            for (int r = lane; r < m; r += 32) zsm[(size_t)c * m + r] = Zt[(size_t)c * ldz + r];
         Zt = zsm;
         ld = m;
     }
-    if (tid == 0) {
-        double t = 0;
-        for (int i = 0; i < m; ++i)
-            t = fmax(t, fabs(d[i]) + (i > 0 ? fabs(e[i - 1]) : 0.0) + (i < m - 1 ? fabs(e[i]) : 0.0));
-        s_tn = t;
-    }
     __syncthreads();
-    const double ortol = 1e-3 * s_tn;
-    int cs = 0;
-    for (int j = 0; j < nev; ++j) {
-        if (j > 0 && eval[j] - eval[j - 1] > ortol) cs = j;
-        double *zj = Zt + (size_t)j * ld;
-        const int np = j - cs;
+    for (int np = 0; np < end - first; ++np) {
+        double *zj = Zt + (size_t)np * ld;
         if (np > 0) {
             for (int pass = 0; pass < 2; ++pass) {
                 for (int q = wid; q < np; q += nw) {
-                    const double *zi = Zt + (size_t)(cs + q) * ld;
+                    const double *zi = Zt + (size_t)q * ld;
                     double s = 0;
                     for (int r = lane; r < m; r += 32) s = fma(zi[r], zj[r], s);
                     for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
@@ -1105,7 +1491,7 @@ k_cluster_orth(int m, const double *__restrict__ d, const double *__restrict__ e
                 __syncthreads();
                 for (int r = tid; r < m; r += blockDim.x) {
                     double acc = zj[r];
-                    for (int q = 0; q < np && q < 1024; ++q) acc -= coef[q] * Zt[(size_t)(cs + q) * ld + r];
+                    for (int q = 0; q < np && q < 1024; ++q) acc -= coef[q] * Zt[(size_t)q * ld + r];
                     zj[r] = acc;
                 }
                 __syncthreads();
@@ -1126,39 +1512,67 @@ k_cluster_orth(int m, const double *__restrict__ d, const double *__restrict__ e
         for (int r = tid; r < m; r += blockDim.x) zj[r] *= inv;
         __syncthreads();
     }
-    if (SMEM)
-        for (long t = tid; t < (long)m * nev; t += blockDim.x) Zg[(t / m) * ldz + t % m] = zsm[t];
-}
-
-// Z = Q Zt with Q = H_0 H_1 ... H_{m-3}; one warp per column, reflectors in reverse.
-__global__ void __launch_bounds__(256)
-k_backtransform(int m, const double *__restrict__ Aw, const double *__restrict__ tau, int nev,
-                const double *__restrict__ Zt, int ldzt, double *__restrict__ Z, int ldz)
-{
-    const int lane = threadIdx.x & 31;
-    const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (c >= nev) return;
-    double *z = Z + (size_t)c * ldz;
-    const double *zt = Zt + (size_t)c * ldzt;
-    for (int r = lane; r < m; r += 32) z[r] = zt[r];
-    __syncwarp();
-    for (int i = m - 3; i >= 0; --i) {
-        const double t = tau[i];
-        if (t == 0.0) continue;
-        const double *v = Aw + (size_t)i * m;   // v[i+1] = 1, v[i+2:] stored
-        double s = 0;
-        for (int r = i + 1 + lane; r < m; r += 32) s = fma(r == i + 1 ? 1.0 : v[r], z[r], s);
-        for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
-        const double f = t * s;
-        for (int r = i + 1 + lane; r < m; r += 32) z[r] -= f * (r == i + 1 ? 1.0 : v[r]);
-        __syncwarp();
+    if (SMEM) {
+        double *Zo = Zg + (size_t)first * ldz;
+        for (int c = wid; c < end - first; c += nw)
+            for (int r = lane; r < m; r += 32) Zo[(size_t)c * ldz + r] = zsm[(size_t)c * m + r];
     }
 }
 
-__global__ void k_check_finite(int m, int nev, const double *Z, int ldz, int *info)
+// Z = Q Zt with Q = H_0 H_1 ... H_{m-3}; a block of one warp per column (its FP64
+// chain alone on an SM), reflectors in reverse. The vector stays in shared memory and
+// the next BT_AHEAD reflectors are on their way there (with both in global memory a step
+// waited for two trips to L2: 33 us for 13 vectors of 30, here 22). A non-finite result
+// sets info.
+#define BT_AHEAD 4
+__device__ __forceinline__ void bt_fetch(double *slot, const double *v, int i, int m)
 {
-    for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < (long)m * nev; t += (long)gridDim.x * blockDim.x)
-        if (!isfinite(Z[(t % m) + (t / m) * (long)ldz])) atomicExch(info, 2);
+    for (int r = i + 2 + (int)threadIdx.x; r < m; r += 32)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(slot + r)),
+                     "l"(v + r)
+                     : "memory");
+}
+__global__ void __launch_bounds__(32)
+k_backtransform(int m, const double *__restrict__ Aw, const double *__restrict__ tau, int nev,
+                const double *__restrict__ Zt, int ldzt, double *__restrict__ Z, int ldz, int *info)
+{
+    extern __shared__ double bsm[];                      // z, then BT_AHEAD + 1 reflectors
+    const int lane = threadIdx.x, c = blockIdx.x;
+    double *z = bsm, *ring = bsm + m;
+    const double *zt = Zt + (size_t)c * ldzt;
+    for (int q = 0; q < BT_AHEAD; ++q) {
+        const int i = m - 3 - q;
+        if (i >= 0) bt_fetch(ring + (size_t)q * m, Aw + (size_t)i * m, i, m);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    for (int r = lane; r < m; r += 32) z[r] = zt[r];
+    __syncwarp();
+    int slot = 0, fill = BT_AHEAD;
+    for (int i = m - 3; i >= 0; --i) {
+        const int ahead = i - BT_AHEAD;
+        if (ahead >= 0) bt_fetch(ring + (size_t)fill * m, Aw + (size_t)ahead * m, ahead, m);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const double t = tau[i];
+        asm volatile("cp.async.wait_group %0;" ::"n"(BT_AHEAD) : "memory");
+        __syncwarp();
+        const double *v = ring + (size_t)slot * m;       // v[i+1] = 1, v[i+2:] stored
+        if (t != 0.0) {
+            double s = 0;
+            for (int r = i + 1 + lane; r < m; r += 32) s = fma(r == i + 1 ? 1.0 : v[r], z[r], s);
+            for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
+            const double f = t * s;
+            for (int r = i + 1 + lane; r < m; r += 32) z[r] -= f * (r == i + 1 ? 1.0 : v[r]);
+        }
+        __syncwarp();
+        slot = slot == BT_AHEAD ? 0 : slot + 1;
+        fill = fill == BT_AHEAD ? 0 : fill + 1;
+    }
+    bool bad = false;
+    for (int r = lane; r < m; r += 32) {
+        bad |= !isfinite(z[r]);
+        Z[r + (size_t)c * ldz] = z[r];
+    }
+    if (bad) atomicExch(info, 2);
 }
 
 // Reorthogonalisation of many inverse-iteration vectors by Cholesky-QR.
@@ -1189,8 +1603,7 @@ static int cholqr_reorth(gcge_gpu_ctx *ctx, int m, int nev, double *Zt, double *
         double *src = pass == 0 ? Zt : Zq, *dst = pass == 0 ? Zq : Zt;
         int st = gb_small_gemm(ctx, 'T', 'N', nev, nev, m, 1.0, src, m, src, m, 0.0, G, nev);
         if (st) return st;
-        GB_LAUNCH(ctx, k_chol_deflate, 1, 512, 2 * nev * sizeof(int), nev, G, nev, Tq, kept_dev, 0.0, 1e-10, cw,
-                  cw + (size_t)nev * nev, ratio_dev);
+        if ((st = cd_launch(ctx, nev, G, nev, Tq, kept_dev, 0.0, 1e-10, cw, ratio_dev))) return st;
         struct { int kept; int pad; double ratio; } h = {0, 0, 0.0};
         if (cudaMemcpyAsync(&h.kept, kept_dev, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess ||
             cudaMemcpyAsync(&h.ratio, ratio_dev, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess ||
@@ -1237,26 +1650,23 @@ extern "C" int gb_syevx_guess(gcge_gpu_ctx *ctx, int m, const double *H, int ldh
         static bool td_attr = false;
         if (!td_attr) {
             if (cudaFuncSetAttribute(k_tridiag_smem, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)td_smem_bytes(TD_SMEM_MAX_M)) != cudaSuccess)
+                                     (int)td_smem_bytes(TD_SMEM_MAX_M)) != cudaSuccess ||
+                cudaFuncSetAttribute(k_tridiag_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)ts_smem_bytes(TS_MAX_M)) != cudaSuccess)
                 return gb_fail(ctx, GCGE_GPU_ERR_CUDA);
             td_attr = true;
         }
-        if (m <= TD_SMEM_MAX_M)
+        if (m <= TS_MAX_M)
+            GB_LAUNCH(ctx, k_tridiag_small, 1, TS_THREADS, ts_smem_bytes(m), m, H, ldh, Aw, d, e, tau);
+        else if (m <= TD_SMEM_MAX_M)
             GB_LAUNCH(ctx, k_tridiag_smem, 1, tthreads, td_smem_bytes(m), m, H, ldh, Aw, d, e, tau);
         else
             GB_LAUNCH(ctx, k_tridiag, 1, tthreads, 2 * m * sizeof(double), m, H, ldh, Aw, d, e, tau);
     }
-    const int warps_per_block = 1;     // one eigenvalue per SM: the Sturm chains use the FP64 pipe
     GB_PROF(ctx, GB_K_EIG, 0.0, 0.0);
-    GB_LAUNCH(ctx, k_bisect, (nev + warps_per_block - 1) / warps_per_block, 32 * warps_per_block,
-              2 * m * sizeof(double), m, d, e, il, iu, eval, info_dev, guess);
+    GB_LAUNCH(ctx, k_bisect, nev, 32 * BI_WARPS, 2 * m * sizeof(double), m, d, e, il, iu, eval, info_dev, guess);
     GB_PROF(ctx, GB_K_EIG, 0.0, 0.0);
-    // inverse iteration: one eigenvalue per one-warp block, so that the chains spread
-    // over the SMs (the FP64 pipe of an SM is narrow: chains sharing one SM queue
-    // on it); working arrays in shared memory
-    const size_t per_eig = (size_t)m * (6 * sizeof(double) + sizeof(int));
-    const int IV = 1;
-    const size_t ismem = per_eig * IV;
+    const size_t ismem = (size_t)m * (6 * sizeof(double) + sizeof(int));
     // the 48 KB default covers static + dynamic shared memory together: both kernels
     // are opened once to the most they can ask for (k_invit <= 156 KB at m = 3000,
     // k_cluster_orth<true> <= 160 KB + its 8.3 KB static)
@@ -1264,11 +1674,12 @@ extern "C" int gb_syevx_guess(gcge_gpu_ctx *ctx, int m, const double *H, int ldh
     if (!attrs) {
         if (cudaFuncSetAttribute(k_invit, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess ||
             cudaFuncSetAttribute(k_cluster_orth<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) !=
-                cudaSuccess)
+                cudaSuccess ||
+            cudaFuncSetAttribute(k_backtransform, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess)
             return gb_fail(ctx, GCGE_GPU_ERR_CUDA);
         attrs = true;
     }
-    GB_LAUNCH(ctx, k_invit, (nev + IV - 1) / IV, 32, ismem, m, d, e, nev, eval, Zt, m, IV);
+    GB_LAUNCH(ctx, k_invit, nev, 32, ismem, m, d, e, nev, eval, Zt, m);
     GB_PROF(ctx, GB_K_EIG, 0.0, 0.0);
     int reorth_done = 0;
     if (nev >= CQ_MIN_NEV) {
@@ -1276,15 +1687,16 @@ extern "C" int gb_syevx_guess(gcge_gpu_ctx *ctx, int m, const double *H, int ldh
         if (st) return st;
     }
     const size_t osmem = sizeof(double) * (size_t)m * nev;
+    const int othreads = m > 1024 ? 1024 : (m + 31) / 32 * 32;
     if (reorth_done) {
         // the vectors are orthonormal: Cholesky-QR over all of them
     } else if (osmem <= 160 * 1024) {
-        GB_LAUNCH(ctx, k_cluster_orth<true>, 1, 1024, osmem, m, d, e, nev, eval, Zt, m);
+        GB_LAUNCH(ctx, k_cluster_orth<true>, nev, othreads, osmem, m, d, e, nev, eval, Zt, m);
     } else {
-        GB_LAUNCH(ctx, k_cluster_orth<false>, 1, 1024, 0, m, d, e, nev, eval, Zt, m);
+        GB_LAUNCH(ctx, k_cluster_orth<false>, nev, othreads, 0, m, d, e, nev, eval, Zt, m);
     }
     GB_PROF(ctx, GB_K_EIG, 0.0, 0.0);
-    GB_LAUNCH(ctx, k_backtransform, (nev * 32 + 255) / 256, 256, 0, m, Aw, tau, nev, Zt, m, Z, ldz);
-    GB_LAUNCH(ctx, k_check_finite, 64, 256, 0, m, nev, Z, ldz, info_dev);
+    GB_LAUNCH(ctx, k_backtransform, nev, 32, sizeof(double) * (size_t)m * (BT_AHEAD + 2), m, Aw, tau, nev, Zt, m, Z, ldz,
+              info_dev);
     return GCGE_GPU_OK;
 }

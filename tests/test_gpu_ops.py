@@ -347,3 +347,20 @@ def test_bcg_fp64_on_the_sides_of_its_forms(ctx, shape, k, rounds, rate):
     assert rel(out[0][0], x) < 1e-11
     assert np.linalg.norm(out[0][1] - res) < 1e-11 * np.linalg.norm(R0)
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("n,k,dep", [(400, 1, 0), (400, 33, 4), (900, 129, 7), (900, 160, 0), (900, 161, 5), (2500, 250, 9)])
+def test_orthonormalize_widths(ctx, n, k, dep):
+    """Blocks at the sides of the Cholesky's forms (a warp's columns, all of a block's, the
+    widest in shared memory and the first past it), with columns that repeat others: the
+    kept ones are orthonormal to a few roundings a row and span the rest."""
+    rng = np.random.default_rng(k)
+    W0 = rng.standard_normal((n, k))
+    for i in range(dep):
+        W0[:, k - 1 - 2 * i] = W0[:, i] * 2.0 - W0[:, i + 1]
+    w = ctx.multivec(n, k, W0)
+    end = G.orthonormalize(w, 0, k)
+    assert end == k - dep
+    Q = w.download(0, end)
+    assert np.max(np.abs(Q.T @ Q - np.eye(end))) < 1e-13
+    assert np.linalg.norm(W0 - Q @ (Q.T @ W0)) < 1e-11 * np.linalg.norm(W0)

@@ -179,6 +179,34 @@ def test_table_dense_eigensolver_matches_lapack(env, m):
         assert abs(abs(Z[j, :m] @ U[:, j]) - 1.0) < 1e-10
 
 
+@pytest.mark.parametrize("m,split", [(1, 0), (2, 0), (3, 0), (32, 0), (33, 0), (34, 1), (64, 0), (65, 1), (97, 0), (127, 1)])
+def test_table_dense_eigensolver_widths(env, m, split):
+    """Every eigenpair at the sides of the small reduction's rows a warp, and where the matrix
+    all but splits into a diagonal part and the rest (a Rayleigh-Ritz matrix near
+    convergence): residuals and orthogonality to a modest multiple of m eps ||M||."""
+    ctx, tab = env
+    rng = np.random.default_rng(100 + m)
+    M = rng.standard_normal((m, m))
+    M = M + M.T
+    if split:
+        h = m // 2
+        M[:h, :h] = np.diag(np.sort(rng.uniform(1.0, 2.0, h)))
+        M[:h, h:] *= 1e-9
+        M[h:, :h] = M[:h, h:].T
+    a = np.ascontiguousarray(M.T)
+    ev, Z = np.zeros(m), np.zeros((m, m))
+    nev, info, dummy = C.c_int(), C.c_int(), C.c_double()
+    iv = lambda v: C.byref(C.c_int(v))  # noqa: E731
+    tab.DenseMatEigenSolver(b"V", b"I", b"U", iv(m), a.ctypes.data_as(PD), iv(m), C.byref(dummy), C.byref(dummy), iv(1),
+                            iv(m), C.byref(dummy), C.byref(nev), ev.ctypes.data_as(PD), Z.ctypes.data_as(PD), iv(m), None,
+                            None, iv(8 * m), None, None, None, C.byref(info))
+    assert info.value == 0 and nev.value == m
+    scale = max(1.0, np.abs(M).sum(1).max())
+    assert np.max(np.abs(M @ Z.T - Z.T * ev)) <= 1e-13 * m * scale
+    assert np.max(np.abs(Z @ Z.T - np.eye(m))) <= 1e-11
+    assert np.max(np.abs(ev - np.linalg.eigvalsh(M))) <= 1e-13 * m * scale
+
+
 def test_table_linear_solver_hook(env):
     """GCGE_GPU_OpsSetLinearSolver installs a device Jacobi-preconditioned CG in the
     table's LinearSolver member (the hook GCGE calls per W column in place of its
