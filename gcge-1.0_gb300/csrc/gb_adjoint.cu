@@ -14,20 +14,13 @@
 // which GCGE_GPU_PatternGrad evaluates; GCGE_GPU_EigvecAdjoint computes mu.
 #include "gb_coop.h"
 #include "gb_internal.h"
+#include "gb_launch.h"
 
 #include <cuda_runtime.h>
 #include <float.h>
 #include <math.h>
 #include <stdlib.h>
 #include <string.h>
-
-#define GB_LAUNCH(ctx, kern, grid, block, smem, ...)                                   \
-    do {                                                                               \
-        kern<<<(grid), (block), (smem), (ctx)->stream>>>(__VA_ARGS__);                 \
-        (ctx)->launches++;                                                             \
-        int _st = gb_check_launch(ctx);                                                \
-        if (_st) return _st;                                                           \
-    } while (0)
 
 #define AD_CUDA(ctx, call)                                                             \
     do {                                                                               \
@@ -55,6 +48,7 @@ k_pattern_grad(int n, const int *__restrict__ rp, const int *__restrict__ ci, co
                long ldu, const double *__restrict__ V, long ldv, int r, const double *__restrict__ s, int acc,
                double *__restrict__ grad, int rows)
 {
+    GB_PDL();
     extern __shared__ double us[];      // [rows][r | 1]
     __shared__ unsigned char row_of[PG_CHUNK];
     __shared__ int first[PG_ROWS + 1];
@@ -167,6 +161,7 @@ static int av_grid(gcge_gpu_ctx *ctx, long work)
 // y = a x + b y (b == 0: y = a x, y not read)
 __global__ void k_av_axpby(long n, double a, const double *__restrict__ x, double b, double *__restrict__ y)
 {
+    GB_PDL();
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
         y[i] = b == 0.0 ? a * x[i] : fma(a, x[i], b * y[i]);
 }
@@ -175,6 +170,7 @@ __global__ void k_av_axpby(long n, double a, const double *__restrict__ x, doubl
 __global__ void __launch_bounds__(AV_THREADS)
 k_av_dot_part(long n, const double *__restrict__ x, const double *__restrict__ y, double *__restrict__ part)
 {
+    GB_PDL();
     __shared__ double red[AV_THREADS / 32];
     double s = 0.0;
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
@@ -193,6 +189,7 @@ k_av_dot_part(long n, const double *__restrict__ x, const double *__restrict__ y
 // out[0] = sum of nparts partials (one warp, fixed order)
 __global__ void k_av_sum(int nparts, const double *__restrict__ part, double *__restrict__ out)
 {
+    GB_PDL();
     double s = 0.0;
     for (int i = threadIdx.x; i < nparts; i += 32) s += part[i];
 #pragma unroll
@@ -206,6 +203,7 @@ __global__ void __launch_bounds__(AV_THREADS)
 k_av_xtv_part(long n, int m, const double *__restrict__ X, long ldx, const double *__restrict__ v,
               double *__restrict__ part)
 {
+    GB_PDL();
     __shared__ double red[AV_THREADS / 32][64];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     double s0 = 0.0, s1 = 0.0;
@@ -229,6 +227,7 @@ k_av_xtv_part(long n, int m, const double *__restrict__ X, long ldx, const doubl
 // c[j] = sum of the partials of column j (thread per column, fixed order)
 __global__ void k_av_xtv_sum(int nparts, int m, const double *__restrict__ part, double *__restrict__ c)
 {
+    GB_PDL();
     const int j = threadIdx.x;
     if (j >= m) return;
     double t = 0.0;
@@ -241,6 +240,7 @@ __global__ void __launch_bounds__(AV_THREADS)
 k_av_v_minus_xc(long n, int m, const double *__restrict__ X, long ldx, const double *__restrict__ c,
                 const double *__restrict__ v, double *__restrict__ y)
 {
+    GB_PDL();
     __shared__ double cs[64];
     if (threadIdx.x < m) cs[threadIdx.x] = c[threadIdx.x];
     __syncthreads();
@@ -540,6 +540,7 @@ __device__ __forceinline__ double ac_minus(const ac_args &a, const double *M, lo
 __global__ void __launch_bounds__(AC_ROWS, 4)
 k_adjoint_cg(const ac_args a)
 {
+    GB_PDL();
     __shared__ double red[AC_WARPS][64], tile[AC_ROWS], cs[64];
     const int n = a.n, m = a.m;
     const long stride = (long)gridDim.x * AC_ROWS, first = (long)blockIdx.x * AC_ROWS;

@@ -9,15 +9,8 @@
 #include <cuda_runtime.h>
 
 #include "gb_internal.h"
+#include "gb_launch.h"
 #include "gb_orth.h"
-
-#define GB_LAUNCH(ctx, kern, grid, block, smem, ...)                                   \
-    do {                                                                               \
-        kern<<<(grid), (block), (smem), (ctx)->stream>>>(__VA_ARGS__);                 \
-        (ctx)->launches++;                                                             \
-        int _st = gb_check_launch(ctx);                                                \
-        if (_st) return _st;                                                           \
-    } while (0)
 
 #define CUDA_TRY(ctx, call)                                                            \
     do {                                                                               \
@@ -369,6 +362,7 @@ extern "C" int GCGE_GPU_ProfileRead(gcge_gpu_ctx *ctx, int nclass, double *ms, l
 // ---------------------------------------------------------------- matrices
 __global__ void k_d2f_vals(long n, const double *a, float *b)
 {
+    GB_PDL();
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x)
         b[t] = (float)a[t];
 }
@@ -377,6 +371,7 @@ __global__ void k_d2f_vals(long n, const double *a, float *b)
 // decreases or a column lies outside [0, n); res[1] = the longest row
 __global__ void k_csr_check(int n, int nnz, const int *__restrict__ rp, const int *__restrict__ ci, int *res)
 {
+    GB_PDL();
     int bad = 0, mr = 0;
     const long stride = (long)gridDim.x * blockDim.x;
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -591,6 +586,7 @@ extern "C" int GCGE_GPU_MultiVecDestroy(gcge_gpu_mv *m)
 // column-major (ld n) <-> row-major block columns, through a tiled transpose
 __global__ void k_cm_to_rm(int n, int k, const double *__restrict__ src, double *__restrict__ dst, long ld)
 {
+    GB_PDL();
     __shared__ double t[32][33];
     const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
     for (int q = threadIdx.y; q < 32; q += blockDim.y) {
@@ -605,6 +601,7 @@ __global__ void k_cm_to_rm(int n, int k, const double *__restrict__ src, double 
 }
 __global__ void k_rm_to_cm(int n, int k, const double *__restrict__ src, long ld, double *__restrict__ dst)
 {
+    GB_PDL();
     __shared__ double t[32][33];
     const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
     for (int q = threadIdx.y; q < 32; q += blockDim.y) {
@@ -747,6 +744,7 @@ extern "C" int GCGE_GPU_MultiVecInnerProd(const gcge_gpu_mv *V, const gcge_gpu_m
 
 __global__ void k_swap_cols(int n, int k, double *A, long lda, double *B, long ldb)
 {
+    GB_PDL();
     const long total = (long)n * k;
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
         const long r = t / k;
@@ -993,6 +991,7 @@ extern "C" int gb_orth_kind(const char *t)
 __global__ void k_eig_inv_sqrt(int k, const double *__restrict__ Q, int ldq, const double *__restrict__ theta,
                                double tol, double *__restrict__ T, int ldt, int *__restrict__ kept)
 {
+    GB_PDL();
     __shared__ int f;
     if (threadIdx.x == 0) {
         const double rel = theta[k - 1] > 0.0 ? 1e-12 * theta[k - 1] : 0.0;

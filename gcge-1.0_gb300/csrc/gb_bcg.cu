@@ -21,6 +21,7 @@
 
 #include "gb_bcg.h"
 #include "gb_internal.h"
+#include "gb_launch.h"
 
 #define RED_ROWS 128
 
@@ -31,15 +32,6 @@ static inline int cdiv(long a, long b) { return (int)((a + b - 1) / b); }
 #define GB_PROF(ctx, cls, bytes, flops) \
     do { if ((ctx)->prof) gb_prof_begin((ctx), (cls), (bytes), (flops)); } while (0)
 
-#define GB_LAUNCH(ctx, kern, grid, block, smem, ...)                                   \
-    do {                                                                               \
-        kern<<<(grid), (block), (smem), (ctx)->stream>>>(__VA_ARGS__);                 \
-        (ctx)->launches++;                                                             \
-        if ((ctx)->prof) gb_prof_end(ctx);                                             \
-        int _st = gb_check_launch(ctx);                                                \
-        if (_st) return _st;                                                           \
-    } while (0)
-
 // warp-per-row loop over an n x k block: lanes walk the columns of one row
 #define ROWS_BY_WARP(n, r)                                                             \
     for (long r = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < (n);         \
@@ -47,29 +39,29 @@ static inline int cdiv(long a, long b) { return (int)((a + b - 1) / b); }
 
 // p = r + beta p on active columns (beta = 0 on the first round: p = r);
 // beta[c] = rho2[c] / rho1[c] was formed once per column by k_finalize
-template <typename T>
-__global__ void k_pupdate(int n, int k, const T *__restrict__ R, T *__restrict__ P, long ld,
+__global__ void k_pupdate(int n, int k, const float *__restrict__ R, float *__restrict__ P, long ld,
                           const double *__restrict__ beta, const int *__restrict__ nact, int first,
-                          const T *__restrict__ dinv)
+                          const float *__restrict__ dinv)
 {
+    GB_PDL();
     const int ka = min(*nact, k);
     if (ka <= 0) return;
     const int lane = threadIdx.x & 31;
     ROWS_BY_WARP(n, r)
     {
-        const T *rr = R + r * ld;
-        T *pr = P + r * ld;
-        const T dr = dinv ? dinv[r] : (T)1;                // z = D^-1 r (Jacobi) or r
-        for (int c = lane; c < ka; c += 32) pr[c] = first ? dr * rr[c] : dr * rr[c] + (T)beta[c] * pr[c];
+        const float *rr = R + r * ld;
+        float *pr = P + r * ld;
+        const float dr = dinv ? dinv[r] : 1.0f;            // z = D^-1 r (Jacobi) or r
+        for (int c = lane; c < ka; c += 32) pr[c] = first ? dr * rr[c] : dr * rr[c] + (float)beta[c] * pr[c];
     }
 }
 
 // partial sums of a*b over row slabs, active columns only
-template <typename T>
 __global__ void __launch_bounds__(256)
-k_dot_partial(int n, int k, const T *__restrict__ A, const T *__restrict__ B, long ld,
-              const int *__restrict__ nact, double *__restrict__ part, const T *__restrict__ wdiag = nullptr)
+k_dot_partial(int n, int k, const float *__restrict__ A, const float *__restrict__ B, long ld,
+              const int *__restrict__ nact, double *__restrict__ part, const float *__restrict__ wdiag)
 {
+    GB_PDL();
     __shared__ double sh[8][33];
     const int ka = nact ? *nact : k;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -79,7 +71,7 @@ k_dot_partial(int n, int k, const T *__restrict__ A, const T *__restrict__ B, lo
     if (c < k && c < ka) {
         long r = r0 + ty;
         while (r < r1) {
-            T run = 0;
+            float run = 0;
 #pragma unroll
             for (int q = 0; q < 8; ++q, r += 8)
                 if (r < r1) run = fma(A[r * ld + c], wdiag ? wdiag[r] * B[r * ld + c] : B[r * ld + c], run);
@@ -97,12 +89,12 @@ k_dot_partial(int n, int k, const T *__restrict__ A, const T *__restrict__ B, lo
 
 // x += alpha p, r -= alpha w (alpha = rho2/ptw) on active columns, with the
 // partial sums of the new r.r
-template <typename T>
 __global__ void __launch_bounds__(256)
-k_xr_update(int n, int k, T *__restrict__ X, T *__restrict__ R, const T *__restrict__ P,
-            const T *__restrict__ W, long ld, const double *__restrict__ alpha,
-            const int *__restrict__ nact, double *__restrict__ part, const T *__restrict__ dinv)
+k_xr_update(int n, int k, float *__restrict__ X, float *__restrict__ R, const float *__restrict__ P,
+            const float *__restrict__ W, long ld, const double *__restrict__ alpha,
+            const int *__restrict__ nact, double *__restrict__ part, const float *__restrict__ dinv)
 {
+    GB_PDL();
     __shared__ double sh[8][33];
     const int ka = *nact;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -110,16 +102,16 @@ k_xr_update(int n, int k, T *__restrict__ X, T *__restrict__ R, const T *__restr
     const long r0 = (long)blockIdx.x * RED_ROWS, r1 = min((long)n, r0 + RED_ROWS);
     double s = 0;
     if (c < k && c < ka) {
-        const T a = (T)alpha[c];
+        const float a = (float)alpha[c];
         long r = r0 + ty;
         while (r < r1) {
-            T run = 0;
+            float run = 0;
 #pragma unroll
             for (int q = 0; q < 8; ++q, r += 8) {
                 if (r < r1) {
                     const long o = r * ld + c;
                     X[o] = X[o] + a * P[o];
-                    const T rn = R[o] - a * W[o];
+                    const float rn = R[o] - a * W[o];
                     R[o] = rn;
                     run = fma(rn, dinv ? dinv[r] * rn : rn, run);   // r.z, z = D^-1 r or r
                 }
@@ -141,6 +133,7 @@ k_xr_update(int n, int k, T *__restrict__ X, T *__restrict__ R, const T *__restr
 __global__ void __launch_bounds__(256)
 k_colsum(int nblk, int k, const double *__restrict__ part, const int *__restrict__ nact, double *__restrict__ out)
 {
+    GB_PDL();
     __shared__ double sh[256];
     const int c = blockIdx.x;
     if (nact && c >= *nact) return;
@@ -159,6 +152,7 @@ k_colsum(int nblk, int k, const double *__restrict__ part, const int *__restrict
 __global__ void k_sum_active(int k, const int *__restrict__ nact, const double *__restrict__ ptw,
                              const double *__restrict__ rho2, double *__restrict__ alpha)
 {
+    GB_PDL();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= k || c >= *nact) return;
     alpha[c] = rho2[c] / ptw[c];
@@ -167,6 +161,7 @@ __global__ void k_sum_active(int k, const int *__restrict__ nact, const double *
 // initial residual norms: rho2 = column sums, err = sqrt(rho2), nact = k
 __global__ void k_init_state(int k, const double *__restrict__ sums, double *rho2, double *err, int *nact)
 {
+    GB_PDL();
     for (int c = threadIdx.x; c < k; c += blockDim.x) {
         rho2[c] = sums[c];
         err[c] = sqrt(sums[c]);
@@ -178,6 +173,7 @@ __global__ void k_init_state(int k, const double *__restrict__ sums, double *rho
 __global__ void k_finalize(int k, const double *__restrict__ sums, double *rho1, double *rho2,
                            const double *__restrict__ err, int *nact, double rate, double *beta)
 {
+    GB_PDL();
     __shared__ int cnt;
     const int ka = *nact;
     if (threadIdx.x == 0) cnt = 0;
@@ -199,6 +195,7 @@ __global__ void k_finalize(int k, const double *__restrict__ sums, double *rho1,
 // X += (double) D
 __global__ void k_add_f2d(int n, int k, const float *__restrict__ D, long ldd, double *__restrict__ X, long ldx)
 {
+    GB_PDL();
     const int lane = threadIdx.x & 31;
     ROWS_BY_WARP(n, r)
     for (int c = lane; c < k; c += 32) X[r * ldx + c] += (double)D[r * ldd + c];
@@ -289,6 +286,7 @@ k_pupdate_v(int n, int k, const float *__restrict__ R, float *__restrict__ P, lo
             const double *__restrict__ beta, const int *__restrict__ nact, int first,
             const float *__restrict__ dinv)
 {
+    GB_PDL();
     constexpr int RPB = VB_THREADS / TPR;
     const int ka = min(*nact, k);
     const int cg = threadIdx.x % TPR, rs = threadIdx.x / TPR;
@@ -340,6 +338,7 @@ k_xr_update_v(int n, int k, float *__restrict__ X, float *__restrict__ R, const 
               const float *__restrict__ W, long ld, const double *__restrict__ alpha, const int *__restrict__ nact,
               double *__restrict__ part, const float *__restrict__ dinv)
 {
+    GB_PDL();
     constexpr int RPB = VB_THREADS / TPR;
     const int ka = min(*nact, k);
     const int cg = threadIdx.x % TPR, rs = threadIdx.x / TPR;
@@ -394,6 +393,7 @@ k_spmm32_long(const int *__restrict__ rp, const int *__restrict__ ci, const floa
               const float *__restrict__ P, float *__restrict__ W, long ld, int k, const int *__restrict__ nact,
               double *__restrict__ part, int part_row0, const int *__restrict__ lrows, int nlong)
 {
+    GB_PDL();
     constexpr int RPB = VB_THREADS / L, COLS = 4 * L * NV, UNR = 4;
     __shared__ float rs[RPB * COLS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -467,6 +467,7 @@ k_spmm32_dot(int n, const int *__restrict__ rp, const int *__restrict__ ci, cons
              const float *__restrict__ P, float *__restrict__ W, long ld, int k, const int *__restrict__ nact,
              double *__restrict__ part, int lim)
 {
+    GB_PDL();
     constexpr int RPB = VB_THREADS / L, COLS = 4 * L * NV, UNR = 4;
     __shared__ double red[RPB][COLS + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -561,6 +562,7 @@ __global__ void __launch_bounds__(256)
 k_colsum_alpha(int nblk, int k, const double *__restrict__ part, const int *__restrict__ nact,
                const double *__restrict__ rho2, double *__restrict__ ptw, double *__restrict__ alpha)
 {
+    GB_PDL();
     __shared__ double sh[256];
     const int c = blockIdx.x;
     if (c >= *nact) return;
@@ -584,6 +586,7 @@ __global__ void __launch_bounds__(1024)
 k_colsum_finalize(int nblk, int k, const double *__restrict__ part, double *sums, double *rho1, double *rho2,
                   const double *__restrict__ err, int *nact, double rate, double *beta)
 {
+    GB_PDL();
     __shared__ int cnt;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ka = *nact;
@@ -688,15 +691,16 @@ static int bcg_rounds32_wide(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, float *R,
     dim3 rgrid(nblk, (k + 31) / 32);
     for (int it = 1; it < a->max_it; ++it) {
         GB_PROF(ctx, GB_K_BCGVEC, 12.0 * n * k, 2.0 * n * k);
-        GB_LAUNCH(ctx, k_pupdate<float>, row_grid(ctx, n), 256, 0, n, k, R, P, ld, s->beta, s->nact, it == 1, a->dinv32);
+        GB_LAUNCH(ctx, k_pupdate, row_grid(ctx, n), 256, 0, n, k, R, P, ld, s->beta, s->nact, it == 1, a->dinv32);
         int st = gb_spmm32(ctx, A, P, ld, W, ld, k, s->nact);
         if (st) return st;
         GB_PROF(ctx, GB_K_BCGVEC, 8.0 * n * k, 2.0 * n * k);
-        GB_LAUNCH(ctx, k_dot_partial<float>, rgrid, 256, 0, n, k, P, W, ld, s->nact, s->part);
+        GB_LAUNCH(ctx, k_dot_partial, rgrid, 256, 0, n, k, P, W, ld, s->nact, s->part,
+                  (const float *)nullptr);
         GB_LAUNCH(ctx, k_colsum, k, 256, 0, nblk, k, s->part, s->nact, s->ptw);
         GB_LAUNCH(ctx, k_sum_active, (k + 127) / 128, 128, 0, k, s->nact, s->ptw, s->rho2, s->alpha);
         GB_PROF(ctx, GB_K_BCGVEC, 24.0 * n * k, 6.0 * n * k);
-        GB_LAUNCH(ctx, k_xr_update<float>, rgrid, 256, 0, n, k, X, R, P, W, ld, s->alpha, s->nact, s->part, a->dinv32);
+        GB_LAUNCH(ctx, k_xr_update, rgrid, 256, 0, n, k, X, R, P, W, ld, s->alpha, s->nact, s->part, a->dinv32);
         GB_LAUNCH(ctx, k_colsum, k, 256, 0, nblk, k, s->part, s->nact, s->sums);
         GB_LAUNCH(ctx, k_finalize, 1, 256, 0, k, s->sums, s->rho1, s->rho2, s->err, s->nact, a->rate, s->beta);
     }
@@ -748,7 +752,7 @@ extern "C" int gb_bcg(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, double *RHS, lon
     if ((st = gb_convert_d2f(ctx, n, k, RHS, ldr, R, ld))) return st;
     if (cudaMemsetAsync(D, 0, (size_t)n * ld * sizeof(float), ctx->stream) != cudaSuccess)
         return gb_fail(ctx, GCGE_GPU_ERR_CUDA);
-    GB_LAUNCH(ctx, k_dot_partial<float>, dim3(nblk, (k + 31) / 32), 256, 0, n, k, R, R, ld, (const int *)nullptr, s.part,
+    GB_LAUNCH(ctx, k_dot_partial, dim3(nblk, (k + 31) / 32), 256, 0, n, k, R, R, ld, (const int *)nullptr, s.part,
               a->dinv32);
     GB_LAUNCH(ctx, k_colsum, k, 256, 0, nblk, k, s.part, (const int *)nullptr, s.sums);
     GB_LAUNCH(ctx, k_init_state, 1, 256, 0, k, s.sums, s.rho2, s.err, s.nact);
@@ -760,6 +764,7 @@ extern "C" int gb_bcg(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, double *RHS, lon
 
 __global__ void k_axpy32(int n, int k, float a, const float *__restrict__ X, float *__restrict__ Y, long ld)
 {
+    GB_PDL();
     const int lane = threadIdx.x & 31;
     ROWS_BY_WARP(n, r)
     for (int c = lane; c < k; c += 32) Y[r * ld + c] += a * X[r * ld + c];
@@ -777,6 +782,7 @@ extern "C" int gb_axpy32(gcge_gpu_ctx *ctx, int n, int k, float a, const float *
 __global__ void k_diag_inv(int n, const int *__restrict__ rp, const int *__restrict__ ci,
                            const double *__restrict__ v, double *__restrict__ dinv, float *__restrict__ dinv32)
 {
+    GB_PDL();
     for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (long)gridDim.x * blockDim.x) {
         double dg = 0.0;
         for (int e = rp[r]; e < rp[r + 1]; ++e)

@@ -30,6 +30,7 @@
 #include "gb_bcg.h"
 #include "gb_coop.h"
 #include "gb_internal.h"
+#include "gb_launch.h"
 
 #define PB_THREADS 256
 #define PB_WARPS (PB_THREADS / 32)
@@ -293,6 +294,7 @@ template <int L, int Q, bool FUSED>
 __global__ void __launch_bounds__(PB_THREADS, 3)
 k_bcg_persist(const pb_args a)
 {
+    GB_PDL();
     constexpr int RPB = PB_THREADS / L, C = L * Q;
     __shared__ double red[16][C];
     __shared__ double sh[PB_THREADS];

@@ -15,19 +15,11 @@
 #include <cuda_runtime.h>
 
 #include "gb_internal.h"
+#include "gb_launch.h"
 
 #define FULL 0xffffffffu
 
 static inline int ceil_div_l(long a, long b) { return (int)((a + b - 1) / b); }
-
-#define GB_LAUNCH(ctx, kern, grid, block, smem, ...)                                   \
-    do {                                                                               \
-        kern<<<(grid), (block), (smem), (ctx)->stream>>>(__VA_ARGS__);                 \
-        (ctx)->launches++;                                                             \
-        if ((ctx)->prof) gb_prof_end(ctx);                                             \
-        int _st = gb_check_launch(ctx);                                                \
-        if (_st) return _st;                                                           \
-    } while (0)
 
 // profile the next launch (no-op unless profiling is enabled on the context)
 #define GB_PROF(ctx, cls, bytes, flops) \
@@ -41,6 +33,7 @@ k_spmm(int n, const int *__restrict__ rp, const int *__restrict__ ci, const VT *
        const XT *__restrict__ X, long ldx, XT *__restrict__ Y, long ldy, int k, AT alpha,
        const double *__restrict__ alpha_col, AT beta, const int *__restrict__ ncols_dev)
 {
+    GB_PDL();
     const int lane = threadIdx.x & 31;
     const long warp = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nchunks = (k + 63) >> 6;
@@ -95,6 +88,7 @@ k_spmm_vec(int n, const int *__restrict__ rp, const int *__restrict__ ci, const 
            const T *__restrict__ X, long ldx, T *__restrict__ Y, long ldy, int k, T alpha,
            const double *__restrict__ alpha_col, T beta, const int *__restrict__ ncols_dev)
 {
+    GB_PDL();
     typedef typename vec16<T>::type V;
     constexpr int VW = 16 / sizeof(T);
     constexpr int RPW = 32 / L;
@@ -175,6 +169,7 @@ k_spmv(int n, const int *__restrict__ rp, const int *__restrict__ ci, const VT *
        const XT *__restrict__ X, long ldx, XT *__restrict__ Y, long ldy, AT alpha,
        const double *__restrict__ alpha_col, AT beta, const int *__restrict__ ncols_dev)
 {
+    GB_PDL();
     const int lane = threadIdx.x & 31;
     const long row = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (row >= n) return;
@@ -243,6 +238,7 @@ k_spmm64_lv(int n, const int *__restrict__ rp, const int *__restrict__ ci, const
             const double *__restrict__ X, long ldx, double *__restrict__ Y, long ldy, int k, double alpha,
             const double *__restrict__ alpha_col, double beta, const int *__restrict__ ncols_dev)
 {
+    GB_PDL();
     constexpr int RPW = 32 / L;
     const int lane = threadIdx.x & 31;
     const int sub = lane / L, sl = lane % L;
@@ -305,6 +301,7 @@ __device__ __forceinline__ double pair_f2d(float f, int s)
 __global__ void __launch_bounds__(256)
 k_pair_split(int n, int k, const double *__restrict__ X, long ldx, float2 *__restrict__ Xs, int *flag, int epoch)
 {
+    GB_PDL();
     int bad = 0;
     const int lane = threadIdx.x & 31, c = blockIdx.y * 32 + lane;
     const int rstride = gridDim.x * (blockDim.x >> 5);
@@ -317,6 +314,7 @@ k_pair_split(int n, int k, const double *__restrict__ X, long ldx, float2 *__res
 // matrix values: max |a| (as ordered bits of a non-negative double), then the split
 __global__ void k_pair_absmax(int nnz, const double *__restrict__ v, unsigned long long *meta)
 {
+    GB_PDL();
     unsigned long long m = 0;
     for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += (long)gridDim.x * blockDim.x) {
         const unsigned long long b = (unsigned long long)__double_as_longlong(fabs(v[e]));
@@ -331,6 +329,7 @@ __global__ void k_pair_absmax(int nnz, const double *__restrict__ v, unsigned lo
 
 __global__ void k_pair_vals(int nnz, const double *__restrict__ v, float2 *__restrict__ vp, int *meta)
 {
+    GB_PDL();
     const unsigned long long mb = *(const unsigned long long *)meta;
     // s with max |a| 2^-s in [0.5, 1); s = 0 for an all-zero matrix; non-finite
     // values or |s| > 700 leave s = 4096, which sends every product to the FP64 loop
@@ -356,6 +355,7 @@ k_spmm_pair(int n, const int *__restrict__ rp, const int *__restrict__ ci, const
             const double *__restrict__ X, long ldx, double *__restrict__ Y, long ldy, int k,
             const int *__restrict__ flag, int epoch)
 {
+    GB_PDL();
     constexpr int RPW = 32 / L;
     const int lane = threadIdx.x & 31;
     const int sub = lane / L, sl = lane % L;
@@ -655,6 +655,7 @@ extern "C" int gb_spmm32(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, const float *
 __global__ void k_axpby(int n, int k, double a, const double *__restrict__ X, long ldx, double b,
                         double *__restrict__ Y, long ldy)
 {
+    GB_PDL();
     const int lane = threadIdx.x & 31;
     ROWS_BY_WARP(n, r)
     for (int c = lane; c < k; c += 32) {
@@ -713,6 +714,7 @@ __device__ __forceinline__ void gather_setup(int k, const int *idx, const double
 __global__ void k_gather_cols(int n, int k, const double *__restrict__ X, long ldx, const int *__restrict__ idx,
                               double *__restrict__ Y, long ldy, const double *__restrict__ eval, int mode)
 {
+    GB_PDL();
     extern __shared__ double gsm[];
     double *ss = gsm;
     int *si = (int *)(gsm + k);
@@ -743,6 +745,7 @@ __global__ void k_w_residual(int n, int k, const double *__restrict__ AX, long l
                              const double *__restrict__ BX, long ldbx, const int *__restrict__ bi,
                              const double *__restrict__ lam, double *__restrict__ R, long ldr)
 {
+    GB_PDL();
     extern __shared__ double gsm[];
     double *ss = gsm;
     int *si = (int *)(gsm + k);
@@ -768,6 +771,7 @@ extern "C" int gb_w_residual(gcge_gpu_ctx *ctx, int n, int k, const double *AX, 
 
 __global__ void k_fill_random(int n, int k, double *X, long ldx, int col0, unsigned long long seed)
 {
+    GB_PDL();
     const long total = (long)n * k;
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
         const long r = t / k;
@@ -791,12 +795,14 @@ extern "C" int gb_fill_random(gcge_gpu_ctx *ctx, int n, int k, double *X, long l
 
 __global__ void k_d2f(int n, int k, const double *__restrict__ X, long ldx, float *__restrict__ Y, long ldy)
 {
+    GB_PDL();
     const int lane = threadIdx.x & 31;
     ROWS_BY_WARP(n, r)
     for (int c = lane; c < k; c += 32) Y[r * ldy + c] = (float)X[r * ldx + c];
 }
 __global__ void k_f2d(int n, int k, const float *__restrict__ X, long ldx, double *__restrict__ Y, long ldy)
 {
+    GB_PDL();
     const int lane = threadIdx.x & 31;
     ROWS_BY_WARP(n, r)
     for (int c = lane; c < k; c += 32) Y[r * ldy + c] = (double)X[r * ldx + c];
@@ -819,6 +825,7 @@ extern "C" int gb_convert_f2d(gcge_gpu_ctx *ctx, int n, int k, const float *X, l
 __global__ void k_dirichlet(int n, const int *arp, const double *av, const int *brp, const double *bv, int k,
                             double *X, long ldx)
 {
+    GB_PDL();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         bool zero_b = true;
         for (int j = brp[i]; j < brp[i + 1]; ++j)
@@ -851,8 +858,9 @@ template <int MODE, bool THIN>
 __global__ void __launch_bounds__(THIN ? 32 : 256)
 k_coldot_partial(int n, int k, const double *__restrict__ X, long ldx, const double *__restrict__ Y, long ldy,
                  const double *__restrict__ Z, long ldz, const double *__restrict__ eval,
-                 const int *__restrict__ idx, double *__restrict__ part, int bnorm = 0)
+                 const int *__restrict__ idx, double *__restrict__ part, int bnorm)
 {
+    GB_PDL();
     // MODE 0: sum X*Y. MODE 1: residual triple (sum (Y - l Z)^2, sum X^2, sum Z^2), Z may be NULL (= X);
     // bnorm != 0 ("BR": only the residual and the B-norm are used) skips X (when Z is given) and sum X^2
     // (reported as sum Z^2): three FP64 operations per entry instead of four, the FP64 pipe being the
@@ -913,6 +921,7 @@ k_coldot_partial(int n, int k, const double *__restrict__ X, long ldx, const dou
 // classes: 1, or 8 for the thin form's partials
 __global__ void k_sum_partials(int nblk, int width, int classes, const double *__restrict__ part, double *__restrict__ out)
 {
+    GB_PDL();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= width) return;
     double s = 0;
@@ -944,10 +953,10 @@ extern "C" int gb_col_dots(gcge_gpu_ctx *ctx, int n, int k, const double *X, lon
     GB_PROF(ctx, GB_K_REDUCE, 16.0 * n * k, 2.0 * n * k);
     if (thin)
         GB_LAUNCH(ctx, (k_coldot_partial<0, true>), grid, 32, 0, n, k, X, ldx, Y, ldy, (const double *)nullptr, 0L,
-                  (const double *)nullptr, (const int *)nullptr, ctx->scratch);
+                  (const double *)nullptr, (const int *)nullptr, ctx->scratch, 0);
     else
         GB_LAUNCH(ctx, (k_coldot_partial<0, false>), grid, 256, 0, n, k, X, ldx, Y, ldy, (const double *)nullptr, 0L,
-                  (const double *)nullptr, (const int *)nullptr, ctx->scratch);
+                  (const double *)nullptr, (const int *)nullptr, ctx->scratch, 0);
     GB_LAUNCH(ctx, k_sum_partials, (k + 31) / 32, 32, 0, nblk, k, thin ? 8 : 1, ctx->scratch, out_dev);
     return GCGE_GPU_OK;
 }
@@ -979,8 +988,9 @@ extern "C" int gb_residual_norms(gcge_gpu_ctx *ctx, int n, int k, const double *
 __global__ void __launch_bounds__(256)
 k_gram_partial(int n, int k1, int k2, const double *__restrict__ V, long ldv, const double *__restrict__ W,
                long ldw, double *__restrict__ part, long rows_per_split, int sym,
-               const int *__restrict__ run = nullptr)
+               const int *__restrict__ run)
 {
+    GB_PDL();
     const int ti = blockIdx.x, tj = blockIdx.y, split = blockIdx.z;
     if (sym && ti > tj) return;
     if (run && !*run) return;                              // the tensor-core form has the product
@@ -1019,8 +1029,9 @@ k_gram_partial(int n, int k1, int k2, const double *__restrict__ V, long ldv, co
 }
 
 __global__ void k_gram_reduce(int k1, int k2, int nsplit, const double *__restrict__ part, double *a, int lda,
-                              int sym, const int *__restrict__ run = nullptr)
+                              int sym, const int *__restrict__ run)
 {
+    GB_PDL();
     if (run && !*run) return;
     const long total = (long)k1 * k2;
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
@@ -1059,9 +1070,9 @@ extern "C" int gb_gram(gcge_gpu_ctx *ctx, int n, int k1, int k2, const double *V
     if (st) return st;
     dim3 grid(ti, tj, (unsigned)nsplit);
     GB_PROF(ctx, GB_K_GRAM, 8.0 * n * (k1 + k2), sym ? 1.0 * n * k1 * (k1 + 1) : 2.0 * n * k1 * k2);
-    GB_LAUNCH(ctx, k_gram_partial, grid, 256, 0, n, k1, k2, V, ldv, W, ldw, ctx->scratch, rps, sym);
+    GB_LAUNCH(ctx, k_gram_partial, grid, 256, 0, n, k1, k2, V, ldv, W, ldw, ctx->scratch, rps, sym, nullptr);
     GB_LAUNCH(ctx, k_gram_reduce, elem_grid(ctx, (long)k1 * k2), 256, 0, k1, k2, (int)nsplit, ctx->scratch,
-              a_dev, lda, sym);
+              a_dev, lda, sym, nullptr);
     return GCGE_GPU_OK;
 }
 
@@ -1071,6 +1082,7 @@ __global__ void __launch_bounds__(256)
 k_lincomb(int n, int k1, int k2, const double *__restrict__ X, long ldx, const double *__restrict__ C, int ldc,
           double alpha, double beta, double *__restrict__ Y, long ldy, int upper)
 {
+    GB_PDL();
     __shared__ double Xs[64][33];
     __shared__ double Cs[32][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -1135,6 +1147,7 @@ extern "C" int gb_lincomb(gcge_gpu_ctx *ctx, int n, int k1, int k2, const double
 // Frobenius norm of a small column-major block (one block, fixed order)
 __global__ void k_frobenius(int m, int n, const double *a, int lda, double *out)
 {
+    GB_PDL();
     __shared__ double sh[256];
     double s = 0;
     for (long t = threadIdx.x; t < (long)m * n; t += 256) {
@@ -1158,6 +1171,7 @@ extern "C" int gb_frobenius(gcge_gpu_ctx *ctx, int m, int n, const double *a, in
 // out[c] = src[idx[c]] (eigenvalues of the unlocked columns)
 __global__ void k_select(int k, const double *src, const int *idx, double *out)
 {
+    GB_PDL();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c < k) out[c] = src[idx[c]];
 }
@@ -1172,6 +1186,7 @@ extern "C" int gb_select(gcge_gpu_ctx *ctx, int k, const double *src, const int 
 __global__ void k_scale_cols(int n, int k, const double *__restrict__ X, long ldx, const double *__restrict__ s,
                              double *Y, long ldy)
 {
+    GB_PDL();
     const int lane = threadIdx.x & 31;
     ROWS_BY_WARP(n, r)
     for (int c = lane; c < k; c += 32) Y[r * ldy + c] = s[c] * X[r * ldx + c];
@@ -1219,7 +1234,7 @@ extern "C" int gb_gram_fixed_partials(cudaStream_t stream, int num_sms, int n, i
     *st = nsplit ? GCGE_GPU_OK : GCGE_GPU_ERR_ARG;
     if (!nsplit) return 0;
     dim3 grid((k1 + 31) / 32, (k2 + 31) / 32, (unsigned)nsplit);
-    k_gram_partial<<<grid, 256, 0, stream>>>(n, k1, k2, V, ldv, W, ldw, part, rps, sym, run);
+    gb_launch(stream, grid, 256, 0, k_gram_partial, n, k1, k2, V, ldv, W, ldw, part, rps, sym, run);
     if (cudaGetLastError() != cudaSuccess) *st = GCGE_GPU_ERR_CUDA;
     return *st ? 0 : (int)nsplit;
 }
@@ -1230,7 +1245,7 @@ extern "C" int gb_gram_fixed_reduce(cudaStream_t stream, int num_sms, int k1, in
 {
     long g = ((long)k1 * k2 + 255) / 256;
     if (g > (long)num_sms * 16) g = (long)num_sms * 16;
-    k_gram_reduce<<<(int)(g > 0 ? g : 1), 256, 0, stream>>>(k1, k2, nsplit, part, a_dev, lda, sym, run);
+    gb_launch(stream, (int)(g > 0 ? g : 1), 256, 0, k_gram_reduce, k1, k2, nsplit, part, a_dev, lda, sym, run);
     return cudaGetLastError() != cudaSuccess ? GCGE_GPU_ERR_CUDA : GCGE_GPU_OK;
 }
 
@@ -1238,6 +1253,6 @@ extern "C" int gb_gram_fixed_reduce(cudaStream_t stream, int num_sms, int k1, in
 extern "C" int gb_gram_reduce_launch(gcge_gpu_ctx *ctx, int k1, int k2, int nsplit, const double *part,
                                      double *a_dev, int lda, int sym)
 {
-    GB_LAUNCH(ctx, k_gram_reduce, elem_grid(ctx, (long)k1 * k2), 256, 0, k1, k2, nsplit, part, a_dev, lda, sym);
+    GB_LAUNCH(ctx, k_gram_reduce, elem_grid(ctx, (long)k1 * k2), 256, 0, k1, k2, nsplit, part, a_dev, lda, sym, nullptr);
     return GCGE_GPU_OK;
 }

@@ -21,20 +21,12 @@
 #include <cuda_runtime.h>
 
 #include "gb_internal.h"
+#include "gb_launch.h"
 
 #define FULL 0xffffffffu
 
 #define GB_PROF(ctx, cls, bytes, flops) \
     do { if ((ctx)->prof) gb_prof_begin((ctx), (cls), (bytes), (flops)); } while (0)
-
-#define GB_LAUNCH(ctx, kern, grid, block, smem, ...)                                   \
-    do {                                                                               \
-        kern<<<(grid), (block), (smem), (ctx)->stream>>>(__VA_ARGS__);                 \
-        (ctx)->launches++;                                                             \
-        if ((ctx)->prof) gb_prof_end(ctx);                                             \
-        int _st = gb_check_launch(ctx);                                                \
-        if (_st) return _st;                                                           \
-    } while (0)
 
 // ---------------------------------------------------------------- small GEMM
 // C = alpha op(A) op(B) + beta C for the projected matrices (m, n, k of a few hundred
@@ -48,6 +40,7 @@ __global__ void __launch_bounds__(256)
 k_small_gemm(char ta, char tb, int m, int n, int k, double alpha, const double *__restrict__ A, int lda,
              const double *__restrict__ B, int ldb, double beta, double *__restrict__ C, int ldc)
 {
+    GB_PDL();
     __shared__ double part[4][SG_T * SG_T];
     const int t = threadIdx.x, o = t & 63, sl = t >> 6;
     const int i = blockIdx.x * SG_T + (o & 7), j = blockIdx.y * SG_T + (o >> 3);
@@ -91,6 +84,7 @@ extern "C" int gb_small_gemm(gcge_gpu_ctx *ctx, char ta, char tb, int m, int n, 
 // ---------------------------------------------------------------- misc helpers
 __global__ void k_set_zero(double *a, size_t count)
 {
+    GB_PDL();
     for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < count; t += (size_t)gridDim.x * blockDim.x)
         a[t] = 0.0;
 }
@@ -111,6 +105,7 @@ extern "C" int gb_copy_d(gcge_gpu_ctx *ctx, double *dst, const double *src, size
 }
 __global__ void k_set_diag(double *H, int ldh, int count, const double *vals)
 {
+    GB_PDL();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
         H[i + (long)i * ldh] = vals[i];
 }
@@ -124,6 +119,7 @@ extern "C" int gb_set_diag_from(gcge_gpu_ctx *ctx, double *H, int ldh, int count
 // kept in nu and turned into lambda = -1/nu (ascending as well)
 __global__ void k_neg_recip(int count, double *v, double *nu)
 {
+    GB_PDL();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         const double x = v[i];
         nu[i] = x;
@@ -140,6 +136,7 @@ extern "C" int gb_neg_recip(gcge_gpu_ctx *ctx, int count, double *v, double *nu)
 // locked Ritz vectors); C[:, 0:s] = e_0 .. e_(s-1); C[0:s, s:iu] = 0
 __global__ void k_soft_lock(double *H, int ldh, int m, int w0, int s, double *C, int ldc, int iu)
 {
+    GB_PDL();
     const long nh = (long)(m - w0) * s, nc = (long)m * s, nz = (long)(iu - s) * s;
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < nh + nc + nz; t += (long)gridDim.x * blockDim.x) {
         if (t < nh) {
@@ -165,6 +162,7 @@ extern "C" int gb_soft_lock(gcge_gpu_ctx *ctx, double *H, int ldh, int m, int w0
 }
 __global__ void k_sym_upper(double *H, int ldh, int m)
 {
+    GB_PDL();
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < (long)m * m; t += (long)gridDim.x * blockDim.x) {
         const int i = (int)(t % m), j = (int)(t / m);
         if (i > j) H[i + (long)j * ldh] = H[j + (long)i * ldh];
@@ -179,6 +177,7 @@ extern "C" int gb_symmetrize_from_upper(gcge_gpu_ctx *ctx, double *H, int ldh, i
 }
 __global__ void k_copy_block(int rows, int cols, const double *src, int lds, double *dst, int ldd)
 {
+    GB_PDL();
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < (long)rows * cols; t += (long)gridDim.x * blockDim.x) {
         const int i = (int)(t % rows), j = (int)(t / rows);
         dst[i + (long)j * ldd] = src[i + (long)j * lds];
@@ -198,6 +197,7 @@ extern "C" int gb_copy_block(gcge_gpu_ctx *ctx, int rows, int cols, const double
 // p_start+cp.
 __global__ void k_p_coef(double *coef, int ldc, int p_start, int p_ncols, int xx_nrows, const int *unlock)
 {
+    GB_PDL();
     const long total = (long)p_ncols * ldc;
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
         const int r = (int)(t % ldc), cp = (int)(t / ldc);
@@ -250,6 +250,7 @@ __global__ void __launch_bounds__(CD_THREADS)
 k_chol_deflate(int k, const double *__restrict__ G, int ldg, double *__restrict__ T, int *kept_out,
                double zero_tol, double rel_tol, double *work, double *__restrict__ min_ratio)
 {
+    GB_PDL();
     extern __shared__ double cd_sm[];
     const int ld = k | 1;
     double *piv = cd_sm, *diag = piv + k, *rinv = diag + k;      // pivots d, G's diagonal, 1 / R[j, j]
@@ -388,6 +389,7 @@ __global__ void __launch_bounds__(1024)
 k_tridiag(int m, const double *__restrict__ H, int ldh, double *__restrict__ Aw, double *__restrict__ d,
           double *__restrict__ e, double *__restrict__ tau)
 {
+    GB_PDL();
     extern __shared__ double sm[];
     double *v = sm;          // m
     double *w = sm + m;      // m
@@ -497,6 +499,7 @@ __global__ void __launch_bounds__(1024)
 k_tridiag_smem(int m, const double *__restrict__ H, int ldh, double *__restrict__ Aw, double *__restrict__ d,
                double *__restrict__ e, double *__restrict__ tau)
 {
+    GB_PDL();
     extern __shared__ double sm[];
     double *L = sm;                                   // packed lower triangle
     double *v = sm + (size_t)m * (m + 1) / 2;         // m
@@ -618,6 +621,7 @@ __global__ void __launch_bounds__(TS_THREADS)
 k_tridiag_small(int m, const double *__restrict__ H, int ldh, double *__restrict__ Aw, double *__restrict__ d,
                 double *__restrict__ e, double *__restrict__ tau)
 {
+    GB_PDL();
     extern __shared__ double sm[];
     const int ld = m | 1;
     double *A = sm, *vb = sm + (size_t)m * ld, *w = vb + 2 * m, *part = w + m;   // v of both parities, w, partials [4][m]
@@ -821,6 +825,7 @@ __global__ void __launch_bounds__(TD_THREADS)
 k_tridiag_cluster(int m, const double *__restrict__ H, int ldh, double *__restrict__ Aw, double *__restrict__ d,
                   double *__restrict__ e, double *__restrict__ tau)
 {
+    GB_PDL();
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
     const int TC = (int)cl.num_blocks(), b = (int)cl.block_rank();
@@ -1130,6 +1135,7 @@ __global__ void __launch_bounds__(32 * BI_WARPS)
 k_bisect(int m, const double *__restrict__ dg, const double *__restrict__ eg, int il, int iu,
          double *__restrict__ eval, int *info, const double *__restrict__ guess)
 {
+    GB_PDL();
     extern __shared__ double sm[];
     double *d = sm, *e2 = sm + m;
     __shared__ double px[BI_WARPS][32], pq[BI_WARPS][32], plo[BI_WARPS], phi[BI_WARPS];
@@ -1273,6 +1279,7 @@ __device__ __forceinline__ double start_value(int j, int i)
 
 __global__ void k_recip_probe(int n, const double *__restrict__ x, double *__restrict__ r)
 {
+    GB_PDL();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) r[i] = nr_recip(x[i]);
 }
@@ -1309,6 +1316,7 @@ __global__ void __launch_bounds__(32)
 k_invit(int m, const double *__restrict__ d, const double *__restrict__ e, int nev,
         const double *__restrict__ eval, double *__restrict__ Zt, int ldz)
 {
+    GB_PDL();
     extern __shared__ double ism[];
     const int lane = threadIdx.x, j = blockIdx.x;
     double *dl = ism, *dd = dl + m, *du = dd + m, *du2 = du + m, *inv = du2 + m, *z = inv + m;
@@ -1428,6 +1436,7 @@ __global__ void __launch_bounds__(1024)
 k_cluster_orth(int m, const double *__restrict__ d, const double *__restrict__ e, int nev,
                const double *__restrict__ eval, double *__restrict__ Zg, int ldz)
 {
+    GB_PDL();
     extern __shared__ double zsm[];
     __shared__ double coef[1024];
     __shared__ double red[32];
@@ -1536,6 +1545,7 @@ __global__ void __launch_bounds__(32)
 k_backtransform(int m, const double *__restrict__ Aw, const double *__restrict__ tau, int nev,
                 const double *__restrict__ Zt, int ldzt, double *__restrict__ Z, int ldz, int *info)
 {
+    GB_PDL();
     extern __shared__ double bsm[];                      // z, then BT_AHEAD + 1 reflectors
     const int lane = threadIdx.x, c = blockIdx.x;
     double *z = bsm, *ring = bsm + m;

@@ -45,19 +45,11 @@
 #include <cuda_runtime.h>
 
 #include "gb_internal.h"
+#include "gb_launch.h"
 #include "gb_tc05.h"
 
 #define GB_PROF(ctx, cls, bytes, flops) \
     do { if ((ctx)->prof) gb_prof_begin((ctx), (cls), (bytes), (flops)); } while (0)
-
-#define GB_LAUNCH(ctx, kern, grid, block, smem, ...)                                   \
-    do {                                                                               \
-        kern<<<(grid), (block), (smem), (ctx)->stream>>>(__VA_ARGS__);                 \
-        (ctx)->launches++;                                                             \
-        if ((ctx)->prof) gb_prof_end(ctx);                                             \
-        int _st = gb_check_launch(ctx);                                                \
-        if (_st) return _st;                                                           \
-    } while (0)
 
 extern "C" int gb_gram_reduce_launch(gcge_gpu_ctx *ctx, int k1, int k2, int nsplit, const double *part,
                                      double *a_dev, int lda, int sym);
@@ -254,6 +246,7 @@ __global__ void __launch_bounds__(256)
 k_col_exponent(int n, int k1, const double *__restrict__ V, long ldv, int k2, const double *__restrict__ W, long ldw,
                int *__restrict__ exps)
 {
+    GB_PDL();
     __shared__ int se[8][CE_COLS];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int k = blockIdx.y ? k2 : k1;
@@ -291,6 +284,7 @@ k_col_exponent(int n, int k1, const double *__restrict__ V, long ldv, int k2, co
 __global__ void k_gram_init(int *__restrict__ exps, int cols, unsigned *__restrict__ ticket, int tiles,
                             ulonglong2 *__restrict__ sums, long total)
 {
+    GB_PDL();
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < cols) exps[i] = OZ_NO_EXP;
     if (i < tiles) ticket[i] = 0;
@@ -331,6 +325,7 @@ k_gram_tc(int n, int k1, int k2, const double *__restrict__ V, long ldv, const d
           unsigned *__restrict__ ticket, double *__restrict__ a, int lda, long rows_per_split, int mt, int sym,
           int *__restrict__ err, int stall)
 {
+    GB_PDL();
     extern __shared__ __align__(1024) uint8_t tc_smem[];
     uint8_t *sm = tc_smem;
     const int i0 = blockIdx.x * mt, j0 = blockIdx.y * TC_N, iend = min(k1, i0 + mt);
@@ -613,6 +608,7 @@ extern "C" size_t gb_gram_fixed_ctl_bytes(void) { return sizeof(gn_ctl); }
 
 __global__ void k_gn_init(gn_ctl *ctl, int cols, ulonglong2 *__restrict__ sums, long total)
 {
+    GB_PDL();
     const long c = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c == 0) {
         ctl->skip = 0;
@@ -633,6 +629,7 @@ __global__ void __launch_bounds__(256)
 k_col_stats(int n, int k1, const double *__restrict__ V, long ldv, int k2, const double *__restrict__ W, long ldw,
             gn_ctl *ctl)
 {
+    GB_PDL();
     __shared__ int se[8][CE_COLS], sc[8][CE_COLS], ss[8][CE_COLS];
     __shared__ int done, wide;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -742,10 +739,10 @@ extern "C" int gb_gram_fixed(cudaStream_t stream, int num_sms, int n, int k1, in
             if (cudaFuncSetAttribute(k_gram_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, GR_SMEM) != cudaSuccess)
                 return GCGE_GPU_ERR_CUDA;
             const long most = total > k1 + k2 ? total : k1 + k2;
-            k_gn_init<<<(int)((most < 65536 ? most : 65536) + 255) / 256, 256, 0, stream>>>(
-                ctl, k1 + k2, (ulonglong2 *)part, nsplit > 1 ? total : 0);
-            k_col_stats<<<dim3(num_sms * 4, 2), 256, 0, stream>>>(n, k1, V, ldv, k2, W, ldw, ctl);
-            k_gram_tc<<<dim3(ti, tj, (unsigned)nsplit), TC_THREADS, GR_SMEM, stream>>>(
+            gb_launch(stream, (int)((most < 65536 ? most : 65536) + 255) / 256, 256, 0, k_gn_init, ctl, k1 + k2,
+                      (ulonglong2 *)part, nsplit > 1 ? total : 0L);
+            gb_launch(stream, dim3(num_sms * 4, 2), 256, 0, k_col_stats, n, k1, V, ldv, k2, W, ldw, ctl);
+            gb_launch(stream, dim3(ti, tj, (unsigned)nsplit), TC_THREADS, GR_SMEM, k_gram_tc,
                 n, k1, k2, V, ldv, W, ldw, ctl->e, ctl->e + k1, (unsigned long long *)part, ctl->ticket, a_dev, lda,
                 rps, gram_tc_mt(k1), sym, &ctl->skip, 0);
             if (cudaGetLastError() != cudaSuccess) return GCGE_GPU_ERR_CUDA;
@@ -785,6 +782,7 @@ __global__ void __launch_bounds__(256)
 k_lc_coef_split(int k1, int k2, const double *__restrict__ C, int ldc, int upper, int nst, int *__restrict__ g_out,
                 int *__restrict__ f_out, uint32_t *__restrict__ Bd)
 {
+    GB_PDL();
     __shared__ int gs[LC_MAX_K];
     __shared__ int fs[TC_N];
     const int s = blockIdx.x, jt = blockIdx.y, j0 = jt * TC_N;
@@ -852,6 +850,7 @@ k_lincomb_tc(int n, int k1, int k2, const double *__restrict__ X, long ldx, cons
              const int *__restrict__ g_in, const int *__restrict__ ec, double alpha, double beta,
              double *__restrict__ Y, long ldy, int nst, int *__restrict__ err, int stall)
 {
+    GB_PDL();
     extern __shared__ __align__(1024) uint8_t tc_smem[];
     uint8_t *sm = tc_smem;
     if (*(volatile int *)err) return;                    // an earlier launch timed out: do nothing
