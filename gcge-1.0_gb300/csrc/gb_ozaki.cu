@@ -22,7 +22,7 @@
 //  * 16 warps, one CTA per SM; warps 0-14 split FP64 operands into f16 digit
 //    planes in shared memory (two stages of K = 32, no-swizzle K-major core
 //    matrices), lane 0 of warp 15 issues the digit-pair MMAs of a stage
-//    (M = 128, N = 64, K = 16, accumulators: 8 levels x 64 TMEM columns), and
+//    (M = 128, K = 16, accumulators: 8 levels x N TMEM columns, N = 16 .. 64), and
 //    all 16 warps drain TMEM (warp w: lanes 32 (w % 4) .. +31, columns 4 (w / 4)
 //    .. +3 of every 16, so that a narrow output is shared by all of them);
 //  * hand-offs through mbarriers: full[b] (stage b written, 480 arrivals),
@@ -56,10 +56,10 @@ extern "C" int gb_gram_reduce_launch(gcge_gpu_ctx *ctx, int k1, int k2, int nspl
 
 // ---------------------------------------------------------------- tile geometry
 #define TC_M 128                                     // MMA M, TMEM lanes
-#define TC_N 64                                      // MMA N (max), TMEM columns per level
+#define TC_N 64                                      // columns of a tile (max), TMEM columns per level
 #define TC_KS 32                                     // K per pipeline stage
 #define TC_APLANE (TC_M * TC_KS * 2)                 // bytes of one f16 digit plane, A operand
-#define TC_BPLANE (TC_N * TC_KS * 2)                 // bytes of one f16 digit plane, B operand
+#define TC_BPLANE (TC_N * TC_KS * 2)                 // and, at most, B operand
 #define TC_STAGE (OZ_DIGITS * (TC_APLANE + TC_BPLANE))
 #define TC_HDR 1024                                  // mbarriers, TMEM address, flags, scales
 #define TC_WARPS 16
@@ -113,16 +113,48 @@ __device__ __forceinline__ void tc_setup(tc_hdr *h)
     }
 }
 
+// the digit-pair MMAs of the stage whose planes begin at a0 (see tc_issue_stage)
+template <int LEVELS, int N>
+__device__ __forceinline__ void tc_issue_mmas(uint32_t a0, uint32_t tmem, bool first)
+{
+    constexpr int GROUP = 256 / N < OZ_DIGITS ? 256 / N : OZ_DIGITS;   // B digits of one MMA
+    const uint32_t b0 = a0 + OZ_DIGITS * TC_APLANE;
+#pragma unroll
+    for (int ks = 0; ks < TC_KS / 16; ++ks) {
+        const bool over = first && ks == 0;
+#pragma unroll
+        for (int p = 0; p < OZ_DIGITS; ++p) {
+            const int qmax = (LEVELS - 1 - p < OZ_DIGITS - 1) ? LEVELS - 1 - p : OZ_DIGITS - 1;
+            const uint64_t ad = tc_sdesc(a0 + p * TC_APLANE + ks * 256, TC_LBO, TC_SBO);
+#pragma unroll
+            for (int q0 = 0; q0 <= qmax; q0 += GROUP) {
+                const int nq = qmax - q0 + 1 < GROUP ? qmax - q0 + 1 : GROUP;
+                const bool begins = p == 1 && q0 + nq == OZ_DIGITS;    // its last pair begins level OZ_DIGITS
+                const uint64_t bd = tc_sdesc(b0 + q0 * (N * TC_KS * 2) + ks * 256, TC_LBO, TC_SBO);
+                if (begins && over) {
+                    if (nq > 1) tc_mma_kf16(tmem + (p + q0) * N, ad, bd, tc_idesc_f16(TC_M, N * (nq - 1)), 1u);
+                    tc_mma_kf16(tmem + OZ_DIGITS * N, ad,
+                                tc_sdesc(b0 + (OZ_DIGITS - 1) * (N * TC_KS * 2) + ks * 256, TC_LBO, TC_SBO),
+                                tc_idesc_f16(TC_M, N), 0u);
+                } else {
+                    tc_mma_kf16(tmem + (p + q0) * N, ad, bd, tc_idesc_f16(TC_M, N * nq), p == 0 && over ? 0u : 1u);
+                }
+            }
+        }
+    }
+}
+
 // MMA issue of stage s (lane 0 of the MMA warp): wait for the stage's planes
 // (and, at the first stage of a chunk, for the previous chunk's drain), issue the
 // digit pairs with p + q < LEVELS x TC_KS / 16 K steps, commit to empty[buf].
-// The B digit planes of a stage lie back to back with the same 512-byte stride
-// between 8-row groups, and level L of the accumulator is TMEM columns 64 L ..
-// 64 L + 63, so the pairs (p, q0) .. (p, q0 + 3) are one MMA with N = 64 x 4
-// whose D starts at level p + q0: 11 MMAs per K step (10 for the Gram's seven
-// levels) instead of 34 (28), and each A plane is read from shared memory once
-// per such group instead of once per pair. The first K step of a chunk keeps
-// the pairwise order, whose first MMA into every level overwrites it.
+// The B digit planes of a stage (N rows, N a multiple of 16) lie back to back with the
+// same 512-byte stride between 8-row groups, and level L of the accumulator is TMEM
+// columns N L .. N L + N - 1, so the pairs (p, q0) .. (p, q0 + j - 1) are one MMA with
+// N j <= 256 columns whose D starts at level p + q0: 11 MMAs per K step at N = 64 and
+// 7 at N = 16 instead of 34, and each A plane is read from shared memory once per such group instead of once per pair. The first K
+// step of a chunk overwrites: with p = 0, and the one level that begins with p = 1 by
+// an MMA of its own. (With planes of 64 rows whatever N, and the first step pairwise, a
+// stage's MMAs ended 2.2 us after its split at any N.)
 // stall (test hook, GCGE_GPU_TestStallTensorWait): before the first stage the
 // issuing thread waits for the first drain, an arrival that cannot come before
 // the MMAs it would issue, so that bounded wait runs out and the CTA takes the
@@ -146,52 +178,24 @@ __device__ __forceinline__ void tc_issue_stage(tc_hdr *h, uint32_t sbase, uint32
         return;
     }
     tc_fence_after_sync();
-    (void)N;
-    const uint32_t a0 = sbase + buf * TC_STAGE, b0 = a0 + OZ_DIGITS * TC_APLANE;
-    const uint32_t idesc = tc_idesc_f16(TC_M, TC_N);
-#pragma unroll
-    for (int ks = 0; ks < TC_KS / 16; ++ks) {
-        if (cs == 0 && ks == 0) {
-#pragma unroll
-            for (int p = 0; p < OZ_DIGITS; ++p) {
-                const uint64_t ad = tc_sdesc(a0 + p * TC_APLANE, TC_LBO, TC_SBO);
-#pragma unroll
-                for (int q = 0; q < OZ_DIGITS; ++q) {
-                    if (p + q < LEVELS) {
-                        const uint64_t bd = tc_sdesc(b0 + q * TC_BPLANE, TC_LBO, TC_SBO);
-                        // the first MMA into level L is (p, q) = (max(0, L - 6), min(L, 6))
-                        const bool first = p == (p + q > OZ_DIGITS - 1 ? p + q - (OZ_DIGITS - 1) : 0);
-                        tc_mma_kf16(tmem + (p + q) * TC_N, ad, bd, idesc, first ? 0u : 1u);
-                    }
-                }
-            }
-        } else {
-#pragma unroll
-            for (int p = 0; p < OZ_DIGITS; ++p) {
-                const int qmax = (LEVELS - 1 - p < OZ_DIGITS - 1) ? LEVELS - 1 - p : OZ_DIGITS - 1;
-                const uint64_t ad = tc_sdesc(a0 + p * TC_APLANE + ks * 256, TC_LBO, TC_SBO);
-#pragma unroll
-                for (int q0 = 0; q0 <= qmax; q0 += 4) {
-                    const int nq = qmax - q0 + 1 < 4 ? qmax - q0 + 1 : 4;
-                    const uint64_t bd = tc_sdesc(b0 + q0 * TC_BPLANE + ks * 256, TC_LBO, TC_SBO);
-                    tc_mma_kf16(tmem + (p + q0) * TC_N, ad, bd, tc_idesc_f16(TC_M, TC_N * nq), 1u);
-                }
-            }
-        }
-    }
+    const uint32_t a0 = sbase + buf * TC_STAGE;
+    if (N == 16) tc_issue_mmas<LEVELS, 16>(a0, tmem, cs == 0);
+    else if (N == 32) tc_issue_mmas<LEVELS, 32>(a0, tmem, cs == 0);
+    else if (N == 48) tc_issue_mmas<LEVELS, 48>(a0, tmem, cs == 0);
+    else tc_issue_mmas<LEVELS, 64>(a0, tmem, cs == 0);
     tc_mma_commit(empty);
     ++commits[buf];
 }
 
 // TMEM read-out of 4 columns x LEVELS levels for this thread's lane (row of the tile)
 template <int LEVELS>
-__device__ __forceinline__ void tc_load_levels4(uint32_t taddr, uint32_t v[][4])
+__device__ __forceinline__ void tc_load_levels4(uint32_t taddr, int N, uint32_t v[][4])
 {
 #pragma unroll
     for (int L = 0; L < LEVELS; ++L)
         asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
                      : "=r"(v[L][0]), "=r"(v[L][1]), "=r"(v[L][2]), "=r"(v[L][3])
-                     : "r"(taddr + L * TC_N));
+                     : "r"(taddr + L * N));
     tc_tmem_wait_ld();
 #pragma unroll
     for (int L = 0; L < LEVELS; ++L) asm volatile("" : "+r"(v[L][0]), "+r"(v[L][1]), "+r"(v[L][2]), "+r"(v[L][3]));
@@ -337,25 +341,9 @@ k_gram_tc(int n, int k1, int k2, const double *__restrict__ V, long ldv, const d
     const long re = min((long)n, rb + rows_per_split);
     const int nst = (int)((re - rb + TC_KS - 1) / TC_KS);
     const int N = min(TC_N, (k2 - j0 + 15) & ~15);
-    tc_setup(h);
-    int *sbs = (int *)(sm + 2 * TC_STAGE + 128);         // shift bases of the tile's columns of V, then of W
-    for (int c = tid; c < TC_M + TC_N; c += TC_THREADS) {
-        const int col = c < TC_M ? i0 + c : j0 + c - TC_M;
-        sbs[c] = col < (c < TC_M ? iend : k2) ? (c < TC_M ? ev : ew)[col] + OZ_SHIFT0 : OZ_SHIFT_NONE;
-    }
-    // digit planes of both buffers start at zero: core matrices wholly outside the
-    // columns of V or W (the padding of a short tile) are never split and keep
-    // zero digits; the split threads' first proxy fence covers these writes
-    if (tid < TC_SPLIT_THREADS)
-        for (int i = tid; i < 2 * TC_STAGE / 16; i += TC_SPLIT_THREADS)
-            reinterpret_cast<uint4 *>(sm)[i] = make_uint4(0u, 0u, 0u, 0u);
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
-    const uint32_t tmem = h->tmem, sbase = tc_smem_addr(sm);
+    const uint32_t sbase = tc_smem_addr(sm);
     const bool mma_warp = warp == TC_SPLIT_WARPS;
     const int quarter = warp & 3, col0 = (warp >> 2) * 4;    // drained: columns col0 .. +3 of every 16
-    const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16) + col0;
     int commits[3] = {0, 0, 0};                          // empty[0], empty[1], drained chunks
     long long hi[TC_COLS_PER_WARP], lo[TC_COLS_PER_WARP];
 #pragma unroll
@@ -397,15 +385,28 @@ k_gram_tc(int n, int k1, int k2, const double *__restrict__ V, long ldv, const d
 #pragma unroll
         for (int cc = 0; cc < GR_CORES_PER_WARP; ++cc) copy_core(0, cc);
     }
+    // set-up while the first copies are on their way. (The digits of the padding -- core matrices
+    // past the tile's columns -- are whatever is there: they reach only the sums of the padding.)
+    tc_setup(h);
+    int *sbs = (int *)(sm + 2 * TC_STAGE + 128);         // shift bases of the tile's columns of V, then of W
+    for (int c = tid; c < TC_M + TC_N; c += TC_THREADS) {
+        const int col = c < TC_M ? i0 + c : j0 + c - TC_M;
+        sbs[c] = col < (c < TC_M ? iend : k2) ? (c < TC_M ? ev : ew)[col] + OZ_SHIFT0 : OZ_SHIFT_NONE;
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem = h->tmem, trow = tmem + ((uint32_t)(quarter * 32) << 16) + col0;
+    const int bplane = N * TC_KS * 2;
 
+    // A chunk is drained after the stage that follows it has been split: the split runs while
+    // the chunk's last MMAs do, and the next MMAs are ready to go when the drain ends.
+    // (262144 x 178 x 64: 484 -> 445 us, 10000 x 30 x 10: 13.4 -> 10.1 us in the kernel, both
+    // together with planes of the tile's width and two stages a split instead of four.)
     const uint8_t *raw = sm + 2 * TC_STAGE + TC_HDR + 16 * lane;
-    for (int s = 0; s < nst; ++s) {
+    for (int s = 0; s <= nst; ++s) {
         const int buf = s & 1, cs = s % TC_CHUNK_STAGES;
-        const bool chunk_end = cs == TC_CHUNK_STAGES - 1 || s == nst - 1;
-        if (mma_warp) {
-            if (lane == 0) tc_issue_stage<GR_LEVELS, false>(h, sbase, tmem, N, s, cs, commits, err, stall);
-            __syncwarp();
-        } else {
+        if (s < nst && !mma_warp) {
             if (s >= 2 && !tc_mbar_wait(tc_smem_addr(h->bar) + 16 + 8 * buf, ((s >> 1) - 1) & 1, TC_WAIT_NS))
                 tc_fail(h, err);
             uint8_t *A = sm + buf * TC_STAGE;
@@ -421,22 +422,22 @@ k_gram_tc(int n, int k1, int k2, const double *__restrict__ V, long ldv, const d
                     uint32_t d[OZ_DIGITS];
                     oz_pack(oz_bias(xv.x, sb), oz_bias(xv.y, sb), d);
                     uint32_t *dst = (uint32_t *)((isA ? A : B) + q * 128 + i8 * 16 + rp * 4);
-                    constexpr int pl[2] = {TC_BPLANE / 4, TC_APLANE / 4};
+                    const int pl = (isA ? TC_APLANE : bplane) / 4;
 #pragma unroll
-                    for (int p = 0; p < OZ_DIGITS; ++p) dst[p * pl[isA]] = d[p];
+                    for (int p = 0; p < OZ_DIGITS; ++p) dst[p * pl] = d[p];
                 }
                 copy_core(s + 1, cc);
             }
             tc_fence_async_smem();
             tc_mbar_arrive(tc_smem_addr(h->bar) + 8 * buf);
         }
-        if (chunk_end) {
-            if (!tc_wait_chunk(h, s, err)) break;
+        if (s > 0 && (cs == 0 || s == nst)) {
+            if (!tc_wait_chunk(h, s - 1, err)) break;
 #pragma unroll
             for (int g4 = 0; g4 < TC_COLS_PER_WARP / 4; ++g4) {
                 if (col0 + g4 * 16 < N) {
                     uint32_t v[GR_LEVELS][4];
-                    tc_load_levels4<GR_LEVELS>(trow + g4 * 16, v);
+                    tc_load_levels4<GR_LEVELS>(trow + g4 * 16, N, v);
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         float lev[GR_LEVELS];
@@ -454,6 +455,10 @@ k_gram_tc(int n, int k1, int k2, const double *__restrict__ V, long ldv, const d
             tc_fence_before_sync();
             tc_mbar_arrive(tc_smem_addr(h->bar) + 32);
             ++commits[2];
+        }
+        if (s < nst && mma_warp) {
+            if (lane == 0) tc_issue_stage<GR_LEVELS, false>(h, sbase, tmem, N, s, cs, commits, err, stall);
+            __syncwarp();
         }
         if (*(volatile int *)&h->flag) break;
     }
@@ -515,7 +520,8 @@ k_gram_tc(int n, int k1, int k2, const double *__restrict__ V, long ldv, const d
     tc_release(h, tmem, mma_warp, commits, nullptr);
 }
 
-// Row splits of the tensor-core Gram and the rows of each: about one CTA per SM. int64 headroom: a row adds < 2^28.2 to the level 0-2 sum (units
+// Row splits of the tensor-core Gram and the rows of each: about one CTA per SM, of two
+// stages at least (one: the same to 1%; four: a 30 x 30 grid's solve 1% slower). int64 headroom: a row adds < 2^28.2 to the level 0-2 sum (units
 // of 2^-16), so a split holds at most GR_MAX_ROWS rows (the level 3-7 sum is
 // carried into it after every chunk).
 #define GR_MAX_ROWS (1L << 20)
@@ -533,7 +539,7 @@ static long gram_tc_splits(int num_sms, int n, int k1, int k2, int sym, long *rp
             if (!sym || a * gram_tc_mt(k1) <= b * TC_N + TC_N - 1) ++tiles;
     if (tiles < 1) tiles = 1;
     long nsplit = ((long)num_sms + tiles - 1) / tiles;
-    const long max_split = (n + 4 * TC_KS - 1) / (4 * TC_KS);
+    const long max_split = (n + 2 * TC_KS - 1) / (2 * TC_KS);
     if (nsplit > max_split) nsplit = max_split;
     const long min_split = (n + GR_MAX_ROWS - 1) / GR_MAX_ROWS;
     if (nsplit < min_split) nsplit = min_split;
@@ -776,7 +782,7 @@ extern "C" int gb_gram_fixed(cudaStream_t stream, int num_sms, int n, int k1, in
 // C (k1 x k2, column-major, only i <= j when upper) -> row scales g (all blocks
 // compute them; block (0, 0) stores them), column scales F of 2^-g C (block
 // (0, jt) stores its 64) and digit planes Bd[jt][stage][digit] of 2^-g C in
-// the core-matrix layout (N = 64 rows j, K = 32 entries i per stage).
+// the core-matrix layout (N = 16 .. 64 rows j, K = 32 entries i per stage).
 // grid (stages, column tiles), 256 threads, k1 <= LC_MAX_K.
 __global__ void __launch_bounds__(256)
 k_lc_coef_split(int k1, int k2, const double *__restrict__ C, int ldc, int upper, int nst, int *__restrict__ g_out,
@@ -814,11 +820,14 @@ k_lc_coef_split(int k1, int k2, const double *__restrict__ C, int ldc, int upper
         }
     }
     __syncthreads();
+    // planes of N rows back to back, each stage's at a fixed place
     uint32_t *out = Bd + (size_t)(jt * nst + s) * OZ_DIGITS * (TC_BPLANE / 4);
+    const int N = min(TC_N, (k2 - j0 + 15) & ~15);
     const int n8 = lane >> 2, kp = lane & 3;
     for (int cc = 0; cc < 4; ++cc) {
         const int core = warp * 4 + cc, g = core >> 2, c = core & 3;
         const int jj = g * 8 + n8, j = j0 + jj, i = s * TC_KS + c * 8 + 2 * kp;
+        if (8 * g >= N) break;
         unsigned long long u0 = OZ_ZERO, u1 = OZ_ZERO;
         if (j < k2) {
             if (i < k1 && (!upper || i <= j)) u0 = oz_bias(C[i + (long)j * ldc], fs[jj] + gs[i] + OZ_SHIFT0);
@@ -828,7 +837,7 @@ k_lc_coef_split(int k1, int k2, const double *__restrict__ C, int ldc, int upper
         uint32_t d[OZ_DIGITS];
         oz_pack(u0, u1, d);
 #pragma unroll
-        for (int q = 0; q < OZ_DIGITS; ++q) out[q * (TC_BPLANE / 4) + w] = d[q];
+        for (int q = 0; q < OZ_DIGITS; ++q) out[q * (N * TC_KS / 2) + w] = d[q];
     }
 }
 
@@ -864,6 +873,39 @@ k_lincomb_tc(int n, int k1, int k2, const double *__restrict__ X, long ldx, cons
     const long ntiles = ((long)n + TC_M - 1) / TC_M;
     // one exact accumulation over all of K when it is short enough
     const int chunk_stages = k1 <= OZ_EXACT_TERMS ? nst : TC_CHUNK_STAGES;
+
+    const bool mma_warp = warp == TC_SPLIT_WARPS;
+    // split-warp geometry: core q = warp + 15 cc (A cores only); lane (r8, kp):
+    // row 8g + r8, entries 8c + 2 kp and 8c + 2 kp + 1
+    const int r8 = lane >> 2, kp = lane & 3;
+    double xv[LC_CORES_PER_WARP][2];
+    int off[LC_CORES_PER_WARP];                          // of the lane's entries from the stage's first one
+#pragma unroll
+    for (int cc = 0; cc < LC_CORES_PER_WARP; ++cc) {
+        const int q = warp + TC_SPLIT_WARPS * cc;
+        off[cc] = (8 * (q >> 2) + r8) * (int)ldx + 8 * (q & 3) + 2 * kp;
+    }
+    auto load_stage = [&](long row0, int s) {
+        const double *Xs = X + row0 * ldx + s * TC_KS;
+        if (row0 + TC_M <= n && (s + 1) * TC_KS <= k1) {
+#pragma unroll
+            for (int cc = 0; cc < LC_CORES_PER_WARP; ++cc)
+                if (warp + TC_SPLIT_WARPS * cc < TC_ACORES) {
+                    xv[cc][0] = Xs[off[cc]];
+                    xv[cc][1] = Xs[off[cc] + 1];
+                }
+        } else {
+#pragma unroll
+            for (int cc = 0; cc < LC_CORES_PER_WARP; ++cc) {
+                const int q = warp + TC_SPLIT_WARPS * cc, left = k1 - s * TC_KS - (8 * (q & 3) + 2 * kp);
+                const bool in = q < TC_ACORES && row0 + 8 * (q >> 2) + r8 < n;
+                xv[cc][0] = in && left > 0 ? Xs[off[cc]] : 0.0;
+                xv[cc][1] = in && left > 1 ? Xs[off[cc] + 1] : 0.0;
+            }
+        }
+    };
+    // the first stage's values, on their way during the set-up and the scale pass
+    if (!mma_warp) load_stage((long)blockIdx.x * TC_M, 0);
 
     tc_setup(h);
     // a zero row of C contributes nothing, nor do the entries past k1: no digits
@@ -904,7 +946,6 @@ k_lincomb_tc(int n, int k1, int k2, const double *__restrict__ X, long ldx, cons
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = h->tmem, sbase = tc_smem_addr(sm);
-    const bool mma_warp = warp == TC_SPLIT_WARPS;
     const int quarter = warp & 3, col0 = (warp >> 2) * 4;    // drained: columns col0 .. +3 of every 16
     const int my_row = quarter * 32 + lane;
     const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16) + col0;
@@ -916,36 +957,7 @@ k_lincomb_tc(int n, int k1, int k2, const double *__restrict__ X, long ldx, cons
     int commits[3] = {0, 0, 0};
     int copies[2] = {0, 0};                              // bulk copies per buffer (thread 0)
 
-    // split-warp geometry: core q = warp + 15 cc (A cores only); lane (r8, kp):
-    // row 8g + r8, entries 8c + 2 kp and 8c + 2 kp + 1
-    const int r8 = lane >> 2, kp = lane & 3;
-    double xv[LC_CORES_PER_WARP][2];
     unsigned pw[LC_CORES_PER_WARP][2];                   // high words of the next tile's entries, in flight
-    int off[LC_CORES_PER_WARP];                          // of the lane's entries from the stage's first one
-#pragma unroll
-    for (int cc = 0; cc < LC_CORES_PER_WARP; ++cc) {
-        const int q = warp + TC_SPLIT_WARPS * cc;
-        off[cc] = (8 * (q >> 2) + r8) * (int)ldx + 8 * (q & 3) + 2 * kp;
-    }
-    auto load_stage = [&](long row0, int s) {
-        const double *Xs = X + row0 * ldx + s * TC_KS;
-        if (row0 + TC_M <= n && (s + 1) * TC_KS <= k1) {
-#pragma unroll
-            for (int cc = 0; cc < LC_CORES_PER_WARP; ++cc)
-                if (warp + TC_SPLIT_WARPS * cc < TC_ACORES) {
-                    xv[cc][0] = Xs[off[cc]];
-                    xv[cc][1] = Xs[off[cc] + 1];
-                }
-        } else {
-#pragma unroll
-            for (int cc = 0; cc < LC_CORES_PER_WARP; ++cc) {
-                const int q = warp + TC_SPLIT_WARPS * cc, left = k1 - s * TC_KS - (8 * (q & 3) + 2 * kp);
-                const bool in = q < TC_ACORES && row0 + 8 * (q >> 2) + r8 < n;
-                xv[cc][0] = in && left > 0 ? Xs[off[cc]] : 0.0;
-                xv[cc][1] = in && left > 1 ? Xs[off[cc] + 1] : 0.0;
-            }
-        }
-    };
     auto load_words = [&](long row0, int s) {
         const unsigned *Xs = reinterpret_cast<const unsigned *>(X + row0 * ldx + s * TC_KS) + 1;
         const bool full = row0 + TC_M <= n && (s + 1) * TC_KS <= k1;
@@ -971,8 +983,6 @@ k_lincomb_tc(int n, int k1, int k2, const double *__restrict__ X, long ldx, cons
             }
         }
     };
-    if (!mma_warp) load_stage((long)blockIdx.x * TC_M, 0);
-
     // Stages g of this CTA over all its tiles (lt: its tile, s: the stage in it). A chunk
     // is drained after the next stage has been split: the split of that one -- the next
     // tile's first, mostly -- runs while the chunk's last MMAs do, and the next MMAs are
@@ -1004,9 +1014,9 @@ k_lincomb_tc(int n, int k1, int k2, const double *__restrict__ X, long ldx, cons
             // the pre-split C planes of this stage: one bulk copy, completing on copied[buf]
             if (tid == 0) {
                 const uint32_t copied = tc_smem_addr(h->bar) + 40 + 8 * buf;
-                tc_mbar_arrive_expect_tx(copied, OZ_DIGITS * TC_BPLANE);
+                tc_mbar_arrive_expect_tx(copied, OZ_DIGITS * N * TC_KS * 2);
                 tc_bulk_g2s(tc_smem_addr(B), Bd + (size_t)(jt * nst + s) * (OZ_DIGITS * TC_BPLANE / 16),
-                            OZ_DIGITS * TC_BPLANE, copied);
+                            OZ_DIGITS * N * TC_KS * 2, copied);
                 ++copies[buf];
             }
 #pragma unroll
@@ -1052,7 +1062,7 @@ k_lincomb_tc(int n, int k1, int k2, const double *__restrict__ X, long ldx, cons
             for (int g4 = 0; g4 < TC_COLS_PER_WARP / 4; ++g4) {
                 if (col0 + g4 * 16 < N) {
                     uint32_t v[LC_LEVELS][4];
-                    tc_load_levels4<LC_LEVELS>(trow + g4 * 16, v);
+                    tc_load_levels4<LC_LEVELS>(trow + g4 * 16, N, v);
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         int lev[LC_LEVELS];

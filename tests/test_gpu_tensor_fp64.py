@@ -138,6 +138,18 @@ def test_tensor_lincomb_exact_on_integers(ctx):
     assert np.array_equal(lincomb(ctx, X, C), X @ C)
 
 
+@pytest.mark.parametrize("k2", [1, 16, 17, 33, 48, 49, 64, 65, 100])
+@pytest.mark.parametrize("n,k1", [(1, 1), (33, 8), (161, 9), (353, 128), (20011, 129), (129, 187)])
+def test_tensor_integers_at_tile_widths(ctx, n, k1, k2):
+    """Integers below 2^8 have at most three digits in either factor, whatever the equilibration: every
+    width of the digit planes and every length of the last stage gives the product itself."""
+    rng = np.random.default_rng(1000 * k1 + k2)
+    V, W = rng.integers(-255, 256, (n, k1)), rng.integers(-255, 256, (n, k2))
+    assert np.array_equal(gram(ctx, V.astype(float), W.astype(float)), (V.T @ W).astype(float))
+    C = rng.integers(1, 256, (k1, k2)) * rng.choice([-1, 1], (k1, k2))
+    assert np.array_equal(lincomb(ctx, V.astype(float), C.astype(float)), (V @ C).astype(float))
+
+
 def test_tensor_lincomb_wide_dynamic_range(ctx):
     """Row entries spanning 2^-40 .. 1: errors bounded by the row and column scales."""
     rng = np.random.default_rng(9)
