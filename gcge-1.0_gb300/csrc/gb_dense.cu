@@ -1428,7 +1428,10 @@ k_invit(int m, const double *__restrict__ d, const double *__restrict__ e, int n
 // reorthogonalise inside clusters (gap <= 1e-3 ||T||_1, as dstein) by two
 // classical Gram-Schmidt passes, then normalise; a block per cluster (the b-th run of
 // close eigenvalues to block b), vectors in order; with SMEM the cluster's vectors are
-// worked on in shared memory. m <= 1024: a thread per row. (All vectors in one block of
+// worked on in shared memory. m <= 1024: a thread per row, and eight warps at least: the
+// products with the earlier vectors, four to a warp and one tree of additions for the four,
+// keep all quarters of the SM at their FP64. (Two warps at m = 60, a tree per product: 185
+// us for 25 vectors in one cluster, now 104. All vectors in one block of
 // 1,024 threads spent 2.3 us on each, mostly barriers and a serial sum of 32 warps, although
 // most of them belong to no cluster: 73 us for 13 vectors of 30, here 12.)
 template <bool SMEM>
@@ -1490,12 +1493,25 @@ k_cluster_orth(int m, const double *__restrict__ d, const double *__restrict__ e
         double *zj = Zt + (size_t)np * ld;
         if (np > 0) {
             for (int pass = 0; pass < 2; ++pass) {
-                for (int q = wid; q < np; q += nw) {
-                    const double *zi = Zt + (size_t)q * ld;
-                    double s = 0;
-                    for (int r = lane; r < m; r += 32) s = fma(zi[r], zj[r], s);
-                    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
-                    if (lane == 0 && q < 1024) coef[q] = s;
+                for (int q = wid; q < np; q += 4 * nw) {
+                    // four vectors a warp: lanes with bits 4 and 3 equal to (u & 1, u >> 1) end with
+                    // vector u's sum, the halves added in the order of a butterfly of its own
+                    double s[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const double *zi = Zt + (size_t)min(q + u * nw, np - 1) * ld;
+                        s[u] = 0;
+                        if (q + u * nw < np)
+                            for (int r = lane; r < m; r += 32) s[u] = fma(zi[r], zj[r], s[u]);
+                    }
+                    const bool b4 = lane & 16, b3 = lane & 8;
+                    const double t0 = (b4 ? s[1] : s[0]) + __shfl_xor_sync(FULL, b4 ? s[0] : s[1], 16);
+                    const double t1 = (b4 ? s[3] : s[2]) + __shfl_xor_sync(FULL, b4 ? s[2] : s[3], 16);
+                    double t = (b3 ? t1 : t0) + __shfl_xor_sync(FULL, b3 ? t0 : t1, 8);
+#pragma unroll
+                    for (int o = 4; o; o >>= 1) t += __shfl_xor_sync(FULL, t, o);
+                    const int c = q + ((b4 ? 1 : 0) + (b3 ? 2 : 0)) * nw;
+                    if ((lane & 7) == 0 && c < np && c < 1024) coef[c] = t;
                 }
                 __syncthreads();
                 for (int r = tid; r < m; r += blockDim.x) {
@@ -1697,7 +1713,7 @@ extern "C" int gb_syevx_guess(gcge_gpu_ctx *ctx, int m, const double *H, int ldh
         if (st) return st;
     }
     const size_t osmem = sizeof(double) * (size_t)m * nev;
-    const int othreads = m > 1024 ? 1024 : (m + 31) / 32 * 32;
+    const int othreads = m > 1024 ? 1024 : m > 256 ? (m + 31) / 32 * 32 : 256;
     if (reorth_done) {
         // the vectors are orthonormal: Cholesky-QR over all of them
     } else if (osmem <= 160 * 1024) {

@@ -240,10 +240,40 @@ __device__ __forceinline__ void tc_release(tc_hdr *h, uint32_t tmem, int mma_war
 // ---------------------------------------------------------------- Gram column scales
 // exps[c] = smallest e with |X[r, c]| < 2^e for all rows (OZ_NO_EXP for an
 // all-zero column; subnormal entries count as zero). exps must hold OZ_NO_EXP
-// on entry. A warp reads whole rows (lane l: columns c0 + l + 32 j, 8 independent
-// loads per row in flight) over 256-column chunks, so each row's bytes stream
+// on entry. A warp reads whole rows over 256-column chunks, so each row's bytes stream
 // once per chunk; each block reduces its warps and issues one atomic per column.
 #define CE_COLS 256
+
+// f(j, entry) for the entries of columns lane + 32 j < kc of the warp's rows (zeros past
+// them), eight loads in flight: of one row when it has more than 128 columns, of eight when
+// it has 32. (One row at a time, 110592 x 60 and x 20 kept two loads and one: 28.3 -> 16.1 us.)
+template <int NJ, class F>
+__device__ __forceinline__ void ce_walk(int n, int kc, const double *__restrict__ X, long ldx, long warp, long nw, F f)
+{
+    constexpr int U = CE_COLS / 32 / NJ;
+    const int lane = threadIdx.x & 31;
+    for (long r = warp; r < n; r += U * nw) {
+        double v[U][NJ];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int j = 0; j < NJ; ++j)
+                v[u][j] = r + u * nw < n && lane + 32 * j < kc ? __ldg(X + (r + u * nw) * ldx + lane + 32 * j) : 0.0;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) f(j, v[u][j]);
+    }
+}
+template <class F>
+__device__ __forceinline__ void ce_rows(int n, int kc, const double *__restrict__ X, long ldx, long warp, long nw, F f)
+{
+    if (kc <= 32) ce_walk<1>(n, kc, X, ldx, warp, nw, f);
+    else if (kc <= 64) ce_walk<2>(n, kc, X, ldx, warp, nw, f);
+    else if (kc <= 128) ce_walk<4>(n, kc, X, ldx, warp, nw, f);
+    else ce_walk<CE_COLS / 32>(n, kc, X, ldx, warp, nw, f);
+}
+
 // grid (blocks, 2): blockIdx.y = 0 the columns of V (exps[0:k1]), 1 those of W
 // (exps[k1:]) -- one launch, so that the two short passes share the chip.
 __global__ void __launch_bounds__(256)
@@ -263,14 +293,8 @@ k_col_exponent(int n, int k1, const double *__restrict__ V, long ldv, int k2, co
         int e[CE_COLS / 32];
 #pragma unroll
         for (int j = 0; j < CE_COLS / 32; ++j) e[j] = OZ_NO_EXP;
-        for (long r = warp; r < n; r += nw) {
-            const double *xr = X + r * ldx + c0 + lane;
-            double v[CE_COLS / 32];
-#pragma unroll
-            for (int j = 0; j < CE_COLS / 32; ++j) v[j] = c0 + lane + 32 * j < k ? __ldg(xr + 32 * j) : 0.0;
-#pragma unroll
-            for (int j = 0; j < CE_COLS / 32; ++j) e[j] = max(e[j], oz_exponent(v[j]));
-        }
+        ce_rows(n, min(CE_COLS, k - c0), X + c0, ldx, warp, nw,
+                [&](int j, double x) { e[j] = max(e[j], oz_exponent(x)); });
 #pragma unroll
         for (int j = 0; j < CE_COLS / 32; ++j) se[w][lane + 32 * j] = e[j];
         __syncthreads();
@@ -629,8 +653,7 @@ __global__ void k_gn_init(gn_ctl *ctl, int cols, ulonglong2 *__restrict__ sums, 
     for (long t = c; t < total; t += (long)gridDim.x * blockDim.x) sums[t] = make_ulonglong2(0, 0);
 }
 
-// grid (blocks, 2): blockIdx.y = 0 the columns of V, 1 those of W. A warp reads
-// whole rows, eight independent loads per lane in flight, as k_col_exponent.
+// grid (blocks, 2): blockIdx.y = 0 the columns of V, 1 those of W; rows as k_col_exponent.
 __global__ void __launch_bounds__(256)
 k_col_stats(int n, int k1, const double *__restrict__ V, long ldv, int k2, const double *__restrict__ W, long ldw,
             gn_ctl *ctl)
@@ -652,23 +675,16 @@ k_col_stats(int n, int k1, const double *__restrict__ V, long ldv, int k2, const
             cnt[j] = 0;
             sum[j] = 0;
         }
-        for (long r = warp; r < n; r += nw) {
-            const double *xr = X + r * ldx + c0 + lane;
-            double v[CE_COLS / 32];
-#pragma unroll
-            for (int j = 0; j < CE_COLS / 32; ++j) v[j] = c0 + lane + 32 * j < k ? __ldg(xr + 32 * j) : 0.0;
-#pragma unroll
-            for (int j = 0; j < CE_COLS / 32; ++j) {
-                // a subnormal entry has no digits: counted as not finite
-                int x = oz_exponent(v[j]);
-                if (x == OZ_NO_EXP && (__double_as_longlong(v[j]) << 1)) x = 1025;
-                if (x != OZ_NO_EXP) {
-                    e[j] = max(e[j], x);
-                    ++cnt[j];
-                    sum[j] += x;
-                }
+        ce_rows(n, min(CE_COLS, k - c0), X + c0, ldx, warp, nw, [&](int j, double v) {
+            // a subnormal entry has no digits: counted as not finite
+            int x = oz_exponent(v);
+            if (x == OZ_NO_EXP && (__double_as_longlong(v) << 1)) x = 1025;
+            if (x != OZ_NO_EXP) {
+                e[j] = max(e[j], x);
+                ++cnt[j];
+                sum[j] += x;
             }
-        }
+        });
 #pragma unroll
         for (int j = 0; j < CE_COLS / 32; ++j) {
             se[w][lane + 32 * j] = e[j];
@@ -784,6 +800,9 @@ extern "C" int gb_gram_fixed(cudaStream_t stream, int num_sms, int n, int k1, in
 // (0, jt) stores its 64) and digit planes Bd[jt][stage][digit] of 2^-g C in
 // the core-matrix layout (N = 16 .. 64 rows j, K = 32 entries i per stage).
 // grid (stages, column tiles), 256 threads, k1 <= LC_MAX_K.
+// One block or two at a solve's sizes, so only latency counts: each of the three passes over C
+// has its loads in flight together, the first along C's columns (60 x 20: 8.2 -> 4.8 us;
+// a call at 10000 x 178 x 64 90 -> 75 us).
 __global__ void __launch_bounds__(256)
 k_lc_coef_split(int k1, int k2, const double *__restrict__ C, int ldc, int upper, int nst, int *__restrict__ g_out,
                 int *__restrict__ f_out, uint32_t *__restrict__ Bd)
@@ -793,30 +812,44 @@ k_lc_coef_split(int k1, int k2, const double *__restrict__ C, int ldc, int upper
     __shared__ int fs[TC_N];
     const int s = blockIdx.x, jt = blockIdx.y, j0 = jt * TC_N;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int i = warp; i < k1; i += 8) {
+    // row exponents: lanes along the rows (contiguous in C), columns dealt to the warps
+    for (int i = threadIdx.x; i < k1; i += 256) gs[i] = OZ_NO_EXP;
+    __syncthreads();
+    for (int i0 = 0; i0 < k1; i0 += 32) {
+        const int i = i0 + lane;
         int e = OZ_NO_EXP;
-        for (int j = (upper ? i : 0) + lane; j < k2; j += 32) e = max(e, oz_exponent(C[i + (long)j * ldc]));
-        e = __reduce_max_sync(0xffffffffu, e);
-        if (lane == 0) {
-            gs[i] = e;
-            if (s == 0 && jt == 0) g_out[i] = e;
-        }
+#pragma unroll 4
+        for (int j = (upper ? i0 : 0) + warp; j < k2; j += 8)
+            if (i < k1 && (!upper || i <= j)) e = max(e, oz_exponent(C[i + (long)j * ldc]));
+        if (e != OZ_NO_EXP) atomicMax(gs + i, e);
     }
     __syncthreads();
-    for (int cc = 0; cc < TC_N / 8; ++cc) {
-        const int jj = warp * (TC_N / 8) + cc, j = j0 + jj;
-        int e = OZ_NO_EXP;
-        if (j < k2) {
-            const int iend = upper ? min(k1, j + 1) : k1;
-            for (int i = lane; i < iend; i += 32) {
-                const int ex = oz_exponent(C[i + (long)j * ldc]);
-                if (ex != OZ_NO_EXP) e = max(e, ex - gs[i]);
+    if (s == 0 && jt == 0)
+        for (int i = threadIdx.x; i < k1; i += 256) g_out[i] = gs[i];
+    // column scales: a warp has columns warp, warp + 8, ..
+    {
+        int e[TC_N / 8];
+#pragma unroll
+        for (int cc = 0; cc < TC_N / 8; ++cc) e[cc] = OZ_NO_EXP;
+        for (int i = lane; i < k1; i += 32) {
+            const int g = gs[i];
+            int ex[TC_N / 8];
+#pragma unroll
+            for (int cc = 0; cc < TC_N / 8; ++cc) {
+                const int j = j0 + warp + 8 * cc;
+                ex[cc] = j < k2 && (!upper || i <= j) ? oz_exponent(C[i + (long)j * ldc]) : OZ_NO_EXP;
             }
+#pragma unroll
+            for (int cc = 0; cc < TC_N / 8; ++cc)
+                if (ex[cc] != OZ_NO_EXP) e[cc] = max(e[cc], ex[cc] - g);
         }
-        e = __reduce_max_sync(0xffffffffu, e);
-        if (lane == 0) {
-            fs[jj] = e;
-            if (s == 0 && j < k2) f_out[j] = e;
+#pragma unroll
+        for (int cc = 0; cc < TC_N / 8; ++cc) {
+            const int jj = warp + 8 * cc, m = __reduce_max_sync(0xffffffffu, e[cc]);
+            if (lane == 0) {
+                fs[jj] = m;
+                if (s == 0 && j0 + jj < k2) f_out[j0 + jj] = m;
+            }
         }
     }
     __syncthreads();
@@ -824,20 +857,24 @@ k_lc_coef_split(int k1, int k2, const double *__restrict__ C, int ldc, int upper
     uint32_t *out = Bd + (size_t)(jt * nst + s) * OZ_DIGITS * (TC_BPLANE / 4);
     const int N = min(TC_N, (k2 - j0 + 15) & ~15);
     const int n8 = lane >> 2, kp = lane & 3;
-    for (int cc = 0; cc < 4; ++cc) {
-        const int core = warp * 4 + cc, g = core >> 2, c = core & 3;
-        const int jj = g * 8 + n8, j = j0 + jj, i = s * TC_KS + c * 8 + 2 * kp;
-        if (8 * g >= N) break;
-        unsigned long long u0 = OZ_ZERO, u1 = OZ_ZERO;
-        if (j < k2) {
-            if (i < k1 && (!upper || i <= j)) u0 = oz_bias(C[i + (long)j * ldc], fs[jj] + gs[i] + OZ_SHIFT0);
-            if (i + 1 < k1 && (!upper || i + 1 <= j)) u1 = oz_bias(C[i + 1 + (long)j * ldc], fs[jj] + gs[i + 1] + OZ_SHIFT0);
-        }
-        const int w = (core * 128 + n8 * 16 + kp * 4) / 4;
-        uint32_t d[OZ_DIGITS];
-        oz_pack(u0, u1, d);
+    double x[4][2];
 #pragma unroll
-        for (int q = 0; q < OZ_DIGITS; ++q) out[q * (N * TC_KS / 2) + w] = d[q];
+    for (int cc = 0; cc < 4; ++cc) {
+        const int core = warp + 8 * cc, jj = (core >> 2) * 8 + n8, j = j0 + jj, i = s * TC_KS + (core & 3) * 8 + 2 * kp;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            x[cc][h] = j < k2 && i + h < k1 && (!upper || i + h <= j) ? C[i + h + (long)j * ldc] : 0.0;
+    }
+#pragma unroll
+    for (int cc = 0; cc < 4; ++cc) {
+        const int core = warp + 8 * cc, jj = (core >> 2) * 8 + n8, i = s * TC_KS + (core & 3) * 8 + 2 * kp;
+        if (core >> 2 < N / 8) {
+            uint32_t d[OZ_DIGITS];
+            oz_pack(oz_bias(x[cc][0], i < k1 ? fs[jj] + gs[i] + OZ_SHIFT0 : OZ_SHIFT_NONE),
+                    oz_bias(x[cc][1], i + 1 < k1 ? fs[jj] + gs[i + 1] + OZ_SHIFT0 : OZ_SHIFT_NONE), d);
+#pragma unroll
+            for (int q = 0; q < OZ_DIGITS; ++q) out[q * (N * TC_KS / 2) + (core * 128 + n8 * 16 + kp * 4) / 4] = d[q];
+        }
     }
 }
 

@@ -181,7 +181,6 @@ __device__ __forceinline__ unsigned long long oz_bias(double x, int sb)
 // significant first: byte b goes under 0x64 as 0x64bb = 1024 + b, from which 1152 is
 // subtracted, both exact. A byte permute pairs two bytes of both entries, a second one
 // spreads each pair over the constant: 11 for seven digits.
-#define OZ_ZERO 0x8080808080808080ULL                // oz_digits of nothing
 __device__ __forceinline__ void oz_pack(unsigned long long u0, unsigned long long u1, uint32_t d[OZ_DIGITS])
 {
     const uint32_t l0 = (uint32_t)u0, h0 = (uint32_t)(u0 >> 32), l1 = (uint32_t)u1, h1 = (uint32_t)(u1 >> 32);
