@@ -128,6 +128,42 @@ k_xr_update(int n, int k, float *__restrict__ X, float *__restrict__ R, const fl
     }
 }
 
+// v[b0] + v[b0 + step] + ... (b < nblk, row stride k) in that order, U loads in flight:
+// the additions are a chain, the loads need not wait for them
+template <int U>
+__device__ __forceinline__ double cs_strided(const double *__restrict__ v, int k, int b0, int nblk, int step)
+{
+    double s = 0;
+    for (int b = b0; b < nblk; b += U * step) {
+        double x[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) x[u] = b + u * step < nblk ? v[(long)(b + u * step) * k] : 0.0;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (b + u * step < nblk) s += x[u];
+    }
+    return s;
+}
+
+// the sum of 256 threads' s in thread 0, pairs at distance 128, 64, .. 1; the last
+// five levels lie within a warp
+__device__ __forceinline__ double cs_tree(double s, double *sh)
+{
+    const int t = threadIdx.x;
+    sh[t] = s;
+    __syncthreads();
+    if (t < 128) sh[t] = s = s + sh[t + 128];
+    __syncthreads();
+    if (t < 64) sh[t] = s = s + sh[t + 64];
+    __syncthreads();
+    if (t < 32) {
+        s += sh[t + 32];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    }
+    return s;
+}
+
 // second stage of the per-column sums, one block per column: each thread adds a
 // fixed strided subset of the row-slab partials, then a fixed tree (deterministic)
 __global__ void __launch_bounds__(256)
@@ -137,15 +173,9 @@ k_colsum(int nblk, int k, const double *__restrict__ part, const int *__restrict
     __shared__ double sh[256];
     const int c = blockIdx.x;
     if (nact && c >= *nact) return;
-    double s = 0;
-    for (int b = threadIdx.x; b < nblk; b += 256) s += part[(long)b * k + c];
-    sh[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) out[c] = sh[0];
+    double s = cs_strided<4>(part + c, k, threadIdx.x, nblk, 256);
+    s = cs_tree(s, sh);
+    if (threadIdx.x == 0) out[c] = s;
 }
 
 // ptw[c] (summed by k_colsum) for active c, and alpha[c] = rho2[c] / ptw[c]
@@ -166,7 +196,10 @@ __global__ void k_init_state(int k, const double *__restrict__ sums, double *rho
         rho2[c] = sums[c];
         err[c] = sqrt(sums[c]);
     }
-    if (threadIdx.x == 0) *nact = k;
+    if (threadIdx.x == 0) {
+        nact[0] = k;
+        nact[1] = 0;                                       // k_colsum_finalize's count of blocks
+    }
 }
 
 // end of a round: rho1 = rho2, rho2 = new r.r (active columns); recount over all columns
@@ -255,6 +288,14 @@ static int vec_blocks(gcge_gpu_ctx *ctx, const void *fn, int n, int ctiles)
     return (int)(g < cap ? g : cap);
 }
 
+// blocks of k_xr_update_v: two per SM at four threads a row, else three
+static int xr_blocks(gcge_gpu_ctx *ctx, int tpr, int n, int ctiles)
+{
+    long g = cdiv(n > 0 ? n : 1, RED_ROWS), cap = (long)ctx->num_sms * (tpr == 4 ? 2 : 3) / (ctiles > 0 ? ctiles : 1);
+    if (cap < 1) cap = 1;
+    return (int)(g < cap ? g : cap);
+}
+
 // sum the per-thread column partials s[4] (thread (rs, cg) holds columns
 // c0 + 4 cg .. +3 of its row slot) over the row slots in a fixed order; the block's
 // partials of the kact active columns go to row blockIdx.x of part (row stride k,
@@ -296,44 +337,40 @@ k_pupdate_v(int n, int k, const float *__restrict__ R, float *__restrict__ P, lo
 #pragma unroll
     for (int q = 0; q < 4; ++q) b[q] = (!first && c0 + q < ka) ? (float)beta[c0 + q] : 0.f;
     const bool full = c0 + 4 <= ka;
-    for (long r = (long)blockIdx.x * RPB + rs; r < n; r += (long)gridDim.x * RPB) {
-        float4 rv = *reinterpret_cast<const float4 *>(R + r * ld + c0);
-        if (dinv) {                                // z = D^-1 r (Jacobi)
-            const float dr = dinv[r];
-            rv.x *= dr; rv.y *= dr; rv.z *= dr; rv.w *= dr;
-        }
-        float4 *pp = reinterpret_cast<float4 *>(P + r * ld + c0);
-        if (first) {                               // p = r: the old p (uninitialised) is not read
-            if (full) {
-                *pp = rv;
-            } else {
-                float *pe = reinterpret_cast<float *>(pp);
-                const float *re = &rv.x;
+    const long step = (long)gridDim.x * RPB;
+    for (long r = (long)blockIdx.x * RPB + rs; r < n; r += 2 * step) {
+        // two rows' loads in flight
+        float4 rv[2], pv[2];
+        float dr[2];
 #pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    if (c0 + q < ka) pe[q] = re[q];
+        for (int u = 0; u < 2; ++u)
+            if (r + u * step < n) {
+                rv[u] = *reinterpret_cast<const float4 *>(R + (r + u * step) * ld + c0);
+                if (dinv) dr[u] = dinv[r + u * step];
+                // p = r on the first round: the old p (uninitialised) is not read
+                if (!first || !full) pv[u] = *reinterpret_cast<const float4 *>(P + (r + u * step) * ld + c0);
             }
-            continue;
-        }
-        float4 pv = *pp;
-        if (full) {
-            pv.x = rv.x + b[0] * pv.x; pv.y = rv.y + b[1] * pv.y;
-            pv.z = rv.z + b[2] * pv.z; pv.w = rv.w + b[3] * pv.w;
-        } else {
-            float *pe = &pv.x;
-            const float *re = &rv.x;
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (c0 + q < ka) pe[q] = re[q] + b[q] * pe[q];
+        for (int u = 0; u < 2; ++u) {
+            if (r + u * step >= n) break;
+            float *pe = &pv[u].x, *re = &rv[u].x;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (dinv) re[q] *= dr[u];                  // z = D^-1 r (Jacobi)
+                if (full || c0 + q < ka) pe[q] = first ? re[q] : re[q] + b[q] * pe[q];
+            }
+            *reinterpret_cast<float4 *>(P + (r + u * step) * ld + c0) = pv[u];
         }
-        *pp = pv;
     }
 }
 
 // x += alpha p, r -= alpha w on the active columns, with block partials of r.r
 // (FP32 products summed over runs of 8 rows, the runs summed in FP64)
+// The next row's loads go out before this row is worked on, and the grid is xr_blocks() whatever
+// the registers: the row slots are the sums' association. (20 columns of 48^3
+// cells, in L2: 14.5 -> 12.4 us.)
 template <int TPR>
-__global__ void __launch_bounds__(VB_THREADS)
+__global__ void __launch_bounds__(VB_THREADS, 3)
 k_xr_update_v(int n, int k, float *__restrict__ X, float *__restrict__ R, const float *__restrict__ P,
               const float *__restrict__ W, long ld, const double *__restrict__ alpha, const int *__restrict__ nact,
               double *__restrict__ part, const float *__restrict__ dinv)
@@ -350,12 +387,22 @@ k_xr_update_v(int n, int k, float *__restrict__ X, float *__restrict__ R, const 
         for (int q = 0; q < 4; ++q) a[q] = c0 + q < ka ? (float)alpha[c0 + q] : 0.f;
         float run[4] = {0, 0, 0, 0};
         int cnt = 0;
-        for (long r = (long)blockIdx.x * RPB + rs; r < n; r += (long)gridDim.x * RPB) {
+        const long step = (long)gridDim.x * RPB;
+        long r = (long)blockIdx.x * RPB + rs;
+        float4 nx, nr, np, nv;
+        auto load = [&](long row) {
+            const long o = row * ld + c0;
+            nx = *reinterpret_cast<const float4 *>(X + o);
+            nr = *reinterpret_cast<const float4 *>(R + o);
+            np = *reinterpret_cast<const float4 *>(P + o);
+            nv = *reinterpret_cast<const float4 *>(W + o);
+        };
+        if (r < n) load(r);
+        for (; r < n; r += step) {
             const long o = r * ld + c0;
-            float4 xv = *reinterpret_cast<const float4 *>(X + o);
-            float4 rv = *reinterpret_cast<const float4 *>(R + o);
-            const float4 pv = *reinterpret_cast<const float4 *>(P + o);
-            const float4 wv = *reinterpret_cast<const float4 *>(W + o);
+            float4 xv = nx, rv = nr;
+            const float4 pv = np, wv = nv;
+            if (r + step < n) load(r + step);
             float *xe = &xv.x, *re = &rv.x;
             const float *pe = &pv.x, *we = &wv.x;
             const float dr = dinv ? dinv[r] : 1.0f;
@@ -566,42 +613,46 @@ k_colsum_alpha(int nblk, int k, const double *__restrict__ part, const int *__re
     __shared__ double sh[256];
     const int c = blockIdx.x;
     if (c >= *nact) return;
-    double s = 0;
-    for (int b = threadIdx.x; b < nblk; b += 256) s += part[(long)b * k + c];
-    sh[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
-    }
+    double s = cs_strided<4>(part + c, k, threadIdx.x, nblk, 256);
+    s = cs_tree(s, sh);
     if (threadIdx.x == 0) {
-        ptw[c] = sh[0];
-        alpha[c] = rho2[c] / sh[0];
+        ptw[c] = s;
+        alpha[c] = rho2[c] / s;
     }
 }
 
-// column sums of the r.r partials (a warp per column, fixed order), then the
-// end-of-round update of k_finalize in the same block
-__global__ void __launch_bounds__(1024)
+// column sums of the r.r partials (a warp per column, fixed order); the block that comes
+// last (nact[1] counts them and is left at zero) does the end-of-round update of
+// k_finalize. Four warps a block, one on each quarter of the SM: a sum's some twenty
+// additions occupy a quarter for 64 clocks each, and in one block of 32 warps they
+// queued. (20 columns, 456 partials: 7.9 -> 6.6 us.)
+#define CF_WARPS 4
+__global__ void __launch_bounds__(32 * CF_WARPS)
 k_colsum_finalize(int nblk, int k, const double *__restrict__ part, double *sums, double *rho1, double *rho2,
                   const double *__restrict__ err, int *nact, double rate, double *beta)
 {
     GB_PDL();
-    __shared__ int cnt;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ int cnt, last;
+    const int lane = threadIdx.x & 31, c0 = blockIdx.x * CF_WARPS + (threadIdx.x >> 5);
     const int ka = *nact;
-    if (threadIdx.x == 0) cnt = 0;
-    for (int c = warp; c < ka; c += 32) {
-        double s = 0;
-        for (int b = lane; b < nblk; b += 32) s += part[(long)b * k + c];
+    if (c0 < ka) {
+        double s = cs_strided<8>(part + c0, k, lane, nblk, 32);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) sums[c] = s;
+        if (lane == 0) sums[c0] = s;
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        cnt = 0;
+        last = atomicAdd(nact + 1, 1) == (int)gridDim.x - 1;
     }
     __syncthreads();
+    if (!last) return;
+    __threadfence();
     for (int c = threadIdx.x; c < k; c += blockDim.x) {
         if (c < ka) {
-            const double s = sums[c];
+            const double s = __ldcg(sums + c);
             rho1[c] = rho2[c];
             rho2[c] = s;
             beta[c] = s / rho1[c];   // the next round's beta (src/gcge_cg.c:219)
@@ -610,7 +661,10 @@ k_colsum_finalize(int nblk, int k, const double *__restrict__ part, double *sums
         if (lerr / err[c] >= rate) atomicAdd(&cnt, 1);
     }
     __syncthreads();
-    if (threadIdx.x == 0) *nact = cnt;
+    if (threadIdx.x == 0) {
+        nact[0] = cnt;
+        nact[1] = 0;
+    }
 }
 
 typedef void (*pupdate_fn)(int, int, const float *, float *, long, const double *, const int *, int,
@@ -640,7 +694,7 @@ static int bcg_rounds32(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, float *R, floa
                         : k <= 128 ? k_spmm32_dot<16, 2> : k_spmm32_dot<32, 2>;
     const int Gp = vec_blocks(ctx, (const void *)pup, n, ctiles);
     const int Gs = vec_blocks(ctx, (const void *)spm, n, 1);
-    const int Gx = vec_blocks(ctx, (const void *)xru, n, ctiles);
+    const int Gx = xr_blocks(ctx, tpr, n, ctiles);
     // rows longer than GB_LONG_ROW: a launch of their own before the grid-stride
     // product (one wave of blocks over the sorted list); its p.w partials follow
     // the Gs rows of the other launch in part, which holds LONG_PART_ROWS rows
@@ -677,7 +731,7 @@ static int bcg_rounds32(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, float *R, floa
         GB_PROF(ctx, GB_K_BCGVEC, 24.0 * n * k, 6.0 * n * k);
         GB_LAUNCH(ctx, xru, dim3(Gx, ctiles), VB_THREADS, 0, n, k, X, R, P, W, ld, s->alpha, s->nact, s->part,
                   a->dinv32);
-        GB_LAUNCH(ctx, k_colsum_finalize, 1, 1024, 0, Gx, k, s->part, s->sums, s->rho1, s->rho2, s->err, s->nact,
+        GB_LAUNCH(ctx, k_colsum_finalize, cdiv(k, CF_WARPS), 32 * CF_WARPS, 0, Gx, k, s->part, s->sums, s->rho1, s->rho2, s->err, s->nact,
                   a->rate, s->beta);
     }
     return GCGE_GPU_OK;

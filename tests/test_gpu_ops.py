@@ -349,6 +349,28 @@ def test_bcg_fp64_on_the_sides_of_its_forms(ctx, shape, k, rounds, rate):
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
 
 
+@pytest.mark.parametrize("shape,k", [((1, 1), 1), ((43, 3), 3), ((30, 30), 4), ((91, 77), 5), ((91, 77), 13), ((120, 90), 20),
+                                     ((300, 280), 33), ((300, 280), 64), ((91, 77), 65), ((91, 77), 130), ((60, 50), 256)])
+def test_bcg_mixed_precision_widths(ctx, shape, k):
+    """Every width of the FP32 rounds' kernels, a part of a float4 group and of a block of
+    column sums included. Condition numbers are at most 25 and nothing leaves the active range:
+    six rounds with rows of five entries lose a few hundred units of 2^-24 of the correction
+    at most, 2e-5; 1e-4 is above that and far below any wrong term. Twice the same bits."""
+    A, _ = P.laplace2d(*shape)
+    A = P.CSR.from_scipy(A.to_scipy() + 4.0 * __import__("scipy.sparse").sparse.identity(A.n))
+    rng = np.random.default_rng(k)
+    R0, W0 = rng.standard_normal((A.n, k)), 0.1 * rng.standard_normal((A.n, k))
+    dA = ctx.matrix(A, keep_fp32=True)
+    out = []
+    for _ in range(2):
+        r, w = ctx.multivec(A.n, k, R0), ctx.multivec(A.n, k, W0)
+        G.bcg(dA, r, 0, w, 0, k, cg_max_it=7, cg_rate=1e-30, precision=1)
+        out.append(w.download())
+    x, _ = _block_cg(A.to_scipy(), R0, W0, 6, 1e-30)
+    assert np.linalg.norm(out[0] - x) < 1e-4 * np.linalg.norm(x - W0)
+    assert np.array_equal(out[0], out[1])
+
+
 @pytest.mark.parametrize("n,k,dep", [(400, 1, 0), (400, 33, 4), (900, 129, 7), (900, 160, 0), (900, 161, 5), (2500, 250, 9)])
 def test_orthonormalize_widths(ctx, n, k, dep):
     """Blocks at the sides of the Cholesky's forms (a warp's columns, all of a block's, the
