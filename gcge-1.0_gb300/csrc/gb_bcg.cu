@@ -14,9 +14,10 @@
 //
 // precision 0: FP64 vectors and values, all rounds in one launch
 // (gb_bcg_persist.cu). precision 1: the residual of the initial guess is formed in
-// FP64, then CG runs on the correction with FP32 vectors and the FP32 copy of the matrix values; products are formed in FP32 and summed in
-// FP32 over runs of 8 rows, then accumulated in FP64 (FP64-reduced dot products);
-// the correction is added to the FP64 solution at the end.
+// FP64, then CG runs on the correction with FP32 vectors and the FP32 copy of the
+// matrix values; products are formed in FP32 and summed in FP32 over runs of 8 rows,
+// then accumulated in FP64 (FP64-reduced dot products); the correction is added to
+// the FP64 solution at the end.
 #include <cuda_runtime.h>
 
 #include "gb_bcg.h"

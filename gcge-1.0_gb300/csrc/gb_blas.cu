@@ -1049,7 +1049,7 @@ extern "C" int gb_gram(gcge_gpu_ctx *ctx, int n, int k1, int k2, const double *V
                        long ldw, double *a_dev, int lda, int sym)
 {
     if (k1 <= 0 || k2 <= 0) return GCGE_GPU_OK;
-    if (ctx->tc) {
+    if (ctx->tc && ldv < GB_TC_MAX_LD && ldw < GB_TC_MAX_LD) {
         int st = gb_iscratch(ctx, gb_gram_tc_ints(k1, k2));
         if (st) return st;
         return gb_gram_tc(ctx, n, k1, k2, V, ldv, W, ldw, a_dev, lda, sym, ctx->iscratch);
@@ -1125,9 +1125,9 @@ k_lincomb(int n, int k1, int k2, const double *__restrict__ X, long ldx, const d
     }
 }
 
-extern "C" int gb_lincomb_inplace_ok(const gcge_gpu_ctx *ctx, int k1, int k2)
+extern "C" int gb_lincomb_inplace_ok(const gcge_gpu_ctx *ctx, int k1, int k2, long ldx)
 {
-    return ctx->tc && gb_lincomb_tc_inplace_ok(k1, k2);
+    return ctx->tc && gb_lincomb_tc_inplace_ok(k1, k2, ldx);
 }
 
 extern "C" int gb_lincomb(gcge_gpu_ctx *ctx, int n, int k1, int k2, const double *X, long ldx,
@@ -1136,7 +1136,7 @@ extern "C" int gb_lincomb(gcge_gpu_ctx *ctx, int n, int k1, int k2, const double
 {
     if (n <= 0 || k2 <= 0) return GCGE_GPU_OK;
     if (k1 <= 0) return gb_axpby(ctx, n, k2, 0.0, Y, ldy, beta, Y, ldy);
-    if (ctx->tc && gb_lincomb_tc_ok(k1)) return gb_lincomb_tc(ctx, n, k1, k2, X, ldx, C_dev, ldc, alpha, beta, Y, ldy, upper);
+    if (ctx->tc && gb_lincomb_tc_ok(k1, ldx)) return gb_lincomb_tc(ctx, n, k1, k2, X, ldx, C_dev, ldc, alpha, beta, Y, ldy, upper);
     dim3 grid(ceil_div_l(n, 64), (k2 + 31) / 32);
     GB_PROF(ctx, GB_K_LINCOMB, 8.0 * n * k1 + (beta != 0.0 ? 16.0 : 8.0) * n * k2,
             upper ? 1.0 * n * k1 * (k2 + 1) : 2.0 * n * k1 * k2);

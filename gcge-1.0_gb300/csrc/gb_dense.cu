@@ -13,8 +13,8 @@
 //  * gb_syevx: partial symmetric eigensolver with the structure of LAPACK's
 //    dsyevx for a range of indices (the routine the reference calls in
 //    GCGE_Default_DenseMatEigenSolver, src/gcge_ops.c:302-316): Householder
-//    tridiagonalisation, bisection on Sturm counts (32-way multisection per
-//    warp), inverse iteration with reorthogonalisation inside clusters of close
+//    tridiagonalisation, bisection on Sturm counts (32-way multisection, four
+//    rounds a pass), inverse iteration with reorthogonalisation inside clusters of close
 //    eigenvalues, and back-transformation by the stored reflectors.
 #include <cfloat>
 #include <cooperative_groups.h>
@@ -1128,8 +1128,9 @@ __device__ __forceinline__ int sturm_count(int m, const double *d, const double 
 // warps takes as long as one: warp L counts at the points of the L-th round from
 // here, along the path that an estimate of the eigenvalue predicts (at first the guess,
 // then the zero of det(T - x I) by inverse interpolation through the four points
-// around its sign change; the last ratio alone says nothing where T all but splits). Rounds whose predicted interval turns out to be the actual one are
-// done; the first always is. m = 33: 149 us (one round a pass, IEEE divisions) -> 92.
+// around its sign change; the last ratio alone says nothing where T all but splits).
+// Rounds whose predicted interval turns out to be the actual one are done; the first
+// always is. m = 33: 149 us (one round a pass, IEEE divisions) -> 92.
 #define BI_WARPS 4
 __global__ void __launch_bounds__(32 * BI_WARPS)
 k_bisect(int m, const double *__restrict__ dg, const double *__restrict__ eg, int il, int iu,

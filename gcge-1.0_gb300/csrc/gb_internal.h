@@ -132,12 +132,14 @@ int gb_gram_tc(gcge_gpu_ctx *ctx, int n, int k1, int k2, const double *V, long l
 size_t gb_gram_fixed_ctl_bytes(void);
 int gb_gram_fixed(cudaStream_t stream, int num_sms, int n, int k1, int k2, const double *V, long ldv, const double *W,
                   long ldw, double *a_dev, int lda, int sym, double *part, size_t part_cap, void *ctl_dev);
-/* FP64-accurate Y = alpha X C + beta Y on the tensor cores (gb_ozaki.cu), for k1 where
- * gb_lincomb_tc_ok(k1) holds */
-int gb_lincomb_tc_ok(int k1);
-int gb_lincomb_tc_inplace_ok(int k1, int k2);
+/* FP64-accurate Y = alpha X C + beta Y on the tensor cores (gb_ozaki.cu), where
+ * gb_lincomb_tc_ok(k1, ldx) holds */
+int gb_lincomb_tc_ok(int k1, long ldx);
+int gb_lincomb_tc_inplace_ok(int k1, int k2, long ldx);
 /* 1 when gb_lincomb may write Y over columns of X (same rows, same ld) */
-int gb_lincomb_inplace_ok(const gcge_gpu_ctx *ctx, int k1, int k2);
+int gb_lincomb_inplace_ok(const gcge_gpu_ctx *ctx, int k1, int k2, long ldx);
+/* row strides that the tensor-core kernels take: offsets within a tile's 128 rows fit an int */
+#define GB_TC_MAX_LD (1L << 24)
 int gb_lincomb_tc(gcge_gpu_ctx *ctx, int n, int k1, int k2, const double *X, long ldx, const double *C, int ldc,
                   double alpha, double beta, double *Y, long ldy, int upper);
 

@@ -746,7 +746,7 @@ extern "C" int gb_gram_fixed(cudaStream_t stream, int num_sms, int n, int k1, in
     gn_ctl *ctl = (gn_ctl *)ctl_dev;
     int st = GCGE_GPU_OK;
     const int *run = nullptr;
-    if (k1 + k2 <= GB_GRAM_FIXED_COLS) {
+    if (k1 + k2 <= GB_GRAM_FIXED_COLS && ldv < GB_TC_MAX_LD && ldw < GB_TC_MAX_LD) {
         const int ti = (k1 + TC_M - 1) / TC_M, tj = (k2 + TC_N - 1) / TC_N;
         long rps = 0;
         const long nsplit = gram_tc_splits(num_sms, n, k1, k2, sym, &rps), total = (long)k1 * k2;
@@ -1137,12 +1137,12 @@ k_lincomb_tc(int n, int k1, int k2, const double *__restrict__ X, long ldx, cons
     tc_release(h, tmem, mma_warp, commits, copies);
 }
 
-extern "C" int gb_lincomb_tc_ok(int k1) { return k1 <= LC_MAX_K; }
+extern "C" int gb_lincomb_tc_ok(int k1, long ldx) { return k1 <= LC_MAX_K && ldx < GB_TC_MAX_LD; }
 // Y may overlap X's columns (the same rows, the same leading dimension) when one
 // column tile covers the output: a CTA reads every entry of its row tile before
 // its drain writes that tile's rows, and walks only its own tiles (the
 // next-tile prefetch and scale pass included)
-extern "C" int gb_lincomb_tc_inplace_ok(int k1, int k2) { return k1 <= LC_MAX_K && k2 <= TC_N; }
+extern "C" int gb_lincomb_tc_inplace_ok(int k1, int k2, long ldx) { return gb_lincomb_tc_ok(k1, ldx) && k2 <= TC_N; }
 
 // Y = alpha X C + beta Y (C: k1 x k2 column-major on the device, upper: only
 // i <= j of C is used) to FP64 accuracy on the tensor cores.
