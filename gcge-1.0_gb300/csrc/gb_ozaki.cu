@@ -735,9 +735,12 @@ extern "C" int gb_gram_fixed_reduce(cudaStream_t stream, int num_sms, int k1, in
 // Gram V^T W with caller-provided partials (part_cap doubles), control block and
 // stream: no context, no allocation; part_cap >= 2 k1 k2. The tensor-core form where
 // its estimate is the shorter one. Measured on the GB300: a CTA takes a stage of 32
-// rows in 2.6 us for a few columns and 4.6 us for a full tile, and the form has 40 us
-// of launches, scales and drain beside it; the FP64 pipe takes 8.2 us for 32 rows of
-// a 32 x 32 tile on each SM, and 12 us.
+// rows, its share of the column pass included, in 1.4 us for a few columns and 3.8 us for
+// a full tile, and the form has 22 us of launches, scales and drain beside it, 36 for many
+// outputs; the FP64 pipe takes 8.2 us for 32 rows of a 32 x 32 tile on each SM, 0.055 us
+// a split to sum, and 8 us. Both sides, us, tensor cores / FP64 pipe: 3,500 rows, 3 x 3
+// 25 / 22, 33 x 16 30 / 33, 64 x 64 42 / 42; 5,000 rows 26 / 34, 31 / 46, 45 / 64;
+// 1,000 rows of 178 x 64 41 / 33, 2,000 43 / 58.
 extern "C" long gb_gram_fixed_splits(int num_sms, int n, int k1, int k2, int sym, size_t part_cap, long *rps_out);
 extern "C" int gb_gram_fixed(cudaStream_t stream, int num_sms, int n, int k1, int k2, const double *V, long ldv,
                              const double *W, long ldw, double *a_dev, int lda, int sym, double *part,
@@ -752,11 +755,13 @@ extern "C" int gb_gram_fixed(cudaStream_t stream, int num_sms, int n, int k1, in
         const long nsplit = gram_tc_splits(num_sms, n, k1, k2, sym, &rps), total = (long)k1 * k2;
         const double waves = (double)(((long)ti * tj * nsplit + num_sms - 1) / num_sms);
         const double fill = (double)((k1 < TC_M ? k1 : TC_M) + (k2 < TC_N ? k2 : TC_N)) / (TC_M + TC_N);
-        const double t_tc = 40.0 + waves * (double)(rps / TC_KS) * (2.6 + 2.0 * fill);
+        const double t_tc = 22.0 + 14.0 * (total < 8192 ? (double)total / 8192 : 1.0) +
+                            waves * (double)(rps / TC_KS) * (1.35 + 2.5 * fill);
         long rps64 = 0;
         const long n64 = gb_gram_fixed_splits(num_sms, n, k1, k2, sym, part_cap, &rps64);
         const long b64 = n64 * ((k1 + 31) / 32) * ((k2 + 31) / 32);
-        const double t_64 = 12.0 + 8.2 * (double)(rps64 / 32) * (double)((b64 + num_sms - 1) / num_sms);
+        const double t_64 = 8.0 + 0.055 * (double)n64 +
+                            8.2 * (double)(rps64 / 32) * (double)((b64 + num_sms - 1) / num_sms);
         if (t_tc < t_64) {
             if (cudaFuncSetAttribute(k_gram_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, GR_SMEM) != cudaSuccess)
                 return GCGE_GPU_ERR_CUDA;

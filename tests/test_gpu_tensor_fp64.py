@@ -264,6 +264,12 @@ def test_no_alloc_gram_sides_of_the_tiles(n, k1, k2):
     assert np.all(np.isfinite(got))
 
 
+@pytest.mark.parametrize("n,k1,k2", [(3500, 3, 3), (5000, 3, 3), (2000, 33, 16), (3500, 33, 16), (1000, 178, 64), (2000, 178, 64)])
+def test_no_alloc_gram_on_both_sides_of_the_line(n, k1, k2):
+    """The shortest blocks that go to the tensor cores and the longest that do not: the same bound."""
+    test_no_alloc_gram_sides_of_the_tiles(n, k1, k2)
+
+
 @pytest.mark.parametrize("what", ["spike", "range", "nan", "inf", "subnormal", "zero"])
 def test_no_alloc_gram_columns_that_a_scale_does_not_serve(what):
     """Columns whose entries lie far below the largest, and entries without digits, get
