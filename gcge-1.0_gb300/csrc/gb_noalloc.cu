@@ -7,9 +7,9 @@
 // point computes the same Gram block as GCGE_GPU_MultiVecInnerProd into memory
 // the caller passes, with its partial sums in a fixed file-scope device array
 // instead of the library's context scratch, and allocates nothing. It runs on the
-// tensor cores (gb_ozaki.cu: gb_gram_fixed) where that is the shorter way and every
-// column's entries lie close enough together for the digits that a column scale
-// leaves them, and on the FP64 pipe (k_gram_partial, plain FP64 fused multiply-adds
+// tensor cores (gb_ozaki.cu: gb_gram_fixed) where that is the shorter way and the
+// operands prove that the digits which column scales leave them keep every entry within
+// the bound of a plain FP64 sum, and on the FP64 pipe (k_gram_partial, plain FP64 fused multiply-adds
 // with a fixed-order second stage) otherwise: at 262,144 x (178, 64) 5.45 ms on the
 // FP64 pipe, 0.64 ms on the tensor cores; at 600,000 x (256, 128) 32.7 and 2.5 ms.
 //

@@ -616,17 +616,26 @@ extern "C" int gb_gram_tc(gcge_gpu_ctx *ctx, int n, int k1, int k2, const double
 // The allocation-free Gram on the tensor cores. What the FP64-pipe form took at
 // 262,144 x (178, 64) was the FP64 pipe itself: 5.44 ms at 1.1 of 1.2 TFLOP/s.
 //
-// Column scales serve every row of a column, so an entry far below its column's
-// largest keeps fewer bits than FP64 would. k_col_stats therefore forms, beside the
-// scale e (max |x| < 2^e), the mean exponent of the nonzero entries, and the block
-// that finishes last sets ctl->skip when a column's mean lies more than
-// GN_SPREAD below its e, or an entry is not finite or subnormal: the FP64-pipe kernel that
-// follows then does the work, and nothing otherwise. With GN_SPREAD = 5 the digits
-// of a typical entry end 2^-49 below it and their roundings are independent, so
-// their sum over n rows stays under the FP64 form's own summation error (normal
-// and smooth columns, n from 1,000 to 600,000: 0.4 to 0.02 of it). A bounded wait
+// Column scales serve every row of a column: an entry x of a column with scale e (|x| < 2^e) is
+// held to 2^(e - 54), so a small one keeps fewer bits than FP64 would, and a product of two
+// such entries may be all that a sum consists of. The tensor form is therefore taken
+// only where the data prove the bound of a plain FP64 sum, n 2^-53 sum |v w|, for every
+// entry of the result. k_col_stats forms, beside a column's scale e, the number q of its
+// nonzeros and the sum g of their gaps (e less the entry's exponent, |x| >= 2^(e - 1 - gap)).
+// With q >= a n, g <= G n for every column of V that is not all zero and q' >= a' n,
+// g' <= G' n for W's, at least s n = (a + a' - 1) n rows have both factors, and by the
+// arithmetic-geometric mean over them
+//   sum |v w| >= s n 2^(e + f - 2 - (G + G') / s).
+// The digits' error, roundings of the entries at 2^-54 of their scales and dropped pairs at
+// 2^-57.4, is at most 1.05 n 2^(e + f - 53), which lies below (n - 1) 2^-53 sum |v w| where
+//   (G + G') / s <= log2((n - 1) s) - 2.1.
+// GN_SPREAD caps the left side for large n: the digits' roundings are independent as a rule, and with
+// a mean gap of 5 in both factors their sum over n rows stays near the FP64 form's own error (normal
+// and smooth columns, n from 1,000 to 600,000: 0.4 to 0.02 of it). Otherwise, and where an
+// entry is not finite or subnormal, the block that finishes last sets ctl->skip: the
+// FP64-pipe kernel that follows then does the work, and nothing otherwise. A bounded wait
 // that runs out sets skip as well.
-#define GN_SPREAD 5
+#define GN_SPREAD 10.0f
 struct gn_ctl {
     int skip;
     unsigned done;
@@ -660,7 +669,8 @@ k_col_stats(int n, int k1, const double *__restrict__ V, long ldv, int k2, const
 {
     GB_PDL();
     __shared__ int se[8][CE_COLS], sc[8][CE_COLS], ss[8][CE_COLS];
-    __shared__ int done, wide;
+    __shared__ int done, wide, fewest[2];                // of V and of W: the fewest nonzeros, the largest sum of gaps
+    __shared__ unsigned long long gaps[2];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int k = blockIdx.y ? k2 : k1, off = blockIdx.y ? k1 : 0;
     const double *X = blockIdx.y ? W : V;
@@ -713,17 +723,26 @@ k_col_stats(int n, int k1, const double *__restrict__ V, long ldv, int k2, const
     if (threadIdx.x == 0) {
         done = atomicAdd(&ctl->done, 1u) == gridDim.x * 2 - 1;
         wide = 0;
+        fewest[0] = fewest[1] = n;
+        gaps[0] = gaps[1] = 0;
     }
     __syncthreads();
     if (!done) return;
     __threadfence();
     for (int c = threadIdx.x; c < k1 + k2; c += blockDim.x) {
-        const long long q = __ldcg(&ctl->cnt[c]), t = __ldcg(&ctl->sum[c]);
-        const int m = __ldcg(&ctl->e[c]);
-        if (m > 1024 || (long long)m * q - t > GN_SPREAD * q) wide = 1;   // e = 1025: not finite, or subnormal
+        const int q = __ldcg(&ctl->cnt[c]), m = __ldcg(&ctl->e[c]), op = c >= k1;
+        if (m > 1024) wide = 1;                            // e = 1025: not finite, or subnormal
+        if (q && m <= 1024) {
+            atomicMin(&fewest[op], q);
+            atomicMax(&gaps[op], (unsigned long long)((long long)m * q - __ldcg(&ctl->sum[c])));
+        }
     }
     __syncthreads();
-    if (threadIdx.x == 0 && wide) ctl->skip = 1;
+    if (threadIdx.x == 0) {
+        const float both = (float)((long long)fewest[0] + fewest[1] - n);      // s n
+        const float gap = (float)(gaps[0] + gaps[1]);                          // (G + G') n
+        if (wide || !(both > 0.0f) || gap > both * fminf(GN_SPREAD, log2f(both) - 2.1f)) ctl->skip = 1;
+    }
 }
 
 extern "C" int gb_gram_fixed_partials(cudaStream_t stream, int num_sms, int n, int k1, int k2, const double *V,

@@ -316,6 +316,10 @@ int  GCGE_GPU_EigvecAdjoint(const gcge_gpu_mat *A, const gcge_gpu_mat *B, const 
  *          (the multivector layout of this library), n rows, k1 / k2 columns;
  *   a      device pointer, column major with leading dimension lda >= k1;
  *   stream a cudaStream_t (NULL: the default stream); the call is asynchronous.
+ * Every entry is within n 2^-53 sum_r |V(r, i)| |W(r, j)| of the exact one, the bound of a
+ * plain FP64 sum: the tensor cores do the work only where a pass over the operands
+ * has shown that (dense columns without a wide spread), the FP64 pipe otherwise,
+ * and where an entry is not finite or subnormal.
  * Partial sums go to a fixed 8 MiB device array inside the library, with 64 KiB of
  * column scales beside it (held by every GPU that loads it, until exit), so k1*k2
  * may be at most 262,144.

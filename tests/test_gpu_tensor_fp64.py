@@ -300,3 +300,39 @@ def test_no_alloc_gram_columns_that_a_scale_does_not_serve(what):
         np.testing.assert_allclose(got, ref, rtol=n * 2.0 ** -53)
     else:
         np.testing.assert_array_equal(got, ref)
+
+
+@pytest.mark.parametrize("what", ["rows45", "rows40", "smallest", "ones", "third", "two thirds", "nine tenths"])
+def test_no_alloc_gram_small_entries_facing_the_other_factors_nonzeros(what):
+    """A column scale that serves most of a column, and a second factor that is nonzero where
+    it does not: the bound of plain FP64 sums, n 2^-53 sum |v w|, for every entry."""
+    torch = pytest.importorskip("torch")
+    n, k1, k2 = 70000, 130, 66
+    rng = np.random.default_rng(17)
+    v, w = rng.standard_normal((n, k1)), np.zeros((n, k2))
+    if what == "rows45":
+        rows = rng.choice(n, 64, replace=False)
+        v[rows] *= 2.0 ** -45
+        w[rows] = rng.standard_normal((64, k2))
+    elif what == "rows40":                               # 3% of the rows in another unit
+        rows = rng.choice(n, 3 * n // 100, replace=False)
+        v[rows] *= 2.0 ** -40
+        w[rows] = rng.standard_normal((len(rows), k2))
+    elif what == "smallest":                             # the unit vector at a column's smallest entry
+        w[np.abs(v[:, :k2]).argmin(axis=0), np.arange(k2)] = 1.0
+    elif what == "ones":
+        v[:] = 1.0
+        v[11] = 2.0 ** -60
+        w[11] = 1.0
+    elif what == "third":
+        w = rng.standard_normal((n, k2)) * (rng.random((n, k2)) < 0.33)
+    else:                                                # zeros in both factors
+        p = 0.67 if what == "two thirds" else 0.9
+        v *= rng.random((n, k1)) < p
+        w = rng.standard_normal((n, k2)) * (rng.random((n, k2)) < p)
+    got = _no_alloc(torch, torch.from_numpy(v).cuda(), torch.from_numpy(w).cuda(), k1, k2)
+    for j in range(k2):
+        r = np.flatnonzero(w[:, j])
+        for i in (range(k1) if len(r) < 100 else (0, j, k1 - 1)):
+            t = v[r, i].astype(np.longdouble) * w[r, j]
+            assert abs(got[i, j] - t.sum()) <= n * 2.0 ** -53 * float(np.abs(t).sum()), (i, j)
