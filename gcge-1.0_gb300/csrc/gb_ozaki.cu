@@ -308,15 +308,16 @@ k_col_exponent(int n, int k1, const double *__restrict__ V, long ldv, int k2, co
     }
 }
 
-// start of a Gram: column exponents unset, tickets and integer sums zero
+// start of a Gram: column exponents unset, tickets and integer sums zero (a grid of at most
+// 65,536 threads, whatever their number)
 __global__ void k_gram_init(int *__restrict__ exps, int cols, unsigned *__restrict__ ticket, int tiles,
                             ulonglong2 *__restrict__ sums, long total)
 {
     GB_PDL();
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < cols) exps[i] = OZ_NO_EXP;
-    if (i < tiles) ticket[i] = 0;
-    for (long t = i; t < total; t += (long)gridDim.x * blockDim.x) sums[t] = make_ulonglong2(0, 0);
+    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x, step = (long)gridDim.x * blockDim.x;
+    for (long t = i; t < cols; t += step) exps[t] = OZ_NO_EXP;
+    for (long t = i; t < tiles; t += step) ticket[t] = 0;
+    for (long t = i; t < total; t += step) sums[t] = make_ulonglong2(0, 0);
 }
 
 // ---------------------------------------------------------------- Gram V^T W (tcgen05)

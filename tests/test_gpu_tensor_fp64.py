@@ -336,3 +336,17 @@ def test_no_alloc_gram_small_entries_facing_the_other_factors_nonzeros(what):
         for i in (range(k1) if len(r) < 100 else (0, j, k1 - 1)):
             t = v[r, i].astype(np.longdouble) * w[r, j]
             assert abs(got[i, j] - t.sum()) <= n * 2.0 ** -53 * float(np.abs(t).sum()), (i, j)
+
+
+def test_tensor_gram_scales_of_many_columns(ctx):
+    """More columns than the threads that start a Gram's scales, after a Gram with far larger
+    scales in the same scratch: integers below 2^8, so the product itself."""
+    n, k1 = 160, 65600
+    rng = np.random.default_rng(6)
+    V, W = rng.integers(-9, 10, (n, k1)).astype(float), rng.integers(-9, 10, (n, 1)).astype(float)
+    ref = V.T @ W
+    v, w = ctx.multivec(n, k1, V * 2.0 ** 300), ctx.multivec(n, 1, W)
+    big = G.multivec_inner_prod(v, w, (0, 0), (k1, 1), k1)
+    v.upload(V)
+    assert np.array_equal(G.multivec_inner_prod(v, w, (0, 0), (k1, 1), k1), ref[:, 0])
+    assert np.array_equal(big, ref[:, 0] * 2.0 ** 300)
