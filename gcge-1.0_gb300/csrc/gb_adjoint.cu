@@ -62,6 +62,8 @@ k_pattern_grad(int n, const int *__restrict__ rp, const int *__restrict__ ci, co
     for (int i = threadIdx.x; i <= nr; i += PG_THREADS) first[i] = rp[i0 + i];
     __syncthreads();
     const int e0 = first[0], e1 = first[nr], sub = threadIdx.x % LPE;
+    // the lanes of an entry: one k for all of them, but loops over t of unequal length
+    const unsigned group = ((1u << LPE) - 1) << ((threadIdx.x & 31) & ~(LPE - 1));
     for (int base = e0; base < e1; base += PG_CHUNK) {
         const int cnt = min(PG_CHUNK, e1 - base);
         // four threads list a row's entries
@@ -76,7 +78,7 @@ k_pattern_grad(int n, const int *__restrict__ rp, const int *__restrict__ ci, co
 #pragma unroll 4
             for (int t = sub; t < r; t += LPE) sum = fma(ur[t], __ldg(vr + t), sum);
 #pragma unroll
-            for (int o = 1; o < LPE; o <<= 1) sum += __shfl_xor_sync(__activemask(), sum, o, LPE);
+            for (int o = 1; o < LPE; o <<= 1) sum += __shfl_xor_sync(group, sum, o, LPE);
             if (sub == 0) grad[base + k] = acc ? grad[base + k] + sum : sum;
         }
         __syncthreads();

@@ -66,6 +66,20 @@ def test_pattern_grad_row_runs(ctx, r):
         assert np.all(np.abs(g[b:b + 2000] - t.sum(1)) <= (r + 2) * 2.0 ** -52 * np.abs(t).sum(1))
 
 
+@pytest.mark.parametrize("r", [5, 31, 33, 34, 35])
+def test_pattern_grad_uneven_lanes(ctx, r):
+    """Widths that give the lanes of an entry unequal shares, and entries that leave lanes of the last
+    warp without one: within (r + 2) 2^-52 of the sum of the products' magnitudes."""
+    rng = np.random.default_rng(r)
+    for n in (1, 3, 37):
+        A = P.laplace2d(n, 1)[0]
+        U, V, s = rng.standard_normal((n, r)), rng.standard_normal((n, r)), rng.standard_normal(r)
+        g = G.pattern_grad(ctx.matrix(A), ctx.multivec(n, r, U), 0, ctx.multivec(n, r, V), 0, r, s, A.nnz)
+        rows, cols = AD.pattern(A)
+        t = (U[rows].astype(np.longdouble) * V[cols]) * s
+        assert np.all(np.abs(g - t.sum(1)) <= (r + 2) * 2.0 ** -52 * np.abs(t).sum(1))
+
+
 @pytest.mark.parametrize("m,what", [(1, "grid"), (17, "grid"), (33, "B"), (64, "grid"), (65, "B"), (12, "graph")])
 def test_eigvec_adjoint_forms(ctx, m, what):
     """Widths at the lanes' and the launch's limits, with and without B, and rows that take
