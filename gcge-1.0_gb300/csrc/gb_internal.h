@@ -138,8 +138,9 @@ int gb_lincomb_tc_ok(int k1, long ldx);
 int gb_lincomb_tc_inplace_ok(int k1, int k2, long ldx);
 /* 1 when gb_lincomb may write Y over columns of X (same rows, same ld) */
 int gb_lincomb_inplace_ok(const gcge_gpu_ctx *ctx, int k1, int k2, long ldx);
-/* row strides that the tensor-core kernels take: offsets within a tile's 128 rows fit an int */
-#define GB_TC_MAX_LD (1L << 24)
+/* row strides below which the tensor-core kernels' offsets within a stage fit an int (in entries; the lanes
+ * dealt past a tile's 128 rows reach row 151). Wider blocks take the FP64 pipe. */
+#define GB_TC_MAX_LD (1L << 23)
 int gb_lincomb_tc(gcge_gpu_ctx *ctx, int n, int k1, int k2, const double *X, long ldx, const double *C, int ldc,
                   double alpha, double beta, double *Y, long ldy, int upper);
 

@@ -808,6 +808,9 @@ extern "C" int gb_gram_fixed(cudaStream_t stream, int num_sms, int n, int k1, in
 #define LC_OUT_LD (TC_N + 1)                         // doubles per staged output row
 #define LC_CORES_PER_WARP ((TC_ACORES + TC_SPLIT_WARPS - 1) / TC_SPLIT_WARPS)
 #define LC_SCALE_LOADS 48                            // row-scale loads in flight per thread
+// the largest of k_lincomb_tc's int offsets, a lane past the tile's cores among them (k_gram_tc's: 31 rows)
+static_assert((8L * ((TC_SPLIT_WARPS * LC_CORES_PER_WARP - 1) >> 2) + 7) * GB_TC_MAX_LD + TC_KS <= 0x7fffffffL,
+              "row strides of the tensor-core kernels");
 // Levels 0-7 (34 digit pairs; 8 x 64 TMEM columns): the dropped pairs (level >= 8)
 // lie below 2^-55 of the scale product per term; level 7 (weight 2^-56) needs no
 // exactness, levels 0-6 stay exact for OZ_EXACT_TERMS terms.
@@ -1021,14 +1024,15 @@ k_lincomb_tc(int n, int k1, int k2, const double *__restrict__ X, long ldx, cons
 
     unsigned pw[LC_CORES_PER_WARP][2];                   // high words of the next tile's entries, in flight
     auto load_words = [&](long row0, int s) {
-        const unsigned *Xs = reinterpret_cast<const unsigned *>(X + row0 * ldx + s * TC_KS) + 1;
+        const double *Xs = X + row0 * ldx + s * TC_KS;
         const bool full = row0 + TC_M <= n && (s + 1) * TC_KS <= k1;
 #pragma unroll
         for (int cc = 0; cc < LC_CORES_PER_WARP; ++cc) {
             const int q = warp + TC_SPLIT_WARPS * cc, left = k1 - s * TC_KS - (8 * (q & 3) + 2 * kp);
             const bool in = q < TC_ACORES && (full || row0 + 8 * (q >> 2) + r8 < n);
-            pw[cc][0] = in && (full || left > 0) ? __ldg(Xs + 2 * off[cc]) : 0u;
-            pw[cc][1] = in && (full || left > 1) ? __ldg(Xs + 2 * off[cc] + 2) : 0u;
+            const unsigned *xw = reinterpret_cast<const unsigned *>(Xs + off[cc]) + 1;
+            pw[cc][0] = in && (full || left > 0) ? __ldg(xw) : 0u;
+            pw[cc][1] = in && (full || left > 1) ? __ldg(xw + 2) : 0u;
         }
     };
     auto fold_words = [&](int *scales, int s) {          // into the scales of the words' tile

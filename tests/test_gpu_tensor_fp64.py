@@ -350,3 +350,18 @@ def test_tensor_gram_scales_of_many_columns(ctx):
     v.upload(V)
     assert np.array_equal(G.multivec_inner_prod(v, w, (0, 0), (k1, 1), k1), ref[:, 0])
     assert np.array_equal(big, ref[:, 0] * 2.0 ** 300)
+
+
+@pytest.mark.parametrize("ncols", [(1 << 23) - 2, 1 << 23, 8600000])
+def test_tensor_lincomb_row_strides(ctx, ncols):
+    """Row strides at the limit of a tile's int offsets, with a second tile for the one CTA a column tile
+    gets: the same integers on either side."""
+    n, k1, k2 = 130, 40, 64 * 77
+    rng = np.random.default_rng(7)
+    X, Cm = rng.integers(-99, 100, (n, k1)).astype(float), rng.integers(1, 100, (k1, k2)).astype(float)
+    x, y = ctx.multivec(n, ncols), ctx.multivec(n, k2)
+    x.upload(X)
+    G.multivec_linear_comb(x, y, (0, 0), (k1, k2), Cm.ravel(order="F"), k1)
+    out = y.download()
+    x.close()
+    assert np.array_equal(out, X @ Cm)
