@@ -1651,6 +1651,11 @@ static int cholqr_reorth(gcge_gpu_ctx *ctx, int m, int nev, double *Zt, double *
     return GCGE_GPU_OK;
 }
 
+// largest matrix: 52 bytes of shared memory a row in k_invit, 48 in k_backtransform, 16 in k_tridiag (below
+// the default of 48 KB) and k_bisect (above it with its 2.6 KB of static arrays)
+#define SY_MAX_M 3000
+static size_t bi_smem(int m) { return 2 * sizeof(double) * (size_t)m; }
+
 extern "C" int gb_syevx_guess(gcge_gpu_ctx *ctx, int m, const double *H, int ldh, int il, int iu, double *eval,
                               double *Z, int ldz, double *work, int *info_dev, const double *guess);
 extern "C" int gb_syevx(gcge_gpu_ctx *ctx, int m, const double *H, int ldh, int il, int iu, double *eval,
@@ -1663,7 +1668,7 @@ extern "C" int gb_syevx_guess(gcge_gpu_ctx *ctx, int m, const double *H, int ldh
                               double *Z, int ldz, double *work, int *info_dev, const double *guess)
 {
     if (m <= 0 || il < 1 || iu > m || il > iu) return gb_fail(ctx, GCGE_GPU_ERR_ARG);
-    if (m > 3000) return gb_fail(ctx, GCGE_GPU_ERR_ARG);   // dynamic shared memory of k_tridiag / k_bisect (2m doubles)
+    if (m > SY_MAX_M) return gb_fail(ctx, GCGE_GPU_ERR_ARG);
     const int nev = iu - il + 1;
     double *Aw = work, *d = Aw + (size_t)m * m, *e = d + m, *tau = e + m, *Zt = tau + m;
     if (cudaMemsetAsync(info_dev, 0, sizeof(int), ctx->stream) != cudaSuccess) return gb_fail(ctx, GCGE_GPU_ERR_CUDA);
@@ -1690,22 +1695,23 @@ extern "C" int gb_syevx_guess(gcge_gpu_ctx *ctx, int m, const double *H, int ldh
         else
             GB_LAUNCH(ctx, k_tridiag, 1, tthreads, 2 * m * sizeof(double), m, H, ldh, Aw, d, e, tau);
     }
-    GB_PROF(ctx, GB_K_EIG, 0.0, 0.0);
-    GB_LAUNCH(ctx, k_bisect, nev, 32 * BI_WARPS, 2 * m * sizeof(double), m, d, e, il, iu, eval, info_dev, guess);
-    GB_PROF(ctx, GB_K_EIG, 0.0, 0.0);
-    const size_t ismem = (size_t)m * (6 * sizeof(double) + sizeof(int));
-    // the 48 KB default covers static + dynamic shared memory together: both kernels
-    // are opened once to the most they can ask for (k_invit <= 156 KB at m = 3000,
-    // k_cluster_orth<true> <= 160 KB + its 8.3 KB static)
+    // the 48 KB default covers static and dynamic shared memory together: these kernels are
+    // opened once to the most they can ask for (k_bisect 48 KB at m = 3000, k_invit 156 KB,
+    // k_backtransform 144 KB, k_cluster_orth<true> 160 KB)
     static bool attrs = false;
     if (!attrs) {
-        if (cudaFuncSetAttribute(k_invit, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess ||
+        if (cudaFuncSetAttribute(k_bisect, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bi_smem(SY_MAX_M)) != cudaSuccess ||
+            cudaFuncSetAttribute(k_invit, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess ||
             cudaFuncSetAttribute(k_cluster_orth<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) !=
                 cudaSuccess ||
             cudaFuncSetAttribute(k_backtransform, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess)
             return gb_fail(ctx, GCGE_GPU_ERR_CUDA);
         attrs = true;
     }
+    GB_PROF(ctx, GB_K_EIG, 0.0, 0.0);
+    GB_LAUNCH(ctx, k_bisect, nev, 32 * BI_WARPS, bi_smem(m), m, d, e, il, iu, eval, info_dev, guess);
+    GB_PROF(ctx, GB_K_EIG, 0.0, 0.0);
+    const size_t ismem = (size_t)m * (6 * sizeof(double) + sizeof(int));
     GB_LAUNCH(ctx, k_invit, nev, 32, ismem, m, d, e, nev, eval, Zt, m);
     GB_PROF(ctx, GB_K_EIG, 0.0, 0.0);
     int reorth_done = 0;

@@ -233,3 +233,26 @@ def test_table_linear_solver_hook(env):
     assert ctx.lib.GCGE_GPU_OpsSetLinearSolver(C.byref(tab), 0, 20, 1e-2) == 0
     assert not tab.LinearSolver
     assert ctx.lib.GCGE_GPU_OpsSetLinearSolver(C.byref(tab), 2, 20, 1e-2) == 1
+
+
+@pytest.mark.parametrize("m", [2907, 2908, 3000])
+def test_table_dense_eigensolver_largest(env, m):
+    """The largest matrices that the eigensolver takes: the lowest four pairs of (I - 2 u u^T) D (I - 2 u u^T),
+    whose eigenvalues are D's."""
+    ctx, tab = env
+    rng = np.random.default_rng(m)
+    d = np.sort(rng.uniform(-3.0, 3.0, m))
+    u = rng.standard_normal(m)
+    u /= np.linalg.norm(u)
+    Du = d * u
+    M = np.diag(d) - 2.0 * np.outer(u, Du) - 2.0 * np.outer(Du, u) + 4.0 * (u @ Du) * np.outer(u, u)
+    M = 0.5 * (M + M.T)
+    ev, Z = np.zeros(4), np.zeros((4, m))
+    nev, info, dummy = C.c_int(), C.c_int(), C.c_double()
+    iv = lambda v: C.byref(C.c_int(v))  # noqa: E731
+    tab.DenseMatEigenSolver(b"V", b"I", b"U", iv(m), np.ascontiguousarray(M).ctypes.data_as(PD), iv(m), C.byref(dummy),
+                            C.byref(dummy), iv(1), iv(4), C.byref(dummy), C.byref(nev), ev.ctypes.data_as(PD),
+                            Z.ctypes.data_as(PD), iv(m), None, None, iv(8 * m), None, None, None, C.byref(info))
+    assert info.value == 0 and nev.value == 4
+    assert np.max(np.abs(ev - d[:4])) <= 1e-13 * m * 3.0
+    assert np.max(np.abs(M @ Z.T - Z.T * ev)) <= 1e-13 * m * 3.0
