@@ -359,12 +359,12 @@ static size_t cd_smem(int k, bool array)
 static int cd_launch(gcge_gpu_ctx *ctx, int k, const double *G, int ldg, double *T, int *kept_dev, double zero_tol,
                      double rel_tol, double *work, double *ratio_dev)
 {
-    if (k <= CD_SMEM_K) {
-        if (cudaFuncSetAttribute(k_chol_deflate, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)cd_smem(CD_SMEM_K, true)) != cudaSuccess)
-            return gb_fail(ctx, GCGE_GPU_ERR_CUDA);
-        work = nullptr;
-    }
+    // on either side of CD_SMEM_K (a wide block's pivots pass the default of 48 KB from 1,537 columns on):
+    // 208 KB, the matrix of 160 columns or the pivots of 6,640
+    if (cudaFuncSetAttribute(k_chol_deflate, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)cd_smem(CD_SMEM_K, true)) != cudaSuccess)
+        return gb_fail(ctx, GCGE_GPU_ERR_CUDA);
+    if (k <= CD_SMEM_K) work = nullptr;
     GB_LAUNCH(ctx, k_chol_deflate, 1, CD_THREADS, cd_smem(k, !work), k, G, ldg, T, kept_dev, zero_tol, rel_tol, work,
               ratio_dev);
     return GCGE_GPU_OK;

@@ -386,3 +386,23 @@ def test_orthonormalize_widths(ctx, n, k, dep):
     Q = w.download(0, end)
     assert np.max(np.abs(Q.T @ Q - np.eye(end))) < 1e-13
     assert np.linalg.norm(W0 - Q @ (Q.T @ W0)) < 1e-11 * np.linalg.norm(W0)
+
+
+def test_orthonormalize_wide_block_first_in_a_process():
+    """1,600 columns as a process' first block: no earlier, narrower call has raised a limit."""
+    import subprocess
+    import sys
+    code = """
+import numpy as np, sys
+sys.path[:0] = %r
+import gcge_gb300 as G
+with G.Context(0) as c:
+    n, k = 2000, 1600
+    V = np.random.default_rng(2).standard_normal((n, k))
+    v = c.multivec(n, k, V)
+    assert G.orthonormalize(v, 0, k) == k
+    Q = v.download()
+assert np.max(np.abs(Q.T @ Q - np.eye(k))) < 1e-11
+"""
+    r = subprocess.run([sys.executable, "-c", code % sys.path], capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stderr[-2000:]
