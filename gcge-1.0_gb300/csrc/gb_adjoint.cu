@@ -370,6 +370,7 @@ struct ac_args {
     ac_state *s;
     unsigned *bar;
     int *dev_err;
+    coop_limit limit;
 };
 enum { AC_PLAIN, AC_COEF, AC_PQ, AC_RR };
 
@@ -380,8 +381,9 @@ __device__ int ac_barrier(const ac_args &a, int op, int ns, unsigned &gen)
     __shared__ int last, res;
     __shared__ double sum0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, G = gridDim.x;
+    const unsigned lastn = a.limit.last;
     __syncthreads();
-    if (threadIdx.x == 0) last = coop_arrive(a.bar) == (unsigned)G - 1;
+    if (threadIdx.x == 0) last = coop_arrive(a.bar) == lastn;
     __syncthreads();
     if (last) {
         for (int j = warp; j < ns; j += AC_WARPS) {
@@ -424,7 +426,7 @@ __device__ int ac_barrier(const ac_args &a, int op, int ns, unsigned &gen)
         int spin = 0;
         unsigned long long v;
         while ((unsigned)((v = coop_ld64(a.bar + 2)) >> 32) == gen)
-            if ((++spin & 1023) == 0 && coop_now() - t0 > COOP_WAIT_NS) {
+            if ((++spin & 1023) == 0 && coop_now() - t0 > a.limit.ns) {
                 atomicExch(a.dev_err, 1);
                 v = 0xffffffffull;
                 break;
@@ -667,6 +669,7 @@ static int ad_iterate(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, const gcge_gpu_m
     if (per_sm > AV_BLOCKS_PER_SM) per_sm = AV_BLOCKS_PER_SM;   // the partials' room
     long G = (long)ctx->num_sms * per_sm, tiles = ((long)n + AC_ROWS - 1) / AC_ROWS;
     if (G > tiles) G = tiles;
+    a.limit = gb_coop_limit(ctx, G);
     void *args[] = {&a};
     if (cudaLaunchCooperativeKernel(k_adjoint_cg, dim3((unsigned)G), dim3(AC_ROWS), args, 0, ctx->stream) != cudaSuccess) {
         cudaGetLastError();

@@ -114,6 +114,13 @@ extern "C" int GCGE_GPU_TestStallTensorWait(gcge_gpu_ctx *ctx, int on)
     return GCGE_GPU_OK;
 }
 
+extern "C" int GCGE_GPU_TestStallGridWait(gcge_gpu_ctx *ctx, int on)
+{
+    if (!ctx) return GCGE_GPU_ERR_ARG;
+    ctx->coop_stall = on ? 1 : 0;
+    return GCGE_GPU_OK;
+}
+
 extern "C" int GCGE_GPU_SetPairSpMM(gcge_gpu_ctx *ctx, int on)
 {
     if (!ctx) return GCGE_GPU_ERR_ARG;
@@ -268,7 +275,7 @@ extern "C" const char *GCGE_GPU_ErrorString(int st)
     case GCGE_GPU_ERR_NONFINITE: return "non-finite value";
     case GCGE_GPU_ERR_BREAKDOWN: return "orthogonalisation lost every column";
     case GCGE_GPU_ERR_EIGSOLVE: return "projected eigensolve failed";
-    case GCGE_GPU_ERR_TIMEOUT: return "tensor-core kernel wait timed out";
+    case GCGE_GPU_ERR_TIMEOUT: return "a kernel's bounded wait timed out";
     case GCGE_GPU_ERR_IO: return "file missing, unreadable, truncated or not CSR";
     default: return "unknown status";
     }
@@ -794,7 +801,9 @@ extern "C" int GCGE_GPU_BCG(const gcge_gpu_mat *A, gcge_gpu_mv *RHS, int r_start
     args.precision = precision;
     args.rate = cg_rate;
     int st = gb_bcg(ctx, A, RHS->d + r_start, RHS->ld, W->d + w_start, W->ld, &args, work, bytes);
-    cudaStreamSynchronize(ctx->stream);
+    // the FP64 rounds wait inside their kernel, and do nothing once a wait has run out
+    if (!st && !precision) st = gb_check_device_error(ctx);
+    else cudaStreamSynchronize(ctx->stream);
     gb_dev_free(ctx, work);
     return st;
 }

@@ -22,7 +22,7 @@
 // chunk), the shape with the fewest idle slots: the FP64 pipe issues for idle lanes
 // too. Only p crosses a barrier; x and r of an entry belong to one thread.
 //
-// Every wait is bounded (COOP_WAIT_NS); a block whose wait runs out sets the
+// Every wait is bounded (a.limit); a block whose wait runs out sets the
 // context's device error word and leaves, and so do the others in turn.
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -59,6 +59,7 @@ struct pb_args {
     double *part;              // [column][slab]
     unsigned *bar;             // [0] arrivals, [1] columns' owners done, [2..3] generation and active columns
     int *dev_err;
+    coop_limit limit;
 };
 
 // sqrt(|s|) / err >= rate (src/gcge_cg.c:286-294); far from the line, where rounding
@@ -136,12 +137,12 @@ __device__ __forceinline__ void pb_column(const pb_args &a, int op, int c, doubl
 __device__ int pb_barrier(const pb_args &a, int op, int ka, double *sh, unsigned &gen)
 {
     __shared__ int last, res;
-    const unsigned G = gridDim.x;
+    const unsigned G = gridDim.x, lastn = a.limit.last;
     const bool one = op == PB_PLAIN || (long)a.nslab * ka <= PB_ONE_BLOCK_SUMS;
     const unsigned owners = min((unsigned)ka, G);
     __syncthreads();
     if (threadIdx.x == 0) {
-        last = coop_arrive(a.bar) == G - 1;
+        last = coop_arrive(a.bar) == lastn;
         res = 0;
     }
     __syncthreads();
@@ -167,8 +168,8 @@ __device__ int pb_barrier(const pb_args &a, int op, int ka, double *sh, unsigned
         if (threadIdx.x == 0) {
             const unsigned long long t0 = coop_now();
             int spin = 0;
-            while (coop_ld32(a.bar) != G)
-                if ((++spin & 1023) == 0 && coop_now() - t0 > COOP_WAIT_NS) {
+            while (coop_ld32(a.bar) != lastn + 1)
+                if ((++spin & 1023) == 0 && coop_now() - t0 > a.limit.ns) {
                     atomicExch(a.dev_err, 1);
                     res = -1;
                     break;
@@ -204,7 +205,7 @@ __device__ int pb_barrier(const pb_args &a, int op, int ka, double *sh, unsigned
         int spin = 0;
         unsigned long long v;
         while ((unsigned)((v = coop_ld64(a.bar + 2)) >> 32) == gen)
-            if ((++spin & 1023) == 0 && coop_now() - t0 > COOP_WAIT_NS) {
+            if ((++spin & 1023) == 0 && coop_now() - t0 > a.limit.ns) {
                 atomicExch(a.dev_err, 1);
                 v = 0xffffffffull;
                 break;
@@ -612,6 +613,7 @@ extern "C" int gb_bcg_persist64(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, const 
     long G = (long)ctx->num_sms * per_sm;
     const long items = (long)a.nslab * ((a.k + a.cw - 1) / a.cw);
     if (G > items) G = items;
+    a.limit = gb_coop_limit(ctx, G);
     const double nk = (double)a.n * a.k, rounds = a.max_it > 1 ? a.max_it - 1 : 0;
     GB_PROF(ctx, GB_K_SPMM64, rounds * (12.0 * A->nnz + 4.0 * (A->n + 1) + 88.0 * nk),
             rounds * (2.0 * A->nnz * a.k + 10.0 * nk));

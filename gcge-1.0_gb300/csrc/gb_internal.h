@@ -64,6 +64,7 @@ struct gcge_gpu_ctx {
     int *dev_err;              /* device word: set by a kernel whose bounded wait ran out */
     unsigned *dev_bar;         /* device: counters of a cooperative grid's barrier (gb_bcg_persist.cu) */
     int tc_stall;              /* test hook: the next tensor-core launch withholds an arrival */
+    int coop_stall;            /* the same for the next launch with grid barriers */
     /* FP64 SpMM in FP32-pair arithmetic (1; set by the mixed solver form) or on the
      * FP64 pipe (0, default) */
     int spmm_pair;

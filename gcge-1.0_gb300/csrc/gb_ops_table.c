@@ -362,7 +362,8 @@ static void op_LinearSolverJacobi(void *mat, void *b, void *x, GCGE_GPU_OPS_LAYO
     a.rate = g_ls_rate;
     a.dinv = A->dinv;
     a.dinv32 = A->dinv32;
-    rec(gb_bcg(g_ctx, A, g_ls_rhs->d, g_ls_rhs->ld, colptr(vx), vx->mv->ld, &a, g_ls_work, g_ls_work_bytes));
+    st = gb_bcg(g_ctx, A, g_ls_rhs->d, g_ls_rhs->ld, colptr(vx), vx->mv->ld, &a, g_ls_work, g_ls_work_bytes);
+    rec(st ? st : gb_check_device_error(g_ctx));
 }
 
 int GCGE_GPU_OpsSetLinearSolver(void *gcge_ops, int kind, int max_it, double rate)

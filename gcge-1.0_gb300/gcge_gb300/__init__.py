@@ -20,7 +20,7 @@ OK = 0
 ERR_ARG, ERR_CUDA, ERR_NOMEM, ERR_CSR, ERR_NONFINITE, ERR_BREAKDOWN, ERR_EIGSOLVE, ERR_TIMEOUT, ERR_IO = range(1, 10)
 STATUS = {0: "ok", 1: "invalid argument", 2: "CUDA runtime error", 3: "device allocation failed",
           4: "malformed CSR matrix", 5: "non-finite value", 6: "orthogonalisation lost every column",
-          7: "projected eigensolve failed", 8: "tensor-core kernel wait timed out",
+          7: "projected eigensolve failed", 8: "a kernel's bounded wait timed out",
           9: "file missing, unreadable, truncated or not CSR"}
 
 
@@ -104,6 +104,7 @@ def load():
         "GCGE_GPU_SetTensorEmulation": (_I, [_P, _I]),
         "GCGE_GPU_SetPairSpMM": (_I, [_P, _I]),
         "GCGE_GPU_TestStallTensorWait": (_I, [_P, _I]),
+        "GCGE_GPU_TestStallGridWait": (_I, [_P, _I]),
         "GCGE_GPU_InnerProdNoAlloc": (_I, [_I, _I, _I, _P, C.c_long, _P, C.c_long, _P, _I, _I, _P]),
         "GCGE_GPU_PatternGrad": (_I, [_P, _P, _I, _P, _I, _I, _P, _I, _P]),
         "GCGE_GPU_EigvecAdjoint": (_I, [_P, _P, _P, _I, _P, _I, _P, _I, _P, _I, _D, _D, _I, C.POINTER(_I)]),

@@ -47,7 +47,7 @@ extern "C" {
 #define GCGE_GPU_ERR_NONFINITE 5   /* NaN/Inf met in a reduction or the small eigensolve */
 #define GCGE_GPU_ERR_BREAKDOWN 6   /* orthogonalisation lost every column               */
 #define GCGE_GPU_ERR_EIGSOLVE  7   /* projected eigensolve did not converge             */
-#define GCGE_GPU_ERR_TIMEOUT   8   /* a tensor-core kernel's bounded wait ran out       */
+#define GCGE_GPU_ERR_TIMEOUT   8   /* a kernel's bounded wait ran out                   */
 #define GCGE_GPU_ERR_IO        9   /* file missing, unreadable, truncated or not CSR    */
 
 typedef struct gcge_gpu_ctx gcge_gpu_ctx;  /* device, stream, reduction scratch  */
@@ -124,6 +124,14 @@ int  GCGE_GPU_SetTensorEmulation(gcge_gpu_ctx *ctx, int on);
  * later tensor-core launches on this context do no work. One-shot: the flag is
  * cleared by that launch. No fault, trap or endless wait is involved. */
 int  GCGE_GPU_TestStallTensorWait(gcge_gpu_ctx *ctx, int on);
+
+/* The same for the kernels that wait on a barrier of their own grid (all rounds of
+ * an FP64 block CG, the iteration of the eigenvector adjoint): the next such launch on
+ * this context waits at its first barrier for an arrival that cannot come, with waits of
+ * 0.1 s (20 s otherwise). They run out, the kernel returns, and the call that launched it
+ * reports GCGE_GPU_ERR_TIMEOUT, as do later ones of its kind on this context,
+ * which do no work. One-shot. */
+int  GCGE_GPU_TestStallGridWait(gcge_gpu_ctx *ctx, int on);
 
 /* Sparse products Y = A X with two or more columns either in FP32-pair
  * arithmetic (on = 1: values as hi + lo floats, error-free products and sums on
