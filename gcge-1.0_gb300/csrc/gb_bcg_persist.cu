@@ -63,11 +63,12 @@ struct pb_args {
 };
 
 // sqrt(|s|) / err >= rate (src/gcge_cg.c:286-294); far from the line, where rounding
-// cannot matter, without the square root and the division (0.7 us of the barrier)
+// cannot matter, without the square root and the division (0.7 us of the barrier).
+// Squares compare as the quotient does only for a positive rate.
 __device__ __forceinline__ bool pb_active(double s, double err, double rate)
 {
     const double m = fabs(s), t = rate * err, t2 = t * t;
-    if (t2 > 1e-280 && t2 < 1e280) {
+    if (rate > 0.0 && t2 > 1e-280 && t2 < 1e280) {
         if (m > 1.0000001 * t2 && m < 1e300) return true;
         if (m < 0.9999999 * t2) return false;
     }

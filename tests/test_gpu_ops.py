@@ -406,3 +406,18 @@ assert np.max(np.abs(Q.T @ Q - np.eye(k))) < 1e-11
 """
     r = subprocess.run([sys.executable, "-c", code % sys.path], capture_output=True, text=True, timeout=600)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_bcg_fp64_negative_rate_drops_no_column(ctx):
+    """cg_rate <= 0: ||r|| / ||r0|| >= cg_rate always holds, so every column runs all rounds, the
+    same for 0 and below it."""
+    A, _ = P.laplace2d(43, 31)
+    dA = ctx.matrix(A)
+    R = np.random.default_rng(31).standard_normal((A.n, 9))
+    out = []
+    for rate in (0.0, -1.0, -1e-3):
+        r, w = ctx.multivec(A.n, 9, R), ctx.multivec(A.n, 9)
+        G.bcg(dA, r, 0, w, 0, 9, cg_max_it=40, cg_rate=rate)
+        out.append(w.download())
+    assert np.linalg.norm(A.to_scipy() @ out[0] - R) < 0.5 * np.linalg.norm(R)
+    assert np.array_equal(out[1], out[0]) and np.array_equal(out[2], out[0])
