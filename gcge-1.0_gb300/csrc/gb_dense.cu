@@ -236,11 +236,12 @@ extern "C" int gb_p_coef_assemble(gcge_gpu_ctx *ctx, double *coef, int ldc, int 
 // n / b rounded as IEEE division, y = 1 / b correctly rounded: two corrections of n y by
 // the exact remainder (Markstein, IBM J. Res. Dev. 34, 1990; with a quotient within
 // one ulp and a correctly rounded reciprocal the second is exact), a chain of five
-// operations. Outside the middle of the exponent range the division itself.
+// operations. Operands of which the quotient could leave the range of normal numbers (|n| past 2^+-600, |b|
+// past 2^+-300) take the division itself.
 __device__ __forceinline__ double div_by(double n, double b, double y)
 {
     const int en = __double2hiint(n) & 0x7ff00000, eb = __double2hiint(b) & 0x7ff00000;
-    if (en < (123 << 20) || en > (1923 << 20) || eb < (723 << 20) || eb > (1323 << 20)) return n / b;
+    if (en < (423 << 20) || en > (1622 << 20) || eb < (723 << 20) || eb > (1322 << 20)) return n / b;
     double q = __dmul_rn(n, y);
     q = fma(fma(-b, q, n), y, q);
     return fma(fma(-b, q, n), y, q);
@@ -1072,13 +1073,15 @@ static int td_cluster_launch(gcge_gpu_ctx *ctx, int tc, int m, const double *H, 
 // n / b on the path of the Sturm counts: the hardware reciprocal refined once (Newton-
 // Raphson, about 2^-40), then the quotient corrected by its exact remainder, which
 // leaves an error of 2^-80 before the one rounding -- the IEEE quotient but for values
-// that close to the middle of two doubles. Five FP64 instructions; a quotient is most
-// of a Sturm step, and each instruction takes a quarter of the SM for 64 clocks.
-// Outside the middle of the exponent range the division itself.
+// that close to the middle of two doubles. It falls as b grows, as IEEE's does: quotients of
+// neighbouring divisors are 2^-53 apart or more before the rounding, which keeps their order.
+// Five FP64 instructions; a quotient is most of a Sturm step, and each instruction takes
+// a quarter of the SM for 64 clocks. Operands past 2^+-450, of which the
+// quotient could leave the range of normal numbers, take the division itself.
 __device__ __forceinline__ double sturm_div(double n, double b)
 {
     const int en = __double2hiint(n) & 0x7ff00000, eb = __double2hiint(b) & 0x7ff00000;
-    if (en < (323 << 20) || en > (1723 << 20) || eb < (323 << 20) || eb > (1723 << 20)) return n / b;
+    if (en < (573 << 20) || en > (1472 << 20) || eb < (573 << 20) || eb > (1472 << 20)) return n / b;
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
     r = fma(fma(-b, r, 1.0), r, r);
@@ -1284,26 +1287,43 @@ __global__ void k_recip_probe(int n, const double *__restrict__ x, double *__res
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) r[i] = nr_recip(x[i]);
 }
+__global__ void k_div_probe(int n, int kind, const double *__restrict__ x, const double *__restrict__ y,
+                            double *__restrict__ q)
+{
+    GB_PDL();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) q[i] = kind ? sturm_div(x[i], y[i]) : div_by(x[i], y[i], 1.0 / y[i]);
+}
 
-// Internal check of nr_recip (not part of the public interface): r[i] = nr_recip(x[i])
-// for n host values, on the current device.
-extern "C" int gb_recip_check(int n, const double *x_host, double *r_host)
+// Internal checks of nr_recip and of the two divisions (not part of the public interface), on
+// the current device: r[i] = nr_recip(x[i]); q[i] = div_by (kind 0) or sturm_div (kind 1) of
+// x[i] and y[i], for n host values.
+static int probe(int n, const double *x_host, const double *y_host, int kind, double *r_host)
 {
     if (n <= 0 || !x_host || !r_host) return GCGE_GPU_ERR_ARG;
-    double *dx = nullptr, *dr = nullptr;
+    const size_t bytes = sizeof(double) * n;
+    double *dx = nullptr, *dy = nullptr, *dr = nullptr;
     int st = GCGE_GPU_OK;
-    if (cudaMalloc(&dx, sizeof(double) * n) != cudaSuccess || cudaMalloc(&dr, sizeof(double) * n) != cudaSuccess ||
-        cudaMemcpy(dx, x_host, sizeof(double) * n, cudaMemcpyHostToDevice) != cudaSuccess)
+    if (cudaMalloc(&dx, bytes) != cudaSuccess || cudaMalloc(&dr, bytes) != cudaSuccess ||
+        cudaMemcpy(dx, x_host, bytes, cudaMemcpyHostToDevice) != cudaSuccess ||
+        (y_host && (cudaMalloc(&dy, bytes) != cudaSuccess ||
+                    cudaMemcpy(dy, y_host, bytes, cudaMemcpyHostToDevice) != cudaSuccess)))
         st = GCGE_GPU_ERR_CUDA;
     if (!st) {
-        k_recip_probe<<<(n + 255) / 256, 256>>>(n, dx, dr);
-        if (cudaGetLastError() != cudaSuccess ||
-            cudaMemcpy(r_host, dr, sizeof(double) * n, cudaMemcpyDeviceToHost) != cudaSuccess)
+        if (y_host) k_div_probe<<<(n + 255) / 256, 256>>>(n, kind, dx, dy, dr);
+        else k_recip_probe<<<(n + 255) / 256, 256>>>(n, dx, dr);
+        if (cudaGetLastError() != cudaSuccess || cudaMemcpy(r_host, dr, bytes, cudaMemcpyDeviceToHost) != cudaSuccess)
             st = GCGE_GPU_ERR_CUDA;
     }
     cudaFree(dx);
+    cudaFree(dy);
     cudaFree(dr);
     return st;
+}
+extern "C" int gb_recip_check(int n, const double *x_host, double *r_host) { return probe(n, x_host, nullptr, 0, r_host); }
+extern "C" int gb_div_check(int kind, int n, const double *x_host, const double *y_host, double *q_host)
+{
+    return y_host ? probe(n, x_host, y_host, kind, q_host) : GCGE_GPU_ERR_ARG;
 }
 
 // inverse iteration: a block of one warp per wanted eigenvalue, so that the chains

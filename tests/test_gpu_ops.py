@@ -421,3 +421,60 @@ def test_bcg_fp64_negative_rate_drops_no_column(ctx):
         out.append(w.download())
     assert np.linalg.norm(A.to_scipy() @ out[0] - R) < 0.5 * np.linalg.norm(R)
     assert np.array_equal(out[1], out[0]) and np.array_equal(out[2], out[0])
+
+
+def _quotients(kind, num, den):
+    import ctypes as C
+    lib = G.load()
+    num, den = np.ascontiguousarray(num), np.ascontiguousarray(den)
+    q = np.zeros_like(num)
+    lib.gb_div_check.restype = C.c_int
+    p = lambda a: a.ctypes.data_as(C.c_void_p)  # noqa: E731
+    assert lib.gb_div_check(kind, len(num), p(num), p(den), p(q)) == 0
+    with np.errstate(all="ignore"):
+        return q, num / den
+
+
+def _division_operands(rng, count):
+    """Significands at random and at both ends, exponents over the whole range and around every
+    power that either division's own range ends at; zeros, infinities, NaN and subnormals."""
+    sig = np.where(rng.random(count) < 0.2, rng.choice([1.0, 1.0 + 2.0 ** -52, 2.0 - 2.0 ** -52, 1.5], count),
+                   rng.uniform(1.0, 2.0, count))
+    ex = np.where(rng.random(count) < 0.5, rng.integers(-60, 61, count),
+                  np.where(rng.random(count) < 0.5, rng.integers(-1022, 1024, count),
+                           rng.choice([-900, -700, -600, -450, -300, 300, 450, 600, 700, 900], count) +
+                           rng.integers(-2, 3, count)))
+    x = rng.choice([-1.0, 1.0], count) * np.ldexp(sig, ex)
+    x[:64] = rng.choice([0.0, -0.0, np.inf, -np.inf, np.nan, 5e-324, -1e-310, 2.0 ** -1022, 1.7e308], 64)
+    return x
+
+
+def test_quotient_by_a_known_reciprocal(ctx):
+    """The Cholesky inverse divides by a pivot whose reciprocal it has: IEEE division, bit for bit."""
+    rng = np.random.default_rng(41)
+    q, ref = _quotients(0, _division_operands(rng, 1 << 21), rng.permutation(_division_operands(rng, 1 << 21)))
+    assert np.array_equal(q, ref, equal_nan=True)
+
+
+def test_quotient_of_the_sturm_counts(ctx):
+    """The division of the Sturm counts: its value before the one rounding is within 2^-78 of the quotient, so it is
+    IEEE division but where the quotient lies that close to the middle of two doubles; and never
+    decreasing as the divisor falls through neighbouring doubles, which the bisection relies on."""
+    from fractions import Fraction
+    rng = np.random.default_rng(42)
+    num, den = _division_operands(rng, 1 << 21), rng.permutation(_division_operands(rng, 1 << 21))
+    q, ref = _quotients(1, num, den)
+    bad = np.flatnonzero(~((q == ref) | (np.isnan(q) & np.isnan(ref))))
+    # 2^-25 of random significands are expected there; of the chosen ones 1 / (2 - 2^-52) lies 2^-106 from a middle
+    assert np.sum(np.abs(np.frexp(den[bad])[0]) != 1.0 - 2.0 ** -53) <= 16
+    for i in bad:
+        mid = (Fraction(float(q[i])) + Fraction(float(ref[i]))) / 2
+        ex = Fraction(float(num[i])) / Fraction(float(den[i]))
+        assert abs(ex / mid - 1) <= Fraction(1, 2 ** 78)
+    for e in (0, -40, 449, 450, 451, -449, -450, -451):
+        n1 = float(np.ldexp(rng.uniform(1.0, 2.0), e))
+        d = np.ldexp(2.0 - np.arange(1 << 16) * 2.0 ** -52, e // 3)   # falls, and passes a power of two
+        d = np.concatenate([d, np.ldexp(1.0 + np.arange(1 << 15, -(1 << 15), -1) * 2.0 ** -53, e)])
+        for part in (d[:1 << 16], d[1 << 16:]):
+            q, _ = _quotients(1, np.full(len(part), n1), part)
+            assert np.all(np.diff(q) >= 0)
