@@ -370,7 +370,7 @@ struct ac_args {
     ac_state *s;
     unsigned *bar;
     int *dev_err;
-    coop_limit limit;
+    unsigned long long wait_ns;
 };
 enum { AC_PLAIN, AC_COEF, AC_PQ, AC_RR };
 
@@ -381,9 +381,8 @@ __device__ int ac_barrier(const ac_args &a, int op, int ns, unsigned &gen)
     __shared__ int last, res;
     __shared__ double sum0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, G = gridDim.x;
-    const unsigned lastn = a.limit.last;
     __syncthreads();
-    if (threadIdx.x == 0) last = coop_arrive(a.bar) == lastn;
+    if (threadIdx.x == 0) last = coop_arrive(a.bar) == (unsigned)G - 1;
     __syncthreads();
     if (last) {
         for (int j = warp; j < ns; j += AC_WARPS) {
@@ -426,7 +425,7 @@ __device__ int ac_barrier(const ac_args &a, int op, int ns, unsigned &gen)
         int spin = 0;
         unsigned long long v;
         while ((unsigned)((v = coop_ld64(a.bar + 2)) >> 32) == gen)
-            if ((++spin & 1023) == 0 && coop_now() - t0 > a.limit.ns) {
+            if ((++spin & 1023) == 0 && coop_now() - t0 > a.wait_ns) {
                 atomicExch(a.dev_err, 1);
                 v = 0xffffffffull;
                 break;
@@ -663,13 +662,13 @@ static int ad_iterate(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, const gcge_gpu_m
     a.s = (ac_state *)W->dot;
     a.bar = ctx->dev_bar;
     a.dev_err = ctx->dev_err;
+    a.wait_ns = gb_coop_wait_ns(ctx);
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_adjoint_cg, AC_ROWS, 0) != cudaSuccess || per_sm < 1)
         return gb_fail(ctx, GCGE_GPU_ERR_CUDA);
     if (per_sm > AV_BLOCKS_PER_SM) per_sm = AV_BLOCKS_PER_SM;   // the partials' room
     long G = (long)ctx->num_sms * per_sm, tiles = ((long)n + AC_ROWS - 1) / AC_ROWS;
     if (G > tiles) G = tiles;
-    a.limit = gb_coop_limit(ctx, G);
     void *args[] = {&a};
     if (cudaLaunchCooperativeKernel(k_adjoint_cg, dim3((unsigned)G), dim3(AC_ROWS), args, 0, ctx->stream) != cudaSuccess) {
         cudaGetLastError();

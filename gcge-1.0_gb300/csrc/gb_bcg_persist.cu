@@ -22,7 +22,7 @@
 // chunk), the shape with the fewest idle slots: the FP64 pipe issues for idle lanes
 // too. Only p crosses a barrier; x and r of an entry belong to one thread.
 //
-// Every wait is bounded (a.limit); a block whose wait runs out sets the
+// Every wait is bounded (a.wait_ns); a block whose wait runs out sets the
 // context's device error word and leaves, and so do the others in turn.
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -59,16 +59,16 @@ struct pb_args {
     double *part;              // [column][slab]
     unsigned *bar;             // [0] arrivals, [1] columns' owners done, [2..3] generation and active columns
     int *dev_err;
-    coop_limit limit;
+    unsigned long long wait_ns;
 };
 
 // sqrt(|s|) / err >= rate (src/gcge_cg.c:286-294); far from the line, where rounding
 // cannot matter, without the square root and the division (0.7 us of the barrier).
-// Squares compare as the quotient does only for a positive rate.
+// Squares compare as the quotient does only for a positive rate: t2 keeps its sign.
 __device__ __forceinline__ bool pb_active(double s, double err, double rate)
 {
-    const double m = fabs(s), t = rate * err, t2 = t * t;
-    if (rate > 0.0 && t2 > 1e-280 && t2 < 1e280) {
+    const double m = fabs(s), t = rate * err, t2 = t * fabs(t);
+    if (t2 > 1e-280 && t2 < 1e280) {
         if (m > 1.0000001 * t2 && m < 1e300) return true;
         if (m < 0.9999999 * t2) return false;
     }
@@ -138,12 +138,12 @@ __device__ __forceinline__ void pb_column(const pb_args &a, int op, int c, doubl
 __device__ int pb_barrier(const pb_args &a, int op, int ka, double *sh, unsigned &gen)
 {
     __shared__ int last, res;
-    const unsigned G = gridDim.x, lastn = a.limit.last;
+    const unsigned G = gridDim.x;
     const bool one = op == PB_PLAIN || (long)a.nslab * ka <= PB_ONE_BLOCK_SUMS;
     const unsigned owners = min((unsigned)ka, G);
     __syncthreads();
     if (threadIdx.x == 0) {
-        last = coop_arrive(a.bar) == lastn;
+        last = coop_arrive(a.bar) == G - 1;
         res = 0;
     }
     __syncthreads();
@@ -169,8 +169,8 @@ __device__ int pb_barrier(const pb_args &a, int op, int ka, double *sh, unsigned
         if (threadIdx.x == 0) {
             const unsigned long long t0 = coop_now();
             int spin = 0;
-            while (coop_ld32(a.bar) != lastn + 1)
-                if ((++spin & 1023) == 0 && coop_now() - t0 > a.limit.ns) {
+            while (coop_ld32(a.bar) != G)
+                if ((++spin & 1023) == 0 && coop_now() - t0 > a.wait_ns) {
                     atomicExch(a.dev_err, 1);
                     res = -1;
                     break;
@@ -206,7 +206,7 @@ __device__ int pb_barrier(const pb_args &a, int op, int ka, double *sh, unsigned
         int spin = 0;
         unsigned long long v;
         while ((unsigned)((v = coop_ld64(a.bar + 2)) >> 32) == gen)
-            if ((++spin & 1023) == 0 && coop_now() - t0 > a.limit.ns) {
+            if ((++spin & 1023) == 0 && coop_now() - t0 > a.wait_ns) {
                 atomicExch(a.dev_err, 1);
                 v = 0xffffffffull;
                 break;
@@ -582,6 +582,7 @@ extern "C" int gb_bcg_persist64(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, const 
     a.part = s->part;
     a.bar = ctx->dev_bar;
     a.dev_err = ctx->dev_err;
+    a.wait_ns = gb_coop_wait_ns(ctx);
     int L = 16, Q = 1, per_sm = 0;
     // Items of fewer columns where whole slabs would leave SMs without work: the chunk
     // count with the shortest busiest SM, an item costing its latencies (as much as
@@ -614,7 +615,6 @@ extern "C" int gb_bcg_persist64(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, const 
     long G = (long)ctx->num_sms * per_sm;
     const long items = (long)a.nslab * ((a.k + a.cw - 1) / a.cw);
     if (G > items) G = items;
-    a.limit = gb_coop_limit(ctx, G);
     const double nk = (double)a.n * a.k, rounds = a.max_it > 1 ? a.max_it - 1 : 0;
     GB_PROF(ctx, GB_K_SPMM64, rounds * (12.0 * A->nnz + 4.0 * (A->n + 1) + 88.0 * nk),
             rounds * (2.0 * A->nnz * a.k + 10.0 * nk));

@@ -2,10 +2,10 @@
 // release by a second one that carries a generation and a 32-bit message, so that
 // a waiting block learns both in one trip to L2. Waits are bounded by the callers
 // (COOP_WAIT_NS of %globaltimer; the longest phase of a kernel is below a second). A
-// launch stalled on purpose (GCGE_GPU_TestStallGridWait) waits for an arrival beyond its
-// blocks' and gives its waits COOP_STALL_NS. (The arrival to wait for is an argument, so
-// that a barrier does the same with and without; a test of the block and a flag before the
-// arrival took 60 ns of a barrier's 2.2 us.)
+// launch stalled on purpose (GCGE_GPU_TestStallGridWait) finds the count of arrivals off,
+// so that its first barrier never completes, and waits COOP_STALL_NS. (The barriers
+// themselves are the same: a test of a flag or of an argument before the arrival took 20
+// to 60 ns of a barrier's 2.2 us.)
 #pragma once
 #include <cuda_runtime.h>
 
@@ -13,11 +13,6 @@
 
 #define COOP_WAIT_NS 20000000000ull
 #define COOP_STALL_NS 100000000ull
-
-struct coop_limit {
-    unsigned long long ns;     // of every wait
-    unsigned last;             // what the arrival that completes a barrier finds: blocks - 1
-};
 
 __device__ __forceinline__ unsigned long long coop_now()
 {
@@ -43,12 +38,13 @@ __device__ __forceinline__ unsigned coop_ld32(const unsigned *w)
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(w) : "memory");
     return v;
 }
-// for a launch of G blocks; a stall is for one launch
-static inline coop_limit gb_coop_limit(gcge_gpu_ctx *ctx, long G)
+// the limit of the next launch's waits; a stall is for one launch
+static inline unsigned long long gb_coop_wait_ns(gcge_gpu_ctx *ctx)
 {
-    const coop_limit l = {ctx->coop_stall ? COOP_STALL_NS : COOP_WAIT_NS, ctx->coop_stall ? ~0u : (unsigned)G - 1};
+    if (!ctx->coop_stall) return COOP_WAIT_NS;
     ctx->coop_stall = 0;
-    return l;
+    cudaMemsetAsync(ctx->dev_bar, 0x40, sizeof(unsigned), ctx->stream);
+    return COOP_STALL_NS;
 }
 // word pair w (8-byte aligned): generation gen, message msg
 __device__ __forceinline__ void coop_release(unsigned *w, unsigned gen, unsigned msg)
