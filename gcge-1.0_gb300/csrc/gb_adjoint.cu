@@ -123,8 +123,8 @@ extern "C" int GCGE_GPU_PatternGrad(const gcge_gpu_mat *M, const gcge_gpu_mv *U,
     if (M->nnz == 0) return GCGE_GPU_OK;
     double *g_dev = nullptr, *s_dev = nullptr;
     int st = GCGE_GPU_OK;
-    if (gb_dev_alloc(ctx, (void **)&g_dev, sizeof(double) * (size_t)M->nnz) ||
-        gb_dev_alloc(ctx, (void **)&s_dev, sizeof(double) * (size_t)r)) {
+    if (gb_call_alloc(ctx, (void **)&g_dev, sizeof(double) * (size_t)M->nnz) ||
+        gb_call_alloc(ctx, (void **)&s_dev, sizeof(double) * (size_t)r)) {
         st = gb_fail(ctx, GCGE_GPU_ERR_NOMEM);
         goto done;
     }
@@ -142,8 +142,8 @@ extern "C" int GCGE_GPU_PatternGrad(const gcge_gpu_mat *M, const gcge_gpu_mv *U,
         st = gb_fail(ctx, GCGE_GPU_ERR_CUDA);
 done:
     cudaStreamSynchronize(ctx->stream);
-    gb_dev_free(ctx, g_dev);
-    gb_dev_free(ctx, s_dev);
+    gb_call_free(ctx, g_dev);
+    gb_call_free(ctx, s_dev);
     return st;
 }
 
@@ -774,7 +774,7 @@ extern "C" int GCGE_GPU_EigvecAdjoint(const gcge_gpu_mat *A, const gcge_gpu_mat 
     const size_t vn = ((size_t)n + 31) & ~(size_t)31, vm = ((size_t)m + 31) & ~(size_t)31;
     const size_t np = (((size_t)ctx->num_sms * AV_BLOCKS_PER_SM * (size_t)(m > 1 ? m : 1)) + 31) & ~(size_t)31;
     const size_t nv = 7 * vn + vm + 32 + np + (B ? (((size_t)n * m + 31) & ~(size_t)31) : 0);
-    if (gb_dev_alloc(ctx, (void **)&base, sizeof(double) * nv)) return gb_fail(ctx, GCGE_GPU_ERR_NOMEM);
+    if (gb_call_alloc(ctx, (void **)&base, sizeof(double) * nv)) return gb_fail(ctx, GCGE_GPU_ERR_NOMEM);
     W.y = base;
     W.r = W.y + vn;
     W.p = W.r + vn;
@@ -788,7 +788,7 @@ extern "C" int GCGE_GPU_EigvecAdjoint(const gcge_gpu_mat *A, const gcge_gpu_mat 
     W.BX = B ? W.part + np : nullptr;
     W.h_c = (double *)malloc(sizeof(double) * m);
     if (!W.h_c) {
-        gb_dev_free(ctx, base);
+        gb_call_free(ctx, base);
         return gb_fail(ctx, GCGE_GPU_ERR_NOMEM);
     }
     // the projections are n x m by one column: FP64-pipe Gram and combination
@@ -799,7 +799,7 @@ extern "C" int GCGE_GPU_EigvecAdjoint(const gcge_gpu_mat *A, const gcge_gpu_mat 
                   tol, max_it, iters, &W);
     ctx->tc = tc;
     cudaStreamSynchronize(ctx->stream);
-    gb_dev_free(ctx, base);
+    gb_call_free(ctx, base);
     free(W.h_c);
     return st;
 }

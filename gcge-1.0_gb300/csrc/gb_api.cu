@@ -172,7 +172,7 @@ extern "C" int GCGE_GPU_Init(int device, gcge_gpu_ctx **out)
 // cudaFree, so repeated solves on a context reuse it rather than paying
 // cudaMalloc/cudaFree of every block each time. Blocks are used on the context's
 // stream only, so handing one to a later request is stream-ordered.
-extern "C" int gb_dev_alloc(gcge_gpu_ctx *ctx, void **p, size_t bytes)
+static int dev_alloc(gcge_gpu_ctx *ctx, void **p, size_t bytes, int call)
 {
     *p = nullptr;
     if (bytes == 0) bytes = 8;
@@ -212,10 +212,13 @@ extern "C" int gb_dev_alloc(gcge_gpu_ctx *ctx, void **p, size_t bytes)
         ctx->blk = nb;
         ctx->blk_cap = nc;
     }
-    ctx->blk[ctx->nblk++] = gb_block{q, bytes, 1};
+    ctx->blk[ctx->nblk++] = gb_block{q, bytes, 1, call};
     *p = q;
     return GCGE_GPU_OK;
 }
+
+extern "C" int gb_dev_alloc(gcge_gpu_ctx *ctx, void **p, size_t bytes) { return dev_alloc(ctx, p, bytes, 0); }
+extern "C" int gb_call_alloc(gcge_gpu_ctx *ctx, void **p, size_t bytes) { return dev_alloc(ctx, p, bytes, 1); }
 
 extern "C" void gb_dev_free(gcge_gpu_ctx *ctx, void *p)
 {
@@ -226,6 +229,24 @@ extern "C" void gb_dev_free(gcge_gpu_ctx *ctx, void *p)
             return;
         }
     cudaFree(p);
+}
+
+extern "C" void gb_call_free(gcge_gpu_ctx *ctx, void *p)
+{
+    if (!p) return;
+    gb_dev_free(ctx, p);
+    // newest first: what does not fit is given back
+    size_t kept = 0;
+    for (int i = ctx->nblk - 1; i >= 0; --i) {
+        const gb_block b = ctx->blk[i];
+        if (b.call && !b.used && kept + b.bytes > GB_CALL_KEEP) {
+            cudaFree(b.p);
+            memmove(ctx->blk + i, ctx->blk + i + 1, sizeof(gb_block) * (ctx->nblk - 1 - i));
+            --ctx->nblk;
+        } else if (b.call && !b.used) {
+            kept += b.bytes;
+        }
+    }
 }
 
 extern "C" int GCGE_GPU_Finalize(gcge_gpu_ctx *ctx)
@@ -792,7 +813,7 @@ extern "C" int GCGE_GPU_BCG(const gcge_gpu_mat *A, gcge_gpu_mv *RHS, int r_start
     if (k <= 0) return GCGE_GPU_OK;
     size_t bytes = gb_bcg_work_bytes(A->n, k, precision);
     void *work = nullptr;
-    if (gb_dev_alloc(ctx, &work, bytes)) return gb_fail(ctx, GCGE_GPU_ERR_CUDA);
+    if (gb_call_alloc(ctx, &work, bytes)) return gb_fail(ctx, GCGE_GPU_ERR_CUDA);
     gb_bcg_args args;
     memset(&args, 0, sizeof(args));
     args.n = A->n;
@@ -804,7 +825,7 @@ extern "C" int GCGE_GPU_BCG(const gcge_gpu_mat *A, gcge_gpu_mv *RHS, int r_start
     // the FP64 rounds wait inside their kernel, and do nothing once a wait has run out
     if (!st && !precision) st = gb_check_device_error(ctx);
     else cudaStreamSynchronize(ctx->stream);
-    gb_dev_free(ctx, work);
+    gb_call_free(ctx, work);
     return st;
 }
 

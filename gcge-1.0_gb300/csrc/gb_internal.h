@@ -30,6 +30,7 @@ typedef struct {
     void *p;
     size_t bytes;
     int used;
+    int call;                  /* allocated for a call of its own (gb_call_alloc) */
 } gb_block;
 
 struct gcge_gpu_ctx {
@@ -107,6 +108,12 @@ struct gcge_gpu_mv {
  * all are freed by GCGE_GPU_Finalize (and unused ones when cudaMalloc fails) */
 int  gb_dev_alloc(gcge_gpu_ctx *ctx, void **p, size_t bytes);
 void gb_dev_free(gcge_gpu_ctx *ctx, void *p);
+/* the same for the workspace of a call of its own (block CG, gradients): of the blocks first allocated
+ * for such calls the newest stay, GB_CALL_KEEP bytes in all; larger ones are freed as the
+ * call ends. gb_call_free: the stream's work on p is done. */
+#define GB_CALL_KEEP ((size_t)256 << 20)
+int  gb_call_alloc(gcge_gpu_ctx *ctx, void **p, size_t bytes);
+void gb_call_free(gcge_gpu_ctx *ctx, void *p);
 
 /* profiling hooks around a launch: class, algorithmic bytes and flops */
 void gb_prof_begin(gcge_gpu_ctx *ctx, int cls, double bytes, double flops);

@@ -478,3 +478,34 @@ def test_quotient_of_the_sturm_counts(ctx):
         for part in (d[:1 << 16], d[1 << 16:]):
             q, _ = _quotients(1, np.full(len(part), n1), part)
             assert np.all(np.diff(q) >= 0)
+
+
+@pytest.mark.parametrize("op", ["bcg", "grad", "adjoint", "widths"])
+def test_large_workspaces_go_back_after_the_call(op):
+    """Single calls' workspaces are kept for later ones up to 256 MiB in all: after a call that needs
+    more, or calls of growing widths, the device has the rest of its memory again (other buffers of
+    the calls: within 300 MiB)."""
+    torch = pytest.importorskip("torch")
+    with G.Context(0) as c:
+        A, _ = P.laplace2d(1200, 1000)
+        n = A.n
+        if op == "bcg":
+            dA, x, y = c.matrix(A), c.multivec(n, 64), c.multivec(n, 64)
+            run = lambda: G.bcg(dA, x, 0, y, 0, 64, cg_max_it=2)  # noqa: E731
+        elif op == "widths":
+            dA, x, y = c.matrix(A), c.multivec(n, 12), c.multivec(n, 12)
+            run = lambda: [G.bcg(dA, x, 0, y, 0, k, cg_max_it=2) for k in (4, 8, 12)]  # noqa: E731
+        elif op == "grad":
+            import scipy.sparse as sp
+            M = P.CSR.from_scipy(sp.csr_matrix(sp.diags([np.ones(n)] * 41, range(41), shape=(n, n))))
+            dA, x = c.matrix(M), c.multivec(n, 2)
+            run = lambda: G.pattern_grad(dA, x, 0, x, 0, 1, [1.0], M.nnz)  # noqa: E731
+        else:
+            dA, x, y = c.matrix(A), c.multivec(n, 40), c.multivec(n, 2)
+            dB = c.matrix(P.CSR(np.arange(n + 1), np.arange(n), np.ones(n)))
+            run = lambda: G.eigvec_adjoint(dA, dB, x, 40, np.arange(40.0), 0, y, 0, y, 1, max_it=1)  # noqa: E731
+        c.sync()
+        before = torch.cuda.mem_get_info()[0]
+        run()
+        c.sync()
+        assert before - torch.cuda.mem_get_info()[0] <= 300 << 20
