@@ -805,7 +805,6 @@ extern "C" int gb_gram_fixed(cudaStream_t stream, int num_sms, int n, int k1, in
 #define LC_ER 8                                      // tiles whose row scales are kept
 #define LC_HDR (80 + 4 * (LC_ER * TC_M + TC_N) + 48) // tc_hdr, er, ecs
 #define LC_SMEM (2 * TC_STAGE + LC_HDR + 4 * LC_MAX_K)
-#define LC_OUT_LD (TC_N + 1)                         // doubles per staged output row
 #define LC_CORES_PER_WARP ((TC_ACORES + TC_SPLIT_WARPS - 1) / TC_SPLIT_WARPS)
 #define LC_SCALE_LOADS 48                            // row-scale loads in flight per thread
 // the largest of k_lincomb_tc's int offsets, a lane past the tile's cores among them (k_gram_tc's: 31 rows)

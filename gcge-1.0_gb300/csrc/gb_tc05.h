@@ -30,20 +30,7 @@ __device__ __forceinline__ void tc_tmem_dealloc(uint32_t taddr, uint32_t ncols)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
-// 32 lanes x 8 consecutive 32-bit columns (lane = warp's quarter of the 128 lanes);
-// the values may be used only after tc_tmem_wait8 on the same registers
-__device__ __forceinline__ void tc_tmem_ld8(uint32_t taddr, uint32_t r[8])
-{
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr));
-}
 __device__ __forceinline__ void tc_tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// ties registers loaded by tc_tmem_ld8 to a point after tc_tmem_wait_ld
-__device__ __forceinline__ void tc_reg_fence8(uint32_t r[8])
-{
-    asm volatile("" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]));
-}
 
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void tc_mbar_init(uint32_t bar, uint32_t count)
@@ -84,21 +71,12 @@ __device__ __forceinline__ void tc_cp8(uint32_t dst_smem, const void *src, uint3
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst_smem), "l"(src), "r"(src_bytes) : "memory");
 }
-__device__ __forceinline__ void tc_cp16(uint32_t dst_smem, const void *src)
-{
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
-}
 __device__ __forceinline__ void tc_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 // until at most PENDING of this thread's groups are in flight
 template <int PENDING>
 __device__ __forceinline__ void tc_cp_wait()
 {
     asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
-}
-// barrier over the first `count` threads of the CTA (named barrier `id`, 1..15)
-__device__ __forceinline__ void tc_bar_sync(int id, int count)
-{
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
 // bounded wait for the phase of the given parity; false after limit_ns
 __device__ __forceinline__ bool tc_mbar_wait(uint32_t bar, uint32_t parity, uint64_t limit_ns)
@@ -119,12 +97,7 @@ __device__ __forceinline__ uint64_t tc_sdesc(uint32_t saddr, uint32_t lbo, uint3
     return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) |
            (1ull << 46);
 }
-// instruction descriptor of kind::f16: bf16 x bf16 -> f32, both K-major, M x N
-__host__ __device__ constexpr uint32_t tc_idesc_bf16(int M, int N)
-{
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
-// the same for f16 x f16 -> f32
+// instruction descriptor of kind::f16: f16 x f16 -> f32, both K-major, M x N
 __host__ __device__ constexpr uint32_t tc_idesc_f16(int M, int N)
 {
     return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
