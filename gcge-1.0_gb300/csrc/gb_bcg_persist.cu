@@ -292,15 +292,17 @@ __device__ __forceinline__ void pb_row(const pb_args &a, int beg, int end, int s
     const long slab = is;                             \
     const int c0 = (int)((item - is * nch) * a.cw), kc = min(a.cw, (cols) - c0);
 
-template <int L, int Q, bool FUSED>
-__global__ void __launch_bounds__(PB_THREADS, 3)
+// MB blocks an SM (the registers for it): two for matrices without long rows where that takes no
+// more waves of items than three do, see gb_bcg_persist64
+template <int L, int Q, bool FUSED, int MB>
+__global__ void __launch_bounds__(PB_THREADS, MB)
 k_bcg_persist(const pb_args a)
 {
     GB_PDL();
     constexpr int RPB = PB_THREADS / L, C = L * Q;
     __shared__ double red[16][C];
     __shared__ double sh[PB_THREADS];
-    __shared__ int lflag[RPB];
+    __shared__ int lflag[MB == 3 ? RPB : 1];
     __shared__ uint8_t flip[FUSED ? PB_FUSED_K : 1];     // the buffer that holds a column's p
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int sl = lane % L, slot = threadIdx.x / L;
@@ -395,11 +397,11 @@ k_bcg_persist(const pb_args a)
                     double acc[Q];
 #pragma unroll
                     for (int q = 0; q < Q; ++q) acc[q] = 0;
-                    const bool lng = a.long_rows && end - beg > GB_LONG_ROW;
+                    const bool lng = MB == 3 && a.long_rows && end - beg > GB_LONG_ROW;
                     if (!lng) pb_row<L, Q, FUSED>(a, beg, end, L, sl, gmask, col, pold, bq, first, acc);
                     // rows longer than GB_LONG_ROW: all groups of the block on one row, the
                     // group sums added by shuffles and then warp by warp, in row order
-                    if (a.long_rows && __syncthreads_or(lng)) {
+                    if (MB == 3 && a.long_rows && __syncthreads_or(lng)) {
                         if (sl == 0) lflag[slot] = lng;
                         __syncthreads();
                         for (int q0 = 0; q0 < RPB; ++q0) {
@@ -538,19 +540,19 @@ static void pb_shape(int k, int maxq, int *Lo, int *Qo)
     }
 }
 
-static const void *pb_kernel(int L, int Q, bool fused)
+static const void *pb_kernel(int L, int Q, bool fused, int mb)
 {
-#define PB_K4(LL, F) (const void *)k_bcg_persist<LL, 1, F>, (const void *)k_bcg_persist<LL, 2, F>, \
-                     (const void *)k_bcg_persist<LL, 3, F>, (const void *)k_bcg_persist<LL, 4, F>
-#define PB_K8(LL) {PB_K4(LL, false), (const void *)k_bcg_persist<LL, 5, false>, \
-                   (const void *)k_bcg_persist<LL, 6, false>, (const void *)k_bcg_persist<LL, 7, false>, \
-                   (const void *)k_bcg_persist<LL, 8, false>}
-    static const void *const tab[3][8] = {PB_K8(4), PB_K8(8), PB_K8(16)};
-    static const void *const tabf[3][4] = {{PB_K4(4, true)}, {PB_K4(8, true)}, {PB_K4(16, true)}};
+#define PB_K4(LL, F, MB) (const void *)k_bcg_persist<LL, 1, F, MB>, (const void *)k_bcg_persist<LL, 2, F, MB>, \
+                         (const void *)k_bcg_persist<LL, 3, F, MB>, (const void *)k_bcg_persist<LL, 4, F, MB>
+#define PB_K8(LL, MB) {PB_K4(LL, false, MB), (const void *)k_bcg_persist<LL, 5, false, MB>, \
+                       (const void *)k_bcg_persist<LL, 6, false, MB>, (const void *)k_bcg_persist<LL, 7, false, MB>, \
+                       (const void *)k_bcg_persist<LL, 8, false, MB>}
+    static const void *const tab[2][3][8] = {{PB_K8(4, 2), PB_K8(8, 2), PB_K8(16, 2)}, {PB_K8(4, 3), PB_K8(8, 3), PB_K8(16, 3)}};
+    static const void *const tabf[3][4] = {{PB_K4(4, true, 3)}, {PB_K4(8, true, 3)}, {PB_K4(16, true, 3)}};
 #undef PB_K4
 #undef PB_K8
     const int i = L == 4 ? 0 : L == 8 ? 1 : 2;
-    return fused ? tabf[i][Q - 1] : tab[i][Q - 1];
+    return fused ? tabf[i][Q - 1] : tab[mb - 2][i][Q - 1];
 }
 
 extern "C" int gb_bcg_persist64(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, const gb_bcg_args *b, const bcg_state *s,
@@ -609,11 +611,20 @@ extern "C" int gb_bcg_persist64(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, const 
                        (double)A->nnz / a.n * L * Q * items_sm < PB_FUSED_WORK;
     if (!fused) pb_shape(a.cw, 8, &L, &Q);
     if (a.cw > L * Q) a.cw = L * Q;
-    const void *fn = pb_kernel(L, Q, fused);
+    const long items = (long)a.nslab * ((a.k + a.cw - 1) / a.cw);
+    // Three blocks an SM hide more of the gathers' latency, two have registers for all their loads in
+    // flight (three spill 96 to 220 bytes) and leave a last item less often alone on its SM.
+    // Two where that takes no more waves of items: 27-point 40^3, k = 64 (500 items) 336 -> 261 us
+    // a round, eight separate kernels took 293; 7-point 40^3, k = 32 103 -> 82 (101); one wave either way 2
+    // to 7%. One wave more and two lose: 27-point 36^3, k = 32 (365) 108 -> 126, 5-point 200^2, k = 24 46 ->
+    // 57; from 12 items an SM on both are within 13%. Long rows keep three: 20,000-node
+    // graph, k = 20 84 against 109 us.
+    auto waves = [&](int b) { return (items + b * sms - 1) / (b * sms); };
+    const int mb = !fused && !a.long_rows && waves(2) == waves(3) ? 2 : 3;
+    const void *fn = pb_kernel(L, Q, fused, mb);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, PB_THREADS, 0) != cudaSuccess || per_sm < 1)
         return gb_fail(ctx, GCGE_GPU_ERR_CUDA);
     long G = (long)ctx->num_sms * per_sm;
-    const long items = (long)a.nslab * ((a.k + a.cw - 1) / a.cw);
     if (G > items) G = items;
     const double nk = (double)a.n * a.k, rounds = a.max_it > 1 ? a.max_it - 1 : 0;
     GB_PROF(ctx, GB_K_SPMM64, rounds * (12.0 * A->nnz + 4.0 * (A->n + 1) + 88.0 * nk),

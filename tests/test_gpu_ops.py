@@ -509,3 +509,10 @@ def test_large_workspaces_go_back_after_the_call(op):
         run()
         c.sync()
         assert before - torch.cuda.mem_get_info()[0] <= 300 << 20
+
+
+@pytest.mark.parametrize("items,k", [(152, 2), (304, 3), (305, 3), (456, 2), (457, 5), (608, 1), (609, 2), (304, 33), (500, 9)])
+def test_bcg_fp64_two_or_three_blocks_an_sm(ctx, items, k):
+    """Row slabs on either side of where two blocks an SM take a wave more than three (304 and 608 slabs of
+    128 rows on 152 SMs), the last slab of one row: as test_bcg_fp64_on_the_sides_of_its_forms."""
+    test_bcg_fp64_on_the_sides_of_its_forms(ctx, (128 * (items - 1) + 1, 1), k, 4, 1e-30)
