@@ -248,20 +248,12 @@ static int row_grid(gcge_gpu_ctx *ctx, long rows)
 // cdiv(n, RED_ROWS) rows of the other kernels)
 #define LONG_PART_ROWS 2048
 
-// the FP64 rounds may form p where it is gathered (a second buffer of p) up to this
-// many entries of a block; which calls do is decided at the launch, by their work
-#define FUSE_MAX 400000L
-static bool fuse_direction(int n, int k) { return (long)n * ((k + 3) & ~3) <= FUSE_MAX; }
-
 extern "C" size_t gb_bcg_work_bytes(int n, int k, int precision)
 {
     long ldk = (k + 3) & ~3;   // 16-byte rows for the vectorised SpMM
     size_t vec = precision ? sizeof(float) : sizeof(double);
     size_t nblk = (size_t)cdiv(n > 0 ? n : 1, RED_ROWS) + (precision ? LONG_PART_ROWS : 0);
-    // FP32: R, X, P, W; FP64: P, W and, where it is used, P2 -- never less for more
-    // columns, as the solver sizes the workspace for its widest block
-    size_t blocks = (precision ? 4 : 2) * (size_t)n * ldk * vec;
-    if (!precision && blocks < 3 * vec * FUSE_MAX) blocks = 3 * vec * (fuse_direction(n, k) ? (size_t)n * ldk : FUSE_MAX);
+    size_t blocks = (precision ? 4 : 2) * (size_t)n * ldk * vec;   // FP32: R, X, P, W; FP64: P, W
     size_t state = (7 * (size_t)k + nblk * (size_t)k + 8) * sizeof(double) + 64;
     return blocks + state + 16 * 256;   // every sub-buffer is aligned to 256 bytes (10 of them)
 }
@@ -787,11 +779,10 @@ extern "C" int gb_bcg(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, double *RHS, lon
     if (a->precision == 0) {
         double *P = (double *)take((size_t)n * ld * vec);
         double *W = (double *)take((size_t)n * ld * vec);
-        double *P2 = fuse_direction(n, k) ? (double *)take((size_t)n * ld * vec) : nullptr;
         if ((size_t)(w - (char *)work) > work_bytes) return gb_fail(ctx, GCGE_GPU_ERR_ARG);
         // R = RHS - A X, in place in RHS (the reference overwrites RHS with the residual)
         int st = a->rhs_is_residual ? 0 : gb_spmm(ctx, A, X, ldx, RHS, ldr, k, -1.0, nullptr, 1.0, nullptr);
-        return st ? st : gb_bcg_persist64(ctx, A, a, &s, RHS, ldr, X, ldx, P, P2, W, ld);
+        return st ? st : gb_bcg_persist64(ctx, A, a, &s, RHS, ldr, X, ldx, P, W, ld);
     }
     // Mixed precision as defect correction: the residual r0 = RHS - A X is formed in
     // FP64, block CG runs in FP32 on A D = r0 from D = 0, and X += D in FP64. The

@@ -13,9 +13,8 @@ struct bcg_state {
 };
 
 /* all FP64 rounds in one cooperative launch, on R (the initial residual) and X in
- * place; s->part: ceil(n / 128) doubles per column. P2 (a second buffer of p, or NULL)
- * selects the form with two barriers a round */
+ * place; s->part: ceil(n / 128) doubles per column */
 extern "C" int gb_bcg_persist64(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, const gb_bcg_args *b, const bcg_state *s,
-                                double *R, long ldr, double *X, long ldx, double *P, double *P2, double *W, long ld);
+                                double *R, long ldr, double *X, long ldx, double *P, double *W, long ld);
 
 #endif

@@ -7,11 +7,13 @@
 // persistent grid (every block resident, so that blocks may wait on one another) and
 // the sums are formed inside the grid barrier (2.2 us, 4 to 6 with sums). A call that
 // has no active column left ends there. Time of a round, us, separate launches -> here:
-//   100 x 100 grid, k = 10: 52 -> 26 (latency)   30 x 30 grid, k = 6: 51 -> 20
-//   7-point 64^3, k = 32: 373 -> 283             FEM 40^3, k = 20: 129 -> 104
-//   FEM 64^3, k = 50: 1,095 -> 956 (the product alone is 9.2e9 flops: 0.86 of the
-//   FP64 pipe's 1.2 TFLOP/s over the whole round's 1.0e10)
-//   power-law graph of 100,000, k = 44: 705 -> 318 (rows past GB_LONG_ROW by a block)
+//   100 x 100 grid, k = 10: 52 -> 25 (latency)   30 x 30 grid, k = 6: 51 -> 20
+//   7-point 64^3, k = 32: 371 -> 283             FEM 40^3, k = 20: 117 -> 96
+//   FEM 64^3, k = 50: 1,001 -> 798 (4.1e8 FP64 multiply-adds: 0.85 of the pipe's 6e11 a second)
+//   power-law graph of 100,000, k = 44: 674 -> 319 (rows past GB_LONG_ROW by a block)
+// (Forming p where it is gathered, b p + r from two buffers, saves a barrier and a pass and
+// costs a multiply-add more per entry and lane slot: 2 to 4% faster below 30 x 30 x 6, 5% slower
+// at 100 x 100 x 10 and up to 36% beyond; that form is gone.)
 //
 // Mapping. A block owns slabs of 128 rows. In the vector phases a thread owns eight
 // rows of a column, spaced by eight (a unit): its 16 or 32 loads are all in flight,
@@ -35,7 +37,6 @@
 #define PB_THREADS 256
 #define PB_WARPS (PB_THREADS / 32)
 #define PB_SLAB 128
-#define PB_FUSED_K 1024                                   // widest block of the fused form
 // partials (slabs x columns) up to which the block that arrives last sums them all;
 // beyond, one block per column does (a trip more, but side by side)
 #define PB_ONE_BLOCK_SUMS 1024
@@ -43,7 +44,6 @@
 #define GB_PROF(ctx, cls, bytes, flops) \
     do { if ((ctx)->prof) gb_prof_begin((ctx), (cls), (bytes), (flops)); } while (0)
 
-#define PB_FUSED_WORK 125.0
 enum { PB_PLAIN, PB_INIT, PB_ALPHA, PB_BETA };
 
 struct pb_args {
@@ -52,8 +52,8 @@ struct pb_args {
     double rate;
     const int *rp, *ci;
     const double *val;
-    double *R, *X, *P, *P2, *W; // residual, solution, direction (P2: its other buffer, fused form), A p
-    long ldr, ldx, ld;         // of R, of X, of P, P2 and W
+    double *R, *X, *P, *W;     // residual, solution, direction, A p
+    long ldr, ldx, ld;         // of R, of X, of P and W
     const double *dinv;
     double *rho2, *err, *alpha, *beta;
     double *part;              // [column][slab]
@@ -247,12 +247,10 @@ __device__ __forceinline__ void pb_slab_partials(const pb_args &a, double (*red)
     __syncthreads();
 }
 
-// entries [beg, end) of a row in steps of `step` by a group of L lanes. FUSED: p is
-// formed where it is gathered, b p + z from the buffer that holds the old one.
-template <int L, int Q, bool FUSED>
+// entries [beg, end) of a row in steps of `step` by a group of L lanes
+template <int L, int Q>
 __device__ __forceinline__ void pb_row(const pb_args &a, int beg, int end, int step, int sl, unsigned gmask,
-                                       const int col[Q], const double *const pold[Q], const double b[Q], bool first,
-                                       double acc[Q])
+                                       const int col[Q], double acc[Q])
 {
     for (int base = beg; base < end; base += step) {
         const int e = base + sl;
@@ -267,18 +265,9 @@ __device__ __forceinline__ void pb_row(const pb_args &a, int beg, int end, int s
         for (int t = 0; t < m; ++t) {
             const int jj = __shfl_sync(gmask, j, t, L);
             const double vv = __shfl_sync(gmask, v, t, L);
-            if (FUSED) {
-                const double *r = a.R + (long)jj * a.ldr;
+            const double *p = a.P + (long)jj * a.ld;
 #pragma unroll
-                for (int q = 0; q < Q; ++q) {
-                    const double z = a.dinv ? __dmul_rn(a.dinv[jj], r[col[q]]) : r[col[q]];
-                    acc[q] = fma(vv, first ? z : fma(b[q], pold[q][(long)jj * a.ld], z), acc[q]);
-                }
-            } else {
-                const double *p = a.P + (long)jj * a.ld;
-#pragma unroll
-                for (int q = 0; q < Q; ++q) acc[q] = fma(vv, p[col[q]], acc[q]);
-            }
+            for (int q = 0; q < Q; ++q) acc[q] = fma(vv, p[col[q]], acc[q]);
         }
     }
 }
@@ -294,7 +283,7 @@ __device__ __forceinline__ void pb_row(const pb_args &a, int beg, int end, int s
 
 // MB blocks an SM (the registers for it): two for matrices without long rows where that takes no
 // more waves of items than three do, see gb_bcg_persist64
-template <int L, int Q, bool FUSED, int MB>
+template <int L, int Q, int MB>
 __global__ void __launch_bounds__(PB_THREADS, MB)
 k_bcg_persist(const pb_args a)
 {
@@ -303,7 +292,6 @@ k_bcg_persist(const pb_args a)
     __shared__ double red[16][C];
     __shared__ double sh[PB_THREADS];
     __shared__ int lflag[MB == 3 ? RPB : 1];
-    __shared__ uint8_t flip[FUSED ? PB_FUSED_K : 1];     // the buffer that holds a column's p
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int sl = lane % L, slot = threadIdx.x / L;
     const unsigned gmask = (L == 32) ? 0xffffffffu : (((1u << L) - 1u) << ((lane / L) * L));
@@ -333,14 +321,12 @@ k_bcg_persist(const pb_args a)
             pb_slab_partials<C>(a, red, c0, kc, slab);
         }
     }
-    if (FUSED)
-        for (int c = threadIdx.x; c < k; c += PB_THREADS) flip[c] = 0;
     int ka = pb_barrier(a, PB_INIT, k, sh, gen);
 
     for (int it = 1; ka > 0 && it < a.max_it; ++it) {
         const bool first = it == 1;
         // p = z + beta p on the active columns (p = z first; z = r, or D^-1 r)
-        if (!FUSED) {
+        {
             PB_ITEMS(ka)
             {
                 PB_ITEM(ka)
@@ -366,27 +352,16 @@ k_bcg_persist(const pb_args a)
                     }
                 }
             }
-            if (pb_barrier(a, PB_PLAIN, ka, sh, gen) < 0) return;
         }
+        if (pb_barrier(a, PB_PLAIN, ka, sh, gen) < 0) return;
         // w = A p and the column sums of p.w
         {
             PB_ITEMS(ka)
             {
                 PB_ITEM(ka)
                 int col[Q];
-                const double *pold[Q];
-                double bq[Q];
 #pragma unroll
-                for (int q = 0; q < Q; ++q) {
-                    col[q] = c0 + min(sl + L * q, kc - 1);   // idle slots: a column again
-                    if (FUSED) {
-                        bq[q] = first ? 0.0 : __ldcg(a.beta + col[q]);
-                        pold[q] = (flip[col[q]] ? a.P2 : a.P) + col[q];
-                    } else {
-                        bq[q] = 0;
-                        pold[q] = nullptr;
-                    }
-                }
+                for (int q = 0; q < Q; ++q) col[q] = c0 + min(sl + L * q, kc - 1);   // idle slots: a column again
                 for (int b = 0; b < PB_SLAB; b += RPB) {
                     const long r0 = slab * PB_SLAB + b, r = r0 + slot;
                     int beg = 0, end = 0;
@@ -398,7 +373,7 @@ k_bcg_persist(const pb_args a)
 #pragma unroll
                     for (int q = 0; q < Q; ++q) acc[q] = 0;
                     const bool lng = MB == 3 && a.long_rows && end - beg > GB_LONG_ROW;
-                    if (!lng) pb_row<L, Q, FUSED>(a, beg, end, L, sl, gmask, col, pold, bq, first, acc);
+                    if (!lng) pb_row<L, Q>(a, beg, end, L, sl, gmask, col, acc);
                     // rows longer than GB_LONG_ROW: all groups of the block on one row, the
                     // group sums added by shuffles and then warp by warp, in row order
                     if (MB == 3 && a.long_rows && __syncthreads_or(lng)) {
@@ -410,7 +385,7 @@ k_bcg_persist(const pb_args a)
                             double la[Q];
 #pragma unroll
                             for (int q = 0; q < Q; ++q) la[q] = 0;
-                            pb_row<L, Q, FUSED>(a, lb + slot * L, le, PB_THREADS, sl, gmask, col, pold, bq, first, la);
+                            pb_row<L, Q>(a, lb + slot * L, le, PB_THREADS, sl, gmask, col, la);
                             __syncwarp();
 #pragma unroll
                             for (int q = 0; q < Q; ++q) {
@@ -442,32 +417,12 @@ k_bcg_persist(const pb_args a)
                 {
                     const pb_unit x = pb_decode(u, kc);
                     const int c = c0 + x.c;
-                    const double *po = (FUSED && flip[c] ? a.P2 : a.P) + c;
                     double p[8], w[8], run = 0;
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
                         const long r = slab * PB_SLAB + x.row + 8 * i;
-                        p[i] = r < n && !(FUSED && first) ? po[r * a.ld] : 0.0;
+                        p[i] = r < n ? a.P[r * a.ld + c] : 0.0;
                         w[i] = r < n ? a.W[r * a.ld + c] : 0.0;
-                    }
-                    if (FUSED) {
-                        double *pn = (flip[c] ? a.P : a.P2) + c;
-                        const double b = first ? 0.0 : __ldcg(a.beta + c);
-                        double z[8];
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            const long r = slab * PB_SLAB + x.row + 8 * i;
-                            z[i] = r < n ? a.R[r * a.ldr + c] : 0.0;
-                        }
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            const long r = slab * PB_SLAB + x.row + 8 * i;
-                            if (r < n) {
-                                const double zz = a.dinv ? __dmul_rn(a.dinv[r], z[i]) : z[i];
-                                p[i] = first ? zz : fma(b, p[i], zz);
-                                pn[r * a.ld] = p[i];
-                            }
-                        }
                     }
 #pragma unroll
                     for (int i = 0; i < 8; ++i)
@@ -488,13 +443,12 @@ k_bcg_persist(const pb_args a)
                     const pb_unit x = pb_decode(u, kc);
                     const int c = c0 + x.c;
                     const double al = __ldcg(a.alpha + c);
-                    const double *pc = (FUSED && !flip[c] ? a.P2 : a.P) + c;
                     double xv[8], rv[8], p[8], w[8], run = 0;
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
                         const long r = slab * PB_SLAB + x.row + 8 * i;
                         const bool in = r < n;
-                        p[i] = in ? pc[r * a.ld] : 0.0;
+                        p[i] = in ? a.P[r * a.ld + c] : 0.0;
                         w[i] = in ? a.W[r * a.ld + c] : 0.0;
                         xv[i] = in ? a.X[r * a.ldx + c] : 0.0;
                         rv[i] = in ? a.R[r * a.ldr + c] : 0.0;
@@ -514,12 +468,7 @@ k_bcg_persist(const pb_args a)
                 pb_slab_partials<C>(a, red, c0, kc, slab);
             }
         }
-        const int was = ka;
         ka = pb_barrier(a, PB_BETA, ka, sh, gen);
-        if (FUSED) {
-            for (int c = threadIdx.x; c < was; c += PB_THREADS) flip[c] ^= 1;
-            __syncthreads();
-        }
     }
 }
 
@@ -540,23 +489,19 @@ static void pb_shape(int k, int maxq, int *Lo, int *Qo)
     }
 }
 
-static const void *pb_kernel(int L, int Q, bool fused, int mb)
+static const void *pb_kernel(int L, int Q, int mb)
 {
-#define PB_K4(LL, F, MB) (const void *)k_bcg_persist<LL, 1, F, MB>, (const void *)k_bcg_persist<LL, 2, F, MB>, \
-                         (const void *)k_bcg_persist<LL, 3, F, MB>, (const void *)k_bcg_persist<LL, 4, F, MB>
-#define PB_K8(LL, MB) {PB_K4(LL, false, MB), (const void *)k_bcg_persist<LL, 5, false, MB>, \
-                       (const void *)k_bcg_persist<LL, 6, false, MB>, (const void *)k_bcg_persist<LL, 7, false, MB>, \
-                       (const void *)k_bcg_persist<LL, 8, false, MB>}
+#define PB_K4(LL, q, MB) (const void *)k_bcg_persist<LL, q, MB>, (const void *)k_bcg_persist<LL, q + 1, MB>, \
+                         (const void *)k_bcg_persist<LL, q + 2, MB>, (const void *)k_bcg_persist<LL, q + 3, MB>
+#define PB_K8(LL, MB) {PB_K4(LL, 1, MB), PB_K4(LL, 5, MB)}
     static const void *const tab[2][3][8] = {{PB_K8(4, 2), PB_K8(8, 2), PB_K8(16, 2)}, {PB_K8(4, 3), PB_K8(8, 3), PB_K8(16, 3)}};
-    static const void *const tabf[3][4] = {{PB_K4(4, true, 3)}, {PB_K4(8, true, 3)}, {PB_K4(16, true, 3)}};
 #undef PB_K4
 #undef PB_K8
-    const int i = L == 4 ? 0 : L == 8 ? 1 : 2;
-    return fused ? tabf[i][Q - 1] : tab[mb - 2][i][Q - 1];
+    return tab[mb - 2][L == 4 ? 0 : L == 8 ? 1 : 2][Q - 1];
 }
 
 extern "C" int gb_bcg_persist64(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, const gb_bcg_args *b, const bcg_state *s,
-                                double *R, long ldr, double *X, long ldx, double *P, double *P2, double *W, long ld)
+                                double *R, long ldr, double *X, long ldx, double *P, double *W, long ld)
 {
     pb_args a = {};
     a.n = b->n;
@@ -573,7 +518,6 @@ extern "C" int gb_bcg_persist64(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, const 
     a.X = X;
     a.ldx = ldx;
     a.P = P;
-    a.P2 = P2;
     a.W = W;
     a.ld = ld;
     a.dinv = b->dinv;
@@ -602,14 +546,7 @@ extern "C" int gb_bcg_persist64(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, const 
         }
     }
     if (best == 0 || (long)a.nslab >= 4 * sms) a.cw = a.k;
-    pb_shape(a.cw, 4, &L, &Q);
-    // forming p where it is gathered saves a barrier and a pass (5 us) and costs one more
-    // FMA per entry and lane slot on the busiest SM (16 clocks per warp: an item's 128
-    // rows of nnz / n entries)
-    const long items_sm = (a.nslab * (long)((a.k + a.cw - 1) / a.cw) + sms - 1) / sms;
-    const bool fused = P2 && a.k <= PB_FUSED_K && a.cw <= L * Q &&
-                       (double)A->nnz / a.n * L * Q * items_sm < PB_FUSED_WORK;
-    if (!fused) pb_shape(a.cw, 8, &L, &Q);
+    pb_shape(a.cw, 8, &L, &Q);
     if (a.cw > L * Q) a.cw = L * Q;
     const long items = (long)a.nslab * ((a.k + a.cw - 1) / a.cw);
     // Three blocks an SM hide more of the gathers' latency, two have registers for all their loads in
@@ -620,8 +557,8 @@ extern "C" int gb_bcg_persist64(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, const 
     // 57; from 12 items an SM on both are within 13%. Long rows keep three: 20,000-node
     // graph, k = 20 84 against 109 us.
     auto waves = [&](int b) { return (items + b * sms - 1) / (b * sms); };
-    const int mb = !fused && !a.long_rows && waves(2) == waves(3) ? 2 : 3;
-    const void *fn = pb_kernel(L, Q, fused, mb);
+    const int mb = !a.long_rows && waves(2) == waves(3) ? 2 : 3;
+    const void *fn = pb_kernel(L, Q, mb);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, PB_THREADS, 0) != cudaSuccess || per_sm < 1)
         return gb_fail(ctx, GCGE_GPU_ERR_CUDA);
     long G = (long)ctx->num_sms * per_sm;
