@@ -11,7 +11,7 @@
 // operands prove that the digits which column scales leave them keep every entry within
 // the bound of a plain FP64 sum, and on the FP64 pipe (k_gram_partial, plain FP64 fused multiply-adds
 // with a fixed-order second stage) otherwise: at 262,144 x (178, 64) 5.45 ms on the
-// FP64 pipe, 0.64 ms on the tensor cores; at 600,000 x (256, 128) 32.7 and 2.5 ms.
+// FP64 pipe, 0.42 ms on the tensor cores; at 600,000 x (256, 128) 33.0 and 1.82 ms.
 //
 // The array is GB_NOALLOC_DOUBLES doubles (8 MiB) and a control block of 64 KiB beside
 // it (column scales); every GPU that loads the library holds them until the process
