@@ -550,7 +550,7 @@ extern "C" int gb_bcg_persist64(gcge_gpu_ctx *ctx, const gcge_gpu_mat *A, const 
     if (a.cw > L * Q) a.cw = L * Q;
     const long items = (long)a.nslab * ((a.k + a.cw - 1) / a.cw);
     // Three blocks an SM hide more of the gathers' latency, two have registers for all their loads in
-    // flight (three spill 96 to 220 bytes) and leave a last item less often alone on its SM.
+    // flight (three spill 108 to 224 bytes) and leave a last item less often alone on its SM.
     // Two where that takes no more waves of items: 27-point 40^3, k = 64 (500 items) 336 -> 261 us
     // a round, eight separate kernels took 293; 7-point 40^3, k = 32 103 -> 82 (101); one wave either way 2
     // to 7%. One wave more and two lose: 27-point 36^3, k = 32 (365) 108 -> 126, 5-point 200^2, k = 24 46 ->
